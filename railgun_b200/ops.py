@@ -2250,6 +2250,44 @@ def prefill_attention_tc(q, out, kv_cache, block_table, tiles, positions, nh: in
         _stream()), "prefill_attention_tc")
 
 
+def prefill_attention_wide_ok(q, out, kv_cache, d: int, page_size: int) -> bool:
+    """Can the tcgen05 flash kernel for head size 128 take this?  bfloat16, pages of 8, 16, 32, 64 or 128 tokens, rows
+    and pointers in whole 16 bytes."""
+    return (q.is_cuda and q.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and d == 128
+            and page_size in (8, 16, 32, 64, 128) and q.dim() == 2 and q.stride(1) == 1 and q.stride(0) % 8 == 0
+            and q.data_ptr() % 16 == 0 and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0 and kv_cache.is_contiguous())
+
+
+def prefill_attention_wide(q, out, kv_cache, block_table, tiles, positions, nh: int, nkv: int, d: int, window: int,
+                           scale: float, keep_first: int = 0, sink=None, gate=None, out_scale: float = 1.0,
+                           chunk: int = 0) -> None:
+    """``prefill_attention`` (without pooled entries) at head size 128 on the tcgen05 tensor cores.  ``q`` [T, at least
+    nh * d], head h at column h * d; ``tiles`` [n, 3] = (first row, rows <= 128, request index).  Its waits are
+    bounded; ``tc_gemm_check()`` raises if one gave up."""
+    page_size = kv_cache.shape[3]
+    if not prefill_attention_wide_ok(q, out, kv_cache, d, page_size):
+        raise KernelError("prefill_attention_wide: bfloat16, head size 128, page size 8..128 dividing 128, 16-byte rows")
+    _check(kv_cache, "kv_cache", q.dtype)
+    _check(block_table, "block_table", torch.int32)
+    _check(tiles, "tiles", torch.int32)
+    _check(positions, "positions", torch.int32)
+    _check_out_view(out, out.shape[0], nh * d, q.dtype, "prefill_attention_wide")
+    gate_ld = _sink_and_gate(sink, gate, nh, out.shape[0], q.dtype)
+    if tuple(kv_cache.shape[1:]) != (2, nkv, page_size, d) or q.shape[1] < nh * d:
+        raise KernelError(f"kv cache {tuple(kv_cache.shape)} or q {tuple(q.shape)} does not match heads {nh} and {nkv} x {d}")
+    err = _tc_err.get(q.device)
+    if err is None:
+        err = _tc_err[q.device] = torch.zeros(1, dtype=torch.int32, device=q.device)
+    global _tc_unchecked
+    _tc_unchecked = True
+    _ok(_fn("attention_tcgen05_wide", "rg_prefill_attention_wide")(
+        _ptr(q), c_int(q.stride(0)), c_int(q.shape[0]), _ptr(out), c_int(out.stride(0)), _ptr(kv_cache),
+        c_int(kv_cache.shape[0]), _ptr(block_table), c_int(block_table.shape[1]), _ptr(tiles), c_int(tiles.shape[0]),
+        _ptr(positions), c_int(nh), c_int(nkv), c_int(d), c_int(page_size), c_int(_reach(window, chunk, keep_first)),
+        c_int(keep_first if window else 0), c_float(scale), _ptr(sink), _ptr(gate), c_int(gate_ld), c_float(out_scale),
+        _ptr(err), _stream()), "prefill_attention_wide")
+
+
 def probe_sm100(device="cuda:0") -> dict:
     """Cycle counts of the building blocks of the tcgen05 kernels on this GPU
     (csrc/kernels/probe_sm100.cu): a diagnostic, on no product path."""

@@ -26,6 +26,15 @@ from .registry import register_mixer, POSITION_ENCODINGS
 USE_TC_ATTENTION = os.environ.get("RAILGUN_B200_TC_ATTENTION", "1") != "0"
 
 
+def use_wide_attention(q, out, batch, cache, d: int) -> bool:
+    """Whether portions of prompts take the tcgen05 kernel for head size 128 (where it can).  It pays for its set-up
+    from contexts of about two of its 128-key stages: one prompt of 100 tokens takes 11.5 us against 9.5 on the mma.sync
+    kernel (32 heads on 8), of 200 13.6 against 14.2, of 400 17.7 against 25.9, of 2,048 59 against 208; 16 tokens
+    behind 1,024 28.0 against 49.7."""
+    return (USE_TC_ATTENTION and batch.num_prefill_tiles128 > 0 and batch.max_context_len > 128
+            and ops.prefill_attention_wide_ok(q, out, cache.kv, d, cache.page_size))
+
+
 class PagedAttention(Mixer):
     """params: ``hidden_size``, ``num_heads``, ``num_kv_heads``, ``head_dim``,
     ``window`` (0: none), ``scale`` (None: head_dim^-0.5), ``position``
@@ -125,6 +134,9 @@ class PagedAttention(Mixer):
                     qkv, cache.kv, d, cache.page_size):
                 ops.prefill_attention_tc(qkv, out, cache.kv, table, batch.prefill_tiles128, batch.positions,
                                          nh, nkv, d, self.window, self.scale)
+            elif use_wide_attention(qkv, out, batch, cache, d):
+                ops.prefill_attention_wide(qkv, out, cache.kv, table, batch.prefill_tiles128, batch.positions,
+                                           nh, nkv, d, self.window, self.scale)
             else:
                 ops.prefill_attention(qkv, qkv.shape[1], out, cache.kv, table, batch.prefill_tiles, batch.positions,
                                       nh, nkv, d, self.window, self.scale)
@@ -391,8 +403,13 @@ class NormedAttention(Mixer):
         if self.chunk:
             reach = min(reach, self.chunk)
         if batch.num_prefill_tiles:
-            ops.prefill_attention(q, q.shape[1], out, cache.kv, table, batch.prefill_tiles, batch.positions,
-                                  H, G, D, self.window, 1.0, self.keep_first, **more)
+            if pooled is None and use_wide_attention(q, out, batch, cache, D):
+                ops.prefill_attention_wide(q, out, cache.kv, table, batch.prefill_tiles128, batch.positions, H, G, D,
+                                           self.window, 1.0, self.keep_first, sink=self.sink, gate=gate,
+                                           out_scale=out_scale, chunk=self.chunk)
+            else:
+                ops.prefill_attention(q, q.shape[1], out, cache.kv, table, batch.prefill_tiles, batch.positions,
+                                      H, G, D, self.window, 1.0, self.keep_first, **more)
         n = batch.num_tokens if batch.decode_only else batch.num_decode_rows
         if n:
             ops.decode_attention(q, q.shape[1], out, cache.kv, table, None if batch.decode_only else batch.decode_rows,

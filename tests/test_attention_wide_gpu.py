@@ -1,0 +1,124 @@
+"""The tcgen05 prefill attention for head size 128 against a 64-bit statement, where it can go wrong: tiles of 128
+queries, passes of 64 keys and stages of 128, one or two heads to a block, windows, chunks and kept first tokens at the
+passes' edges, rows whose first keys are masked, references that have to be raised."""
+import pytest
+import torch
+
+from test_kernels_gpu import DEV, make_paged_case, rel_err
+
+pytestmark = pytest.mark.gpu
+D = 128
+# bfloat16 weights (2^-9 each, averaged) and one rounding of the output (2^-9): 4e-3 in the 2-norm, with a margin
+BOUND = 1e-2
+
+
+def statement(c, nh, nkv, page, window, scale, keep_first=0, chunk=0, sink=None, gate=None):
+    kv, q = c["kv"].double().to(DEV), c["q"].double().to(DEV)
+    out = torch.zeros(c["T"], nh, D, dtype=torch.float64, device=DEV)
+    first = 0
+    for r in sorted(set(c["req"])):
+        n = c["req"].count(r)
+        pos = torch.tensor(c["positions"][first:first + n], device=DEV)[:, None]
+        j = torch.arange(int(pos.max()) + 1, device=DEV)
+        pages = torch.tensor(c["tables"][r], device=DEV)[j // page]
+        K, V = (kv[pages, x, :, j % page].repeat_interleave(nh // nkv, 1) for x in (0, 1))
+        s = torch.einsum("thd,khd->htk", q[first:first + n], K) * scale
+        see = j <= pos
+        if window:
+            see &= (j > pos - window) | (j < keep_first)
+        if chunk:
+            see &= j >= pos // chunk * chunk
+        s = s.masked_fill(~see, float("-inf"))
+        if sink is not None:
+            s = torch.cat([s, sink.double()[:, None, None].expand(nh, n, 1)], 2)
+        p = torch.softmax(s, 2)[:, :, :len(j)]
+        out[first:first + n] = torch.einsum("htk,khd->thd", p, V)
+        first += n
+    if gate is not None:
+        out *= torch.sigmoid(gate.double())[:, :, None]
+    return out.reshape(c["T"], nh * D)
+
+
+def tiles_of(q_lens):
+    tiles, off = [], 0
+    for r, n in enumerate(q_lens):
+        tiles += [(off + k, min(128, n - k), r) for k in range(0, n, 128)]
+        off += n
+    return torch.tensor(tiles, dtype=torch.int32, device=DEV)
+
+
+def run(c, nh, nkv, q_lens, window, scale, wide=True, out_cols=0, **more):
+    from railgun_b200 import ops
+    q = c["q"].reshape(c["T"], nh * D).to(DEV)
+    if wide:                                                     # q beside k and v, as a fused projection leaves it
+        q = torch.cat([q, torch.zeros(c["T"], 2 * nkv * D, dtype=torch.bfloat16, device=DEV)], 1)
+    out = torch.full((c["T"], nh * D + out_cols), float("nan"), dtype=torch.bfloat16, device=DEV)[:, :nh * D]
+    ops.prefill_attention_wide(q, out, c["kv"].to(DEV), c["bt"].to(DEV), tiles_of(q_lens),
+                               torch.tensor(c["positions"], dtype=torch.int32, device=DEV), nh, nkv, D, window, scale, **more)
+    ops.tc_gemm_check()
+    return out
+
+
+CASES = [
+    # nh, nkv, page, ctx_lens, q_lens, window, keep_first, chunk
+    (2, 1, 16, [128], [128], 0, 0, 0),
+    (1, 1, 16, [64], [64], 0, 0, 0),                              # one head to a block, one pass
+    (3, 1, 8, [65, 129, 2], [65, 129, 2], 0, 0, 0),               # an odd group; a stage of one pass
+    (4, 2, 32, [1000, 193, 64], [500, 130, 3], 0, 0, 0),          # portions that start inside a context
+    (8, 2, 64, [700], [260], 100, 0, 0),                          # a window
+    (8, 1, 128, [400], [400], 37, 5, 0),                          # a window that keeps the first tokens
+    (4, 2, 16, [900, 300], [300, 300], 256, 70, 0),               # two passes of kept tokens
+    (4, 4, 16, [520], [520], 0, 0, 96),                           # chunks that end inside a pass
+    (32, 8, 16, [1500], [1500], 0, 0, 0),
+]
+
+
+@pytest.mark.parametrize("case_id", range(len(CASES)))
+def test_against_the_statement(case_id):
+    nh, nkv, page, ctx, ql, window, keep, chunk = CASES[case_id]
+    c = make_paged_case(len(ctx), ctx, ql, nh, nkv, D, page, torch.bfloat16, seed=900 + case_id)
+    out = run(c, nh, nkv, ql, window, D ** -0.5, keep_first=keep, chunk=chunk)
+    assert rel_err(out, statement(c, nh, nkv, page, window, D ** -0.5, keep, chunk).cpu()) < BOUND
+
+
+@pytest.mark.parametrize("case_id", [2, 3, 5, 8])
+def test_sink_gate_scale_and_output_view(case_id):
+    nh, nkv, page, ctx, ql, window, keep, chunk = CASES[case_id]
+    c = make_paged_case(len(ctx), ctx, ql, nh, nkv, D, page, torch.bfloat16, seed=950 + case_id)
+    g = torch.Generator(device=DEV).manual_seed(case_id)
+    sink = 3 * torch.randn(nh, device=DEV, generator=g)
+    sink[0] = 60.0                                               # far above every score
+    gate = torch.randn(c["T"], nh, device=DEV, generator=g).to(torch.bfloat16)
+    out = run(c, nh, nkv, ql, window, D ** -0.5, wide=False, out_cols=64, keep_first=keep, sink=sink, gate=gate, out_scale=0.5)
+    ref = 0.5 * statement(c, nh, nkv, page, window, D ** -0.5, keep, chunk, sink, gate).cpu()
+    assert rel_err(out, ref) < BOUND
+    assert (out[:, :D].abs() < 1e-12).all()                      # head 0: the sink has all the weight
+
+
+def test_the_reference_is_raised_and_masked_rows_find_theirs():
+    """Keys that align with some queries ever more strongly, and a window whose first pass many rows do not see while
+    all scores are far below zero: a row may not take zero as its reference there."""
+    nh, nkv, page, T = 2, 1, 16, 300
+    c = make_paged_case(1, [T], [T], nh, nkv, D, page, torch.bfloat16, seed=77)
+    for kp, strength, row in ((70, 1.0, 299), (130, 2.0, 299), (200, 3.0, 299), (290, 4.0, 299), (100, 3.0, 150), (3, 2.0, 40)):
+        c["kv"][c["tables"][0][kp // page], 0, 0, kp % page] = (c["q"][row, 0] * strength).to(torch.bfloat16)
+    assert rel_err(run(c, nh, nkv, [T], 0, D ** -0.5), statement(c, nh, nkv, page, 0, D ** -0.5).cpu()) < BOUND
+    low = make_paged_case(1, [900], [300], nh, nkv, D, page, torch.bfloat16, seed=78)
+    low["q"] = low["q"] * 0.1 + 1.0
+    low["kv"][:, 0] = low["kv"][:, 0] * 0.1 - 4.0                # scores near -512 / 11.3 = -45, 65 in powers of two
+    for window, scale in ((40, D ** -0.5), (129, 0.5)):          # and near -256, far below what 32-bit weights hold
+        ref = statement(low, nh, nkv, page, window, scale).cpu()
+        assert rel_err(run(low, nh, nkv, [300], window, scale), ref) < 2 * BOUND     # fewer keys to average over
+
+
+def test_what_it_refuses():
+    from railgun_b200 import ops
+    q = torch.zeros(4, 3 * 64, dtype=torch.bfloat16, device=DEV)
+    kv = torch.zeros(2, 2, 1, 16, 64, dtype=torch.bfloat16, device=DEV)
+    assert not ops.prefill_attention_wide_ok(q, q, kv, 64, 16)
+    kv = torch.zeros(2, 2, 1, 12, D, dtype=torch.bfloat16, device=DEV)
+    q = torch.zeros(4, D, dtype=torch.bfloat16, device=DEV)
+    assert not ops.prefill_attention_wide_ok(q, q, kv, D, 12)
+    odd = torch.zeros(4, D + 4, dtype=torch.bfloat16, device=DEV)[:, 4:]
+    assert not ops.prefill_attention_wide_ok(odd, q, kv, D, 16)
+    assert not ops.prefill_attention_wide_ok(q, odd, kv, D, 16)
