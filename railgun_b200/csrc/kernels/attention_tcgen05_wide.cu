@@ -164,6 +164,19 @@ fa_wide_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
         for (int j = 0; j < n_kt && ok; ++j) {
             const int J = j >> 1, half = j & 1, s = J % FW_V_STAGES;
             if (half == 0) ok = mbar_wait_all(v_full0 + 8 * s, (J / FW_V_STAGES) & 1, err, 24, &abort_flag);
+            if (ok && j == n_kt - 1) {
+                // The rows of V behind the tile's last key are some other request's, or what an earlier one left: their
+                // weights are 0, and 0 times an infinity is a NaN, so zeros take their place.  Both groups' warps may
+                // write the same zeros.
+                const int over0 = hi + 1 - first_key(j);
+                for (int i = lane; i < (FW_BN - over0) * 16; i += 32) {
+                    const int key = over0 + (i >> 4);                        // 8 pieces of 16 bytes in each half of a row
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};"
+                                 ::"r"(sV0 + s * STAGE_BYTES + half * SUB + ((i >> 3) & 1) * KV_HALF + key * 128 + (i & 7) * 16), "r"(0) : "memory");
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // before the product reads them
+                __syncwarp();
+            }
             const bool next = (half == 1 || j == n_kt - 1) && J + 1 < n_st;
             if (ok && next) ok = mbar_wait_all(k_full0 + 8 * ((J + 1) % FW_K_STAGES), ((J + 1) / FW_K_STAGES) & 1, err, 22, &abort_flag);
             if (ok) ok = mbar_wait_all(p_full0 + 16 * g + 8 * half, J & 1, err, 23, &abort_flag);

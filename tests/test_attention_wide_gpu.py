@@ -111,6 +111,19 @@ def test_the_reference_is_raised_and_masked_rows_find_theirs():
         assert rel_err(run(low, nh, nkv, [300], window, scale), ref) < 2 * BOUND     # fewer keys to average over
 
 
+@pytest.mark.parametrize("n,page", [(129, 16), (191, 8), (200, 128), (257, 64), (320, 32), (383, 16)])
+def test_what_lies_behind_the_context_does_not_matter(n, page):
+    """NaN and infinities in other requests' pages and behind the last token in its own page."""
+    c = make_paged_case(1, [n], [n], 4, 2, D, page, torch.bfloat16, seed=n)
+    want = run(c, 4, 2, [n], 0, D ** -0.5)
+    used = torch.zeros(c["kv"].shape[0], page, dtype=torch.bool)
+    for j in range(n):
+        used[c["tables"][0][j // page], j % page] = True
+    for bad in (float("nan"), float("inf")):
+        c["kv"] = torch.where(used[:, None, None, :, None], c["kv"], torch.full_like(c["kv"], bad))
+        assert torch.equal(run(c, 4, 2, [n], 0, D ** -0.5), want)
+
+
 def test_what_it_refuses():
     from railgun_b200 import ops
     q = torch.zeros(4, 3 * 64, dtype=torch.bfloat16, device=DEV)
