@@ -270,8 +270,9 @@ fa_wide_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
             float row_sum = 0.f;
             if (!redo) {
                 row_sum = pass(m_ref == -INFINITY ? 0.f : m_ref);
-                // also catches inf, NaN and a row that has seen no key so far and so has no reference
-                redo = __any_sync(0xffffffffu, !(row_sum <= 256.f) || m_ref == -INFINITY);
+                // also catches inf, NaN and a row that has seen no key so far and so has no reference; the lanes behind
+                // the tile's rows hold some other request's queries and have no say in how this one's are rounded
+                redo = __any_sync(0xffffffffu, row < nrows && (!(row_sum <= 256.f) || m_ref == -INFINITY));
             }
             if (redo) {
                 // the row's maximum on the raw scores (scale > 0, so the maximum commutes with it)
