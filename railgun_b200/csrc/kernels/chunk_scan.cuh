@@ -23,6 +23,43 @@ __device__ __forceinline__ bool find_chunk(const int* __restrict__ cu, int R, in
     return false;
 }
 
+// c_i of the chunk's tokens for head h (64-bit), by the block's first warp; dt of the tokens (without dt: 1) into sdt.
+// a_t is loga's number, or fixed's of the head, or without either -exp(A_log) dt_t.  Where a decay is 0 (its logarithm
+// minus infinity) a number whose exponential is 0 takes its place, so that differences are numbers.
+__device__ __forceinline__ void chunk_sums(const float* __restrict__ dt, const float* __restrict__ loga,
+                                           const float* __restrict__ A_log, const double* __restrict__ fixed, int lo, int n, int H, int h,
+                                           double* __restrict__ cum, float* __restrict__ sdt) {
+    if (threadIdx.x < 32) {
+        const int i0 = 2 * threadIdx.x, i1 = i0 + 1;
+        const float d0 = i0 < n ? (dt ? dt[(size_t)(lo + i0) * H + h] : 1.f) : 0.f;
+        const float d1 = i1 < n ? (dt ? dt[(size_t)(lo + i1) * H + h] : 1.f) : 0.f;
+        double a0, a1;
+        if (loga) {
+            a0 = i0 < n ? (double)loga[(size_t)(lo + i0) * H + h] : 0.0;
+            a1 = i1 < n ? (double)loga[(size_t)(lo + i1) * H + h] : 0.0;
+        } else if (fixed) {
+            a0 = i0 < n ? fixed[h] : 0.0;
+            a1 = i1 < n ? fixed[h] : 0.0;
+        } else {
+            const float rate = -expf(A_log[h]);
+            a0 = (double)(rate * d0);
+            a1 = (double)(rate * d1);
+        }
+        a0 = a0 < -1e4 ? -1e4 : a0;
+        a1 = a1 < -1e4 ? -1e4 : a1;
+        double s = a0 + a1;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double up = __shfl_up_sync(0xffffffffu, s, o);
+            if ((int)threadIdx.x >= o) s += up;
+        }
+        cum[i0] = s - a1;
+        cum[i1] = s;
+        sdt[i0] = d0;
+        sdt[i1] = d1;
+    }
+}
+
 // dst[k][i] = src row i, number k0 + k (rows ld apart, n rows of N numbers; zeros elsewhere), for 64 x 64, times scale[i].
 // A warp reads 4 rows x 8 neighbouring numbers at a time and writes 32 different banks.
 __device__ __forceinline__ void load_transposed(float (*__restrict__ dst)[PITCH], const float* __restrict__ src, size_t ld,

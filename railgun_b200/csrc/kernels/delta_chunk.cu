@@ -1,0 +1,335 @@
+// The gated delta rule over portions of prompts in chunks of 64 tokens, instead of token by token:
+//
+//   S <- g_t S,  u_t = beta_t (v_t - S^T k_t),  S <- S + k_t u_t^T,  o_t = S^T q_t,   g_t = exp(a_t)
+//
+// With c_i = a_1 + .. + a_i inside a chunk and S0 the state before it, the u of a chunk solve a triangular system,
+//   (I + A) U = beta V - (beta exp(c) K) S0,   A_ij = beta_i exp(c_i - c_j) k_i . k_j  for j < i,
+// so that U = X - W S0 with X = (I + A)^-1 (beta V) and W = (I + A)^-1 (beta exp(c) K), which need no state, and
+//   S1 = exp(c_L) S0 + sum_j exp(c_L - c_j) k_j u_j^T,
+//   o_i = exp(c_i) S0^T q_i + sum_(j <= i) exp(c_i - c_j) (k_j . q_i) u_j
+// (the block form of Yang et al., "Parallelizing Linear Transformers with the Delta Rule over Sequence Length").
+//   delta_solve    per (chunk, head): X and W by forward substitution; per (chunk, query/key head): all k_j . q_i
+//   delta_states   per (request, head, 16 columns of S): chunk after chunk, U, the state before every chunk, and the last
+//                  one into the request's slot
+// and chunk_outputs (ssd_chunk.cu) with U in the place of the values.  Everything is 32-bit fused multiply-adds; the
+// exponents' sums are 64-bit.
+//
+// What bounds it: the 32-bit multiply-adds (128 a cycle and SM, packed or not), and in delta_states the chain from chunk to
+// chunk, 2 x 64 x d of them per column and chunk.  16 columns a block fill 128 of 148 SMs at 16 heads of 128 columns;
+// narrower blocks fetch the same W and K more often.  Measured (2,048 tokens, 16 heads of 128 x 128 on 8): 88 us the
+// systems, 132 the states and 202 until the outputs are there, each from when its blocks may start, beside the kernel
+// before; the token-by-token kernel (state_mixers.cu) took 908.  Steps whose longest portion is shorter than 128 tokens stay
+// on that one.
+#include "chunk_scan.cuh"
+
+#define DC_CB 16              // columns of S per block of delta_states
+#define DC_WP 72              // pitch of W's rows (k) in shared memory: four neighbouring k lie in different banks
+#define DC_MAX_D 128
+
+// q, k: rows q_ld, k_ld apart, head h of the H reads head h / (H / Hqk).  beta, loga [T, H].  x_out [T, H, dv] = X;
+// w_out [chunks, H, d, 64] = W transposed; factors [chunks, H, 64] = exp(c_L - c_i) (1 beyond the chunk's tokens), decays
+// [chunks, H] = exp(c_L); dots [chunks, Hqk, 64, 64] = k_j . q_i at [j][i].  grid: chunks, H (systems) and then Hqk (dots).
+template <typename V>
+__global__ void __launch_bounds__(NTH, 2)
+delta_solve_kernel(const float* __restrict__ q, int q_ld, const float* __restrict__ k, int k_ld, const V* __restrict__ v,
+                   int v_ld, const float* __restrict__ beta, const float* __restrict__ loga, const int* __restrict__ cu,
+                   int R, float* __restrict__ x_out, float* __restrict__ w_out, float* __restrict__ factors,
+                   float* __restrict__ decays, float* __restrict__ dots, int H, int Hqk, int d, int dv) {
+    __shared__ __align__(16) float sA[CH][PITCH];
+    __shared__ __align__(16) float sB[CH][PITCH];
+    __shared__ double cum[CH];
+    __shared__ float sbeta[CH], grown[CH];
+    pdl_wait();
+    pdl_trigger();
+    int r, lo, n;
+    if (!find_chunk(cu, R, blockIdx.x, r, lo, n)) return;
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+    const bool system = (int)blockIdx.y < H;
+    const int h = blockIdx.y, hq = system ? h / (H / Hqk) : h - H;
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    // k_j . k_i, or k_j . q_i: thread (ty, tx) has j = 4 ty .., i = 4 tx ..
+    const float* kh = k + (size_t)lo * k_ld + (size_t)hq * d;
+    const float* other = system ? kh : q + (size_t)lo * q_ld + (size_t)hq * d;
+    for (int k0 = 0; k0 < d; k0 += TILE) {
+        load_transposed(sA, kh, k_ld, n, d, k0, nullptr);
+        if (!system) load_transposed(sB, other, q_ld, n, d, k0, nullptr);
+        __syncthreads();
+        multiply<1>(acc, sA, system ? sA : sB, min(TILE, d - k0), ty, tx);
+        __syncthreads();
+    }
+    if (!system) {
+        float* out = dots + ((size_t)blockIdx.x * Hqk + hq) * CH * CH;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<float4*>(out + (4 * ty + i) * CH + 4 * tx) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        return;
+    }
+    chunk_sums(nullptr, loga, nullptr, nullptr, lo, n, H, h, cum, grown);
+    if (threadIdx.x >= 64 && threadIdx.x < 128) {
+        const int i = threadIdx.x - 64;
+        sbeta[i] = i < n ? beta[(size_t)(lo + i) * H + h] : 0.f;
+    }
+    __syncthreads();
+    // A transposed: sB[j][i], zero for i <= j (and beyond the chunk's tokens, whose beta is 0)
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int j = 4 * ty + a, i = 4 * tx + b;
+            sB[j][i] = j < i && i < n ? sbeta[i] * expf((float)(cum[i] - cum[j])) * acc[a][b] : 0.f;
+        }
+    if (threadIdx.x < CH) {
+        const size_t at = (size_t)blockIdx.x * H + h;
+        const double end = cum[CH - 1];
+        grown[threadIdx.x] = sbeta[threadIdx.x] * expf((float)cum[threadIdx.x]);
+        factors[at * CH + threadIdx.x] = expf((float)(end - cum[threadIdx.x]));
+        if (threadIdx.x == 0) decays[at] = expf((float)end);
+    }
+    __syncthreads();
+    // one column of the right-hand sides per thread, 64 unknowns in registers: each solved unknown is taken out of the
+    // rows below it (independent multiply-adds; A's numbers are the same address for the whole warp)
+    const uint32_t sb = (uint32_t)__cvta_generic_to_shared(&sB[0][0]);
+    for (int col = threadIdx.x; col < dv + d; col += NTH) {
+        float y[CH];
+        if (col < dv) {
+            const V* src = v + (size_t)lo * v_ld + (size_t)h * dv + col;
+#pragma unroll
+            for (int i = 0; i < CH; ++i, src += v_ld) y[i] = i < n ? sbeta[i] * to_f32(*src) : 0.f;
+        } else {
+            const float* src = kh + col - dv;
+#pragma unroll
+            for (int i = 0; i < CH; ++i, src += k_ld) y[i] = i < n ? grown[i] * *src : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < CH - 1; ++j) {
+            const float yj = y[j];
+#pragma unroll
+            for (int i4 = (j + 1) / 4; i4 < CH / 4; ++i4) {
+                float4 a;                                 // (volatile: the loads stay beside their use)
+                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w)
+                             : "r"(sb + (uint32_t)(j * PITCH + 4 * i4) * 4u));
+                if (4 * i4 > j) y[4 * i4] -= a.x * yj;
+                if (4 * i4 + 1 > j) y[4 * i4 + 1] -= a.y * yj;
+                if (4 * i4 + 2 > j) y[4 * i4 + 2] -= a.z * yj;
+                y[4 * i4 + 3] -= a.w * yj;
+            }
+        }
+        if (col < dv) {
+            float* dst = x_out + ((size_t)lo * H + h) * dv + col;
+#pragma unroll
+            for (int i = 0; i < CH; ++i, dst += H * dv)
+                if (i < n) *dst = y[i];
+        } else {
+            float* dst = w_out + (((size_t)blockIdx.x * H + h) * d + (col - dv)) * CH;
+#pragma unroll
+            for (int i = 0; i < CH; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(y[i], y[i + 1], y[i + 2], y[i + 3]);
+        }
+    }
+}
+
+// 16 bytes from global to shared memory, zeros where there are none
+__device__ __forceinline__ void dc_copy16(float* dst, const float* src, bool there) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(dst);
+    const int n = there ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(a), "l"(src), "r"(n));
+}
+
+// u [T, H, dv]: X on entry, U on return.  before [chunks, H, dv, d]: the state before every chunk.  d % 4 == 0, d <= 128,
+// dv % 4 == 0, rows of k 16-byte aligned.  grid: requests, H, groups of DC_CB columns; a chunk's W, K, X and factors are
+// fetched (cp.async) while the chunk before it is worked on.
+__global__ void __launch_bounds__(NTH)
+delta_states_kernel(const float* __restrict__ k, int k_ld, const float* __restrict__ w, const float* __restrict__ factors,
+                    const float* __restrict__ decays, float* __restrict__ u, float* __restrict__ before,
+                    float* __restrict__ state, const int* __restrict__ cu, const int* __restrict__ start_pos,
+                    const int* __restrict__ slots, int H, int Hqk, int d, int dv) {
+    extern __shared__ __align__(16) float sm[];
+    const int KP = d + 16;                              // pitch of K's rows: two neighbouring tokens lie 16 banks apart
+    const int stage_floats = d * DC_WP + CH * KP + CH * DC_CB + CH;
+    float* sS = sm + 2 * stage_floats;                  // [d][16], S
+    float* sU = sS + d * DC_CB;                         // [64][16], exp(c_L - c_i) u_i
+    pdl_wait();
+    pdl_trigger();
+    const int r = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * DC_CB, hq = h / (H / Hqk);
+    const int first = cu[r], last = cu[r + 1];
+    if (last <= first) return;
+    int c0 = 0;
+    for (int x = 0; x < r; ++x) c0 += (cu[x + 1] - cu[x] + CH - 1) / CH;
+    const int nc = (last - first + CH - 1) / CH;
+    const int cols = min(DC_CB, dv - j0);               // a multiple of 4
+    const int d4 = d / 4;
+    auto issue = [&](int c) {
+        float* st = sm + (c & 1) * stage_floats;
+        const int lo = first + c * CH, n = min(CH, last - lo);
+        const size_t at = (size_t)(c0 + c) * H + h;
+        for (int e = threadIdx.x; e < d * (CH / 4); e += NTH) {
+            const int kk = e / (CH / 4), i = e % (CH / 4) * 4;
+            dc_copy16(st + kk * DC_WP + i, w + (at * d + kk) * CH + i, true);
+        }
+        st += d * DC_WP;
+        for (int e = threadIdx.x; e < CH * d4; e += NTH) {
+            const int i = e / d4, kk = (e - i * d4) * 4;
+            dc_copy16(st + i * KP + kk, k + (size_t)(lo + min(i, n - 1)) * k_ld + (size_t)hq * d + kk, i < n);
+        }
+        st += CH * KP;
+        for (int e = threadIdx.x; e < CH * (DC_CB / 4); e += NTH) {
+            const int i = e / (DC_CB / 4), j = e % (DC_CB / 4) * 4;
+            const bool there = i < n && j < cols;
+            dc_copy16(st + i * DC_CB + j, u + ((size_t)(lo + min(i, n - 1)) * H + h) * dv + j0 + (j < cols ? j : 0), there);
+        }
+        if (threadIdx.x < CH / 4) dc_copy16(st + CH * DC_CB + 4 * threadIdx.x, factors + at * CH + 4 * threadIdx.x, true);
+        asm volatile("cp.async.commit_group;\n" ::);
+    };
+    issue(0);
+    // S: thread (k tile kt, column tile jt, half ih) keeps rows 4 kt .. + 3 of columns 4 jt + 2 ih and + 1
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ih = lane >> 4, jt = lane & 3, kt = warp * 4 + ((lane >> 2) & 3);
+    const bool owner = kt < d4;
+    const int slot = slots[r];
+    float S[2][4];
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+        const int j = 4 * jt + 2 * ih + b;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (owner && j < cols && slot >= 0 && start_pos[r] > 0)
+            x = *reinterpret_cast<const float4*>(state + (((size_t)slot * H + h) * dv + j0 + j) * d + 4 * kt);
+        S[b][0] = x.x; S[b][1] = x.y; S[b][2] = x.z; S[b][3] = x.w;
+    }
+    // the products W S0: thread (token tile it, column tile ju, quarter kq of the k, interleaved)
+    const int kq = lane >> 3, ju = lane & 3, it = warp * 2 + ((lane >> 2) & 1);
+    for (int c = 0; c < nc; ++c) {
+        const int lo = first + c * CH, n = min(CH, last - lo);
+        if (c + 1 < nc) issue(c + 1);
+        if (owner) {
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+                *reinterpret_cast<float2*>(sS + (4 * kt + a) * DC_CB + 4 * jt + 2 * ih) = make_float2(S[0][a], S[1][a]);
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                const int j = 4 * jt + 2 * ih + b;
+                if (j < cols)
+                    *reinterpret_cast<float4*>(before + (((size_t)(c0 + c) * H + h) * dv + j0 + j) * d + 4 * kt) =
+                        make_float4(S[b][0], S[b][1], S[b][2], S[b][3]);
+            }
+        }
+        if (c + 1 < nc) asm volatile("cp.async.wait_group 1;\n" ::);
+        else asm volatile("cp.async.wait_group 0;\n" ::);
+        __syncthreads();
+        const float* sW = sm + (c & 1) * stage_floats;
+        const float* sK = sW + d * DC_WP;
+        const float* sX = sK + CH * KP;
+        const float* sF = sX + CH * DC_CB;
+        {
+            float acc[4][4];
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) acc[a][b] = 0.f;
+#pragma unroll 8
+            for (int kk = kq; kk < d; kk += 4) {
+                const float4 wv = *reinterpret_cast<const float4*>(sW + kk * DC_WP + 4 * it);
+                const float4 sv = *reinterpret_cast<const float4*>(sS + kk * DC_CB + 4 * ju);
+                acc[0][0] += wv.x * sv.x; acc[0][1] += wv.x * sv.y; acc[0][2] += wv.x * sv.z; acc[0][3] += wv.x * sv.w;
+                acc[1][0] += wv.y * sv.x; acc[1][1] += wv.y * sv.y; acc[1][2] += wv.y * sv.z; acc[1][3] += wv.y * sv.w;
+                acc[2][0] += wv.z * sv.x; acc[2][1] += wv.z * sv.y; acc[2][2] += wv.z * sv.z; acc[2][3] += wv.z * sv.w;
+                acc[3][0] += wv.w * sv.x; acc[3][1] += wv.w * sv.y; acc[3][2] += wv.w * sv.z; acc[3][3] += wv.w * sv.w;
+            }
+            // the four quarters' sums: lane kq ends up with token 4 it + kq
+            float half[2][4], one[4];
+            const bool up2 = kq >> 1, up1 = kq & 1;
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    const float give = up2 ? acc[a][b] : acc[a + 2][b], keep = up2 ? acc[a + 2][b] : acc[a][b];
+                    half[a][b] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+                }
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const float give = up1 ? half[0][b] : half[1][b], keep = up1 ? half[1][b] : half[0][b];
+                one[b] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+            }
+            const int i = 4 * it + kq;
+            const float4 xv = *reinterpret_cast<const float4*>(sX + i * DC_CB + 4 * ju);
+            const float4 uv = make_float4(xv.x - one[0], xv.y - one[1], xv.z - one[2], xv.w - one[3]);
+            const float f = sF[i];
+            if (i < n && 4 * ju < cols) *reinterpret_cast<float4*>(u + ((size_t)(lo + i) * H + h) * dv + j0 + 4 * ju) = uv;
+            *reinterpret_cast<float4*>(sU + i * DC_CB + 4 * ju) =
+                i < n ? make_float4(f * uv.x, f * uv.y, f * uv.z, f * uv.w) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        __syncthreads();
+        {
+            const float g = decays[(size_t)(c0 + c) * H + h];
+            float acc[4][4];
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) acc[a][b] = 0.f;
+            if (owner) {
+#pragma unroll 8
+                for (int i = ih; i < n; i += 2) {
+                    const float4 kv = *reinterpret_cast<const float4*>(sK + i * KP + 4 * kt);
+                    const float4 uv = *reinterpret_cast<const float4*>(sU + i * DC_CB + 4 * jt);
+                    acc[0][0] += kv.x * uv.x; acc[0][1] += kv.x * uv.y; acc[0][2] += kv.x * uv.z; acc[0][3] += kv.x * uv.w;
+                    acc[1][0] += kv.y * uv.x; acc[1][1] += kv.y * uv.y; acc[1][2] += kv.y * uv.z; acc[1][3] += kv.y * uv.w;
+                    acc[2][0] += kv.z * uv.x; acc[2][1] += kv.z * uv.y; acc[2][2] += kv.z * uv.z; acc[2][3] += kv.z * uv.w;
+                    acc[3][0] += kv.w * uv.x; acc[3][1] += kv.w * uv.y; acc[3][2] += kv.w * uv.z; acc[3][3] += kv.w * uv.w;
+                }
+            }
+            // the two halves' sums: each keeps its two columns
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const float give = ih ? acc[a][b] : acc[a][2 + b], keep = ih ? acc[a][2 + b] : acc[a][b];
+                    S[b][a] = g * S[b][a] + (keep + __shfl_xor_sync(0xffffffffu, give, 16));
+                }
+        }
+        __syncthreads();                                // the stage and S may be overwritten
+    }
+    if (owner && slot >= 0) {
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            const int j = 4 * jt + 2 * ih + b;
+            if (j < cols)
+                *reinterpret_cast<float4*>(state + (((size_t)slot * H + h) * dv + j0 + j) * d + 4 * kt) =
+                    make_float4(S[b][0], S[b][1], S[b][2], S[b][3]);
+        }
+    }
+}
+
+// q, k [T, Hqk * d] float rows q_ld, k_ld apart; v [T, H * dv] float or bfloat16, rows v_ld apart; beta, loga [T, H];
+// state [slots, H, dv, d].  Results and scratch of the caller (chunks at least T / 64 + R, rounded down): u [T, H, dv],
+// before [chunks, H, dv, d], dots [chunks, Hqk, 64, 64]; w [chunks, H, d, 64], factors [chunks, H, 64], decays [chunks, H].
+// Takes d and dv in multiples of 4, d up to 128, rows of k and the state on 16-byte boundaries.
+extern "C" int rg_delta_chunk(const float* q, int q_ld, const float* k, int k_ld, const void* v, int v_dtype, int v_ld,
+                              const float* beta, const float* loga, float* state, const int* cu_seqlens, const int* start_pos,
+                              const int* slots, float* u, float* before, float* dots, float* w, float* factors, float* decays,
+                              int T, int R, int H, int Hqk, int d, int dv, void* stream) {
+    if (T <= 0 || R <= 0) return 0;
+    if (H < 1 || Hqk < 1 || H % Hqk || d < 4 || d % 4 || d > DC_MAX_D || dv < 4 || dv % 4 || H + Hqk > 65535 || k_ld % 4 ||
+        ((uintptr_t)k & 15) || ((uintptr_t)state & 15) || ((uintptr_t)u & 15) || ((uintptr_t)before & 15))
+        return RG_ERR_UNSUPPORTED;
+    const int groups = (dv + DC_CB - 1) / DC_CB;
+    if (groups > 65535) return RG_ERR_UNSUPPORTED;
+    cudaStream_t s = (cudaStream_t)stream;
+    dim3 g1(T / CH + R, H + Hqk);
+    int e;
+    if (v_dtype == RG_DTYPE_F32)
+        e = rg_launch(delta_solve_kernel<float>, g1, dim3(NTH), 0, s, 1, q, q_ld, k, k_ld, (const float*)v, v_ld, beta, loga,
+                      cu_seqlens, R, u, w, factors, decays, dots, H, Hqk, d, dv);
+    else if (v_dtype == RG_DTYPE_BF16)
+        e = rg_launch(delta_solve_kernel<bf16>, g1, dim3(NTH), 0, s, 1, q, q_ld, k, k_ld, (const bf16*)v, v_ld, beta, loga,
+                      cu_seqlens, R, u, w, factors, decays, dots, H, Hqk, d, dv);
+    else
+        return RG_ERR_UNSUPPORTED;
+    if (e) return e;
+    const size_t smem = ((size_t)2 * (d * DC_WP + CH * (d + 16) + CH * DC_CB + CH) + (d + CH) * DC_CB) * sizeof(float);
+    cudaError_t ce = cudaFuncSetAttribute(delta_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (ce != cudaSuccess) return (int)ce;
+    return rg_launch(delta_states_kernel, dim3(R, H, groups), dim3(NTH), smem, s, 1, k, k_ld, (const float*)w,
+                     (const float*)factors, (const float*)decays, u, before, state, cu_seqlens, start_pos, slots, H, Hqk, d, dv);
+}

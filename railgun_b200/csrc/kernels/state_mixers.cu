@@ -6,7 +6,7 @@
 //   conv_state_update  leaves the step's last K - 1 inputs in the slot
 //   retention_prepare  rotation of q and k in pairs (i, i + dims / 2), k times a constant, into 32-bit rows
 //   delta_prepare      q and k to unit length per head (q times a constant), beta = sigmoid(b),
-//                      g = exp(-exp(A) softplus(a + bias)) per head
+//                      g = exp(-exp(A) softplus(a + bias)) per head, or its logarithm
 //   state_scan         per head, token by token, S [d, dv] in 32-bit:
 //                        scalar decay:  S <- g S + beta k v^T;  o = S^T q + skip_h v
 //                                       (retention: g fixed per head, beta 1, skip 0; the state-space duality form of
@@ -22,7 +22,8 @@
 // The step's tokens are packed request by request (cu_seqlens); a request whose start position is 0 begins
 // from zeros whatever its slot holds; a row whose request has slot -1 (padding of a static batch) reads zeros
 // and writes no state.  A token's result depends on its request's earlier tokens only through the state, which
-// is carried in 32-bit, so cutting a prompt into portions changes no bit.
+// is carried in 32-bit, so cutting a prompt into portions changes no bit here (portions of 128 tokens and more run in
+// chunks, ssd_chunk.cu, delta_chunk.cu and channel_chunk.cu, where a cut moves the order of 32-bit sums).
 #include "common.cuh"
 
 __device__ __forceinline__ float sm_sigmoid(float z) { return 1.f / (1.f + expf(-z)); }
@@ -259,12 +260,12 @@ extern "C" int rg_retention_prepare(const void* proj, int dtype, int ld, int q_o
 }
 
 // qk [T, ld] float: q heads (G of d) at column 0, k heads at column G d, in place.  ab: rows ab_ld apart (type A),
-// the H numbers b at b_off and the H numbers a at a_off.  beta, g [T, H] float.
+// the H numbers b at b_off and the H numbers a at a_off.  beta, g (log_g 1: its logarithm) [T, H] float.
 template <typename A>
 __global__ void delta_prepare_kernel(float* __restrict__ qk, int ld, int G, int d, float q_scale, float unit_eps,
                                      const A* __restrict__ ab, int ab_ld, int b_off, int a_off,
                                      const float* __restrict__ A_log, const float* __restrict__ dt_bias,
-                                     float* __restrict__ beta, float* __restrict__ g, int H) {
+                                     float* __restrict__ beta, float* __restrict__ g, int log_g, int H) {
     pdl_wait();
     pdl_trigger();
     const int t = blockIdx.x;
@@ -282,23 +283,24 @@ __global__ void delta_prepare_kernel(float* __restrict__ qk, int ld, int G, int 
         const float bz = to_f32(ab[(size_t)t * ab_ld + b_off + h]);
         const float az = to_f32(ab[(size_t)t * ab_ld + a_off + h]) + dt_bias[h];
         beta[(size_t)t * H + h] = sm_sigmoid(bz);
-        g[(size_t)t * H + h] = expf(-expf(A_log[h]) * sm_softplus(az));
+        const float a = -expf(A_log[h]) * sm_softplus(az);
+        g[(size_t)t * H + h] = log_g ? a : expf(a);
     }
 }
 
 extern "C" int rg_delta_prepare(float* qk, int ld, int G, int d, float q_scale, float unit_eps, const void* ab,
                                 int ab_dtype, int ab_ld, int b_off, int a_off, const float* A_log, const float* dt_bias,
-                                float* beta, float* g, int T, int H, void* stream) {
+                                float* beta, float* g, int log_g, int T, int H, void* stream) {
     if (T <= 0) return 0;
     if (G < 1 || d < 1 || H < 1) return RG_ERR_UNSUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
     const int threads = 2 * G >= 8 ? 256 : 128;
     if (ab_dtype == RG_DTYPE_BF16)
         return rg_launch(delta_prepare_kernel<bf16>, dim3(T), dim3(threads), 0, s, 1, qk, ld, G, d, q_scale, unit_eps,
-                         (const bf16*)ab, ab_ld, b_off, a_off, A_log, dt_bias, beta, g, H);
+                         (const bf16*)ab, ab_ld, b_off, a_off, A_log, dt_bias, beta, g, log_g, H);
     if (ab_dtype == RG_DTYPE_F32)
         return rg_launch(delta_prepare_kernel<float>, dim3(T), dim3(threads), 0, s, 1, qk, ld, G, d, q_scale, unit_eps,
-                         (const float*)ab, ab_ld, b_off, a_off, A_log, dt_bias, beta, g, H);
+                         (const float*)ab, ab_ld, b_off, a_off, A_log, dt_bias, beta, g, log_g, H);
     return RG_ERR_UNSUPPORTED;
 }
 

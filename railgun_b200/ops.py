@@ -1035,11 +1035,11 @@ def retention_prepare(proj: torch.Tensor, q_off: int, k_off: int, freq: torch.Te
 
 
 def delta_prepare(qkv: torch.Tensor, G: int, d: int, q_scale: float, unit_eps: float, ab: torch.Tensor, b_off: int,
-                  a_off: int, A_log: torch.Tensor, dt_bias: torch.Tensor, H: int):
+                  a_off: int, A_log: torch.Tensor, dt_bias: torch.Tensor, H: int, log_g: bool = False):
     """In place on ``qkv`` [T, >= 2 G d] float32: the G query heads (from column 0) and the G key heads (from
     column G d) become unit vectors, x / sqrt(sum(x^2) + ``unit_eps``), the queries times ``q_scale``.  Returns
     beta = sigmoid(ab[:, b_off:b_off + H]) and g = exp(-exp(A_log) softplus(ab[:, a_off:a_off + H] + dt_bias)),
-    both [T, H] float32."""
+    both [T, H] float32 (``log_g``: the logarithm of g in its place)."""
     _check_rows(qkv, "qkv", torch.float32)
     _check_rows(ab, "ab")
     _check(A_log, "A_log", torch.float32)
@@ -1053,7 +1053,7 @@ def delta_prepare(qkv: torch.Tensor, G: int, d: int, q_scale: float, unit_eps: f
     _ok(_fn("state_mixers", "rg_delta_prepare")(
         _ptr(qkv), c_int(qkv.stride(0)), c_int(G), c_int(d), c_float(q_scale), c_float(unit_eps), _ptr(ab),
         c_int(_dtype_code(ab)), c_int(ab.stride(0)), c_int(b_off), c_int(a_off), _ptr(A_log), _ptr(dt_bias), _ptr(beta),
-        _ptr(g), c_int(T), c_int(H), _stream()), "delta_prepare")
+        _ptr(g), c_int(1 if log_g else 0), c_int(T), c_int(H), _stream()), "delta_prepare")
     return beta, g
 
 
@@ -1265,16 +1265,87 @@ def ssd_chunk_scan(xbc: torch.Tensor, dt: torch.Tensor, A_log: torch.Tensor, D: 
     if xbc.shape[1] != inner + 2 * G * N or tuple(dt.shape) != (T, H) or A_log.numel() != H or D.numel() != H \
             or tuple(state.shape[1:]) != (H, dv, N) or H % G:
         raise KernelError("ssd_chunk_scan: sizes do not match")
-    chunks = T // SCAN_CHUNK + R
-    new = lambda *shape: torch.empty(shape, dtype=torch.float32, device=xbc.device)
-    sums, decays, dots = new(chunks, H, dv, N), new(chunks, H), new(chunks, G, SCAN_CHUNK, SCAN_CHUNK)
-    o = new(T, H, dv)
-    _COUNTER.value += 2                              # the launcher runs three kernels
     at = lambda col: c_void_p(xbc.data_ptr() + 4 * col)
+    ld = c_int(xbc.stride(0))
+    return _chunk_scan((at(0), c_int(0), ld), (at(inner), ld), (at(inner + G * N), ld), dt, None, A_log, None, D, state, batch,
+                       T, H, G, N, dv, 0, "ssd_chunk_scan")
+
+
+def _chunk_scan(x, B, C, dt, loga, A_log, fixed, D, state, batch, T, H, G, N, dv, ones, what):
+    """The three kernels of csrc/kernels/ssd_chunk.cu.  ``x``: (pointer, type code, row step), ``B``, ``C``: (pointer, row
+    step).  Returns o [T, H, dv + ones] float32."""
+    R, M = batch.num_requests, dv + ones
+    chunks = T // SCAN_CHUNK + R
+    new = lambda *shape: torch.empty(shape, dtype=torch.float32, device=state.device)
+    sums, decays, dots, o = new(chunks, H, M, N), new(chunks, H), new(chunks, G, SCAN_CHUNK, SCAN_CHUNK), new(T, H, M)
+    _COUNTER.value += 2                              # the launcher runs three kernels
     _ok(_fn("ssd_chunk", "rg_ssd_chunk_scan")(
-        at(0), at(inner), at(inner + G * N), c_int(xbc.stride(0)), _ptr(dt), _ptr(None), _ptr(A_log), _ptr(D), _ptr(state),
-        _ptr(batch.cu_seqlens), _ptr(batch.start_pos), _ptr(batch.state_slots), _ptr(sums), _ptr(decays), _ptr(dots), _ptr(o),
-        c_int(T), c_int(R), c_int(H), c_int(G), c_int(N), c_int(dv), c_int(0), _stream()), "ssd_chunk_scan")
+        *x, *B, *C, _ptr(dt), _ptr(loga), _ptr(A_log), _ptr(fixed), _ptr(D), _ptr(state), _ptr(batch.cu_seqlens),
+        _ptr(batch.start_pos), _ptr(batch.state_slots), _ptr(sums), _ptr(decays), _ptr(dots), _ptr(o), c_int(T), c_int(R),
+        c_int(H), c_int(G), c_int(N), c_int(dv), c_int(ones), _stream()), what)
+    return o
+
+
+def _check_scan_rows(q, k, v, state, H: int, d: int, dv: int, what: str) -> int:
+    """Checks of q, k, v and the state of a recurrence in chunks; the number of query/key heads."""
+    for t, name in ((q, "q"), (k, "k")):
+        _check_rows(t, name, torch.float32)
+    _check_rows(v, "v")
+    _check(state, "state", torch.float32)
+    T, Hqk = q.shape[0], q.shape[1] // d
+    if Hqk < 1 or q.shape[1] != Hqk * d or k.shape != q.shape or v.shape != (T, H * dv) or H % Hqk \
+            or tuple(state.shape[1:]) != (H, dv, d):
+        raise KernelError(f"{what}: q {tuple(q.shape)}, k {tuple(k.shape)}, v {tuple(v.shape)}, state {tuple(state.shape)} do "
+                          f"not match {H} heads of {d} x {dv}")
+    return Hqk
+
+
+def decay_chunk_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, batch, H: int, d: int, dv: int,
+                     log_decay: torch.Tensor) -> torch.Tensor:
+    """S <- decay_h S + k v^T, o = S^T q per head along each request's tokens, as ``state_scan`` with a fixed decay per head
+    computes it token by token, in chunks of 64 tokens side by side.  ``log_decay``: float64 [H], the decays' logarithms
+    (minus infinity: nothing is kept).  q, k, v, state and the result as ``state_scan``'s."""
+    Hqk = _check_scan_rows(q, k, v, state, H, d, dv, "decay_chunk_scan")
+    _check(log_decay, "log_decay", torch.float64)
+    if log_decay.numel() != H:
+        raise KernelError(f"decay_chunk_scan: {log_decay.numel()} decays for {H} heads")
+    return _chunk_scan((_ptr(v), c_int(_dtype_code(v)), c_int(v.stride(0))), (_ptr(k), c_int(k.stride(0))),
+                       (_ptr(q), c_int(q.stride(0))), None, None, None, log_decay, None, state, batch, q.shape[0], H, Hqk, d, dv,
+                       0, "decay_chunk_scan")
+
+
+def delta_chunk_ok(k: torch.Tensor, state: torch.Tensor, d: int, dv: int) -> bool:
+    """Can the delta rule in chunks take these?  Heads of up to 128 in multiples of 4, rows on 16-byte boundaries."""
+    return (d <= 128 and d % 4 == 0 and dv % 4 == 0 and k.stride(0) % 4 == 0 and k.data_ptr() % 16 == 0
+            and state.data_ptr() % 16 == 0)
+
+
+def delta_chunk_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, batch, H: int, d: int, dv: int,
+                     loga: torch.Tensor, beta: torch.Tensor) -> torch.Tensor:
+    """S <- exp(loga) S, u = beta (v - S^T k), S <- S + k u^T, o = S^T q per head along each request's tokens, as
+    ``state_scan`` with the delta rule computes it token by token, in chunks of 64 tokens (csrc/kernels/delta_chunk.cu).
+    ``loga``, ``beta``: float32 [T, H]; q, k, v, state and the result as ``state_scan``'s."""
+    Hqk = _check_scan_rows(q, k, v, state, H, d, dv, "delta_chunk_scan")
+    T, R = q.shape[0], batch.num_requests
+    for t, name in ((loga, "loga"), (beta, "beta")):
+        _check(t, name, torch.float32)
+        if t.numel() != T * H:
+            raise KernelError(f"delta_chunk_scan: {name} has {t.numel()} elements, expected {T * H}")
+    if not delta_chunk_ok(k, state, d, dv):
+        raise KernelError("delta_chunk_scan: heads of up to 128 in multiples of 4, rows on 16-byte boundaries")
+    chunks = T // SCAN_CHUNK + R
+    new = lambda *shape: torch.empty(shape, dtype=torch.float32, device=state.device)
+    u, before, dots, o = new(T, H, dv), new(chunks, H, dv, d), new(chunks, Hqk, SCAN_CHUNK, SCAN_CHUNK), new(T, H, dv)
+    w, factors, decays = new(chunks, H, d, SCAN_CHUNK), new(chunks, H, SCAN_CHUNK), new(chunks, H)
+    _COUNTER.value += 1                              # the launcher runs two kernels
+    _ok(_fn("delta_chunk", "rg_delta_chunk")(
+        _ptr(q), c_int(q.stride(0)), _ptr(k), c_int(k.stride(0)), _ptr(v), c_int(_dtype_code(v)), c_int(v.stride(0)), _ptr(beta),
+        _ptr(loga), _ptr(state), _ptr(batch.cu_seqlens), _ptr(batch.start_pos), _ptr(batch.state_slots), _ptr(u), _ptr(before),
+        _ptr(dots), _ptr(w), _ptr(factors), _ptr(decays), c_int(T), c_int(R), c_int(H), c_int(Hqk), c_int(d), c_int(dv),
+        _stream()), "delta_chunk_scan")
+    _ok(_fn("ssd_chunk", "rg_chunk_outputs")(
+        _ptr(u), c_int(H * dv), _ptr(q), c_int(q.stride(0)), _ptr(loga), _ptr(batch.cu_seqlens), _ptr(before), _ptr(dots),
+        _ptr(o), c_int(T), c_int(R), c_int(H), c_int(Hqk), c_int(d), c_int(dv), _stream()), "delta_chunk_scan")
     return o
 
 
@@ -1325,15 +1396,10 @@ def mlstm_scan(proj: torch.Tensor, ib: torch.Tensor, fb: torch.Tensor, cap: floa
         o = state_scan(proj[:, :k_off], proj[:, k_off:v_off], proj[:, v_off:g_off], state, batch, H, d, dv + 1, g=keep,
                        beta=put, rule="scalar", ones=True)
         return o, m_rows
-    chunks = T // SCAN_CHUNK + R
-    sums, decays, dots = new(chunks, H, dv + 1, d), new(chunks, H), new(chunks, H, SCAN_CHUNK, SCAN_CHUNK)
-    o = new(T, H, dv + 1)
-    _COUNTER.value += 2                              # the launcher runs three kernels
     at = lambda col: c_void_p(proj.data_ptr() + 4 * col)
-    _ok(_fn("ssd_chunk", "rg_ssd_chunk_scan")(
-        at(v_off), at(k_off), at(q_off), c_int(proj.stride(0)), _ptr(put), _ptr(keep), _ptr(None), _ptr(None), _ptr(state),
-        _ptr(batch.cu_seqlens), _ptr(batch.start_pos), _ptr(batch.state_slots), _ptr(sums), _ptr(decays), _ptr(dots), _ptr(o),
-        c_int(T), c_int(R), c_int(H), c_int(H), c_int(d), c_int(dv), c_int(1), _stream()), "mlstm_chunk_scan")
+    ld = c_int(proj.stride(0))
+    o = _chunk_scan((at(v_off), c_int(0), ld), (at(k_off), ld), (at(q_off), ld), put, keep, None, None, None, state, batch, T, H,
+                    H, d, dv, 1, "mlstm_chunk_scan")
     return o, m_rows
 
 

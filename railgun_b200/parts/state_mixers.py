@@ -70,6 +70,7 @@ class Retention(Mixer):
         if len(decay) != self.H:
             raise ValueError(f"{len(decay)} decays for {self.H} heads")
         self.decay = torch.tensor(decay, dtype=torch.float32, device=env.device)
+        self.log_decay = self.decay.double().log() if min(decay) >= 0 else None      # None: no recurrence in chunks
         self.rot_dims = int(p.get("rot_dims") or 0)
         if self.rot_dims % 2 or not 0 <= self.rot_dims <= self.d:
             raise ValueError(f"{self.rot_dims} rotated numbers do not fit a head of {self.d}")
@@ -106,7 +107,10 @@ class Retention(Mixer):
         else:
             q, k = ops.retention_prepare(proj, 0, H * d, self.freq, self.rot_dims, batch.positions, H, d, self.k_scale)
             v = proj[:, 2 * H * d:2 * H * d + H * dv]
-        o = ops.state_scan(q.view(-1, H * d), k.view(-1, H * d), v, cache.state, batch, H, d, dv, decay=self.decay)
+        if self.log_decay is not None and batch.max_query_len >= ops.SCAN_CHUNKED_MIN_TOKENS:
+            o = ops.decay_chunk_scan(q.view(-1, H * d), k.view(-1, H * d), v, cache.state, batch, H, d, dv, self.log_decay)
+        else:
+            o = ops.state_scan(q.view(-1, H * d), k.view(-1, H * d), v, cache.state, batch, H, d, dv, decay=self.decay)
         z = ops.head_norm_gate(o, proj[:, 2 * H * d + H * dv:], self.norm, self.eps, self.env.dtype, whole=self.whole,
                                gate_kind=self.gate)
         return ops.linear(z, self.w_o)
@@ -164,9 +168,14 @@ class GatedDelta(Mixer):
         qkv = ops.causal_conv(proj, 0, self.taps, conv_state, batch, torch.float32, silu=True)
         if writes and conv_state is not None:
             ops.conv_state_update(proj, 0, conv_state, batch)
-        beta, g = ops.delta_prepare(qkv, G, d, self.q_scale, self.unit_eps, ba, 0, H, self.A_log, self.dt_bias, H)
-        o = ops.state_scan(qkv[:, :G * d], qkv[:, G * d:2 * G * d], qkv[:, 2 * G * d:], cache.parts[0].state, batch,
-                           H, d, dv, g=g, beta=beta)
+        q, k, v, state = qkv[:, :G * d], qkv[:, G * d:2 * G * d], qkv[:, 2 * G * d:], cache.parts[0].state
+        chunked = batch.max_query_len >= ops.SCAN_CHUNKED_MIN_TOKENS and ops.delta_chunk_ok(k, state, d, dv)
+        beta, g = ops.delta_prepare(qkv, G, d, self.q_scale, self.unit_eps, ba, 0, H, self.A_log, self.dt_bias, H,
+                                    log_g=chunked)
+        if chunked:
+            o = ops.delta_chunk_scan(q, k, v, state, batch, H, d, dv, g, beta)
+        else:
+            o = ops.state_scan(q, k, v, state, batch, H, d, dv, g=g, beta=beta)
         z = ops.head_norm_gate(o, proj[:, C:], self.norm, self.eps, self.env.dtype)
         return ops.linear(z, self.w_o)
 

@@ -1,0 +1,108 @@
+"""Retention's and the delta rule's recurrences in chunks against the token-by-token loop in 64 bits, where they can go
+wrong: portions of one token to several chunks, chunks of one token, requests that continue or have no slot, heads that share
+keys, sizes that fill no tile, decays of 0 and 1, keys that point the same way."""
+import numpy as np
+import pytest
+import torch
+
+from test_mepatar_gpu import dev, rel, step_batch
+
+pytestmark = pytest.mark.gpu
+# 32-bit sums of up to 64 + 128 terms, through at most five chunks: about 1e-6 is seen; and what the token-by-token kernel
+# is held to
+BOUND = 2e-5
+
+
+def loop(q, k, v, S, g, beta=None):
+    o = np.zeros_like(v)
+    for t in range(q.shape[0]):
+        S *= g[t]
+        S += np.outer(k[t], v[t] if beta is None else beta[t] * (v[t] - S.T @ k[t]))
+        o[t] = S.T @ q[t]
+    return o
+
+
+SIZES = [(4, 4, 32, 16), (4, 2, 16, 8), (3, 1, 8, 24), (5, 5, 12, 20), (2, 2, 128, 128), (4, 2, 64, 136), (2, 1, 100, 72),
+         (1, 1, 4, 4)]
+LENGTHS = [[64, 1, 65], [63, 128, 200], [129], [300, 2]]
+
+
+@pytest.mark.parametrize("rule", ["retention", "delta"])
+@pytest.mark.parametrize("lengths", LENGTHS)
+@pytest.mark.parametrize("H,Hqk,d,dv", SIZES)
+def test_chunks_against_the_loop(H, Hqk, d, dv, lengths, rule):
+    from railgun_b200 import ops
+    rng = np.random.default_rng(H * d + dv + lengths[0])
+    R, T = len(lengths), sum(lengths)
+    q, k = rng.normal(size=(2, T, Hqk, d)) * 0.3
+    v = rng.normal(size=(T, H, dv))
+    if rule == "delta":
+        k += rng.normal(size=(1, Hqk, d)) * 0.6                       # keys that partly point the same way
+        k /= np.linalg.norm(k, axis=-1, keepdims=True)
+        loga = -rng.exponential(size=(T, H)) * np.logspace(-4, 0.5, H)
+        beta = rng.uniform(0.05, 1.0, size=(T, H))
+    else:
+        decay = np.linspace(0.9, 1.0, H) if H != 3 else np.array([0.0, 0.5, 1.0])
+        loga = np.broadcast_to(np.log(np.maximum(decay, 1e-300)), (T, H))
+        beta = None
+    v_type = torch.bfloat16 if d == 128 else torch.float32
+    v = torch.tensor(v, dtype=v_type).double().numpy()
+    slots = [R - 1 - r for r in range(R)]
+    starts = [0 if r == 1 else 7 for r in range(R)]
+    state0 = rng.normal(size=(R + 1, H, dv, d))
+    f32 = lambda a: dev(np.ascontiguousarray(a), torch.float32)
+    state = f32(state0)
+    rows = torch.cat([f32(q.reshape(T, -1)), f32(k.reshape(T, -1)), torch.zeros(T, 4, device=state.device)], 1)   # views
+    qv, kv = rows[:, :Hqk * d], rows[:, Hqk * d:2 * Hqk * d]
+    vv = dev(v.reshape(T, -1), v_type)
+    batch = step_batch(lengths, starts, slots)
+    if rule == "delta":
+        got = ops.delta_chunk_scan(qv, kv, vv, state, batch, H, d, dv, f32(loga), f32(beta))
+    else:
+        got = ops.decay_chunk_scan(qv, kv, vv, state, batch, H, d, dv, f32(decay).double().log())
+    got, state = got.cpu().double().numpy(), state.cpu().double().numpy()
+    assert np.isfinite(got).all()
+    g = np.exp(loga) if rule == "delta" else np.broadcast_to(f32(decay).double().cpu().numpy(), (T, H))
+    lo = 0
+    for r, n in enumerate(lengths):
+        for h in range(H):
+            S = state0[slots[r], h].T.copy() if starts[r] else np.zeros((d, dv))
+            span, hq = slice(lo, lo + n), h // (H // Hqk)
+            ref = loop(q[span, hq], k[span, hq], v[span, h], S, g[span, h], beta[span, h] if rule == "delta" else None)
+            assert rel(got[span, h], ref) < BOUND and rel(state[slots[r], h], S.T) < BOUND, (r, h)
+        lo += n
+    assert np.array_equal(state[R], state0[R].astype(np.float32))     # nobody's slot
+
+
+@pytest.mark.parametrize("rule", ["retention", "delta"])
+def test_no_slot_and_cut_portions(rule):
+    """A row without a slot reads zeros and writes nothing; a prompt in two portions is what it is in one."""
+    from railgun_b200 import ops
+    H, d, dv, T = 2, 32, 32, 210
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = (0.2 * torch.randn(T, H * d, device="cuda", generator=gen) for _ in range(3))
+    k = torch.nn.functional.normalize(k.view(T, H, d), dim=-1).reshape(T, H * d)
+    loga = -torch.rand(T, H, device="cuda", generator=gen) * 0.1
+    beta = torch.rand(T, H, device="cuda", generator=gen)
+    log_decay = torch.tensor([-0.01, -0.2], dtype=torch.float64, device="cuda")
+
+    def run(lo, hi, state, start, slot):
+        batch, part = step_batch([hi - lo], [start], [slot]), slice(lo, hi)
+        if rule == "delta":
+            return ops.delta_chunk_scan(q[part], k[part], v[part], state, batch, H, d, dv, loga[part].contiguous(), beta[part].contiguous())
+        return ops.decay_chunk_scan(q[part], k[part], v[part], state, batch, H, d, dv, log_decay)
+
+    state = torch.full((1, H, dv, d), 9.0, device="cuda")
+    whole = run(0, T, state, 0, 0)
+    kept = state.clone()
+    assert rel(run(0, T, state, 5, -1), whole.cpu().double().numpy()) < 1e-6 and torch.equal(state, kept)
+    two = torch.cat([run(0, 77, state, 0, 0), run(77, T, state, 77, 0)])
+    assert rel(two, whole.cpu().double().numpy()) < BOUND and rel(state, kept.cpu().double().numpy()) < BOUND
+
+
+def test_what_it_refuses():
+    from railgun_b200 import ops
+    state = torch.zeros(1, 1, 4, 6, device="cuda")
+    assert not ops.delta_chunk_ok(torch.zeros(2, 6, device="cuda"), state, 6, 4)
+    assert not ops.delta_chunk_ok(torch.zeros(2, 132, device="cuda"), torch.zeros(1, 1, 4, 132, device="cuda"), 132, 4)
+    assert not ops.delta_chunk_ok(torch.zeros(2, 9, device="cuda")[:, 1:], torch.zeros(1, 1, 4, 8, device="cuda"), 8, 4)
