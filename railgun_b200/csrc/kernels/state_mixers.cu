@@ -241,6 +241,91 @@ __global__ void retention_prepare_kernel(const A* __restrict__ proj, int ld, int
     }
 }
 
+__device__ __forceinline__ void sm_load8(const float* p, float (&v)[8]) {
+    const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void sm_load8(const bf16* p, float (&v)[8]) {
+    const uint4 x = *reinterpret_cast<const uint4*>(p);
+    const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
+        v[2 * i] = f.x; v[2 * i + 1] = f.y;
+    }
+}
+__device__ __forceinline__ void sm_store8(float* p, const float (&v)[8]) {
+    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
+}
+
+// The same, eight neighbouring numbers and their eight partners at a time, where sizes and addresses allow it (d, dims / 2
+// and H dv multiples of 8, rows on 16-byte boundaries).  The form above takes two bytes and two divisions a number; and the
+// angles, the only 64-bit work, are made here before the wait for the kernel before this one (positions were written
+// before the step's first kernel).  Measured (16 heads of 128): 2,048 tokens 39.0 to 11.2 us; 6 tokens of 8 heads 8.4 to 3.5.
+template <typename A>
+__global__ void retention_prepare8_kernel(const A* __restrict__ proj, int ld, int q_off, int k_off,
+                                          const double* __restrict__ freq, int dims, const int* __restrict__ positions,
+                                          float* __restrict__ q_out, float* __restrict__ k_out, int H, int d,
+                                          float k_scale, int act, int v_off, int dv, float* __restrict__ v_out) {
+    extern __shared__ __align__(16) float cs[];      // cos | sin of the token's dims / 2 angles
+    const int t = blockIdx.x;
+    const int half = dims >> 1;
+    const double pos = (double)positions[t];
+    for (int i = threadIdx.x; i < half; i += blockDim.x) rotary_cos_sin(pos, freq[i], &cs[i], &cs[half + i]);
+    pdl_wait();
+    pdl_trigger();
+    __syncthreads();
+    const A* row = proj + (size_t)t * ld;
+    auto activate = [&](float (&v)[8]) {
+        if (act) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] *= sm_sigmoid(v[j]);
+        }
+    };
+    // a head: half / 8 pieces with their partners, then (d - dims) / 8 that are not rotated
+    const int turned = half >> 3, per_head = turned + ((d - dims) >> 3), items = H * per_head;
+    for (int e = threadIdx.x; e < 2 * items; e += blockDim.x) {
+        const bool is_k = e >= items;
+        const int rem = is_k ? e - items : e, h = rem / per_head, c = rem - h * per_head;
+        const A* src = row + (is_k ? k_off : q_off) + (size_t)h * d;
+        float* dst = (is_k ? k_out : q_out) + ((size_t)t * H + h) * d;
+        const float scale = is_k ? k_scale : 1.f;
+        if (c < turned) {
+            const int i = 8 * c;
+            float u[8], v[8], a[8], b[8];
+            sm_load8(src + i, u);
+            sm_load8(src + half + i, v);
+            activate(u);
+            activate(v);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float cosa = cs[i + j], sina = cs[half + i + j];
+                a[j] = (u[j] * cosa - v[j] * sina) * scale;
+                b[j] = (v[j] * cosa + u[j] * sina) * scale;
+            }
+            sm_store8(dst + i, a);
+            sm_store8(dst + half + i, b);
+        } else {
+            const int i = dims + 8 * (c - turned);
+            float u[8];
+            sm_load8(src + i, u);
+            activate(u);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) u[j] *= scale;
+            sm_store8(dst + i, u);
+        }
+    }
+    if (v_out) {
+        for (int e = threadIdx.x; e < H * dv / 8; e += blockDim.x) {
+            float u[8];
+            sm_load8(row + v_off + 8 * e, u);
+            activate(u);
+            sm_store8(v_out + (size_t)t * H * dv + 8 * e, u);
+        }
+    }
+}
+
 extern "C" int rg_retention_prepare(const void* proj, int dtype, int ld, int q_off, int k_off, const double* freq,
                                     int dims, const int* positions, float* q_out, float* k_out, int T, int H, int d,
                                     float k_scale, int act, int v_off, int dv, float* v_out, void* stream) {
@@ -250,6 +335,15 @@ extern "C" int rg_retention_prepare(const void* proj, int dtype, int ld, int q_o
     const size_t smem = (size_t)(dims > 0 ? dims : 1) * sizeof(float);
     if (smem > 48 * 1024) return RG_ERR_UNSUPPORTED;
     const int threads = 2 * H * d >= 512 ? 256 : 128;
+    const bool by8 = d % 8 == 0 && dims % 16 == 0 && ld % 8 == 0 && q_off % 8 == 0 && k_off % 8 == 0 &&
+                     (!v_out || (v_off % 8 == 0 && (H * dv) % 8 == 0)) &&
+                     (((uintptr_t)proj | (uintptr_t)q_out | (uintptr_t)k_out | (uintptr_t)v_out) & 15) == 0;
+    if (by8 && dtype == RG_DTYPE_BF16)
+        return rg_launch(retention_prepare8_kernel<bf16>, dim3(T), dim3(threads), smem, s, 1, (const bf16*)proj, ld, q_off,
+                         k_off, freq, dims, positions, q_out, k_out, H, d, k_scale, act, v_off, dv, v_out);
+    if (by8 && dtype == RG_DTYPE_F32)
+        return rg_launch(retention_prepare8_kernel<float>, dim3(T), dim3(threads), smem, s, 1, (const float*)proj, ld, q_off,
+                         k_off, freq, dims, positions, q_out, k_out, H, d, k_scale, act, v_off, dv, v_out);
     if (dtype == RG_DTYPE_BF16)
         return rg_launch(retention_prepare_kernel<bf16>, dim3(T), dim3(threads), smem, s, 1, (const bf16*)proj, ld, q_off,
                          k_off, freq, dims, positions, q_out, k_out, H, d, k_scale, act, v_off, dv, v_out);
