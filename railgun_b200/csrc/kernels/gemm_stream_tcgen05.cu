@@ -4,10 +4,11 @@
 // streams through a ring of TMA stages exactly once.  At these sizes the product is bound by reading W, and a
 // product with few rows of W (q|k|v, O, down) has too few 128-row tiles to occupy the GPU, so K is split over the
 // CTAs of a thread-block cluster: every CTA accumulates its K range of the cluster's tile, leaves the partial sums
-// in its shared memory, and the cluster's CTAs add them, each for its share of the tokens, reading the others'
-// through distributed shared memory in rank order: one fixed order, no atomics, a token's result does not depend on
-// the batch.  Products with many tiles (gate|up, the head) run unsplit and persistent: a CTA takes tile after tile
-// with two accumulators in tensor memory, so that a tile's epilogue overlaps the next tile's loads.
+// in its shared memory (over the stages, which are done with by then), and the cluster's CTAs add them, each for its
+// share of the tokens, reading the others' through distributed shared memory in rank order: one fixed order, no
+// atomics, a token's result does not depend on the batch.  Products with many tiles (gate|up, the head) run unsplit
+// and persistent: a CTA takes tile after tile with two accumulators in tensor memory, so that a tile's epilogue
+// overlaps the next tile's loads.
 //
 // Roles as in gemm_tcgen05.cu: warps 0-3 epilogue (one lane of tensor memory = one row of W each), warp 4 the TMA
 // producer, warp 5 issues the MMAs and owns the tensor memory.  Epilogues: plain (bfloat16 or 32-bit out) and
@@ -22,7 +23,7 @@
 #define TS_TOK 64                 // tokens per tile (the MMA's N); fewer tokens are padded with zeros by TMA
 #define TS_BK 64
 #define TS_THREADS 192
-#define TS_STAGES 6
+#define TS_MAX_SPLITS 8
 #define TS_EPI_NONE 0
 #define TS_EPI_SILU_MUL 1
 #define TS_EPI_RESIDUAL 2         // out (32-bit) += product; also the next norm's input and sums of squares
@@ -63,156 +64,230 @@ __device__ __forceinline__ float4 ts_ld_remote4(uint32_t addr) {
     return v;
 }
 
-// A tile's sums -> the output, for the tokens m_lo .. m_hi - 1, by `nthreads` threads (a multiple of 32) of which
-// this is thread `tid`.  load4(r, i) gives partial sums i .. i + 3 of CTA r's [token][row] array; they are added in
-// rank order.  inv: 1 / rms per token (TS_PRO_SCALED).
-template <int SPLITS, int EPI, int PRO, typename OUT, typename Load>
-__device__ __forceinline__ void ts_write_out(Load load4, OUT* __restrict__ out, int ldo, int N, int n0, int tile,
-                                             int m_lo, int m_hi, int tid, int nthreads, const float* inv,
-                                             const StreamFusion& fu) {
-    if constexpr (EPI == TS_EPI_ROPE_CACHE) {
-        // rows 16 t .. + 7 and their partners + 8: four rotation pairs at a time
-        const int half = fu.d >> 1;
-        for (int idx = tid; idx < (m_hi - m_lo) * (TS_ROWS / 8); idx += nthreads) {
-            const int m = m_lo + idx / (TS_ROWS / 8), q = idx % (TS_ROWS / 8);
-            const int row = (q >> 1) * 16 + (q & 1) * 4;
-            float4 a[SPLITS], b[SPLITS];
-#pragma unroll
-            for (int r = 0; r < SPLITS; ++r) { a[r] = load4(r, m * TS_ROWS + row); b[r] = load4(r, m * TS_ROWS + row + 8); }
-            float4 as = a[0], bs = b[0];
-#pragma unroll
-            for (int r = 1; r < SPLITS; ++r) {
-                as.x += a[r].x; as.y += a[r].y; as.z += a[r].z; as.w += a[r].w;
-                bs.x += b[r].x; bs.y += b[r].y; bs.z += b[r].z; bs.w += b[r].w;
-            }
-            const float sc = PRO == TS_PRO_SCALED ? inv[m] : 1.f;
-            const float x0[4] = {as.x * sc, as.y * sc, as.z * sc, as.w * sc}, x1[4] = {bs.x * sc, bs.y * sc, bs.z * sc, bs.w * sc};
-            const int f = n0 + row;                                          // output feature of the first pair's first element
-            if (f + 8 >= N) continue;
-            const int head = f / fu.d, e = f - head * fu.d;                  // e: storage index inside the head (a multiple of 4)
-            float y0[4], y1[4];
-            if (head < fu.nh + fu.nkv) {
-                int pos = fu.positions[m];
-                if (pos < 0 || pos >= fu.max_pos) {
-                    if (fu.pos_err) atomicExch(fu.pos_err, 1);
-                    pos = 0;
-                }
-                const int i0 = ((e >> 4) << 3) + (e & 7);                    // the first pair's number = its angle's index
-                const float4 cs = __ldg(reinterpret_cast<const float4*>(fu.rope_table + (size_t)pos * fu.d + i0));
-                const float4 sn = __ldg(reinterpret_cast<const float4*>(fu.rope_table + (size_t)pos * fu.d + half + i0));
-                const float c[4] = {cs.x, cs.y, cs.z, cs.w}, sv[4] = {sn.x, sn.y, sn.z, sn.w};
-#pragma unroll
-                for (int i = 0; i < 4; ++i) { y0[i] = x0[i] * c[i] - x1[i] * sv[i]; y1[i] = x1[i] * c[i] + x0[i] * sv[i]; }
-            } else {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) { y0[i] = x0[i]; y1[i] = x1[i]; }
-            }
-            bf16* dst = nullptr;
-            if (head < fu.nh) {
-                dst = reinterpret_cast<bf16*>(out) + (size_t)m * ldo + f;
-            } else if (fu.slots) {
-                const int slot = fu.slots[m];
-                if (slot >= 0) {
-                    const int kind = head < fu.nh + fu.nkv ? 0 : 1, kvh = head - fu.nh - kind * fu.nkv;
-                    const int page = slot / fu.page_size, off = slot - page * fu.page_size;
-                    dst = fu.kv_cache + ((((size_t)page * 2 + kind) * fu.nkv + kvh) * fu.page_size + off) * fu.d + e;
-                }
-            }
-            if (dst) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) { dst[i] = __float2bfloat16_rn(y0[i]); dst[8 + i] = __float2bfloat16_rn(y1[i]); }
-            }
-        }
-    } else if constexpr (EPI == TS_EPI_SILU_MUL) {
-        // gate rows 16 t .. + 7 and their up rows + 8: four gate values and their four up values at a time
-        for (int idx = tid; idx < (m_hi - m_lo) * (TS_ROWS / 8); idx += nthreads) {
-            const int m = m_lo + idx / (TS_ROWS / 8), q = idx % (TS_ROWS / 8);
-            const int row = (q >> 1) * 16 + (q & 1) * 4;
-            float4 g[SPLITS], u[SPLITS];
-#pragma unroll
-            for (int r = 0; r < SPLITS; ++r) { g[r] = load4(r, m * TS_ROWS + row); u[r] = load4(r, m * TS_ROWS + row + 8); }
-            float4 gs = g[0], us = u[0];
-#pragma unroll
-            for (int r = 1; r < SPLITS; ++r) {
-                gs.x += g[r].x; gs.y += g[r].y; gs.z += g[r].z; gs.w += g[r].w;
-                us.x += u[r].x; us.y += u[r].y; us.z += u[r].z; us.w += u[r].w;
-            }
-            const float sc = PRO == TS_PRO_SCALED ? inv[m] : 1.f;
-            const float gv[4] = {gs.x * sc, gs.y * sc, gs.z * sc, gs.w * sc}, uv[4] = {us.x * sc, us.y * sc, us.z * sc, us.w * sc};
-            OUT* o = out + (size_t)m * ldo + (n0 >> 1) + (q >> 1) * 8 + (q & 1) * 4;
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (n0 + row + i + 8 < N) o[i] = from_f32<OUT>(gv[i] / (1.f + expf(-gv[i])) * uv[i]);
-        }
-    } else {
-    // four consecutive rows of one token at a time; the 32 pieces of a token's 128 rows are one warp's
-    for (int idx = tid; idx < (m_hi - m_lo) * (TS_ROWS / 4); idx += nthreads) {
-        const int m = m_lo + idx / (TS_ROWS / 4), row = (idx % (TS_ROWS / 4)) * 4;
-        float4 p[SPLITS];
-#pragma unroll
-        for (int r = 0; r < SPLITS; ++r) p[r] = load4(r, m * TS_ROWS + row);
-        float4 v = p[0];
-#pragma unroll
-        for (int r = 1; r < SPLITS; ++r) { v.x += p[r].x; v.y += p[r].y; v.z += p[r].z; v.w += p[r].w; }
-        float vv[4] = {v.x, v.y, v.z, v.w};
-        const int n = n0 + row;
-        if (EPI == TS_EPI_RESIDUAL) {
-            float ssq = 0.f;
-            float* o = reinterpret_cast<float*>(out) + (size_t)m * ldo + n;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                if (n + i < N) {
-                    const float r = o[i] + vv[i];
-                    o[i] = r;
-                    ssq += r * r;
-                    if (fu.scaled_out) fu.scaled_out[(size_t)m * ldo + n + i] = __float2bfloat16_rn(r * __ldg(fu.norm_w + n + i));
-                }
-            }
-            ssq = warp_sum(ssq);
-            if ((idx & 31) == 0) fu.ss_out[(size_t)tile * fu.ss_ld + m] = ssq;
+// A tile's sums -> the output, for the tokens m_lo .. m_hi - 1, by 128 threads.  A thread keeps its rows of W: four
+// consecutive ones (plain, residual: a token's 128 rows are one warp's), or four and their partners eight rows on (gate and
+// up, rotation pairs), and goes from token to token.  What it reads from global memory for the next four tokens (residual;
+// angles, cache slots) is requested ahead: for the first four before the tile's product is there, else every token would
+// wait for HBM or L2 once.  (The residual product of 64 rows by 2,048 x 8,192 unsplit, where one CTA writes a tile's 64
+// tokens: 48.2 us before, 41.1 after; in eight splits 13.4 and 12.6.)
+template <int EPI>
+struct TileEpilogue {
+    static constexpr bool PAIRS = EPI == TS_EPI_SILU_MUL || EPI == TS_EPI_ROPE_CACHE;
+    static constexpr int STEP = PAIRS ? 8 : 4;                               // from a thread's token to its next
+    static constexpr int AHEAD = 4;
+    int row, m_off;                                                          // first row of W within the tile; place of the first token
+    float4 resid[EPI == TS_EPI_RESIDUAL ? AHEAD : 1];
+    float4 cosv[EPI == TS_EPI_ROPE_CACHE ? AHEAD : 1], sinv[EPI == TS_EPI_ROPE_CACHE ? AHEAD : 1];
+    int slot[EPI == TS_EPI_ROPE_CACHE ? AHEAD : 1];
+
+    __device__ __forceinline__ explicit TileEpilogue(int tid) {
+        if (PAIRS) {
+            const int q = tid & 15;                                          // rows 16 t .. + 7 and their partners + 8
+            row = (q >> 1) * 16 + (q & 1) * 4;
+            m_off = tid >> 4;
         } else {
-            const float sc = PRO == TS_PRO_SCALED ? inv[m] : 1.f;
-            OUT* o = out + (size_t)m * ldo + n;
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (n + i < N) o[i] = from_f32<OUT>(vv[i] * sc);
+            row = (tid & 31) * 4;
+            m_off = tid >> 5;
         }
     }
+    // four consecutive numbers of the output at n, in one piece where `vec`
+    template <typename T>
+    static __device__ __forceinline__ void put4(T* o, const float (&v)[4], bool vec, int room) {
+        if (vec && room >= 4) {
+            if constexpr (sizeof(T) == 4) {
+                *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+            } else {
+                const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+                *reinterpret_cast<uint2*>(o) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (i < room) o[i] = from_f32<T>(v[i]);
+        }
     }
+    // requests what the tokens m, m + STEP, .. (AHEAD of them) need
+    template <typename OUT>
+    __device__ __forceinline__ void fetch(int m, int m_hi, int n0, int N, const OUT* out, int ldo, bool vec, const StreamFusion& fu) {
+        if constexpr (EPI == TS_EPI_RESIDUAL) {
+            const int n = n0 + row;
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) {
+                const float* o = reinterpret_cast<const float*>(out) + (size_t)(m + u * STEP) * ldo + n;
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (m + u * STEP < m_hi) {
+                    if (vec && n + 4 <= N) {
+                        v = *reinterpret_cast<const float4*>(o);
+                    } else {
+                        if (n < N) v.x = o[0];
+                        if (n + 1 < N) v.y = o[1];
+                        if (n + 2 < N) v.z = o[2];
+                        if (n + 3 < N) v.w = o[3];
+                    }
+                }
+                resid[u] = v;
+            }
+        }
+        if constexpr (EPI == TS_EPI_ROPE_CACHE) {
+            const int f = n0 + row, head = f / fu.d, e = f - head * fu.d, half = fu.d >> 1;
+            const int i0 = ((e >> 4) << 3) + (e & 7);                        // the first pair's number = its angle's index
+            int pos[AHEAD];
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) {
+                const bool there = m + u * STEP < m_hi && f + 8 < N;
+                pos[u] = there && head < fu.nh + fu.nkv ? fu.positions[m + u * STEP] : 0;
+                slot[u] = there && head >= fu.nh && fu.slots ? fu.slots[m + u * STEP] : -1;
+            }
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) {
+                if (pos[u] < 0 || pos[u] >= fu.max_pos) {
+                    if (fu.pos_err) atomicExch(fu.pos_err, 1);
+                    pos[u] = 0;
+                }
+                if (m + u * STEP < m_hi && f + 8 < N && head < fu.nh + fu.nkv) {
+                    cosv[u] = __ldg(reinterpret_cast<const float4*>(fu.rope_table + (size_t)pos[u] * fu.d + i0));
+                    sinv[u] = __ldg(reinterpret_cast<const float4*>(fu.rope_table + (size_t)pos[u] * fu.d + half + i0));
+                }
+            }
+        }
+    }
+    // load4(r, i): partial sums i .. i + 3 of CTA r's [token][row] array; they are added in rank order, and all are requested
+    // before the first is used.  inv: 1 / rms per token (TS_PRO_SCALED).
+    template <bool SPLIT, int PRO, typename OUT, typename Load>
+    __device__ __forceinline__ void write(Load load4, int splits, OUT* __restrict__ out, int ldo, int N, int n0, int tile,
+                                          int m_lo, int m_hi, bool vec, const float* inv, const StreamFusion& fu) {
+        constexpr int MAXS = SPLIT ? TS_MAX_SPLITS : 1;
+        auto sum4 = [&](int i) -> float4 {
+            float4 p[MAXS];
+#pragma unroll
+            for (int r = 0; r < MAXS; ++r) p[r] = r < splits ? load4(r, i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            float4 v = p[0];
+#pragma unroll
+            for (int r = 1; r < MAXS; ++r)
+                if (r < splits) { v.x += p[r].x; v.y += p[r].y; v.z += p[r].z; v.w += p[r].w; }
+            return v;
+        };
+        float norm[4] = {0.f, 0.f, 0.f, 0.f};
+        if constexpr (EPI == TS_EPI_RESIDUAL) {
+            if (fu.scaled_out)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (n0 + row + i < N) norm[i] = __ldg(fu.norm_w + n0 + row + i);
+        }
+        for (int mb = m_lo + m_off; mb - m_off < m_hi; mb += AHEAD * STEP) {
+            const TileEpilogue now = *this;
+            fetch(mb + AHEAD * STEP, m_hi, n0, N, out, ldo, vec, fu);
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) {
+                const int m = mb + u * STEP;
+                if (m >= m_hi) break;                                        // the same for a whole warp, but for PAIRS
+                const float4 s0 = sum4(m * TS_ROWS + row);
+                const float sc = PRO == TS_PRO_SCALED ? inv[m] : 1.f;
+                float a[4] = {s0.x * sc, s0.y * sc, s0.z * sc, s0.w * sc};
+                if constexpr (PAIRS) {
+                    const float4 s1 = sum4(m * TS_ROWS + row + 8);
+                    const float b[4] = {s1.x * sc, s1.y * sc, s1.z * sc, s1.w * sc};
+                    if constexpr (EPI == TS_EPI_SILU_MUL) {
+                        float y[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) y[i] = a[i] / (1.f + expf(-a[i])) * b[i];
+                        put4(out + (size_t)m * ldo + ((n0 + (row & ~15)) >> 1) + (row & 7), y, vec, N - (n0 + row + 8));
+                    } else {
+                        const int f = n0 + row;                              // output feature of the first pair's first element
+                        if (f + 8 >= N) continue;
+                        const int head = f / fu.d, e = f - head * fu.d;      // e: storage index inside the head (a multiple of 4)
+                        float y0[4], y1[4];
+                        if (head < fu.nh + fu.nkv) {
+                            const float c[4] = {now.cosv[u].x, now.cosv[u].y, now.cosv[u].z, now.cosv[u].w};
+                            const float sn[4] = {now.sinv[u].x, now.sinv[u].y, now.sinv[u].z, now.sinv[u].w};
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) { y0[i] = a[i] * c[i] - b[i] * sn[i]; y1[i] = b[i] * c[i] + a[i] * sn[i]; }
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) { y0[i] = a[i]; y1[i] = b[i]; }
+                        }
+                        bf16* dst = nullptr;
+                        if (head < fu.nh) {
+                            dst = reinterpret_cast<bf16*>(out) + (size_t)m * ldo + f;
+                        } else if (now.slot[u] >= 0) {
+                            const int kind = head < fu.nh + fu.nkv ? 0 : 1, kvh = head - fu.nh - kind * fu.nkv;
+                            const int page = now.slot[u] / fu.page_size, off = now.slot[u] - page * fu.page_size;
+                            dst = fu.kv_cache + ((((size_t)page * 2 + kind) * fu.nkv + kvh) * fu.page_size + off) * fu.d + e;
+                        }
+                        if (dst) {                                           // d % 16 == 0: the cache's places are 8-byte aligned
+                            put4(dst, y0, vec, 4);
+                            put4(dst + 8, y1, vec, 4);
+                        }
+                    }
+                } else if constexpr (EPI == TS_EPI_RESIDUAL) {
+                    const int n = n0 + row;
+                    const float r[4] = {now.resid[u].x, now.resid[u].y, now.resid[u].z, now.resid[u].w};
+                    float ssq = 0.f, y[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        a[i] = n + i < N ? r[i] + a[i] : 0.f;
+                        ssq += a[i] * a[i];
+                        y[i] = a[i] * norm[i];
+                    }
+                    put4(reinterpret_cast<float*>(out) + (size_t)m * ldo + n, a, vec, N - n);
+                    if (fu.scaled_out) put4(fu.scaled_out + (size_t)m * ldo + n, y, vec, N - n);
+                    ssq = warp_sum(ssq);
+                    if ((threadIdx.x & 31) == 0) fu.ss_out[(size_t)tile * fu.ss_ld + m] = ssq;
+                } else {
+                    put4(out + (size_t)m * ldo + n0 + row, a, vec, N - (n0 + row));
+                }
+            }
+        }
+    }
+};
+
+// Stages of 24 KB.  Split products leave room for a second CTA on the SM, so that the next kernel's can fetch its weights
+// while this one's still run, and their partial sums take the stages' place.
+__host__ __device__ constexpr int ts_stages(bool split) { return split ? 4 : 6; }
+__host__ __device__ constexpr size_t ts_smem(bool split) {
+    return (size_t)ts_stages(split) * (TS_ROWS + TS_TOK) * TS_BK * 2 + (split ? 0 : TS_TOK * TS_ROWS * 4) +
+           8 * (2 * ts_stages(split) + 4) + 1024;
 }
 
-template <int SPLITS, int EPI, int PRO, typename OUT>
+template <bool SPLIT, int EPI, int PRO, typename OUT>
 __global__ void __launch_bounds__(TS_THREADS)
 tc_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                 OUT* __restrict__ out, int ldo, int M, int N, int K, int* err, const StreamFusion fu) {
+                 OUT* __restrict__ out, int ldo, int M, int N, int K, int splits, int* err, const StreamFusion fu) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ float inv_rms[TS_TOK];
+    constexpr int STAGES = ts_stages(SPLIT);
     constexpr uint32_t W_BYTES = TS_ROWS * TS_BK * 2, X_BYTES = TS_TOK * TS_BK * 2, STAGE_BYTES = W_BYTES + X_BYTES;
+    static_assert(!SPLIT || (uint32_t)TS_TOK * TS_ROWS * 4 <= STAGES * STAGE_BYTES, "the partial sums take the stages' place");
     const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;          // swizzled tiles need 1024-byte alignment
     unsigned char* base_ptr = smem_raw + (base - smem_addr(smem_raw));
-    float* part = reinterpret_cast<float*>(base_ptr + TS_STAGES * STAGE_BYTES);          // [TS_TOK][TS_ROWS]
-    const uint32_t bars = base + TS_STAGES * STAGE_BYTES + TS_TOK * TS_ROWS * 4;
+    // [TS_TOK][TS_ROWS], over the stages or behind them
+    float* part = reinterpret_cast<float*>(base_ptr + (SPLIT ? 0 : STAGES * STAGE_BYTES));
+    const uint32_t bars = base + STAGES * STAGE_BYTES + (SPLIT ? 0 : TS_TOK * TS_ROWS * 4);
     auto full_bar = [&](int s) { return bars + 8u * s; };
-    auto empty_bar = [&](int s) { return bars + 8u * (TS_STAGES + s); };
-    auto acc_full = [&](int b) { return bars + 8u * (2 * TS_STAGES + b); };
-    auto acc_empty = [&](int b) { return bars + 8u * (2 * TS_STAGES + 2 + b); };
+    auto empty_bar = [&](int s) { return bars + 8u * (STAGES + s); };
+    auto acc_full = [&](int b) { return bars + 8u * (2 * STAGES + b); };
+    auto acc_empty = [&](int b) { return bars + 8u * (2 * STAGES + 2 + b); };
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int rank = SPLITS > 1 ? (int)cluster_ctarank() : 0;
+    const int rank = SPLIT ? (int)cluster_ctarank() : 0;
     const int n_tiles = (N + TS_ROWS - 1) / TS_ROWS;
     const int KT_all = (K + TS_BK - 1) / TS_BK;
-    const int kt_lo = KT_all * rank / SPLITS, kt_hi = KT_all * (rank + 1) / SPLITS;       // this CTA's K range, in boxes
+    const int kt_lo = KT_all * rank / splits, kt_hi = KT_all * (rank + 1) / splits;       // this CTA's K range, in boxes
     const int KT = kt_hi - kt_lo;
     // split products: one tile per cluster; unsplit ones: tile after tile
-    const int first_tile = SPLITS > 1 ? (int)(blockIdx.x / SPLITS) : (int)blockIdx.x;
-    const int tile_step = SPLITS > 1 ? n_tiles : (int)gridDim.x;
-    constexpr uint32_t TMEM_COLS = 2 * TS_TOK;
+    const int first_tile = SPLIT ? (int)(blockIdx.x / splits) : (int)blockIdx.x;
+    const int tile_step = SPLIT ? n_tiles : (int)gridDim.x;
+    constexpr uint32_t TMEM_COLS = SPLIT ? TS_TOK : 2 * TS_TOK;
+    const int m_lo = SPLIT ? M * rank / splits : 0, m_hi = SPLIT ? M * (rank + 1) / splits : M;   // the tokens that this CTA writes
+    // four numbers of the output at a time
+    const bool vec = ldo % 4 == 0 && ((uintptr_t)out & (4 * sizeof(OUT) - 1)) == 0 && (((uintptr_t)fu.scaled_out | (uintptr_t)fu.kv_cache) & 7) == 0;
+    TileEpilogue<EPI> epilogue((int)threadIdx.x & 127);
 
     if (threadIdx.x == 0) {
         abort_flag = 0;
-        for (int s = 0; s < TS_STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
+        for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 4); }
         fence_barrier_init();
     }
@@ -229,7 +304,7 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         bool ok = true, waited = false;
         int early = 0;
         if (first_tile < n_tiles) {
-            for (; early < KT && early < TS_STAGES; ++early) {
+            for (; early < KT && early < STAGES; ++early) {
                 mbar_expect_tx(full_bar(early), STAGE_BYTES);
                 tma_load_2d(base + early * STAGE_BYTES, &map_w, full_bar(early), (kt_lo + early) * TS_BK, first_tile * TS_ROWS);
             }
@@ -242,7 +317,7 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         for (int t = first_tile; t < n_tiles && ok; t += tile_step) {
             for (int kt = 0; kt < KT; ++kt, ++it) {
                 if (it < early) continue;                                    // requested above
-                const int s = it % TS_STAGES, r = it / TS_STAGES;
+                const int s = it % STAGES, r = it / STAGES;
                 if (r > 0 && !mbar_wait(empty_bar(s), (r & 1) ^ 1, err, 1, &abort_flag)) { ok = false; break; }
                 mbar_expect_tx(full_bar(s), STAGE_BYTES);
                 const uint32_t sa = base + s * STAGE_BYTES;
@@ -266,7 +341,7 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             tc_fence_after();
             const uint32_t tmem_d = tmem_base + (uint32_t)(b * TS_TOK);
             for (int kt = 0; kt < KT; ++kt, ++it) {
-                const int s = it % TS_STAGES, r = it / TS_STAGES;
+                const int s = it % STAGES, r = it / STAGES;
                 if (!mbar_wait(full_bar(s), r & 1, err, 2, &abort_flag)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t sa = base + s * STAGE_BYTES;
@@ -283,20 +358,22 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         // that what follows reads and writes along rows of W
         int local = 0;
         bool ok = true;
-        if (PRO == TS_PRO_SCALED && threadIdx.x < TS_TOK) {
+        if (PRO == TS_PRO_SCALED && threadIdx.x < M) {
             // 1 / rms of every token from the producer's partial sums of squares, added in their order
             float ssq = 0.f;
+#pragma unroll 8
             for (int p = 0; p < fu.ss_in_blocks; ++p) ssq += fu.ss_in[(size_t)p * fu.ss_ld + threadIdx.x];
             inv_rms[threadIdx.x] = rsqrtf(ssq / (float)K + fu.eps);
         }
         for (int t = first_tile; t < n_tiles && ok; t += tile_step, ++local) {
             const int b = local & 1, u = local >> 1;
+            epilogue.fetch(m_lo + epilogue.m_off, m_hi, t * TS_ROWS, N, out, ldo, vec, fu);
             if (!mbar_wait(acc_full(b), u & 1, err, 3, &abort_flag)) { ok = false; break; }
             tc_fence_after();
             const uint32_t tmem_d = tmem_base + (uint32_t)(b * TS_TOK) + ((uint32_t)(warp * 32) << 16);
-            if (SPLITS == 1 && local > 0) asm volatile("bar.sync 1, 128;" ::: "memory");   // the tile before has been written out
+            if (!SPLIT && local > 0) asm volatile("bar.sync 1, 128;" ::: "memory");       // the tile before has been written out
 #pragma unroll
-            for (int c = 0; c < TS_TOK / 32; ++c) {
+            for (int c = 0; c < TS_TOK / 32; ++c) {      // (split: the stages' copies have landed and been multiplied)
                 uint32_t v[32];
                 tc_ld32(tmem_d + (uint32_t)(c * 32), v);
 #pragma unroll
@@ -305,29 +382,28 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty(b));
-            if (SPLITS == 1) {
+            if (!SPLIT) {
                 // ---- second half, unsplit: the four epilogue warps write the tile out
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 auto load4 = [&](int, int i) { return *reinterpret_cast<const float4*>(part + i); };
-                ts_write_out<1, EPI, PRO, OUT>(load4, out, ldo, N, t * TS_ROWS, t, 0, M, (int)threadIdx.x, 128, inv_rms, fu);
+                epilogue.template write<false, PRO>(load4, 1, out, ldo, N, t * TS_ROWS, t, 0, M, vec, inv_rms, fu);
             }
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (SPLITS > 1) {
+    if (SPLIT) {
         // ---- second half, split over the cluster: CTA `rank` adds the partial sums of its share of the tokens
         cluster_sync_all();                                                 // every CTA's partial sums are in its shared memory
         if (first_tile < n_tiles && !abort_flag) {
             const int n0 = first_tile * TS_ROWS;
-            const int m_lo = M * rank / SPLITS, m_hi = M * (rank + 1) / SPLITS;
             const uint32_t mine = smem_addr(part);
-            uint32_t peer[SPLITS];
+            uint32_t peer[TS_MAX_SPLITS];
 #pragma unroll
-            for (int r = 0; r < SPLITS; ++r) peer[r] = mapa_shared(mine, (uint32_t)r);
+            for (int r = 0; r < TS_MAX_SPLITS; ++r) peer[r] = mapa_shared(mine, (uint32_t)min(r, splits - 1));
             auto load4 = [&](int r, int i) { return ts_ld_remote4(peer[r] + (uint32_t)i * 4u); };
-            ts_write_out<SPLITS, EPI, PRO, OUT>(load4, out, ldo, N, n0, first_tile, m_lo, m_hi, (int)threadIdx.x, TS_THREADS,
-                                                inv_rms, fu);
+            if (threadIdx.x < 128)
+                epilogue.template write<true, PRO>(load4, splits, out, ldo, N, n0, first_tile, m_lo, m_hi, vec, inv_rms, fu);
         }
         cluster_sync_all();                                                 // nobody leaves while its partial sums are being read
     }
@@ -352,26 +428,27 @@ static int ts_num_sms() {
     return num_sms;
 }
 
-template <int SPLITS, int EPI, int PRO, typename OUT>
-static int launch_ts(const CUtensorMap& mw, const CUtensorMap& mx, OUT* out, int ldo, int M, int N, int K, int* err,
+template <bool SPLIT, int EPI, int PRO, typename OUT>
+static int launch_ts(const CUtensorMap& mw, const CUtensorMap& mx, OUT* out, int ldo, int M, int N, int K, int splits, int* err,
                      const StreamFusion& fu, cudaStream_t s) {
-    const size_t smem = (size_t)TS_STAGES * (TS_ROWS * TS_BK * 2 + TS_TOK * TS_BK * 2) + TS_TOK * TS_ROWS * 4 +
-                        8 * (2 * TS_STAGES + 4) + 1024;
-    auto kernel = tc_stream_kernel<SPLITS, EPI, PRO, OUT>;
+    constexpr size_t smem = ts_smem(SPLIT);
+    auto kernel = tc_stream_kernel<SPLIT, EPI, PRO, OUT>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     const int n_tiles = (N + TS_ROWS - 1) / TS_ROWS;
     const int sms = ts_num_sms();
-    const unsigned grid = SPLITS > 1 ? (unsigned)(n_tiles * SPLITS) : (unsigned)(n_tiles < sms ? n_tiles : sms);
-    return rg_launch(kernel, dim3(grid), dim3(TS_THREADS), smem, s, SPLITS, mw, mx, out, ldo, M, N, K, err, fu);
+    const unsigned grid = SPLIT ? (unsigned)(n_tiles * splits) : (unsigned)(n_tiles < sms ? n_tiles : sms);
+    return rg_launch(kernel, dim3(grid), dim3(TS_THREADS), smem, s, splits, mw, mx, out, ldo, M, N, K, splits, err, fu);
 }
 
 static int ts_pick_splits(int splits, int N, int K) {
     const int n_tiles = (N + TS_ROWS - 1) / TS_ROWS, kt = (K + TS_BK - 1) / TS_BK;
     if (splits == 0) {
-        // as many CTAs per tile as keep the whole product in one wave (clusters of 8 start slowly: 4 at most)
+        // As many CTAs per tile as keep the whole product in one wave of one CTA per SM, with at least four boxes of K each.
+        // 64 rows by 2,048 x 2,048 / 2,048 x 8,192: 7.8 / 15.5 us with 4, 6.8 / 12.6 with 8; a second CTA per SM from one
+        // product (16 splits' worth) only delays the product behind it (a 64-row step 1,281 against 1,333 us).
         splits = 1;
-        while (splits < 4 && n_tiles * splits * 2 <= ts_num_sms() && kt >= splits * 2 * 2) splits *= 2;
+        while (splits < TS_MAX_SPLITS && n_tiles * splits * 2 <= ts_num_sms() && kt >= splits * 4) splits *= 2;
     }
     if ((splits != 1 && splits != 2 && splits != 4 && splits != 8) || kt < splits) return -1;
     return splits;
@@ -385,10 +462,8 @@ static int dispatch_ts(const void* x, int ldx, const void* W, OUT* out, int ldo,
     if (e) return e;
     e = rg_make_map(&mx, x, M, K, ldx, TS_TOK);
     if (e) return e;
-    return splits == 1 ? launch_ts<1, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, err, fu, s)
-         : splits == 2 ? launch_ts<2, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, err, fu, s)
-         : splits == 4 ? launch_ts<4, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, err, fu, s)
-                       : launch_ts<8, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, err, fu, s);
+    return splits == 1 ? launch_ts<false, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, 1, err, fu, s)
+                       : launch_ts<true, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, splits, err, fu, s);
 }
 
 static bool ts_operands_ok(const void* x, int ldx, const void* W, int M, int K) {
