@@ -93,6 +93,104 @@ __device__ __forceinline__ void multiply(float (&acc)[4][4 * W], const float (*_
     }
 }
 
+// ---- products of 64 rows by 64 or 128 columns by 128 threads of 8 x 4 or 8 x 8 results each, over rows of both operands as
+// they lie in global memory.  The 4 x 4 results a thread of `multiply` read two 16-byte pieces of shared memory for 16
+// multiply-adds; here 16 pieces serve 256.
+#define MTH 128
+#define MK 32                 // of the contraction at a time
+#define MP (MK + 4)           // pitch of its rows: eight neighbouring rows' 16-byte pieces lie in different banks
+
+// acc[i][q] += sum over k in [k_lo, k_hi) of A[8 ty + i][k] B[tx + 16 q][k], four k at a time; rows PA and PB apart.
+template <int Q, int PA, int PB>
+__device__ __forceinline__ void multiply_rows(float (&acc)[8][Q], const float* __restrict__ A, const float* __restrict__ B, int k_lo,
+                                              int k_hi, int ty, int tx) {
+    const float* a0 = A + 8 * ty * PA;
+    const float* b0 = B + tx * PB;
+#pragma unroll 1
+    for (int k = k_lo; k < k_hi; k += 4) {
+        float4 a[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const float4*>(a0 + i * PA + k);
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            const float4 b = *reinterpret_cast<const float4*>(b0 + 16 * q * PB + k);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                acc[i][q] += a[i].x * b.x;
+                acc[i][q] += a[i].y * b.y;
+                acc[i][q] += a[i].z * b.z;
+                acc[i][q] += a[i].w * b.w;
+            }
+        }
+    }
+}
+
+// dst[row][k] = src row `row`, number k0 + k, for `rows` rows (n of them there) and MK numbers (of N): zeros elsewhere.  VEC:
+// 16 bytes at a time and asynchronously (rows, pitches and N in multiples of four numbers).
+template <bool VEC>
+__device__ __forceinline__ void fetch_rows(float* __restrict__ dst, const float* __restrict__ src, size_t ld, int rows, int n,
+                                           int k0, int N) {
+    if (VEC) {
+        for (int e = threadIdx.x; e < rows * (MK / 4); e += MTH) {
+            const int i = e / (MK / 4), k = e % (MK / 4) * 4;
+            const bool there = i < n && k0 + k < N;
+            const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst + i * MP + k);
+            const float* p = there ? src + (size_t)i * ld + k0 + k : src;
+            const int bytes = there ? 16 : 0;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(p), "r"(bytes));
+        }
+    } else {
+        for (int e = threadIdx.x; e < rows * MK; e += MTH) {
+            const int i = e / MK, k = e % MK;
+            dst[i * MP + k] = i < n && k0 + k < N ? src[(size_t)i * ld + k0 + k] : 0.f;
+        }
+    }
+}
+
+// acc += A B^T over all N numbers of their rows: A has 64 rows (na there), B 16 Q (nb there); two stages of MK numbers in
+// `sm` [2][64 + 16 Q][MP], the next on its way while one is multiplied.
+template <int Q, bool VEC>
+__device__ __forceinline__ void product_of_rows(float (&acc)[8][Q], float* __restrict__ sm, const float* __restrict__ A, size_t lda,
+                                                int na, const float* __restrict__ B, size_t ldb, int nb, int N, int ty, int tx) {
+    constexpr int STAGE = (64 + 16 * Q) * MP;
+    auto fetch = [&](int it) {
+        float* st = sm + (it & 1) * STAGE;
+        fetch_rows<VEC>(st, A, lda, 64, na, it * MK, N);
+        fetch_rows<VEC>(st + 64 * MP, B, ldb, 16 * Q, nb, it * MK, N);
+        if (VEC) asm volatile("cp.async.commit_group;\n" ::);
+    };
+    const int its = (N + MK - 1) / MK;
+    fetch(0);
+    for (int it = 0; it < its; ++it) {
+        if (it + 1 < its) {
+            fetch(it + 1);
+            if (VEC) asm volatile("cp.async.wait_group 1;\n" ::);
+        } else {
+            if (VEC) asm volatile("cp.async.wait_group 0;\n" ::);
+        }
+        __syncthreads();
+        const float* st = sm + (it & 1) * STAGE;
+        multiply_rows<Q, MP, MP>(acc, st, st + 64 * MP, 0, MK, ty, tx);
+        __syncthreads();
+    }
+}
+
+__device__ __forceinline__ float4 four(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 four(const bf16* p) {
+    const uint2 x = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x.x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+// Numbers k .. k + 3 (of N) of row i (of n): zeros where there are none.
+template <bool VEC, typename V>
+__device__ __forceinline__ float4 values4(const V* __restrict__ src, size_t ld, int i, int n, int k, int N) {
+    if (i >= n || k >= N) return make_float4(0.f, 0.f, 0.f, 0.f);
+    const V* p = src + (size_t)i * ld + k;
+    if (VEC) return four(p);
+    return make_float4(to_f32(p[0]), k + 1 < N ? to_f32(p[1]) : 0.f, k + 2 < N ? to_f32(p[2]) : 0.f, k + 3 < N ? to_f32(p[3]) : 0.f);
+}
+
 // sums [chunks, H, M]: each chunk's sum becomes the state before the chunk, and the state after the last one goes into the
 // request's slot (M = dv d numbers per head, S transposed).  decays [chunks, H], or with CHANNEL [chunks, H, d]: one per
 // row of S.  V numbers per thread (with CHANNEL neighbours in a column of S: d % V == 0).

@@ -16,9 +16,8 @@
 //
 // What bounds it: the 32-bit multiply-adds (128 a cycle and SM, packed or not), and in delta_states the chain from chunk to
 // chunk, 2 x 64 x d of them per column and chunk.  16 columns a block fill 128 of 148 SMs at 16 heads of 128 columns;
-// narrower blocks fetch the same W and K more often.  Measured (2,048 tokens, 16 heads of 128 x 128 on 8): 88 us the
-// systems, 132 the states and 202 until the outputs are there, each from when its blocks may start, beside the kernel
-// before; the token-by-token kernel (state_mixers.cu) took 908.  Steps whose longest portion is shorter than 128 tokens stay
+// narrower blocks fetch the same W and K more often.  Measured (2,048 tokens, 16 heads of 128 x 128 on 8): 85 us the
+// systems, 116 the states, 55 the outputs; the token-by-token kernel (state_mixers.cu) took 908.  Steps whose longest portion is shorter than 128 tokens stay
 // on that one.
 #include "chunk_scan.cuh"
 
@@ -28,7 +27,7 @@
 
 // q, k: rows q_ld, k_ld apart, head h of the H reads head h / (H / Hqk).  beta, loga [T, H].  x_out [T, H, dv] = X;
 // w_out [chunks, H, d, 64] = W transposed; factors [chunks, H, 64] = exp(c_L - c_i) (1 beyond the chunk's tokens), decays
-// [chunks, H] = exp(c_L); dots [chunks, Hqk, 64, 64] = k_j . q_i at [j][i].  grid: chunks, H (systems) and then Hqk (dots).
+// [chunks, H] = exp(c_L); dots [chunks, Hqk, 64, 64] = q_i . k_j at [i][j].  grid: chunks, H (systems) and then Hqk (dots).
 template <typename V>
 __global__ void __launch_bounds__(NTH, 2)
 delta_solve_kernel(const float* __restrict__ q, int q_ld, const float* __restrict__ k, int k_ld, const V* __restrict__ v,
@@ -51,14 +50,14 @@ delta_solve_kernel(const float* __restrict__ q, int q_ld, const float* __restric
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-    // k_j . k_i, or k_j . q_i: thread (ty, tx) has j = 4 ty .., i = 4 tx ..
+    // k_j . k_i: thread (ty, tx) has j = 4 ty .., i = 4 tx ..; or q_i . k_j: i = 4 ty .., j = 4 tx ..
     const float* kh = k + (size_t)lo * k_ld + (size_t)hq * d;
     const float* other = system ? kh : q + (size_t)lo * q_ld + (size_t)hq * d;
     for (int k0 = 0; k0 < d; k0 += TILE) {
         load_transposed(sA, kh, k_ld, n, d, k0, nullptr);
         if (!system) load_transposed(sB, other, q_ld, n, d, k0, nullptr);
         __syncthreads();
-        multiply<1>(acc, sA, system ? sA : sB, min(TILE, d - k0), ty, tx);
+        multiply<1>(acc, system ? sA : sB, sA, min(TILE, d - k0), ty, tx);
         __syncthreads();
     }
     if (!system) {

@@ -19,23 +19,38 @@
 // sums that the light blocks of the launches work out.
 //
 // And with one fixed decay per head (retention, lightning attention), its logarithm in 64-bit, and dt 1: 2,048 tokens of 16
-// heads of 128 x 128 take 75 + 42 + 106 us (each from when its blocks may start, beside the kernel before) where the
-// token-by-token kernel took 651.
+// heads of 128 x 128 take 46 + 22 + 55 us (states, pass, outputs) where the token-by-token kernel took 651.
+//
+// What bounds it: 19 us of multiply-adds in the outputs' products, 22 in the states' (128 a cycle and SM); the rest is a
+// block's chain of loads, which is why the products' rows come asynchronously, a stage ahead, and lie in shared memory as
+// they lie in global memory.  With 4 x 4 results a thread and synchronous loads: 67 + 22 + 83 us.
 //
 // The step's tokens are packed request by request (cu_seqlens); a request's chunks start at its first token of the step.
 #include "chunk_scan.cuh"
 
+#define XP (CH + 4)           // pitch of a chunk's values turned (column by token), and of its weights (token by token)
+
+// Shared memory of chunk_states: values [64][68] and B [64][64 W + 4], or two stages of the dots' rows; of chunk_outputs: two
+// stages of C's and S's rows, or weights and values of the chunk.
+__host__ __device__ constexpr size_t states_smem(int W) {
+    const size_t a = (size_t)(CH * (TILE + 4) + CH * (TILE * W + 4)) * 4, b = (size_t)2 * (64 + 64) * MP * 4;
+    return a > b ? a : b;
+}
+__host__ __device__ constexpr size_t outputs_smem(int W) {
+    const size_t a = (size_t)2 * (64 + 64 * W) * MP * 4, b = (size_t)(CH + 64 * W) * XP * 4;
+    return a > b ? a : b;
+}
+
 // x, B, C: rows x_ld, B_ld, C_ld apart (head h's x at column h dv, group g's B and C at column g N).  sums [chunks, H, dv + ones, N],
-// decays [chunks, H], dots [chunks, G, 64, 64] = B_j . C_i at [j][i].  grid: chunks, H (tiles of S: z) and then G (z = 0).
-template <int W, typename V>
-__global__ void __launch_bounds__(NTH)
+// decays [chunks, H], dots [chunks, G, 64, 64] = C_i . B_j at [i][j].  grid: chunks, H (tiles of S, 64 columns by 64 W rows: z)
+// and then G (z = 0).  VEC: rows and sizes allow four numbers at a time.
+template <int W, bool VEC, typename V>
+__global__ void __launch_bounds__(MTH, 4)
 chunk_states_kernel(const V* __restrict__ x, int x_ld, const float* __restrict__ B, int B_ld, const float* __restrict__ C,
                     int C_ld, const float* __restrict__ dt, const float* __restrict__ loga, const float* __restrict__ A_log,
-                    const double* __restrict__ fixed, const int* __restrict__ cu, int R, float* __restrict__ sums, float* __restrict__ decays,
-                    float* __restrict__ dots, int H, int G, int N, int dv, int ntiles, int ones) {
+                    const double* __restrict__ fixed, const int* __restrict__ cu, int R, float* __restrict__ sums,
+                    float* __restrict__ decays, float* __restrict__ dots, int H, int G, int N, int dv, int ntiles, int ones) {
     extern __shared__ __align__(16) float sm[];
-    float (*sA)[PITCH] = reinterpret_cast<float (*)[PITCH]>(sm);                            // [CH][PITCH]
-    float (*sB)[TILE * W + 4] = reinterpret_cast<float (*)[TILE * W + 4]>(sm + CH * PITCH);     // [CH][TILE W + 4]
     __shared__ double cum[CH];
     __shared__ float sdt[CH];
     pdl_wait();
@@ -43,31 +58,21 @@ chunk_states_kernel(const V* __restrict__ x, int x_ld, const float* __restrict__
     int r, lo, n;
     if (!find_chunk(cu, R, blockIdx.x, r, lo, n)) return;
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-    float acc[4][4 * W];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4 * W; ++j) acc[i][j] = 0.f;
     if ((int)blockIdx.y >= H) {
         if (blockIdx.z > 0) return;
         const int g = blockIdx.y - H;
-        float (*sC)[PITCH] = reinterpret_cast<float (*)[PITCH]>(sm + CH * PITCH);
-        float a1[4][4];
+        float a1[8][4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) a1[i][j] = 0.f;
-        for (int k0 = 0; k0 < N; k0 += TILE) {
-            load_transposed(sA, B + (size_t)lo * B_ld + (size_t)g * N, B_ld, n, N, k0, nullptr);
-            load_transposed(sC, C + (size_t)lo * C_ld + (size_t)g * N, C_ld, n, N, k0, nullptr);
-            __syncthreads();
-            multiply<1>(a1, sA, sC, min(TILE, N - k0), ty, tx);
-            __syncthreads();
-        }
+        product_of_rows<4, VEC>(a1, sm, C + (size_t)lo * C_ld + (size_t)g * N, C_ld, n, B + (size_t)lo * B_ld + (size_t)g * N,
+                                B_ld, n, N, ty, tx);
         float* out = dots + ((size_t)blockIdx.x * G + g) * CH * CH;
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-            *reinterpret_cast<float4*>(out + (4 * ty + i) * CH + 4 * tx) = make_float4(a1[i][0], a1[i][1], a1[i][2], a1[i][3]);
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) out[(8 * ty + i) * CH + tx + 16 * q] = a1[i][q];
         if (!ones) return;
         for (int h = g * (H / G); h < (g + 1) * (H / G); ++h) {         // the row of n: every head of the group
             __syncthreads();
@@ -77,7 +82,7 @@ chunk_states_kernel(const V* __restrict__ x, int x_ld, const float* __restrict__
             __syncthreads();
             if (threadIdx.x < n) sdt[threadIdx.x] *= expf((float)(last - cum[threadIdx.x]));
             __syncthreads();
-            for (int k = threadIdx.x; k < N; k += NTH) {
+            for (int k = threadIdx.x; k < N; k += MTH) {
                 float s = 0.f;
 #pragma unroll 8
                 for (int t = 0; t < n; ++t) s += B[(size_t)(lo + t) * B_ld + (size_t)g * N + k] * sdt[t];
@@ -88,29 +93,72 @@ chunk_states_kernel(const V* __restrict__ x, int x_ld, const float* __restrict__
     }
     const int h = blockIdx.y, grp = h / (H / G);
     const int j0 = (blockIdx.z / ntiles) * TILE, n0 = (blockIdx.z % ntiles) * TILE * W;      // columns of S, rows of S
+    // all of the chunk's rows are requested before its decays are worked out
+    float* sA = sm;                                         // [token][column], times what is left of it at the chunk's end
+    float* sB = sm + CH * (TILE + 4);                       // [token][row of S]
+    constexpr int BP = TILE * W + 4;
+    const V* xh = x + (size_t)lo * x_ld + (size_t)h * dv;
+    const float* Bh = B + (size_t)lo * B_ld + (size_t)grp * N;
+    for (int e = threadIdx.x; e < CH * (TILE * W / 4); e += MTH) {
+        const int t = e / (TILE * W / 4), k = e % (TILE * W / 4) * 4;
+        if (VEC) {
+            const bool there = t < n && n0 + k < N;
+            const uint32_t d = (uint32_t)__cvta_generic_to_shared(sB + t * BP + k);
+            const float* p = there ? Bh + (size_t)t * B_ld + n0 + k : Bh;
+            const int bytes = there ? 16 : 0;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(p), "r"(bytes));
+        } else {
+            *reinterpret_cast<float4*>(sB + t * BP + k) = values4<VEC>(Bh, B_ld, t, n, n0 + k, N);
+        }
+    }
+    if (VEC) asm volatile("cp.async.commit_group;\n" ::);
+    constexpr int PER = CH * (TILE / 4) / MTH;
+    float4 xv[PER];
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+        const int e = threadIdx.x + p * MTH;
+        xv[p] = values4<VEC>(xh, x_ld, e / (TILE / 4), n, j0 + e % (TILE / 4) * 4, dv);
+    }
     chunk_sums(dt, loga, A_log, fixed, lo, n, H, h, cum, sdt);
     __syncthreads();
     const double end = cum[CH - 1];
-    for (int e = threadIdx.x; e < CH * TILE; e += NTH) {
-        const int t = e / TILE, j = e - t * TILE;
-        sA[t][j] = t < n && j0 + j < dv
-                       ? to_f32(x[(size_t)(lo + t) * x_ld + (size_t)h * dv + j0 + j]) * sdt[t] * expf((float)(end - cum[t])) : 0.f;
+    if (threadIdx.x == 0 && blockIdx.z == 0) decays[(size_t)blockIdx.x * H + h] = expf((float)end);
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+        const int e = threadIdx.x + p * MTH, t = e / (TILE / 4);
+        const float f = sdt[t] * expf((float)(end - cum[t]));                // 0 beyond the chunk's tokens
+        *reinterpret_cast<float4*>(sA + t * (TILE + 4) + e % (TILE / 4) * 4) =
+            make_float4(xv[p].x * f, xv[p].y * f, xv[p].z * f, xv[p].w * f);
     }
-    for (int e = threadIdx.x; e < CH * TILE * W; e += NTH) {
-        const int t = e / (TILE * W), k = e - t * TILE * W;
-        sB[t][k] = t < n && n0 + k < N ? B[(size_t)(lo + t) * B_ld + (size_t)grp * N + n0 + k] : 0.f;
-    }
+    if (VEC) asm volatile("cp.async.wait_group 0;\n" ::);
     __syncthreads();
-    multiply<W>(acc, sA, sB, n, ty, tx);
+    float acc[8][4 * W];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4 * W; ++j) acc[i][j] = 0.f;
+#pragma unroll 4
+    for (int t = 0; t < n; ++t) {
+        float a[8], b[4 * W];
+        *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(sA + t * (TILE + 4) + 8 * ty);
+        *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(sA + t * (TILE + 4) + 8 * ty + 4);
+#pragma unroll
+        for (int w = 0; w < W; ++w)
+            *reinterpret_cast<float4*>(b + 4 * w) = *reinterpret_cast<const float4*>(sB + t * BP + TILE * w + 4 * tx);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4 * W; ++j) acc[i][j] += a[i] * b[j];
+    }
     float* out = sums + ((size_t)blockIdx.x * H + h) * (dv + ones) * N;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int j = j0 + 4 * ty + i;
+    for (int i = 0; i < 8; ++i) {
+        const int j = j0 + 8 * ty + i;
         if (j >= dv) continue;
 #pragma unroll
         for (int w = 0; w < W; ++w) {
             const int k = n0 + TILE * w + 4 * tx;
-            if (N % 4 == 0) {
+            if (VEC) {
                 if (k < N) *reinterpret_cast<float4*>(out + (size_t)j * N + k) =
                     make_float4(acc[i][4 * w], acc[i][4 * w + 1], acc[i][4 * w + 2], acc[i][4 * w + 3]);
             } else {
@@ -120,84 +168,132 @@ chunk_states_kernel(const V* __restrict__ x, int x_ld, const float* __restrict__
             }
         }
     }
-    if (blockIdx.z == 0 && threadIdx.x == 0) decays[(size_t)blockIdx.x * H + h] = expf((float)end);
 }
 
-// before [chunks, H, dv + ones, N]: the state before every chunk.  o [T, H, dv + ones].  grid: chunks, H, tiles of 64
+// before [chunks, H, dv + ones, N]: the state before every chunk.  o [T, H, dv + ones].  grid: chunks, H, tiles of 64 W
 // columns, and with `ones` a light block for n . C.
-template <typename V>
-__global__ void __launch_bounds__(NTH)
+template <int W, bool VEC, typename V>
+__global__ void __launch_bounds__(MTH, 4)
 chunk_outputs_kernel(const V* __restrict__ x, int x_ld, const float* __restrict__ C, int C_ld, const float* __restrict__ dt,
                      const float* __restrict__ loga, const float* __restrict__ A_log, const double* __restrict__ fixed,
-                     const float* __restrict__ D,
-                     const int* __restrict__ cu, int R, const float* __restrict__ before, const float* __restrict__ dots,
-                     float* __restrict__ o, int H, int G, int N, int dv, int ones) {
-    __shared__ __align__(16) float sA[CH][PITCH];
-    __shared__ __align__(16) float sB[CH][PITCH];
+                     const float* __restrict__ D, const int* __restrict__ cu, int R, const float* __restrict__ before,
+                     const float* __restrict__ dots, float* __restrict__ o, int H, int G, int N, int dv, int ones) {
+    extern __shared__ __align__(16) float sm[];
     __shared__ double cum[CH];
-    __shared__ float sdt[CH], grown[CH];
+    __shared__ float sdt[CH];
     pdl_wait();
     pdl_trigger();
     int r, lo, n;
     if (!find_chunk(cu, R, blockIdx.x, r, lo, n)) return;
-    const int h = blockIdx.y, grp = h / (H / G), j0 = blockIdx.z * TILE;
+    const int h = blockIdx.y, grp = h / (H / G), j0 = blockIdx.z * TILE * W;
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-    chunk_sums(dt, loga, A_log, fixed, lo, n, H, h, cum, sdt);
-    __syncthreads();
+    const float* dd = dots + ((size_t)blockIdx.x * G + grp) * CH * CH;
     if (j0 >= dv) {
-        // n . C_i: four threads a token (neighbouring lanes) share its sums over the chunk's tokens and over n's numbers
-        const float* dd = dots + ((size_t)blockIdx.x * G + grp) * CH * CH;
+        chunk_sums(dt, loga, A_log, fixed, lo, n, H, h, cum, sdt);
+        __syncthreads();
+        // n . C_i: two threads a token (neighbouring lanes) share its sums over the chunk's tokens and over n's numbers
         const float* nb = before + (((size_t)blockIdx.x * H + h) * (dv + 1) + dv) * N;
-        const int i = threadIdx.x >> 2, part = threadIdx.x & 3;
+        const int i = threadIdx.x >> 1, part = threadIdx.x & 1;
         float s = 0.f, b = 0.f;
         if (i < n) {
             const float* c = C + (size_t)(lo + i) * C_ld + (size_t)grp * N;
-            for (int j = part; j <= i; j += 4) s += dd[j * CH + i] * sdt[j] * expf((float)(cum[i] - cum[j]));
-            for (int k = part; k < N; k += 4) b += nb[k] * c[k];
+            for (int j = part; j <= i; j += 2) s += dd[i * CH + j] * sdt[j] * expf((float)(cum[i] - cum[j]));
+            for (int k = part; k < N; k += 2) b += nb[k] * c[k];
             s += b * expf((float)cum[i]);
         }
         s += __shfl_xor_sync(0xffffffffu, s, 1);
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
         if (i < n && part == 0) o[((size_t)(lo + i) * H + h) * (dv + 1) + dv] = s;
         return;
     }
-    if (threadIdx.x < CH) grown[threadIdx.x] = expf((float)cum[threadIdx.x]);
-    // within the chunk
-    const float* d = dots + ((size_t)blockIdx.x * G + grp) * CH * CH;
-    for (int e = threadIdx.x; e < CH * CH; e += NTH) {
-        const int j = e / CH, i = e - j * CH;
-        sA[j][i] = j <= i && i < n ? d[e] * sdt[j] * expf((float)(cum[i] - cum[j])) : 0.f;
-    }
-    for (int e = threadIdx.x; e < CH * TILE; e += NTH) {
-        const int t = e / TILE, j = e - t * TILE;
-        sB[t][j] = t < n && j0 + j < dv ? to_f32(x[(size_t)(lo + t) * x_ld + (size_t)h * dv + j0 + j]) : 0.f;
+    float acc[8][4 * W];                                     // tokens 8 ty + i, columns j0 + tx + 16 q
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int q = 0; q < 4 * W; ++q) acc[i][q] = 0.f;
+    // from the state before the chunk
+    product_of_rows<4 * W, VEC>(acc, sm, C + (size_t)lo * C_ld + (size_t)grp * N, C_ld, n,
+                                before + (((size_t)blockIdx.x * H + h) * (dv + ones) + j0) * N, N, dv - j0, N, ty, tx);
+    chunk_sums(dt, loga, A_log, fixed, lo, n, H, h, cum, sdt);
+    // within it: token j counts for the tokens from j on only.  The values turned, column by token
+    float* sX = sm + CH * XP;
+    const V* xh = x + (size_t)lo * x_ld + (size_t)h * dv;
+#pragma unroll 4
+    for (int e = threadIdx.x; e < CH * (TILE * W / 4); e += MTH) {
+        const int t = e % CH, k = e / CH * 4;
+        const float4 v = values4<VEC>(xh, x_ld, t, n, j0 + k, dv);
+        sX[k * XP + t] = v.x; sX[(k + 1) * XP + t] = v.y; sX[(k + 2) * XP + t] = v.z; sX[(k + 3) * XP + t] = v.w;
     }
     __syncthreads();
-    float acc[4][4];
+#pragma unroll 8
+    for (int e = threadIdx.x; e < CH * CH; e += MTH) {
+        const int i = e / CH, j = e - i * CH;
+        sm[i * XP + j] = j <= i && i < n ? dd[e] * sdt[j] * expf((float)(cum[i] - cum[j])) : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float g = expf((float)cum[8 * ty + i]);
+#pragma unroll
+        for (int q = 0; q < 4 * W; ++q) acc[i][q] *= g;
+    }
+    __syncthreads();
+    multiply_rows<4 * W, XP, XP>(acc, sm, sX, 0, 8 * ty, ty, tx);
+    // the thread's own eight tokens: a triangle
     const float skip = D ? D[h] : 0.f;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int k = 0; k < 8; k += 4) {
+        float4 a[8];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = skip * sB[4 * ty + i][4 * tx + j];
-    multiply<1>(acc, sA, sB, min(n, 4 * (ty | 1) + 4), ty, tx);     // token j counts for the tokens from j on only
-    // from the state before it
-    const float* S = before + (((size_t)blockIdx.x * H + h) * (dv + ones) + j0) * N;
-    for (int k0 = 0; k0 < N; k0 += TILE) {
-        __syncthreads();
-        load_transposed(sA, C + (size_t)lo * C_ld + (size_t)grp * N, C_ld, n, N, k0, grown);
-        load_transposed(sB, S, N, min(TILE, dv - j0), N, k0, nullptr);
-        __syncthreads();
-        multiply<1>(acc, sA, sB, min(TILE, N - k0), ty, tx);
+        for (int i = k; i < 8; ++i) a[i] = *reinterpret_cast<const float4*>(sm + (8 * ty + i) * XP + 8 * ty + k);
+#pragma unroll
+        for (int q = 0; q < 4 * W; ++q) {
+            const float4 b = *reinterpret_cast<const float4*>(sX + (tx + 16 * q) * XP + 8 * ty + k);
+            acc[k][q] += skip * b.x; acc[k + 1][q] += skip * b.y; acc[k + 2][q] += skip * b.z; acc[k + 3][q] += skip * b.w;
+#pragma unroll
+            for (int i = k; i < 8; ++i) {
+                acc[i][q] += a[i].x * b.x;
+                if (i >= k + 1) acc[i][q] += a[i].y * b.y;
+                if (i >= k + 2) acc[i][q] += a[i].z * b.z;
+                if (i >= k + 3) acc[i][q] += a[i].w * b.w;
+            }
+        }
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int t = 4 * ty + i;
+    for (int i = 0; i < 8; ++i) {
+        const int t = 8 * ty + i;
         if (t >= n) continue;
-        float* out = o + ((size_t)(lo + t) * H + h) * (dv + ones) + j0 + 4 * tx;
+        float* out = o + ((size_t)(lo + t) * H + h) * (dv + ones) + j0 + tx;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (j0 + 4 * tx + j < dv) out[j] = acc[i][j];
+        for (int q = 0; q < 4 * W; ++q)
+            if (j0 + tx + 16 * q < dv) out[16 * q] = acc[i][q];
     }
+}
+
+// Four numbers at a time: sizes, pitches and addresses in multiples of four numbers.
+template <typename V>
+static bool by_fours(const V* x, int x_ld, const float* B, int B_ld, const float* C, int C_ld, int N, int dv) {
+    return N % 4 == 0 && dv % 4 == 0 && x_ld % 4 == 0 && B_ld % 4 == 0 && C_ld % 4 == 0 &&
+           ((uintptr_t)x & (4 * sizeof(V) - 1)) == 0 && (((uintptr_t)B | (uintptr_t)C) & 15) == 0;
+}
+template <typename K>
+static int allow(K kernel, size_t smem) {
+    return smem > 46 * 1024 ? (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : 0;
+}
+
+template <typename V>
+static int launch_outputs(const V* x, int x_ld, const float* C, int C_ld, const float* dt, const float* loga, const float* A_log,
+                          const double* fixed, const float* D, const int* cu_seqlens, const float* before, const float* dots,
+                          float* o, int T, int R, int H, int G, int N, int dv, int ones, cudaStream_t s) {
+    // 128 columns a block where that leaves three blocks an SM (2,048 tokens, 16 heads: 55 us), else 64: 30 chunks of 8 heads
+    // take 52 us with 128
+    const int wide = dv > TILE && (long long)(T / CH + R) * H * ((dv + 2 * TILE - 1) / (2 * TILE)) >= 3 * 148 ? 2 : 1;
+    const bool vec = by_fours(x, x_ld, before, 0, C, C_ld, N, dv);
+    auto kernel = wide == 2 ? (vec ? chunk_outputs_kernel<2, true, V> : chunk_outputs_kernel<2, false, V>)
+                            : (vec ? chunk_outputs_kernel<1, true, V> : chunk_outputs_kernel<1, false, V>);
+    const size_t smem = outputs_smem(wide);
+    const int e = allow(kernel, smem);
+    if (e) return e;
+    return rg_launch(kernel, dim3(T / CH + R, H, (dv + TILE * wide - 1) / (TILE * wide) + ones), dim3(MTH), smem, s, 1, x, x_ld, C,
+                     C_ld, dt, loga, A_log, fixed, D, cu_seqlens, R, before, dots, o, H, G, N, dv, ones);
 }
 
 // x [T, H * dv] float or bfloat16, rows x_ld apart; B, C [T, G * N] float, rows B_ld, C_ld apart.  dt [T, H], or null: 1.
@@ -215,14 +311,14 @@ static int chunk_scan(const V* x, int x_ld, const float* B, int B_ld, const floa
     const int jt = (dv + TILE - 1) / TILE, nt = (N + TILE * wide - 1) / (TILE * wide);
     if (jt * nt > 65535) return RG_ERR_UNSUPPORTED;
     dim3 g1(chunks, H + G, jt * nt);
-    const size_t smem = (size_t)CH * (PITCH + TILE * wide + 4) * sizeof(float);
-    auto states = wide == 2 ? chunk_states_kernel<2, V> : chunk_states_kernel<1, V>;
-    if (smem > 46 * 1024) {
-        const cudaError_t ce = cudaFuncSetAttribute(states, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (ce != cudaSuccess) return (int)ce;
-    }
-    int e = rg_launch(states, g1, dim3(NTH), smem, s, 1, x, x_ld, B, B_ld, C, C_ld, dt, loga, A_log, fixed, cu_seqlens, R, sums,
-                      decays, dots, H, G, N, dv, nt, ones);
+    const bool four_each = by_fours(x, x_ld, B, B_ld, C, C_ld, N, dv) && ((uintptr_t)sums & 15) == 0;
+    auto states = wide == 2 ? (four_each ? chunk_states_kernel<2, true, V> : chunk_states_kernel<2, false, V>)
+                            : (four_each ? chunk_states_kernel<1, true, V> : chunk_states_kernel<1, false, V>);
+    const size_t smem = states_smem(wide);
+    int e = allow(states, smem);
+    if (e) return e;
+    e = rg_launch(states, g1, dim3(MTH), smem, s, 1, x, x_ld, B, B_ld, C, C_ld, dt, loga, A_log, fixed, cu_seqlens, R, sums,
+                  decays, dots, H, G, N, dv, nt, ones);
     if (e) return e;
     const int M = (dv + ones) * N;
     const bool vec = M % 4 == 0 && ((uintptr_t)state & 15) == 0;
@@ -231,8 +327,8 @@ static int chunk_scan(const V* x, int x_ld, const float* B, int B_ld, const floa
     e = vec ? rg_launch(chunk_pass_kernel<4, false>, g2, dim3(256), 0, s, 1, sums, (const float*)decays, state, cu_seqlens, start_pos, slots, H, M, N)
             : rg_launch(chunk_pass_kernel<1, false>, g2, dim3(256), 0, s, 1, sums, (const float*)decays, state, cu_seqlens, start_pos, slots, H, M, N);
     if (e) return e;
-    return rg_launch(chunk_outputs_kernel<V>, dim3(chunks, H, jt + ones), dim3(NTH), 0, s, 1, x, x_ld, C, C_ld, dt, loga, A_log,
-                     fixed, D, cu_seqlens, R, (const float*)sums, (const float*)dots, o, H, G, N, dv, ones);
+    return launch_outputs(x, x_ld, C, C_ld, dt, loga, A_log, fixed, D, cu_seqlens, (const float*)sums, (const float*)dots, o, T, R,
+                          H, G, N, dv, ones, s);
 }
 
 extern "C" int rg_ssd_chunk_scan(const void* x, int x_dtype, int x_ld, const float* B, int B_ld, const float* C, int C_ld,
@@ -260,7 +356,6 @@ extern "C" int rg_chunk_outputs(const float* x, int x_ld, const float* C, int C_
                                 void* stream) {
     if (T <= 0 || R <= 0) return 0;
     if (H < 1 || G < 1 || H % G || N < 1 || dv < 1 || H > 65535 || (dv + TILE - 1) / TILE > 65535) return RG_ERR_UNSUPPORTED;
-    return rg_launch(chunk_outputs_kernel<float>, dim3(T / CH + R, H, (dv + TILE - 1) / TILE), dim3(NTH), 0, (cudaStream_t)stream,
-                     1, x, x_ld, C, C_ld, (const float*)nullptr, loga, (const float*)nullptr, (const double*)nullptr,
-                     (const float*)nullptr, cu_seqlens, R, before, dots, o, H, G, N, dv, 0);
+    return launch_outputs(x, x_ld, C, C_ld, (const float*)nullptr, loga, (const float*)nullptr, (const double*)nullptr,
+                          (const float*)nullptr, cu_seqlens, before, dots, o, T, R, H, G, N, dv, 0, (cudaStream_t)stream);
 }
