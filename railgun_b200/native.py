@@ -15,10 +15,12 @@ from __future__ import annotations
 
 import ctypes
 import hashlib
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
@@ -36,12 +38,16 @@ NVCC_FLAGS = [
 GXX_FLAGS = ["-O2", "-std=c++17", "-shared", "-fPIC", "-Wall"]
 
 
+# Host sources that are Python extension modules rather than libraries of C functions.
+PYTHON_MODULES = ("fastcall",)
+
+
 class NativeBuildError(RuntimeError):
     """A native library could not be compiled or loaded."""
 
 
 _lock = threading.Lock()
-_loaded: dict[str, ctypes.CDLL] = {}
+_loaded: dict = {}
 
 
 def _say(msg: str) -> None:
@@ -119,6 +125,8 @@ def library_path(name: str, kind: str) -> tuple[Path, Path, list[str], str]:
     else:
         src = HOST_DIR / f"{name}.cpp"
         flags = list(GXX_FLAGS)
+        if name in PYTHON_MODULES:
+            flags.append(f"-I{sysconfig.get_paths()['include']}")
         compiler = "g++"
     if not src.exists():
         raise NativeBuildError(f"no source file {src}")
@@ -162,6 +170,23 @@ def load(name: str, kind: str = "kernel") -> ctypes.CDLL:
                 raise NativeBuildError(f"cannot load {path}: {e}") from e
             _loaded[key] = lib
         return lib
+
+
+def load_module(name: str):
+    """A Python extension module among the host sources, built first if need be.  Raises, never falls back."""
+    key = f"module:{name}"
+    with _lock:
+        mod = _loaded.get(key)
+        if mod is None:
+            path = build(name, "host")
+            try:
+                spec = importlib.util.spec_from_file_location(name, str(path))
+                mod = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(mod)
+            except (ImportError, OSError) as e:
+                raise NativeBuildError(f"cannot load {path}: {e}") from e
+            _loaded[key] = mod
+        return mod
 
 
 def kernel_sources() -> list[str]:

@@ -8,8 +8,8 @@ or if a library fails to build, these raise.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
-from ctypes import c_int, c_float, c_void_p, c_longlong
 
 import torch
 
@@ -30,7 +30,26 @@ def _dtype_code(t: torch.Tensor) -> int:
     raise KernelError(f"unsupported dtype {t.dtype}: kernels take float32 or bfloat16")
 
 
+# How a launcher (a C function of integers, pointers and floats) is called: through an extension module with plain numbers
+# (csrc/host/fastcall.cpp), or, where that cannot be built (no Python headers), through ctypes.  Either way an argument is
+# written as the C type it has.
+try:
+    _fast = native.load_module("fastcall")
+except native.NativeBuildError:
+    _fast = None
+if _fast is not None:
+    c_int = c_longlong = c_void_p = _fast.same
+    c_float, _ptr = _fast.real, _fast.ptr
+else:
+    from ctypes import c_int, c_float, c_void_p, c_longlong
+
+    def _ptr(t):
+        return c_void_p(0 if t is None else t.data_ptr())
+
+
 def _check(t: torch.Tensor, name: str, dtype=None) -> None:
+    if _fast is not None and _fast.fits(t, dtype):
+        return
     if not t.is_cuda:
         raise KernelError(f"{name} must be a CUDA tensor (there is no CPU path)")
     if not t.is_contiguous():
@@ -49,17 +68,21 @@ def _check_rows(t: torch.Tensor, name: str, dtype=None) -> None:
         raise KernelError(f"{name} must be {dtype}, got {t.dtype}")
 
 
-def _ptr(t) -> c_void_p:
-    return c_void_p(0 if t is None else t.data_ptr())
+def _at(value):
+    """The address of a ctypes value or array that a launcher writes or reads."""
+    return c_void_p(ctypes.addressof(value))
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
-def _stream() -> c_void_p:
+_current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
+
+
+def _stream():
     """The current CUDA stream of the current device (what torch.cuda.stream and graph capture set)."""
     if _raw_stream is not None:
-        return c_void_p(_raw_stream(torch.cuda.current_device()))
+        return c_void_p(_raw_stream(_current_device()))
     return c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
@@ -99,10 +122,12 @@ def _fn(lib_name: str, fn_name: str):
         lib = native.load(lib_name)
         if lib_name not in _pdl_set:
             lib.rg_set_pdl.restype = None
-            lib.rg_set_pdl(c_int(1 if PDL_ENABLED else 0))
+            lib.rg_set_pdl(ctypes.c_int(1 if PDL_ENABLED else 0))
             _pdl_set.add(lib_name)
         fn = getattr(lib, fn_name)
-        fn.restype = c_int
+        fn.restype = ctypes.c_int
+        if _fast is not None:
+            fn = functools.partial(_fast.call, ctypes.cast(fn, ctypes.c_void_p).value)
         _fn_cache[fn_name] = fn
     _COUNTER.value += 1
     return fn
@@ -214,10 +239,10 @@ def norm_sum(ys, weights, consts, eps: float) -> torch.Tensor:
         if tuple(y.shape) != (T, H) or w.numel() != H:
             raise KernelError(f"norm_sum: input {tuple(y.shape)} or weight of {w.numel()} does not match [{T}, {H}]")
     out = torch.empty((T, H), dtype=torch.float32, device=ys[0].device)
-    yp = (c_void_p * n)(*[y.data_ptr() for y in ys])
-    wp = (c_void_p * n)(*[w.data_ptr() for w in weights])
-    cs = (c_float * n)(*[float(c) for c in consts])
-    _ok(_fn("norm", "rg_norm_sum")(yp, wp, cs, c_int(n), c_int(_dtype_code(ys[0])), c_float(eps), _ptr(out), c_int(T),
+    yp = (ctypes.c_void_p * n)(*[y.data_ptr() for y in ys])
+    wp = (ctypes.c_void_p * n)(*[w.data_ptr() for w in weights])
+    cs = (ctypes.c_float * n)(*[float(c) for c in consts])
+    _ok(_fn("norm", "rg_norm_sum")(_at(yp), _at(wp), _at(cs), c_int(n), c_int(_dtype_code(ys[0])), c_float(eps), _ptr(out), c_int(T),
                                    c_int(H), _stream()), "norm_sum")
     return out
 
@@ -1795,10 +1820,10 @@ def skinny_gemm_residual(x: torch.Tensor, weight: torch.Tensor, resid: torch.Ten
     ld = 8 * ((M + 7) // 8)
     partials = torch.empty(((N + 15) // 16, ld), dtype=torch.float32, device=x.device)
     scaled = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
-    blocks = c_int(0)
+    blocks = ctypes.c_int(0)
     _ok(_fn("gemm_skinny_fused", "rg_skinny_gemm_residual")(
         _ptr(weight), _ptr(x), c_int(x.stride(0)), _ptr(resid), c_int(resid.stride(0)), _ptr(norm_weight), _ptr(scaled),
-        c_int(M), c_int(N), c_int(K), _ptr(partials), c_int(ld), ctypes.byref(blocks), _stream()),
+        c_int(M), c_int(N), c_int(K), _ptr(partials), c_int(ld), _at(blocks), _stream()),
         "skinny_gemm_residual")
     return NormedRows(resid, scaled, partials, blocks.value, norm_weight, eps, torch.bfloat16)
 
@@ -2258,10 +2283,10 @@ def tc_stream_gemm_residual(x: torch.Tensor, weight: torch.Tensor, resid: torch.
         err = _tc_err[x.device] = torch.zeros(1, dtype=torch.int32, device=x.device)
     global _tc_unchecked
     _tc_unchecked = True
-    tiles = c_int(0)
+    tiles = ctypes.c_int(0)
     _ok(_fn("gemm_stream_tcgen05", "rg_tc_stream_gemm_residual")(
         _ptr(x), c_int(x.stride(0)), _ptr(weight), _ptr(resid), c_int(resid.stride(0)), _ptr(norm_weight), _ptr(scaled),
-        _ptr(partials), c_int(partials.stride(0)), c_int(M), c_int(N), c_int(K), c_int(splits), ctypes.byref(tiles),
+        _ptr(partials), c_int(partials.stride(0)), c_int(M), c_int(N), c_int(K), c_int(splits), _at(tiles),
         _ptr(err), _stream()), "tc_stream_gemm_residual")
     return NormedRows(resid, scaled, partials, tiles.value, norm_weight, eps, torch.bfloat16)
 
@@ -2369,7 +2394,7 @@ def probe_sm100(device="cuda:0") -> dict:
     err = torch.zeros(1, dtype=torch.int32, device=dev)
     out = (c_double * len(names))()
     with torch.cuda.device(dev):
-        _ok(_fn("probe_sm100", "rg_probe_sm100")(out, _ptr(scratch), _ptr(cyc), _ptr(err), _stream()), "probe_sm100")
+        _ok(_fn("probe_sm100", "rg_probe_sm100")(_at(out), _ptr(scratch), _ptr(cyc), _ptr(err), _stream()), "probe_sm100")
     if int(err.item()) != 0 or any(v < 0 for v in out):
         raise KernelError(f"probe_sm100: a bounded wait gave up (code {int(err.item())})")
     return {n: round(float(v), 1) for n, v in zip(names, out)}
