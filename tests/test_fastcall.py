@@ -45,6 +45,6 @@ def test_what_it_refuses(fast):
         fast.call(1, *[0.5] * 9)
     with pytest.raises(TypeError):
         fast.call(1, "text")
-    with pytest.raises(TypeError):
+    with pytest.raises(ValueError):
         fast.real("text")
     assert fast.ptr(None) == 0 and fast.same(fast) is fast
