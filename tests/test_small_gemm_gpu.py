@@ -1,0 +1,36 @@
+"""The 32-bit product of a few rows by a small matrix, at the edges of its 32 x 32 tiles and 32-wide steps, along and across
+16-byte boundaries, against 64 bits."""
+import pytest
+import torch
+
+from test_kernels_gpu import DEV, rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (1, 500, 96), (67, 160, 96), (32, 32, 32), (33, 33, 33), (31, 65, 511), (128, 1024, 512),
+                                   (16, 96, 256), (2, 7, 4)])
+def test_against_64_bits(M, N, K):
+    from railgun_b200 import ops
+    g = torch.Generator().manual_seed(M + N + K)
+    x, w = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
+    ref = x.double() @ w.double().T
+    y = ops.small_gemm_f32(x, w)
+    # chains of eight products and of at most sixteen of their sums: some 25 x 2^-24 of the largest, 1.5e-6
+    assert y.dtype == torch.float32 and rel_err(y, ref) < 2e-6
+    assert torch.equal(ops.linear(x, w), y)
+    if K <= 128:
+        assert torch.equal(ops.small_gemm_f32(x[M // 2:M // 2 + 1], w)[0], y[M // 2])  # a row on its own
+    wide = torch.full((M, K + 3), float("nan"), device=DEV)                            # rows off 16-byte boundaries
+    wide[:, 1:K + 1] = x
+    assert torch.equal(ops.small_gemm_f32(wide[:, 1:K + 1], w), y)
+
+
+def test_what_it_refuses():
+    from railgun_b200 import ops
+    x, w = torch.zeros(4, 64, device=DEV), torch.zeros(8, 64, device=DEV)
+    assert ops.small_gemm_f32_ok(x, w) and not ops.small_gemm_f32_ok(x.bfloat16(), w.bfloat16())
+    assert not ops.small_gemm_f32_ok(x.t(), w) and not ops.small_gemm_f32_ok(x[:0], w)
+    assert not ops.small_gemm_f32_ok(torch.zeros(8, 256, device=DEV), torch.zeros(64, 256, device=DEV))    # the library's is faster
+    with pytest.raises(ops.KernelError):
+        ops.small_gemm_f32(x, torch.zeros(8, 63, device=DEV))
