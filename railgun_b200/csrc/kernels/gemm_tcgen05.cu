@@ -261,7 +261,7 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int KT = (K + TC_BK - 1) / TC_BK;
     const int m_tiles = (M + 2 * TC_BM - 1) / (2 * TC_BM), n_tiles = (N + BN - 1) / BN;
     const int total_tiles = m_tiles * n_tiles;
-    constexpr uint32_t TMEM_COLS = 2 * BN;
+    constexpr uint32_t TMEM_COLS = BN <= 128 ? 256 : 512;                   // two accumulators; a power of two
 
     if (threadIdx.x == 0) {
         abort_flag = 0;
@@ -373,12 +373,13 @@ static int launch_tc_pair(const CUtensorMap& ma, const CUtensorMap& mb, OUT* out
 // the call, non-zero afterwards if a wait gave up (1 producer, 2 and 4 MMA, 3 epilogue).
 extern "C" int rg_tc_gemm(const void* A, int lda, const void* B, void* out, int ldo, int out_dtype, int epilogue,
                           int M, int N, int K, int wide, int* err, void* stream) {
-    // wide: 0 one CTA per 128 x 128 tile, 1 per 128 x 256; 2 a CTA pair per 256 x 256 tile, 3 per 256 x 128
+    // wide: 0 one CTA per 128 x 128 tile, 1 per 128 x 256; a CTA pair per tile of 256 rows by 2: 256, 3: 128, 4: 224, 5: 192
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || K % 8 || lda % 8 || ((uintptr_t)A & 15) || ((uintptr_t)B & 15)) return RG_ERR_UNSUPPORTED;
     if (epilogue == EPI_SILU_MUL && (N % 16 || out_dtype != RG_DTYPE_BF16)) return RG_ERR_UNSUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
-    const int BN = (wide == 1 || wide == 2) ? 256 : 128;
+    if (wide < 0 || wide > 5) return RG_ERR_UNSUPPORTED;
+    const int BN = wide == 1 || wide == 2 ? 256 : wide == 4 ? 224 : wide == 5 ? 192 : 128;
     CUtensorMap ma, mb;
     int e = rg_make_map(&ma, A, M, K, lda, TC_BM);
     if (e) return e;
@@ -386,8 +387,9 @@ extern "C" int rg_tc_gemm(const void* A, int lda, const void* B, void* out, int 
     if (e) return e;
     if (wide >= 2) {
 #define RG_PAIR(EPI_, OUT_) (wide == 2 ? launch_tc_pair<256, 6, EPI_, OUT_>(ma, mb, (OUT_*)out, ldo, M, N, K, err, s) \
+                           : wide == 4 ? launch_tc_pair<224, 6, EPI_, OUT_>(ma, mb, (OUT_*)out, ldo, M, N, K, err, s) \
+                           : wide == 5 ? launch_tc_pair<192, 7, EPI_, OUT_>(ma, mb, (OUT_*)out, ldo, M, N, K, err, s) \
                                        : launch_tc_pair<128, 8, EPI_, OUT_>(ma, mb, (OUT_*)out, ldo, M, N, K, err, s))
-        if (wide > 3) return RG_ERR_UNSUPPORTED;
         if (epilogue == EPI_SILU_MUL) return RG_PAIR(EPI_SILU_MUL, bf16);
         if (epilogue != EPI_NONE) return RG_ERR_UNSUPPORTED;
         if (out_dtype == RG_DTYPE_BF16) return RG_PAIR(EPI_NONE, bf16);

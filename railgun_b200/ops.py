@@ -2109,7 +2109,25 @@ def tc_gemm_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
             and weight.is_contiguous() and weight.data_ptr() % 16 == 0)
 
 
-TC_TILES = {"128x128": 0, "128x256": 1, "256x256": 2, "256x128": 3}
+TC_TILES = {"128x128": 0, "128x256": 1, "256x256": 2, "256x128": 3, "256x224": 4, "256x192": 5}
+
+
+@functools.lru_cache(maxsize=None)
+def _sm_pairs(device_index: int) -> int:
+    return torch.cuda.get_device_properties(device_index).multi_processor_count // 2
+
+
+def tc_pair_tile(M: int, N: int, device) -> str:
+    """The tile for a product on CTA pairs: 256 x 256, or a narrower one where that leaves the GPU's pairs idle less.  Tiles
+    are worked off in rounds of one per pair, and a round takes about as long as its tiles are wide (and 8 columns more).
+    A narrower tile has to save a twelfth of that: it moves more of x per result, and where nearly every pair is busy the
+    power limit, not the rounds, is the bound.  Back to back with SiLU-mul, 256 / 224 / 192 columns: 1,056 rows by 3,072 x
+    16,384 150 / 135 / 140 us, 1,701 by 2,048 x 16,384 195 / 165 / 172, 2,048 by 4,096 x 28,672 417 / 448 / 473."""
+    pairs = _sm_pairs(device.index if device.index is not None else torch.cuda.current_device())
+    m_tiles = -(-M // 256)
+    cost = {n: -(-(m_tiles * -(-N // n)) // pairs) * (n + 8) for n in (256, 224, 192)}
+    best = min(cost, key=lambda n: (cost[n], -n))
+    return f"256x{best if 12 * cost[best] <= 11 * cost[256] else 256}"
 
 
 def tc_gemm(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, silu_mul: bool = False, wide: bool = True,
@@ -2117,8 +2135,8 @@ def tc_gemm(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, silu_mul: boo
     """y = x W^T on the tcgen05 tensor cores (TMA-fed, accumulators in tensor
     memory).  ``silu_mul``: W is interleaved gate|up storage and y = silu(gate)
     * up.  ``tile`` (rows of x by rows of W): "128x128" or "128x256", one CTA
-    per tile, or "256x256" / "256x128", a pair of CTAs on two SMs per tile
-    (cta_group::2); without it ``wide`` picks between the first two.  The
+    per tile, or "256x256", "256x224", "256x192" or "256x128", a pair of CTAs on
+    two SMs per tile (cta_group::2); without it ``wide`` picks between the first two.  The
     kernel's waits are bounded; ``tc_gemm_check()`` (or ``check=True``, which
     synchronises) raises if one gave up."""
     if tile is None:

@@ -65,7 +65,8 @@ class SwiGLU(FeedForward):
             act = ops.tc_stream_gemm(x, self.w_gate_up, silu_mul=True)
         elif self.interleaved and x.shape[0] >= ops.TC_GEMM_MIN_ROWS and ops.tc_gemm_ok(x, self.w_gate_up):
             # prefill: tcgen05 on CTA pairs, SiLU-mul in the epilogue
-            act = ops.tc_gemm(x, self.w_gate_up, silu_mul=True, tile="256x256")
+            act = ops.tc_gemm(x, self.w_gate_up, silu_mul=True,
+                              tile=ops.tc_pair_tile(x.shape[0], self.w_gate_up.shape[0], x.device))
         else:
             act = ops.silu_mul(ops.linear(x, self.w_gate_up), interleaved=self.interleaved)
         return ops.PendingLinear(act, self.w_down) if defer else ops.linear(act, self.w_down)
