@@ -8,7 +8,7 @@
 //   S1 = exp(c_L) S0 + sum_j exp(c_L - c_j) k_j u_j^T,
 //   o_i = exp(c_i) S0^T q_i + sum_(j <= i) exp(c_i - c_j) (k_j . q_i) u_j
 // (the block form of Yang et al., "Parallelizing Linear Transformers with the Delta Rule over Sequence Length").
-//   delta_solve    per (chunk, head): X and W by forward substitution; per (chunk, query/key head): all k_j . q_i
+//   delta_solve    per (chunk, head): (I + A)^-1 by substitution in blocks, X and W; per (chunk, query/key head): all k_j . q_i
 //   delta_states   per (request, head, 16 columns of S): chunk after chunk, U, the state before every chunk, and the last
 //                  one into the request's slot
 // and chunk_outputs (ssd_chunk.cu) with U in the place of the values.  Everything is 32-bit fused multiply-adds; the
@@ -16,10 +16,11 @@
 //
 // What bounds it: the 32-bit multiply-adds (128 a cycle and SM, packed or not), and in delta_states the chain from chunk to
 // chunk, 2 x 64 x d of them per column and chunk.  16 columns a block fill 128 of 148 SMs at 16 heads of 128 columns;
-// narrower blocks fetch the same W and K more often.  Measured (2,048 tokens, 16 heads of 128 x 128 on 8): 85 us the
-// systems, 116 the states, 55 the outputs; the token-by-token kernel (state_mixers.cu) took 908.  Steps whose longest portion is shorter than 128 tokens stay
-// on that one.
+// narrower blocks fetch the same W and K more often.  Measured (2,048 tokens, 16 heads of 128 x 128 on 8): 58 us the
+// systems, 116 the states, 54 the outputs; the token-by-token kernel (state_mixers.cu) took 908.  Steps whose longest
+// portion is shorter than 128 tokens stay on that one.
 #include "chunk_scan.cuh"
+#include <type_traits>
 
 #define DC_CB 16              // columns of S per block of delta_states
 #define DC_WP 72              // pitch of W's rows (k) in shared memory: four neighbouring k lie in different banks
@@ -28,14 +29,25 @@
 // q, k: rows q_ld, k_ld apart, head h of the H reads head h / (H / Hqk).  beta, loga [T, H].  x_out [T, H, dv] = X;
 // w_out [chunks, H, d, 64] = W transposed; factors [chunks, H, 64] = exp(c_L - c_i) (1 beyond the chunk's tokens), decays
 // [chunks, H] = exp(c_L); dots [chunks, Hqk, 64, 64] = q_i . k_j at [i][j].  grid: chunks, H (systems) and then Hqk (dots).
-template <typename V>
-__global__ void __launch_bounds__(NTH, 2)
+// The inverse T of I + A is made once per system, in blocks of 16: the diagonal blocks by substitution (64 threads, one column
+// each), then row of blocks by row of blocks T_rc = -T_rr sum_k A_rk T_kc; X and W are products with it.  (Substituting
+// all dv + d right-hand sides, one a thread with 64 unknowns in registers, was 2,600 instructions that ran once: 85 us for
+// 528 systems of 2,048 tokens, 58 now.)
+#define DS_TP (CH + 4)        // pitch of T transposed
+#define DS_CP (128 + 4)       // pitch of 128 columns of the right-hand sides
+
+constexpr size_t ds_smem() {
+    const size_t a = (size_t)2 * (64 + 64) * MP * 4, b = (size_t)(CH * DS_TP + CH * DS_CP) * 4;
+    return a > b ? a : b;
+}
+
+template <bool VEC, typename V>
+__global__ void __launch_bounds__(MTH, 4)
 delta_solve_kernel(const float* __restrict__ q, int q_ld, const float* __restrict__ k, int k_ld, const V* __restrict__ v,
                    int v_ld, const float* __restrict__ beta, const float* __restrict__ loga, const int* __restrict__ cu,
                    int R, float* __restrict__ x_out, float* __restrict__ w_out, float* __restrict__ factors,
                    float* __restrict__ decays, float* __restrict__ dots, int H, int Hqk, int d, int dv) {
-    __shared__ __align__(16) float sA[CH][PITCH];
-    __shared__ __align__(16) float sB[CH][PITCH];
+    extern __shared__ __align__(16) float sm[];
     __shared__ double cum[CH];
     __shared__ float sbeta[CH], grown[CH];
     pdl_wait();
@@ -45,87 +57,164 @@ delta_solve_kernel(const float* __restrict__ q, int q_ld, const float* __restric
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
     const bool system = (int)blockIdx.y < H;
     const int h = blockIdx.y, hq = system ? h / (H / Hqk) : h - H;
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-    // k_j . k_i: thread (ty, tx) has j = 4 ty .., i = 4 tx ..; or q_i . k_j: i = 4 ty .., j = 4 tx ..
     const float* kh = k + (size_t)lo * k_ld + (size_t)hq * d;
-    const float* other = system ? kh : q + (size_t)lo * q_ld + (size_t)hq * d;
-    for (int k0 = 0; k0 < d; k0 += TILE) {
-        load_transposed(sA, kh, k_ld, n, d, k0, nullptr);
-        if (!system) load_transposed(sB, other, q_ld, n, d, k0, nullptr);
-        __syncthreads();
-        multiply<1>(acc, system ? sA : sB, sA, min(TILE, d - k0), ty, tx);
-        __syncthreads();
-    }
-    if (!system) {
-        float* out = dots + ((size_t)blockIdx.x * Hqk + hq) * CH * CH;
+    {
+        // k_i . k_j, or q_i . k_j: i = 8 ty .., j = tx + 16 q
+        float acc[8][4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-            *reinterpret_cast<float4*>(out + (4 * ty + i) * CH + 4 * tx) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-        return;
-    }
-    chunk_sums(nullptr, loga, nullptr, nullptr, lo, n, H, h, cum, grown);
-    if (threadIdx.x >= 64 && threadIdx.x < 128) {
-        const int i = threadIdx.x - 64;
-        sbeta[i] = i < n ? beta[(size_t)(lo + i) * H + h] : 0.f;
-    }
-    __syncthreads();
-    // A transposed: sB[j][i], zero for i <= j (and beyond the chunk's tokens, whose beta is 0)
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+            for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+        if (system) product_of_rows<4, true>(acc, sm, kh, k_ld, n, kh, k_ld, n, d, ty, tx);
+        else product_of_rows<4, VEC>(acc, sm, q + (size_t)lo * q_ld + (size_t)hq * d, q_ld, n, kh, k_ld, n, d, ty, tx);
+        if (!system) {
+            float* out = dots + ((size_t)blockIdx.x * Hqk + hq) * CH * CH;
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int j = 4 * ty + a, i = 4 * tx + b;
-            sB[j][i] = j < i && i < n ? sbeta[i] * expf((float)(cum[i] - cum[j])) * acc[a][b] : 0.f;
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) out[(8 * ty + i) * CH + tx + 16 * j] = acc[i][j];
+            return;
         }
+        chunk_sums(nullptr, loga, nullptr, nullptr, lo, n, H, h, cum, grown);
+        if (threadIdx.x >= 64) {
+            const int i = threadIdx.x - 64;
+            sbeta[i] = i < n ? beta[(size_t)(lo + i) * H + h] : 0.f;
+        }
+        __syncthreads();
+        // A as it lies: sm[i][j], zero for j >= i and beyond the chunk's tokens (whose beta is 0)
+#pragma unroll
+        for (int a = 0; a < 8; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const int i = 8 * ty + a, j = tx + 16 * b;
+                sm[i * DS_TP + j] = j < i && i < n ? sbeta[i] * expf((float)(cum[i] - cum[j])) * acc[a][b] : 0.f;
+            }
+    }
+    float* sA = sm;                                      // A, then T transposed
+    float* sT = sm + CH * DS_TP;                         // T, [i][j]; then the right-hand sides
     if (threadIdx.x < CH) {
         const size_t at = (size_t)blockIdx.x * H + h;
         const double end = cum[CH - 1];
-        grown[threadIdx.x] = sbeta[threadIdx.x] * expf((float)cum[threadIdx.x]);
+        grown[threadIdx.x] = expf((float)cum[threadIdx.x]);
         factors[at * CH + threadIdx.x] = expf((float)(end - cum[threadIdx.x]));
         if (threadIdx.x == 0) decays[at] = expf((float)end);
     }
+    for (int e = threadIdx.x; e < CH * DS_TP; e += MTH) sT[e] = 0.f;
     __syncthreads();
-    // one column of the right-hand sides per thread, 64 unknowns in registers: each solved unknown is taken out of the
-    // rows below it (independent multiply-adds; A's numbers are the same address for the whole warp)
-    const uint32_t sb = (uint32_t)__cvta_generic_to_shared(&sB[0][0]);
-    for (int col = threadIdx.x; col < dv + d; col += NTH) {
-        float y[CH];
-        if (col < dv) {
-            const V* src = v + (size_t)lo * v_ld + (size_t)h * dv + col;
+    if (threadIdx.x < CH) {
+        // column c of the diagonal block b
+        const int b0 = threadIdx.x & 48, c = threadIdx.x & 15;
+        float y[16];
 #pragma unroll
-            for (int i = 0; i < CH; ++i, src += v_ld) y[i] = i < n ? sbeta[i] * to_f32(*src) : 0.f;
-        } else {
-            const float* src = kh + col - dv;
+        for (int i = 0; i < 16; ++i) {
+            float t = i == c ? 1.f : 0.f;
 #pragma unroll
-            for (int i = 0; i < CH; ++i, src += k_ld) y[i] = i < n ? grown[i] * *src : 0.f;
+            for (int j = 0; j < i; ++j) t -= sA[(b0 + i) * DS_TP + b0 + j] * y[j];
+            y[i] = t;
         }
 #pragma unroll
-        for (int j = 0; j < CH - 1; ++j) {
-            const float yj = y[j];
+        for (int i = 0; i < 16; ++i) sT[(b0 + i) * DS_TP + b0 + c] = y[i];
+    }
+    __syncthreads();
+    for (int br = 1; br < 4; ++br) {
+        // P_c = sum_(k = c .. br - 1) A_(br, k) T_(k, c) for all c < br: rows 16 br + i, columns 0 .. 16 br - 1, two columns a thread
+        // at a time; then T_(br, c) = -T_(br, br) P_c
+        const int cols = 16 * br, i = threadIdx.x >> 3, c0 = threadIdx.x & 7;       // 16 rows x 8 threads
+        float p[6];
 #pragma unroll
-            for (int i4 = (j + 1) / 4; i4 < CH / 4; ++i4) {
-                float4 a;                                 // (volatile: the loads stay beside their use)
-                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w)
-                             : "r"(sb + (uint32_t)(j * PITCH + 4 * i4) * 4u));
-                if (4 * i4 > j) y[4 * i4] -= a.x * yj;
-                if (4 * i4 + 1 > j) y[4 * i4 + 1] -= a.y * yj;
-                if (4 * i4 + 2 > j) y[4 * i4 + 2] -= a.z * yj;
-                y[4 * i4 + 3] -= a.w * yj;
+        for (int m = 0; m < 6; ++m) {
+            p[m] = 0.f;
+            const int c = c0 + 8 * m;
+            if (c < cols)
+                for (int k2 = c & 48; k2 < cols; ++k2) p[m] += sA[(cols + i) * DS_TP + k2] * sT[k2 * DS_TP + c];
+        }
+        __syncthreads();
+        // P takes A's place in this row of blocks (its columns left of the diagonal block are not needed again)
+#pragma unroll
+        for (int m = 0; m < 6; ++m)
+            if (c0 + 8 * m < cols) sA[(cols + i) * DS_TP + c0 + 8 * m] = p[m];
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+            const int c = c0 + 8 * m;
+            if (c < cols) {
+                float t = 0.f;
+                for (int j = 0; j <= i; ++j) t -= sT[(cols + i) * DS_TP + cols + j] * sA[(cols + j) * DS_TP + c];
+                sT[(cols + i) * DS_TP + c] = t;
             }
         }
-        if (col < dv) {
-            float* dst = x_out + ((size_t)lo * H + h) * dv + col;
+        __syncthreads();
+    }
+    // T transposed and times beta of its columns: sA[j][i]
+    for (int e = threadIdx.x; e < CH * CH; e += MTH) {
+        const int j = e / CH, i = e % CH;
+        sA[j * DS_TP + i] = sT[i * DS_TP + j] * sbeta[j];
+    }
+    // X = T (beta V) and W = T (beta exp(c) K), 128 columns at a time
+    const int vt = (dv + 127) / 128, kt = (d + 127) / 128;
+    for (int t = 0; t < vt + kt; ++t) {
+        const bool values = t < vt;
+        const int col0 = (values ? t : t - vt) * 128, N = values ? dv : d;
+        __syncthreads();
+#pragma unroll 4
+        for (int e = threadIdx.x; e < CH * 32; e += MTH) {
+            const int j = e / 32, c = e % 32 * 4;
+            float4 x;
+            if (values) {
+                x = values4<VEC>(v + (size_t)lo * v_ld + (size_t)h * dv, v_ld, j, n, col0 + c, N);
+            } else {
+                x = values4<true>(kh, k_ld, j, n, col0 + c, N);
+                const float g = grown[j];
+                x.x *= g; x.y *= g; x.z *= g; x.w *= g;
+            }
+            *reinterpret_cast<float4*>(sT + j * DS_CP + c) = x;
+        }
+        __syncthreads();
+        float acc[8][8];
 #pragma unroll
-            for (int i = 0; i < CH; ++i, dst += H * dv)
-                if (i < n) *dst = y[i];
-        } else {
-            float* dst = w_out + (((size_t)blockIdx.x * H + h) * d + (col - dv)) * CH;
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
-            for (int i = 0; i < CH; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(y[i], y[i + 1], y[i + 2], y[i + 3]);
+            for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+        // T is lower triangular: the thread's own eight tokens are a triangle (a later token's infinities stay out of it)
+        auto step = [&](int j, auto from) {
+            float a[8], b[8];
+            *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(sA + j * DS_TP + 8 * ty);
+            *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(sA + j * DS_TP + 8 * ty + 4);
+            *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(sT + j * DS_CP + 4 * tx);
+            *reinterpret_cast<float4*>(b + 4) = *reinterpret_cast<const float4*>(sT + j * DS_CP + 64 + 4 * tx);
+#pragma unroll
+            for (int i = decltype(from)::value; i < 8; ++i)
+#pragma unroll
+                for (int c = 0; c < 8; ++c) acc[i][c] += a[i] * b[c];
+        };
+#pragma unroll 2
+        for (int j = 0; j < 8 * ty; ++j) step(j, std::integral_constant<int, 0>{});
+        step(8 * ty, std::integral_constant<int, 0>{});
+        step(8 * ty + 1, std::integral_constant<int, 1>{});
+        step(8 * ty + 2, std::integral_constant<int, 2>{});
+        step(8 * ty + 3, std::integral_constant<int, 3>{});
+        step(8 * ty + 4, std::integral_constant<int, 4>{});
+        step(8 * ty + 5, std::integral_constant<int, 5>{});
+        step(8 * ty + 6, std::integral_constant<int, 6>{});
+        step(8 * ty + 7, std::integral_constant<int, 7>{});
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const int c = col0 + 64 * half + 4 * tx;
+            if (c >= N) continue;                          // N is a multiple of 4
+            if (values) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (8 * ty + i < n)
+                        *reinterpret_cast<float4*>(x_out + ((size_t)(lo + 8 * ty + i) * H + h) * dv + c) =
+                            make_float4(acc[i][4 * half], acc[i][4 * half + 1], acc[i][4 * half + 2], acc[i][4 * half + 3]);
+            } else {
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    float* dst = w_out + (((size_t)blockIdx.x * H + h) * d + c + m) * CH + 8 * ty;
+                    *reinterpret_cast<float4*>(dst) = make_float4(acc[0][4 * half + m], acc[1][4 * half + m], acc[2][4 * half + m], acc[3][4 * half + m]);
+                    *reinterpret_cast<float4*>(dst + 4) = make_float4(acc[4][4 * half + m], acc[5][4 * half + m], acc[6][4 * half + m], acc[7][4 * half + m]);
+                }
+            }
         }
     }
 }
@@ -317,14 +406,20 @@ extern "C" int rg_delta_chunk(const float* q, int q_ld, const float* k, int k_ld
     cudaStream_t s = (cudaStream_t)stream;
     dim3 g1(T / CH + R, H + Hqk);
     int e;
-    if (v_dtype == RG_DTYPE_F32)
-        e = rg_launch(delta_solve_kernel<float>, g1, dim3(NTH), 0, s, 1, q, q_ld, k, k_ld, (const float*)v, v_ld, beta, loga,
-                      cu_seqlens, R, u, w, factors, decays, dots, H, Hqk, d, dv);
-    else if (v_dtype == RG_DTYPE_BF16)
-        e = rg_launch(delta_solve_kernel<bf16>, g1, dim3(NTH), 0, s, 1, q, q_ld, k, k_ld, (const bf16*)v, v_ld, beta, loga,
-                      cu_seqlens, R, u, w, factors, decays, dots, H, Hqk, d, dv);
-    else
+    const bool q4 = q_ld % 4 == 0 && ((uintptr_t)q & 15) == 0 && v_ld % 4 == 0;
+#define DC_SOLVE(VEC_, V_) { \
+        const cudaError_t ce = cudaFuncSetAttribute(delta_solve_kernel<VEC_, V_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ds_smem()); \
+        if (ce != cudaSuccess) return (int)ce; \
+        e = rg_launch(delta_solve_kernel<VEC_, V_>, g1, dim3(MTH), ds_smem(), s, 1, q, q_ld, k, k_ld, (const V_*)v, v_ld, beta, loga, \
+                      cu_seqlens, R, u, w, factors, decays, dots, H, Hqk, d, dv); }
+    if (v_dtype == RG_DTYPE_F32) {
+        if (q4 && ((uintptr_t)v & 15) == 0) DC_SOLVE(true, float) else DC_SOLVE(false, float)
+    } else if (v_dtype == RG_DTYPE_BF16) {
+        if (q4 && ((uintptr_t)v & 7) == 0) DC_SOLVE(true, bf16) else DC_SOLVE(false, bf16)
+    } else {
         return RG_ERR_UNSUPPORTED;
+    }
+#undef DC_SOLVE
     if (e) return e;
     const size_t smem = ((size_t)2 * (d * DC_WP + CH * (d + 16) + CH * DC_CB + CH) + (d + CH) * DC_CB) * sizeof(float);
     cudaError_t ce = cudaFuncSetAttribute(delta_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
