@@ -1,6 +1,6 @@
-// Weight-streaming matrix product for decode batches of 17 to 64 rows on the 5th-generation tensor cores:
+// Weight-streaming matrix product for steps of 17 to 256 rows on the 5th-generation tensor cores:
 // y[M, N] = x[M, K] W[N, K]^T with the operands swapped, so that 128 rows of W fill the M side of tcgen05.mma
-// and the batch (padded to 64) its N side: D[128 weight rows, 64 tokens] accumulates in tensor memory while W
+// and the step's tokens (padded to 64, 128 or 256) its N side: D[128 weight rows, tokens] accumulates in tensor memory while W
 // streams through a ring of TMA stages exactly once.  At these sizes the product is bound by reading W, and a
 // product with few rows of W (q|k|v, O, down) has too few 128-row tiles to occupy the GPU, so K is split over the
 // CTAs of a thread-block cluster: every CTA accumulates its K range of the cluster's tile, leaves the partial sums
@@ -11,7 +11,8 @@
 // overlaps the next tile's loads.
 //
 // Roles as in gemm_tcgen05.cu: warps 0-3 epilogue (one lane of tensor memory = one row of W each), warp 4 the TMA
-// producer, warp 5 issues the MMAs and owns the tensor memory.  Epilogues: plain (bfloat16 or 32-bit out) and
+// producer, warp 5 issues the MMAs and owns the tensor memory; above 64 tokens warps 8-11 are a second epilogue group, since
+// an epilogue is a chain that one warp per scheduler walks at a quarter of its rate.  Epilogues: plain (bfloat16 or 32-bit out) and
 // SiLU-mul over interleaved gate|up rows (crates/vllm-models/src/llama/architecture.rs:81-85).  The reference runs
 // these products through cuBLAS (crates/vllm-models/src/llama/attention.rs:94-96,133).
 //
@@ -20,9 +21,9 @@
 #include "tcgen05.cuh"
 
 #define TS_ROWS 128               // rows of W per tile (the MMA's M)
-#define TS_TOK 64                 // tokens per tile (the MMA's N); fewer tokens are padded with zeros by TMA
+#define TS_CHUNK 64               // tokens that an unsplit tile's epilogue takes at a time
+#define TS_MAX_TOK 256            // tokens per tile (the MMA's N): 64, 128 or 256; fewer are padded with zeros by TMA
 #define TS_BK 64
-#define TS_THREADS 192
 #define TS_MAX_SPLITS 8
 #define TS_EPI_NONE 0
 #define TS_EPI_SILU_MUL 1
@@ -59,8 +60,9 @@ struct StreamFusion {
 
 __device__ __forceinline__ float4 ts_ld_remote4(uint32_t addr) {
     float4 v;
+    // (volatile: not before the cluster's barrier; no clobber, so that several are in flight between stores)
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
     return v;
 }
 
@@ -153,19 +155,45 @@ struct TileEpilogue {
     }
     // load4(r, i): partial sums i .. i + 3 of CTA r's [token][row] array; they are added in rank order, and all are requested
     // before the first is used.  inv: 1 / rms per token (TS_PRO_SCALED).
-    template <bool SPLIT, int PRO, typename OUT, typename Load>
+    template <bool SPLIT, bool FEW, int PRO, typename OUT, typename Load>
     __device__ __forceinline__ void write(Load load4, int splits, OUT* __restrict__ out, int ldo, int N, int n0, int tile,
                                           int m_lo, int m_hi, bool vec, const float* inv, const StreamFusion& fu) {
-        constexpr int MAXS = SPLIT ? TS_MAX_SPLITS : 1;
-        auto sum4 = [&](int i) -> float4 {
-            float4 p[MAXS];
+        // Four tokens' sums at row `at` of the tile.  A few tokens a thread (FEW): all CTAs' partial sums of one token in
+        // flight at a time; else three CTAs' of all four tokens (two at a time took o's eight splits of 64 rows from 6.8 to
+        // 10.1 us).
+        auto sums = [&](float4 (&v)[AHEAD], int mb, int at) {
+            auto place = [&](int u) { return min(mb + u * STEP, m_hi - 1) * TS_ROWS + at; };
+            auto add = [](float4& a, const float4& b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; };
+            if (!SPLIT || FEW) {
+                constexpr int MAXS = SPLIT ? TS_MAX_SPLITS : 1;
 #pragma unroll
-            for (int r = 0; r < MAXS; ++r) p[r] = r < splits ? load4(r, i) : make_float4(0.f, 0.f, 0.f, 0.f);
-            float4 v = p[0];
+                for (int u = 0; u < AHEAD; ++u) {
+                    if (mb + u * STEP >= m_hi) break;
+                    float4 p[MAXS];
 #pragma unroll
-            for (int r = 1; r < MAXS; ++r)
-                if (r < splits) { v.x += p[r].x; v.y += p[r].y; v.z += p[r].z; v.w += p[r].w; }
-            return v;
+                    for (int r = 0; r < MAXS; ++r) p[r] = r < splits ? load4(r, place(u)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    v[u] = p[0];
+#pragma unroll
+                    for (int r = 1; r < MAXS; ++r)
+                        if (r < splits) add(v[u], p[r]);
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < AHEAD; ++u) v[u] = load4(0, place(u));
+                for (int r0 = 1; r0 < splits; r0 += 3) {
+                    float4 p[3][AHEAD];
+#pragma unroll
+                    for (int r = 0; r < 3; ++r)
+#pragma unroll
+                        for (int u = 0; u < AHEAD; ++u)
+                            if (r0 + r < splits) p[r][u] = load4(r0 + r, place(u));
+#pragma unroll
+                    for (int r = 0; r < 3; ++r)
+#pragma unroll
+                        for (int u = 0; u < AHEAD; ++u)
+                            if (r0 + r < splits) add(v[u], p[r][u]);
+                }
+            }
         };
         float norm[4] = {0.f, 0.f, 0.f, 0.f};
         if constexpr (EPI == TS_EPI_RESIDUAL) {
@@ -177,16 +205,17 @@ struct TileEpilogue {
         for (int mb = m_lo + m_off; mb - m_off < m_hi; mb += AHEAD * STEP) {
             const TileEpilogue now = *this;
             fetch(mb + AHEAD * STEP, m_hi, n0, N, out, ldo, vec, fu);
+            float4 s0[AHEAD], s1[PAIRS ? AHEAD : 1];
+            sums(s0, mb, row);
+            if constexpr (PAIRS) sums(s1, mb, row + 8);
 #pragma unroll
             for (int u = 0; u < AHEAD; ++u) {
                 const int m = mb + u * STEP;
                 if (m >= m_hi) break;                                        // the same for a whole warp, but for PAIRS
-                const float4 s0 = sum4(m * TS_ROWS + row);
                 const float sc = PRO == TS_PRO_SCALED ? inv[m] : 1.f;
-                float a[4] = {s0.x * sc, s0.y * sc, s0.z * sc, s0.w * sc};
+                float a[4] = {s0[u].x * sc, s0[u].y * sc, s0[u].z * sc, s0[u].w * sc};
                 if constexpr (PAIRS) {
-                    const float4 s1 = sum4(m * TS_ROWS + row + 8);
-                    const float b[4] = {s1.x * sc, s1.y * sc, s1.z * sc, s1.w * sc};
+                    const float b[4] = {s1[u].x * sc, s1[u].y * sc, s1[u].z * sc, s1[u].w * sc};
                     if constexpr (EPI == TS_EPI_SILU_MUL) {
                         float y[4];
 #pragma unroll
@@ -241,28 +270,38 @@ struct TileEpilogue {
     }
 };
 
-// Stages of 24 KB.  Split products leave room for a second CTA on the SM, so that the next kernel's can fetch its weights
-// while this one's still run, and their partial sums take the stages' place.
-__host__ __device__ constexpr int ts_stages(bool split) { return split ? 4 : 6; }
-__host__ __device__ constexpr size_t ts_smem(bool split) {
-    return (size_t)ts_stages(split) * (TS_ROWS + TS_TOK) * TS_BK * 2 + (split ? 0 : TS_TOK * TS_ROWS * 4) +
-           8 * (2 * ts_stages(split) + 4) + 1024;
+// The 128 threads of an epilogue group.
+__device__ __forceinline__ void group_sync(int group) {
+    if (group) asm volatile("bar.sync 2, 128;" ::: "memory");
+    else asm volatile("bar.sync 1, 128;" ::: "memory");
 }
 
-template <bool SPLIT, int EPI, int PRO, typename OUT>
-__global__ void __launch_bounds__(TS_THREADS)
+// Stages.  Split products of up to 64 tokens leave room for a second CTA on the SM (four stages of 24 KB), so that the next
+// kernel's can fetch its weights while this one's still run; split products' partial sums take the stages' place.
+__host__ __device__ constexpr int ts_groups(int tok) { return tok > 64 ? 2 : 1; }
+__host__ __device__ constexpr int ts_threads(int tok) { return tok > 64 ? 384 : 192; }
+__host__ __device__ constexpr int ts_stages(bool split, int tok) {
+    return tok == 64 ? (split ? 4 : 6) : tok == 128 ? (split ? 6 : 4) : (split ? 4 : 3);
+}
+__host__ __device__ constexpr size_t ts_smem(bool split, int tok) {
+    return (size_t)ts_stages(split, tok) * (TS_ROWS + tok) * TS_BK * 2 + (split ? 0 : ts_groups(tok) * TS_CHUNK * TS_ROWS * 4) +
+           8 * (2 * ts_stages(split, tok) + 4) + 1024;
+}
+
+template <bool SPLIT, int TOK, int EPI, int PRO, typename OUT>
+__global__ void __launch_bounds__(ts_threads(TOK))
 tc_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                  OUT* __restrict__ out, int ldo, int M, int N, int K, int splits, int* err, const StreamFusion fu) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ float inv_rms[TS_TOK];
-    constexpr int STAGES = ts_stages(SPLIT);
-    constexpr uint32_t W_BYTES = TS_ROWS * TS_BK * 2, X_BYTES = TS_TOK * TS_BK * 2, STAGE_BYTES = W_BYTES + X_BYTES;
-    static_assert(!SPLIT || (uint32_t)TS_TOK * TS_ROWS * 4 <= STAGES * STAGE_BYTES, "the partial sums take the stages' place");
+    __shared__ float inv_rms[TOK];
+    constexpr int STAGES = ts_stages(SPLIT, TOK), GROUPS = ts_groups(TOK);
+    constexpr uint32_t W_BYTES = TS_ROWS * TS_BK * 2, X_BYTES = TOK * TS_BK * 2, STAGE_BYTES = W_BYTES + X_BYTES;
+    static_assert(!SPLIT || (uint32_t)TOK * TS_ROWS * 4 <= STAGES * STAGE_BYTES, "the partial sums take the stages' place");
     const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;          // swizzled tiles need 1024-byte alignment
     unsigned char* base_ptr = smem_raw + (base - smem_addr(smem_raw));
-    // [TS_TOK][TS_ROWS], over the stages or behind them
+    // [TOK][TS_ROWS] over the stages, or [TS_CHUNK][TS_ROWS] per epilogue group behind them
     float* part = reinterpret_cast<float*>(base_ptr + (SPLIT ? 0 : STAGES * STAGE_BYTES));
-    const uint32_t bars = base + STAGES * STAGE_BYTES + (SPLIT ? 0 : TS_TOK * TS_ROWS * 4);
+    const uint32_t bars = base + STAGES * STAGE_BYTES + (SPLIT ? 0 : GROUPS * TS_CHUNK * TS_ROWS * 4);
     auto full_bar = [&](int s) { return bars + 8u * s; };
     auto empty_bar = [&](int s) { return bars + 8u * (STAGES + s); };
     auto acc_full = [&](int b) { return bars + 8u * (2 * STAGES + b); };
@@ -279,8 +318,13 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     // split products: one tile per cluster; unsplit ones: tile after tile
     const int first_tile = SPLIT ? (int)(blockIdx.x / splits) : (int)blockIdx.x;
     const int tile_step = SPLIT ? n_tiles : (int)gridDim.x;
-    constexpr uint32_t TMEM_COLS = SPLIT ? TS_TOK : 2 * TS_TOK;
-    const int m_lo = SPLIT ? M * rank / splits : 0, m_hi = SPLIT ? M * (rank + 1) / splits : M;   // the tokens that this CTA writes
+    constexpr uint32_t TMEM_COLS = SPLIT ? TOK : 2 * TOK;
+    // The tokens that this thread's epilogue group writes: of a split tile the group's half of the CTA's share; of an unsplit one
+    // every GROUPS-th chunk, from its own on.
+    const int group = (int)threadIdx.x >> 8;
+    const int cta_lo = M * rank / splits, cta_hi = M * (rank + 1) / splits;
+    const int m_lo = SPLIT ? cta_lo + (cta_hi - cta_lo) * group / GROUPS : group * TS_CHUNK;
+    const int m_hi = SPLIT ? cta_lo + (cta_hi - cta_lo) * (group + 1) / GROUPS : min(M, (group + 1) * TS_CHUNK);
     // four numbers of the output at a time
     const bool vec = ldo % 4 == 0 && ((uintptr_t)out & (4 * sizeof(OUT) - 1)) == 0 && (((uintptr_t)fu.scaled_out | (uintptr_t)fu.kv_cache) & 7) == 0;
     TileEpilogue<EPI> epilogue((int)threadIdx.x & 127);
@@ -288,7 +332,7 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     if (threadIdx.x == 0) {
         abort_flag = 0;
         for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 4); }
+        for (int b = 0; b < 2; ++b) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 4 * GROUPS); }
         fence_barrier_init();
     }
     if (warp == 5) tmem_alloc(&tmem_base_slot, TMEM_COLS);
@@ -331,15 +375,15 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         pdl_trigger();
     }
     if (warp == 5 && lane == 0) {
-        // ---- MMA issue: D[128 x 64] (+)= W[128 x 16] x[64 x 16]^T, four K steps per stage
-        constexpr uint32_t idesc = make_idesc(TS_ROWS, TS_TOK, false);
+        // ---- MMA issue: D[128 x TOK] (+)= W[128 x 16] x[TOK x 16]^T, four K steps per stage
+        constexpr uint32_t idesc = make_idesc(TS_ROWS, TOK, false);
         int it = 0, local = 0;
         bool ok = true;
         for (int t = first_tile; t < n_tiles && ok; t += tile_step, ++local) {
             const int b = local & 1, u = local >> 1;
             if (u > 0 && !mbar_wait(acc_empty(b), (u & 1) ^ 1, err, 4, &abort_flag)) { ok = false; break; }
             tc_fence_after();
-            const uint32_t tmem_d = tmem_base + (uint32_t)(b * TS_TOK);
+            const uint32_t tmem_d = tmem_base + (uint32_t)(b * TOK);
             for (int kt = 0; kt < KT; ++kt, ++it) {
                 const int s = it % STAGES, r = it / STAGES;
                 if (!mbar_wait(full_bar(s), r & 1, err, 2, &abort_flag)) { ok = false; break; }
@@ -353,41 +397,62 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             }
             if (ok) tc_commit(acc_full(b));
         }
-    } else if (warp < 4) {
+    } else if ((warp & 7) < 4) {
         // ---- epilogue, first half: this warp's 32 rows of the accumulator into shared memory, token-major, so
         // that what follows reads and writes along rows of W
         int local = 0;
         bool ok = true;
-        if (PRO == TS_PRO_SCALED && threadIdx.x < M) {
-            // 1 / rms of every token from the producer's partial sums of squares, added in their order
-            float ssq = 0.f;
+        if (PRO == TS_PRO_SCALED) {
+            // 1 / rms of every token from the producer's partial sums of squares, added in their order (every group all of
+            // them: the same numbers, and no group waits for another)
+            for (int m = threadIdx.x & 127; m < M; m += 128) {
+                float ssq = 0.f;
 #pragma unroll 8
-            for (int p = 0; p < fu.ss_in_blocks; ++p) ssq += fu.ss_in[(size_t)p * fu.ss_ld + threadIdx.x];
-            inv_rms[threadIdx.x] = rsqrtf(ssq / (float)K + fu.eps);
+                for (int p = 0; p < fu.ss_in_blocks; ++p) ssq += fu.ss_in[(size_t)p * fu.ss_ld + m];
+                inv_rms[m] = rsqrtf(ssq / (float)K + fu.eps);
+            }
         }
         for (int t = first_tile; t < n_tiles && ok; t += tile_step, ++local) {
             const int b = local & 1, u = local >> 1;
             epilogue.fetch(m_lo + epilogue.m_off, m_hi, t * TS_ROWS, N, out, ldo, vec, fu);
             if (!mbar_wait(acc_full(b), u & 1, err, 3, &abort_flag)) { ok = false; break; }
             tc_fence_after();
-            const uint32_t tmem_d = tmem_base + (uint32_t)(b * TS_TOK) + ((uint32_t)(warp * 32) << 16);
-            if (!SPLIT && local > 0) asm volatile("bar.sync 1, 128;" ::: "memory");       // the tile before has been written out
+            const uint32_t tmem_d = tmem_base + (uint32_t)(b * TOK) + ((uint32_t)((warp & 3) * 32) << 16);
+            const int row_of = (warp & 3) * 32 + lane;
+            if (SPLIT) {
+                // this group's half of the tokens (the stages' copies have landed and been multiplied)
 #pragma unroll
-            for (int c = 0; c < TS_TOK / 32; ++c) {      // (split: the stages' copies have landed and been multiplied)
-                uint32_t v[32];
-                tc_ld32(tmem_d + (uint32_t)(c * 32), v);
+                for (int c = 0; c < TOK / (32 * GROUPS); ++c) {
+                    const int t0 = group * (TOK / GROUPS) + c * 32;
+                    if (t0 >= M) break;
+                    uint32_t v[32];
+                    tc_ld32(tmem_d + (uint32_t)t0, v);
 #pragma unroll
-                for (int i = 0; i < 32; ++i) part[(c * 32 + i) * TS_ROWS + warp * 32 + lane] = __uint_as_float(v[i]);
+                    for (int i = 0; i < 32; ++i) part[(t0 + i) * TS_ROWS + row_of] = __uint_as_float(v[i]);
+                }
+            } else {
+                float* mine = part + group * TS_CHUNK * TS_ROWS;
+                for (int m0 = group * TS_CHUNK; m0 < M; m0 += GROUPS * TS_CHUNK) {
+                    // what was there has been written out
+                    if (local > 0 || m0 >= GROUPS * TS_CHUNK) group_sync(group);
+#pragma unroll
+                    for (int c = 0; c < TS_CHUNK / 32; ++c) {
+                        uint32_t v[32];
+                        tc_ld32(tmem_d + (uint32_t)(m0 + c * 32), v);
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) mine[(c * 32 + i) * TS_ROWS + row_of] = __uint_as_float(v[i]);
+                    }
+                    // ---- second half, unsplit: the group's warps write the chunk out
+                    group_sync(group);
+                    const int m1 = min(M, m0 + TS_CHUNK);
+                    if (m0 >= GROUPS * TS_CHUNK) epilogue.fetch(m0 + epilogue.m_off, m1, t * TS_ROWS, N, out, ldo, vec, fu);
+                    auto load4 = [&](int, int i) { return *reinterpret_cast<const float4*>(mine + i - m0 * TS_ROWS); };
+                    epilogue.template write<false, false, PRO>(load4, 1, out, ldo, N, t * TS_ROWS, t, m0, m1, vec, inv_rms, fu);
+                }
             }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty(b));
-            if (!SPLIT) {
-                // ---- second half, unsplit: the four epilogue warps write the tile out
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                auto load4 = [&](int, int i) { return *reinterpret_cast<const float4*>(part + i); };
-                epilogue.template write<false, PRO>(load4, 1, out, ldo, N, t * TS_ROWS, t, 0, M, vec, inv_rms, fu);
-            }
         }
     }
     tc_fence_before();
@@ -398,12 +463,9 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         if (first_tile < n_tiles && !abort_flag) {
             const int n0 = first_tile * TS_ROWS;
             const uint32_t mine = smem_addr(part);
-            uint32_t peer[TS_MAX_SPLITS];
-#pragma unroll
-            for (int r = 0; r < TS_MAX_SPLITS; ++r) peer[r] = mapa_shared(mine, (uint32_t)min(r, splits - 1));
-            auto load4 = [&](int r, int i) { return ts_ld_remote4(peer[r] + (uint32_t)i * 4u); };
-            if (threadIdx.x < 128)
-                epilogue.template write<true, PRO>(load4, splits, out, ldo, N, n0, first_tile, m_lo, m_hi, vec, inv_rms, fu);
+            auto load4 = [&](int r, int i) { return ts_ld_remote4(mapa_shared(mine, (uint32_t)r) + (uint32_t)i * 4u); };
+            if ((warp & 7) < 4)
+                epilogue.template write<true, TOK == 64, PRO>(load4, splits, out, ldo, N, n0, first_tile, m_lo, m_hi, vec, inv_rms, fu);
         }
         cluster_sync_all();                                                 // nobody leaves while its partial sums are being read
     }
@@ -428,49 +490,62 @@ static int ts_num_sms() {
     return num_sms;
 }
 
-template <bool SPLIT, int EPI, int PRO, typename OUT>
+template <bool SPLIT, int TOK, int EPI, int PRO, typename OUT>
 static int launch_ts(const CUtensorMap& mw, const CUtensorMap& mx, OUT* out, int ldo, int M, int N, int K, int splits, int* err,
                      const StreamFusion& fu, cudaStream_t s) {
-    constexpr size_t smem = ts_smem(SPLIT);
-    auto kernel = tc_stream_kernel<SPLIT, EPI, PRO, OUT>;
+    constexpr size_t smem = ts_smem(SPLIT, TOK);
+    static_assert(smem <= 227 * 1024, "shared memory of a block");
+    auto kernel = tc_stream_kernel<SPLIT, TOK, EPI, PRO, OUT>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     const int n_tiles = (N + TS_ROWS - 1) / TS_ROWS;
     const int sms = ts_num_sms();
     const unsigned grid = SPLIT ? (unsigned)(n_tiles * splits) : (unsigned)(n_tiles < sms ? n_tiles : sms);
-    return rg_launch(kernel, dim3(grid), dim3(TS_THREADS), smem, s, splits, mw, mx, out, ldo, M, N, K, splits, err, fu);
+    return rg_launch(kernel, dim3(grid), dim3(ts_threads(TOK)), smem, s, splits, mw, mx, out, ldo, M, N, K, splits, err, fu);
 }
 
-static int ts_pick_splits(int splits, int N, int K) {
+static int ts_pick_splits(int splits, int N, int K, int M) {
     const int n_tiles = (N + TS_ROWS - 1) / TS_ROWS, kt = (K + TS_BK - 1) / TS_BK;
     if (splits == 0) {
         // As many CTAs per tile as keep the whole product in one wave of one CTA per SM, with at least four boxes of K each.
         // 64 rows by 2,048 x 2,048 / 2,048 x 8,192: 7.8 / 15.5 us with 4, 6.8 / 12.6 with 8; a second CTA per SM from one
         // product (16 splits' worth) only delays the product behind it (a 64-row step 1,281 against 1,333 us).
         splits = 1;
-        while (splits < TS_MAX_SPLITS && n_tiles * splits * 2 <= ts_num_sms() && kt >= splits * 4) splits *= 2;
+        // Above 64 rows a CTA fills an SM, and clusters of eight such start slowly (180 rows by 2,048 x 2,048: 11.5 us in
+        // four splits, 23.9 in eight).
+        const int most = M <= 64 ? TS_MAX_SPLITS : 4;
+        while (splits < most && n_tiles * splits * 2 <= ts_num_sms() && kt >= splits * 4) splits *= 2;
     }
     if ((splits != 1 && splits != 2 && splits != 4 && splits != 8) || kt < splits) return -1;
     return splits;
 }
 
+template <int TOK, int EPI, int PRO, typename OUT>
+static int dispatch_ts_tok(const void* x, int ldx, const CUtensorMap& mw, OUT* out, int ldo, int M, int N, int K, int splits,
+                           int* err, const StreamFusion& fu, cudaStream_t s) {
+    CUtensorMap mx;
+    const int e = rg_make_map(&mx, x, M, K, ldx, TOK);
+    if (e) return e;
+    return splits == 1 ? launch_ts<false, TOK, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, 1, err, fu, s)
+                       : launch_ts<true, TOK, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, splits, err, fu, s);
+}
+
 template <int EPI, int PRO, typename OUT>
 static int dispatch_ts(const void* x, int ldx, const void* W, OUT* out, int ldo, int M, int N, int K, int splits,
                        int* err, const StreamFusion& fu, cudaStream_t s) {
-    CUtensorMap mw, mx;
-    int e = rg_make_map(&mw, W, N, K, K, TS_ROWS);
+    CUtensorMap mw;
+    const int e = rg_make_map(&mw, W, N, K, K, TS_ROWS);
     if (e) return e;
-    e = rg_make_map(&mx, x, M, K, ldx, TS_TOK);
-    if (e) return e;
-    return splits == 1 ? launch_ts<false, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, 1, err, fu, s)
-                       : launch_ts<true, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, splits, err, fu, s);
+    return M <= 64 ? dispatch_ts_tok<64, EPI, PRO, OUT>(x, ldx, mw, out, ldo, M, N, K, splits, err, fu, s)
+         : M <= 128 ? dispatch_ts_tok<128, EPI, PRO, OUT>(x, ldx, mw, out, ldo, M, N, K, splits, err, fu, s)
+                    : dispatch_ts_tok<256, EPI, PRO, OUT>(x, ldx, mw, out, ldo, M, N, K, splits, err, fu, s);
 }
 
 static bool ts_operands_ok(const void* x, int ldx, const void* W, int M, int K) {
-    return M <= TS_TOK && K > 0 && K % 8 == 0 && ldx % 8 == 0 && !((uintptr_t)x & 15) && !((uintptr_t)W & 15);
+    return M <= TS_MAX_TOK && K > 0 && K % 8 == 0 && ldx % 8 == 0 && !((uintptr_t)x & 15) && !((uintptr_t)W & 15);
 }
 
-// y = x W^T for 1 <= M <= 64 rows of x (bfloat16, rows ldx elements apart), W [N, K] bfloat16 contiguous.
+// y = x W^T for 1 <= M <= 256 rows of x (bfloat16, rows ldx elements apart), W [N, K] bfloat16 contiguous.
 // out_dtype: RG_DTYPE_BF16 or RG_DTYPE_F32; epilogue 0 plain (out [M, N]) or 1 SiLU-mul over interleaved gate|up
 // rows (out [M, N / 2], bfloat16).  splits: 1, 2, 4 or 8 CTAs share a tile's K (K >= 64 x splits); 0 picks.
 // ss_in (may be null): x holds residual rows times a norm's weight and ss_in [ss_in_blocks, ss_ld] their partial
@@ -483,7 +558,7 @@ extern "C" int rg_tc_stream_gemm(const void* x, int ldx, const void* W, void* ou
     if (!ts_operands_ok(x, ldx, W, M, K)) return RG_ERR_UNSUPPORTED;
     if (epilogue == TS_EPI_SILU_MUL && (N % 16 || out_dtype != RG_DTYPE_BF16)) return RG_ERR_UNSUPPORTED;
     if (ss_in && (ss_in_blocks < 1 || ss_ld < M)) return RG_ERR_UNSUPPORTED;
-    splits = ts_pick_splits(splits, N, K);
+    splits = ts_pick_splits(splits, N, K, M);
     if (splits < 0) return RG_ERR_UNSUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
     StreamFusion fu = {};
@@ -498,7 +573,7 @@ extern "C" int rg_tc_stream_gemm(const void* x, int ldx, const void* W, void* ou
     return RG_ERR_UNSUPPORTED;
 }
 
-// The q|k|v projection of M single tokens with the rotary encoding and the cache write in the product's epilogue:
+// The q|k|v projection of M tokens with the rotary encoding and the cache write in the product's epilogue:
 // out [M, N] (bfloat16) receives the rotated q heads (its k and v columns are not written), k (rotated) and v go to
 // kv_cache at slots (null: no write).  W's q and k rows are in the paired8 order.  ss_in as in rg_tc_stream_gemm.
 extern "C" int rg_tc_stream_gemm_rope_cache(const void* x, int ldx, const void* W, void* out, int ldo, int M, int N, int K,
@@ -511,7 +586,7 @@ extern "C" int rg_tc_stream_gemm_rope_cache(const void* x, int ldx, const void* 
         !rope_table || !positions || max_pos < 1 || (slots && (!kv_cache || page_size < 1)) ||
         (ss_in && (ss_in_blocks < 1 || ss_ld < M)))
         return RG_ERR_UNSUPPORTED;
-    splits = ts_pick_splits(splits, N, K);
+    splits = ts_pick_splits(splits, N, K, M);
     if (splits < 0) return RG_ERR_UNSUPPORTED;
     StreamFusion fu = {};
     fu.ss_in = ss_in; fu.ss_in_blocks = ss_in_blocks; fu.ss_ld = ss_ld; fu.eps = eps;
@@ -531,7 +606,7 @@ extern "C" int rg_tc_stream_gemm_residual(const void* x, int ldx, const void* W,
     if (tiles_out) *tiles_out = (N + TS_ROWS - 1) / TS_ROWS;
     if (M <= 0 || N <= 0) return 0;
     if (!ts_operands_ok(x, ldx, W, M, K) || ss_ld < M || !ss_out || !norm_w) return RG_ERR_UNSUPPORTED;
-    splits = ts_pick_splits(splits, N, K);
+    splits = ts_pick_splits(splits, N, K, M);
     if (splits < 0) return RG_ERR_UNSUPPORTED;
     StreamFusion fu = {};
     fu.norm_w = norm_w; fu.scaled_out = (bf16*)scaled_out; fu.ss_out = ss_out; fu.ss_ld = ss_ld;

@@ -1780,12 +1780,13 @@ class NormedRows:
 class PendingLinear:
     """A part's output x W^T, not computed yet: a norm that follows adds it to
     the residual inside the product's own kernel; ``materialize()`` runs the
-    product."""
+    product.  ``max_rows``: up to how many rows the step takes the streaming
+    product for that (None: ``TC_STREAM_AUTO_ROWS``)."""
 
-    __slots__ = ("x", "weight")
+    __slots__ = ("x", "weight", "max_rows")
 
-    def __init__(self, x, weight):
-        self.x, self.weight = x, weight
+    def __init__(self, x, weight, max_rows=None):
+        self.x, self.weight, self.max_rows = x, weight, max_rows
 
     @property
     def shape(self):
@@ -2169,21 +2170,37 @@ def tc_gemm(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, silu_mul: boo
 
 
 TC_STREAM_MAX_ROWS = 64
-# From 17 rows up to here a decode batch's layer products go through the streaming tcgen05 product with the
-# neighbouring operations in its epilogues (residual addition, RMSNorm, rotation and cache write, SiLU-mul).  Alone
-# the product is level with the library's; the step gains what the separate small kernels cost (measured at
-# 1,024-token contexts: 10 % at batch 24, 6 % at 48, 3 % at 64).  RAILGUN_B200_TC_STREAM_ROWS overrides (16: off).
-TC_STREAM_AUTO_ROWS = int(os.environ.get("RAILGUN_B200_TC_STREAM_ROWS", "64"))
+# What the kernel takes.  Plain products above 64 rows are the library's; a step's layer products with the neighbouring
+# operations in their epilogues (residual addition, RMSNorm, rotation and cache write, SiLU-mul) go through this one from 17
+# rows up to what tc_stream_rows says.  Decode batches: up to TC_STREAM_AUTO_ROWS (RAILGUN_B200_TC_STREAM_ROWS; 16: off);
+# they are replayed from graphs, and above 64 rows the library's products are faster on the GPU (100 rows of a 1B-sized
+# layer: about 53 us for the four products here, 47 there with the kernels between them).  Steps that hold prompts and have
+# under 256 tokens are launched one kernel at a time and bound by the host: five launches a layer instead of nine, none of
+# them the library's (15 us of host time each), take one prompt of 100 tokens through a 1B-sized model in 1.50 ms instead
+# of 1.84 and 16 requests with one of 64 tokens through six 3B-sized layers in 0.95 instead of 1.24.  120 rows of width
+# 4,096 are level (0.71 and 0.72 ms) and 250 slower (0.88 and 0.83: the GPU is the bound there), hence the limit on rows
+# times width.
+TC_STREAM_STEP_ROWS = 256
+TC_STREAM_PROMPT_ROWS, TC_STREAM_PROMPT_NUMBERS = 255, 512 * 1024
+TC_STREAM_AUTO_ROWS = min(int(os.environ.get("RAILGUN_B200_TC_STREAM_ROWS", "64")), TC_STREAM_STEP_ROWS)
 
 
-def tc_stream_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
-    """Can the weight-streaming tcgen05 product (up to 64 rows of x) take these operands?"""
-    return 0 < x.shape[0] <= TC_STREAM_MAX_ROWS and tc_gemm_ok(x, weight)
+def tc_stream_rows(batch, width: int) -> int:
+    """Up to how many rows of this width a step's layer products go through the streaming product (``batch`` None: rows that
+    belong to no step)."""
+    if batch is None or batch.decode_only or TC_STREAM_AUTO_ROWS < TC_STREAM_MAX_ROWS:
+        return TC_STREAM_AUTO_ROWS
+    return max(TC_STREAM_AUTO_ROWS, min(TC_STREAM_PROMPT_ROWS, TC_STREAM_PROMPT_NUMBERS // width))
+
+
+def tc_stream_ok(x: torch.Tensor, weight: torch.Tensor, max_rows: int = TC_STREAM_MAX_ROWS) -> bool:
+    """Can the weight-streaming tcgen05 product (up to ``max_rows`` rows of x) take these operands?"""
+    return 0 < x.shape[0] <= min(max_rows, TC_STREAM_STEP_ROWS) and tc_gemm_ok(x, weight)
 
 
 def tc_stream_gemm(x, weight: torch.Tensor, out_dtype=None, silu_mul: bool = False, splits: int = 0,
-                   check: bool = False) -> torch.Tensor:
-    """y = x W^T for up to 64 rows of x on the tcgen05 tensor cores with the operands swapped: 128 rows of W per
+                   check: bool = False, max_rows: int = TC_STREAM_MAX_ROWS) -> torch.Tensor:
+    """y = x W^T for up to ``max_rows`` (at most 256) rows of x on the tcgen05 tensor cores with the operands swapped: 128 rows of W per
     tile stream through once, the rows of x are the narrow side.  ``silu_mul``: W is interleaved gate|up storage
     and y = silu(gate) * up.  ``splits``: 1, 2, 4 or 8 CTAs of a cluster share a tile's K and add their partial
     sums in rank order (0: as many as keep the product in one wave).  A row's result does not depend on the other
@@ -2193,9 +2210,9 @@ def tc_stream_gemm(x, weight: torch.Tensor, out_dtype=None, silu_mul: bool = Fal
     rows = x if isinstance(x, NormedRows) else None
     if rows is not None:
         x = rows.scaled
-    if not tc_stream_ok(x, weight):
+    if not tc_stream_ok(x, weight, max_rows):
         raise KernelError(f"tc_stream_gemm refuses x {tuple(x.shape)} {x.dtype} stride {x.stride()}, "
-                          f"W {tuple(weight.shape)} {weight.dtype}: bfloat16, at most 64 rows, K a multiple of 8")
+                          f"W {tuple(weight.shape)} {weight.dtype}: bfloat16, at most {max_rows} rows, K a multiple of 8")
     M, K = x.shape
     N = weight.shape[0]
     if weight.shape[1] != K:
@@ -2222,25 +2239,25 @@ def tc_stream_gemm(x, weight: torch.Tensor, out_dtype=None, silu_mul: bool = Fal
     return out
 
 
-def tc_stream_rope_ok(x, weight: torch.Tensor, d: int) -> bool:
-    """Can the q|k|v projection of these rows (17 to 64 of them) rotate and write the cache in the streaming
+def tc_stream_rope_ok(x, weight: torch.Tensor, d: int, max_rows: int | None = None) -> bool:
+    """Can the q|k|v projection of these rows (17 to ``max_rows`` of them, default ``TC_STREAM_AUTO_ROWS``) rotate and write the cache in the streaming
     tcgen05 product's own kernel?"""
     if d % 16:
         return False
     if isinstance(x, NormedRows):
         return tc_stream_scaled_ok(x, weight)
-    return SKINNY_AUTO_ROWS < x.shape[0] <= TC_STREAM_AUTO_ROWS and tc_stream_ok(x, weight)
+    return SKINNY_AUTO_ROWS < x.shape[0] <= (max_rows or TC_STREAM_AUTO_ROWS) and tc_stream_ok(x, weight, TC_STREAM_STEP_ROWS)
 
 
 def tc_stream_gemm_rope_cache(x, weight: torch.Tensor, table: torch.Tensor, positions: torch.Tensor, slots, kv_cache,
                               nh: int, nkv: int, d: int, err_flag=None, splits: int = 0) -> torch.Tensor:
-    """``skinny_gemm_rope_cache`` for up to 64 rows: the q|k|v projection with the rotary encoding and the cache
+    """``skinny_gemm_rope_cache`` for up to 256 rows: the q|k|v projection with the rotary encoding and the cache
     write in the product's epilogue.  Returns [M, (nh+2nkv)d] whose q heads are rotated (its k and v columns are
     not written); k (rotated) and v go to ``kv_cache`` at ``slots`` (None: no write).  ``x``: bfloat16 rows or a
     ``NormedRows``; ``weight``'s q and k rows are in ``rope_pair_order``."""
     rows = x if isinstance(x, NormedRows) else None
     xin = rows.scaled if rows is not None else x
-    if d % 16 or not tc_stream_ok(xin, weight):
+    if d % 16 or not tc_stream_ok(xin, weight, TC_STREAM_STEP_ROWS):
         raise KernelError(f"tc_stream_gemm_rope_cache refuses rows {tuple(xin.shape)}, W {tuple(weight.shape)}, head size {d}")
     M, K = xin.shape
     N = weight.shape[0]
@@ -2273,10 +2290,10 @@ def tc_stream_gemm_rope_cache(x, weight: torch.Tensor, table: torch.Tensor, posi
     return out
 
 
-def tc_stream_fused_ok(x: torch.Tensor, weight: torch.Tensor, resid: torch.Tensor) -> bool:
+def tc_stream_fused_ok(x: torch.Tensor, weight: torch.Tensor, resid: torch.Tensor, max_rows: int | None = None) -> bool:
     """Can x W^T be added to ``resid`` inside the streaming tcgen05 product (which then also prepares the next
-    norm)?  Decode batches above the skinny product's and up to ``TC_STREAM_AUTO_ROWS`` rows."""
-    return (SKINNY_AUTO_ROWS < x.shape[0] <= TC_STREAM_AUTO_ROWS and tc_stream_ok(x, weight)
+    norm)?  Steps above the skinny product's and up to ``max_rows`` (default ``TC_STREAM_AUTO_ROWS``)."""
+    return (SKINNY_AUTO_ROWS < x.shape[0] <= (max_rows or TC_STREAM_AUTO_ROWS) and tc_stream_ok(x, weight, TC_STREAM_STEP_ROWS)
             and resid.dtype == torch.float32 and resid.is_contiguous() and resid.shape == (x.shape[0], weight.shape[0])
             and resid.shape[1] % 8 == 0)
 
@@ -2284,8 +2301,8 @@ def tc_stream_fused_ok(x: torch.Tensor, weight: torch.Tensor, resid: torch.Tenso
 def tc_stream_gemm_residual(x: torch.Tensor, weight: torch.Tensor, resid: torch.Tensor, norm_weight: torch.Tensor,
                             eps: float, splits: int = 0) -> NormedRows:
     """resid += x W^T (32-bit, in place), and the RMSNorm (``norm_weight``, ``eps``) of the new rows but for the
-    factor 1 / rms, which the product that reads the result applies (``skinny_gemm_residual`` for 17 to 64 rows)."""
-    if not tc_stream_ok(x, weight):
+    factor 1 / rms, which the product that reads the result applies (``skinny_gemm_residual`` for up to 256 rows)."""
+    if not tc_stream_ok(x, weight, TC_STREAM_STEP_ROWS):
         raise KernelError(f"tc_stream_gemm_residual refuses x {tuple(x.shape)} {x.dtype}, W {tuple(weight.shape)}")
     _check(resid, "resid", torch.float32)
     _check(norm_weight, "norm_weight", torch.float32)
@@ -2294,7 +2311,7 @@ def tc_stream_gemm_residual(x: torch.Tensor, weight: torch.Tensor, resid: torch.
     if weight.shape[1] != K or resid.shape != (M, N) or norm_weight.numel() != N:
         raise KernelError(f"tc_stream_gemm_residual: x {tuple(x.shape)}, W {tuple(weight.shape)}, residual "
                           f"{tuple(resid.shape)}, norm weight {norm_weight.numel()}")
-    partials = torch.empty((-(-N // 128), TC_STREAM_MAX_ROWS), dtype=torch.float32, device=x.device)
+    partials = torch.empty((-(-N // 128), TC_STREAM_MAX_ROWS if M <= TC_STREAM_MAX_ROWS else TC_STREAM_STEP_ROWS), dtype=torch.float32, device=x.device)
     scaled = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
     err = _tc_err.get(x.device)
     if err is None:
@@ -2310,8 +2327,8 @@ def tc_stream_gemm_residual(x: torch.Tensor, weight: torch.Tensor, resid: torch.
 
 
 def tc_stream_scaled_ok(rows: NormedRows, weight: torch.Tensor) -> bool:
-    return (rows.dtype == torch.bfloat16 and SKINNY_AUTO_ROWS < rows.shape[0] <= TC_STREAM_AUTO_ROWS
-            and tc_stream_ok(rows.scaled, weight) and rows.shape[1] == weight.shape[1])
+    return (rows.dtype == torch.bfloat16 and SKINNY_AUTO_ROWS < rows.shape[0] <= max(TC_STREAM_AUTO_ROWS, TC_STREAM_PROMPT_ROWS)
+            and tc_stream_ok(rows.scaled, weight, TC_STREAM_STEP_ROWS) and rows.shape[1] == weight.shape[1])
 
 
 _tc_unchecked = False
@@ -2524,7 +2541,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, bias: torch.Te
         if (out_dtype is None or out_dtype == torch.bfloat16) and skinny_scaled_ok(x, weight):
             return skinny_gemm_scaled(x, weight)              # the norm is finished inside the product
         if tc_stream_scaled_ok(x, weight):
-            return tc_stream_gemm(x, weight, out_dtype)      # likewise, for 17 to 64 rows
+            return tc_stream_gemm(x, weight, out_dtype, max_rows=TC_STREAM_STEP_ROWS)      # likewise, for more rows
         x = x.materialize()
     if not x.is_cuda:
         raise KernelError("linear: CUDA tensors only (there is no CPU path)")

@@ -86,13 +86,15 @@ class PagedAttention(Mixer):
     def forward(self, x, batch, cache, writes=True, defer=False):
         nh, nkv, d = self.nh, self.nkv, self.d
         slots = batch.slot_mapping[cache.group]
+        stream = ops.tc_stream_rows(batch, self.w_o.shape[0])
         if self.paired8 and self.env.dtype == torch.bfloat16 and ops.skinny_rope_ok(x, self.w_qkv, d):
             # a few single tokens: projection, rotation and cache write in one kernel
             qkv = ops.skinny_gemm_rope_cache(x, self.w_qkv, self.position.rotary_table, batch.positions,
                                              slots if writes else None, cache.kv, nh, nkv, d, batch.err_flag)
-        elif (self.paired8 and self.env.dtype == torch.bfloat16 and batch.decode_only
-              and ops.tc_stream_rope_ok(x, self.w_qkv, d)):
-            # 17 to 64 single tokens: the same in the streaming tcgen05 product
+        elif (self.paired8 and self.env.dtype == torch.bfloat16 and (batch.decode_only or x.shape[0] > ops.TC_STREAM_MAX_ROWS)
+              and ops.tc_stream_rope_ok(x, self.w_qkv, d, stream)):
+            # 17 to 64 single tokens, or a step of more with prompts: the same in the streaming tcgen05 product.  (Up to 64
+            # tokens with prompts q and k are rounded once more, before their rotation, as they always were.)
             qkv = ops.tc_stream_gemm_rope_cache(x, self.w_qkv, self.position.rotary_table, batch.positions,
                                                 slots if writes else None, cache.kv, nh, nkv, d, batch.err_flag)
         else:
@@ -108,7 +110,7 @@ class PagedAttention(Mixer):
                 ops.rope_cache_write(qkv, None, batch.positions, slots, cache.kv, nh, nkv, d, cache.page_size,
                                      batch.err_flag)
         out = self.attend(qkv, batch, cache)
-        return ops.PendingLinear(out, self.w_o) if defer else ops.linear(out, self.w_o)
+        return ops.PendingLinear(out, self.w_o, stream) if defer else ops.linear(out, self.w_o)
 
     def attend(self, qkv, batch, cache):
         """Pick the attention kernels for this step's shape and precision:

@@ -1,0 +1,100 @@
+"""The streaming tcgen05 product at 65 to 256 rows (a step that holds short prompts), with the neighbouring operations in its
+epilogues, where it can go wrong: token tiles of 64, 128 and 256, chunks of 64 of them, splits of K, ragged rows of W."""
+import pytest
+import torch
+
+from test_kernels_gpu import DEV, rel_err
+
+pytestmark = pytest.mark.gpu
+F32 = 2e-5                  # 32-bit accumulation over all of K (as the tests of up to 64 rows)
+BF16 = 1e-2                 # one rounding to bfloat16, 2^-9, on values of any size
+
+
+def rows_of(M, H, K, splits, seed, eps=1e-3):
+    from railgun_b200 import ops
+    g = torch.Generator().manual_seed(seed)
+    x = torch.randn(M, K, generator=g).to(torch.bfloat16).to(DEV)
+    w = (torch.randn(H, K, generator=g) / K ** 0.5).to(torch.bfloat16).to(DEV)
+    resid0 = (torch.randn(M, H, generator=g) * 3).to(DEV)
+    nw = (torch.rand(H, generator=g) + 0.5).to(DEV)
+    resid = resid0.clone()
+    rows = ops.tc_stream_gemm_residual(x, w, resid, nw, eps, splits=splits)
+    ops.tc_gemm_check()
+    ref = resid0.double() + x.double() @ w.double().T
+    return g, x, w, resid0, nw, resid, rows, ref, ref * torch.rsqrt((ref ** 2).mean(1, keepdim=True) + eps) * nw.double()
+
+
+@pytest.mark.parametrize("splits", [0, 1, 2, 8])
+@pytest.mark.parametrize("M,H,K", [(65, 200, 520), (128, 2048, 2048), (129, 1000, 1096), (191, 2048, 8192), (256, 3080, 520)])
+def test_residual_then_scaled(M, H, K, splits):
+    from railgun_b200 import ops
+    g, x, w, resid0, nw, resid, rows, ref, normed = rows_of(M, H, K, splits, M + H + K)
+    assert rel_err(resid, ref) < F32
+    assert torch.equal(rows.scaled, (resid * nw).to(torch.bfloat16))           # one rounding, of the 32-bit product
+    assert rel_err(rows.partials[:rows.blocks, :M].double().sum(0), (resid.double() ** 2).sum(1)) < 1e-6
+    alone = resid0[M - 1:].clone()                                              # a row does not depend on its batch
+    ops.tc_stream_gemm_residual(x[M - 1:].contiguous(), w, alone, nw, 1e-3, splits=splits)
+    assert splits == 0 or torch.equal(alone[0], resid[M - 1])                   # (the choice of splits may follow the rows)
+    for N2, silu in ((136, False), (1008, True), (3072, False)):
+        w2 = (torch.randn(N2, H, generator=g) / H ** 0.5).to(torch.bfloat16).to(DEV)
+        assert ops.tc_stream_scaled_ok(rows, w2) == (M < 256)
+        y = ops.tc_stream_gemm(rows, w2, silu_mul=silu, splits=splits if -(-H // 64) >= splits else 0, max_rows=256)
+        ops.tc_gemm_check()
+        z = normed @ w2.double().T
+        if silu:
+            z = z.view(M, N2 // 16, 2, 8)
+            z = (z[:, :, 0] / (1 + torch.exp(-z[:, :, 0])) * z[:, :, 1]).reshape(M, N2 // 2)
+        assert rel_err(y, z) < BF16
+        if not silu and M < 256:
+            assert rel_err(ops.linear(rows, w2), z) < BF16
+
+
+@pytest.mark.parametrize("M", [17, 65, 130, 256])
+@pytest.mark.parametrize("nh,nkv,d,K,page", [(4, 2, 64, 256, 16), (6, 3, 48, 136, 8), (24, 8, 128, 1024, 32)])
+def test_rotation_and_cache_write(M, nh, nkv, d, K, page):
+    """Positions may repeat (portions of several requests); a token without a slot is not stored."""
+    from railgun_b200 import ops
+    from railgun_b200.parts.rope import rope_table
+    g, *_, rows, _, _ = rows_of(M, K, 64, 0, M + d)
+    N, NP, max_pos = (nh + 2 * nkv) * d, 40, 300
+    table = rope_table(d, 500000.0, None, max_pos).to(DEV)
+    w = (torch.randn(N, K, generator=g) / K ** 0.5).to(torch.bfloat16).to(DEV)
+    positions = torch.randint(0, max_pos, (M,), generator=g, dtype=torch.int32).to(DEV)
+    slots = torch.randperm(NP * page, generator=g)[:M].to(torch.int32)
+    slots[1] = -1
+    slots = slots.to(DEV)
+    for x in (torch.randn(M, K, generator=g).to(torch.bfloat16).to(DEV), rows):
+        assert ops.tc_stream_rope_ok(x, w, d, 256) == (x is not rows or M < 256)
+        kv_f = torch.zeros(NP, 2, nkv, page, d, dtype=torch.bfloat16, device=DEV)
+        kv_u = torch.zeros_like(kv_f)
+        fused = ops.tc_stream_gemm_rope_cache(x, w, table, positions, slots, kv_f, nh, nkv, d)
+        ops.tc_gemm_check()
+        plain = ops.tc_stream_gemm(x, w, max_rows=256, check=True)
+        ops.rope_cache_write(plain, table, positions, slots, kv_u, nh, nkv, d, page, paired8=True)
+        # the unfused route rounds the projection to bfloat16 before it rotates: equal within that rounding
+        assert rel_err(fused[:, :nh * d], plain[:, :nh * d].double()) < BF16 and rel_err(kv_f, kv_u.double()) < BF16
+        assert torch.equal(kv_f != 0, kv_u != 0)
+
+
+def test_a_position_outside_the_table_is_flagged_and_too_many_rows_are_refused():
+    from railgun_b200 import ops
+    from railgun_b200.parts.rope import rope_table
+    table = rope_table(64, 1e4, None, 8).to(DEV)
+    x, w = torch.ones(70, 64, dtype=torch.bfloat16, device=DEV), torch.ones(192, 64, dtype=torch.bfloat16, device=DEV)
+    positions = torch.full((70,), 3, dtype=torch.int32, device=DEV)
+    flag = torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.tc_stream_gemm_rope_cache(x, w, table, positions, None, None, 1, 1, 64, flag)
+    assert int(flag) == 0
+    positions[69] = 8
+    ops.tc_stream_gemm_rope_cache(x, w, table, positions, None, None, 1, 1, 64, flag)
+    assert int(flag) == 1
+    with pytest.raises(ops.KernelError):
+        ops.tc_stream_gemm(torch.zeros(257, 64, dtype=torch.bfloat16, device=DEV), w, max_rows=1000)
+
+
+def test_which_steps_take_it():
+    """Decode batches up to 64 rows (they are replayed from graphs); steps with prompts up to 255 of a small width."""
+    from types import SimpleNamespace as Batch
+    from railgun_b200 import ops
+    assert ops.tc_stream_rows(Batch(decode_only=True), 2048) == ops.tc_stream_rows(None, 2048) == 64
+    assert [ops.tc_stream_rows(Batch(decode_only=False), w) for w in (64, 2048, 3072, 4096, 16384)] == [255, 255, 170, 128, 64]
