@@ -23,7 +23,9 @@ convolution per channel over the request's tokens, instead of h.
 Between steps a request keeps, in its state slot and in 32-bit: S of every
 head (transposed, [dv, d]), and the last taps - 1 inputs of every
 convolution.  Everything from the projections' outputs to the rounding
-before the output product is 32-bit.
+before the output product is 32-bit.  The recurrences of retention and of the
+delta rule run token by token, or in chunks of 64 tokens side by side once a
+portion is long (the delta rule's where its sizes allow it).
 """
 from __future__ import annotations
 
