@@ -8,12 +8,9 @@ The reference's counterpart is execute_model_step -> forward_packed
 crates/vllm-models/src/llama/architecture.rs:141-156).
 
 How a step reaches the GPU: steps of single tokens replay a CUDA graph over a
-static batch (``decode_step_flat``; the graph chooses the tokens and copies
-them out; its inputs are copied in ahead of it from one of two host buffers in
-turn, so that a step whose tokens are given is packed and launched while the
-one before it runs: 20 us of a step in which the GPU waited for the host), and
-the step after such a step can be launched before its tokens are known
-(``decode_follow``); large steps whose
+static batch (``decode_step_flat``; the graph copies its inputs in, chooses
+the tokens and copies them out), and the step after such a step can be
+launched before its tokens are known (``decode_follow``); large steps whose
 packed layout repeats replay a graph captured for that layout
 (``_step_shape_graph``); everything else launches its kernels one by one.
 """
@@ -128,10 +125,9 @@ def _bucket(n: int, buckets) -> int:
 
 class StaticDecodeBatch:
     """Device buffers of fixed address for decode steps of up to ``B`` requests
-    whose contexts stay within ``MB`` pages, with two pinned host buffers that
-    are copied into them in turn, each in one transfer: a step can be packed
-    and launched while the step before it runs.  A graph captured over the
-    device buffers can be replayed for any such step.  Layout (int32): token ids | positions |
+    whose contexts stay within ``MB`` pages, with the pinned host buffer that
+    is copied into them in one transfer.  A graph captured over these buffers
+    can be replayed for any such step.  Layout (int32): token ids | positions |
     context lengths | start positions | state slots | per group slot mapping |
     per group block table [B, MB] | the rows' sampling parameters (seed and
     draw counter as 64-bit, temperature, top-k, top-p)."""
@@ -142,10 +138,8 @@ class StaticDecodeBatch:
         self.B, self.MB, self.G = B, MB, G
         self.sampling_off = -(-((5 + G) * B + G * B * MB) // 2) * 2          # even: 64-bit values start there
         n_ints = self.sampling_off + 7 * B
-        self.hosts = [torch.zeros(n_ints, dtype=torch.int32, pin_memory=True) for _ in range(2)]
-        self.hosts_np = [h.numpy() for h in self.hosts]
-        self.copied = [None, None]     # per host buffer: an event after its last copy
-        self.turn = 0
+        self.host = torch.zeros(n_ints, dtype=torch.int32, pin_memory=True)
+        self.host_np = self.host.numpy()
         # the step's tokens and, behind them, the flag that a kernel raises for a position outside its table:
         # one copy by the graph brings both to the host
         self.host_out = torch.zeros(B + 1, dtype=torch.int32, pin_memory=True)
@@ -168,7 +162,7 @@ class StaticDecodeBatch:
         self.sampled = self.out_dev[:B]                                         # the tokens the last step chose
         self.step_graphs = {}          # with sampling parameters or greedy -> CapturedStep
         self.follow = [None, None]     # FollowStep: the same step fed with ``sampled`` instead of host tokens
-        self.in_flight = None          # an event after the last replay, which writes ``host_out``
+        self.in_flight = None          # an event after the last replay that reads ``host`` and writes ``host_out``
 
     def raise_if_flagged(self, host_out_np) -> None:
         code = int(host_out_np[self.B])
@@ -177,22 +171,14 @@ class StaticDecodeBatch:
             host_out_np[self.B] = 0
             raise_device_error(code)
 
-    def next_buffer(self) -> int:
-        """The host buffer whose turn it is; it may be written once its last copy has run."""
-        self.turn ^= 1
-        event = self.copied[self.turn]
-        if event is not None and not event.query():
-            event.synchronize()
-        return self.turn
+    def wait_until_reusable(self) -> None:
+        """The pinned buffers may be written again once the last replay that copies them has run."""
+        if self.in_flight is not None and not self.in_flight.query():
+            self.in_flight.synchronize()
 
-    def upload(self, k: int) -> None:
-        """Copy host buffer ``k`` to the device, behind the last replay on whatever stream that was."""
-        if self.in_flight is not None:
-            torch.cuda.current_stream().wait_event(self.in_flight)
-        self.dev.copy_(self.hosts[k], non_blocking=True)
-        if self.copied[k] is None:
-            self.copied[k] = torch.cuda.Event()
-        self.copied[k].record()
+    def upload(self) -> int:
+        self.dev.copy_(self.host, non_blocking=True)
+        return self.host.numel() * 4
 
 
 def sampling_views(buf, off: int, B: int) -> dict:
@@ -213,7 +199,7 @@ class FollowStep:
 
     def __init__(self, static: StaticDecodeBatch):
         self.static = static
-        self.host_in = torch.zeros(static.dev.numel(), dtype=torch.int32, pin_memory=True)
+        self.host_in = torch.zeros(static.host.numel(), dtype=torch.int32, pin_memory=True)
         self.host_in_np = self.host_in.numpy()
         self.host_out = torch.zeros(static.B + 1, dtype=torch.int32, pin_memory=True)
         self.host_out_np = self.host_out.numpy()
@@ -404,12 +390,12 @@ class ModelRunner:
 
     def _capture(self, static: StaticDecodeBatch, follow: FollowStep | None = None,
                  sampling: bool = False) -> CapturedStep:
-        """Capture one decode step over the static buffers, into which its packed
-        inputs have been copied: the forward pass, the choice of the tokens and
-        their copy to pinned memory, so that a copy, a graph launch and a wait
-        are all the host does.  With ``follow`` the step takes its token ids
-        from the step before it on the device and everything else from
-        ``follow``'s pinned buffer, whose copy is part of the graph.  With ``sampling`` the tokens are drawn with
+        """Capture one decode step over the static buffers: the copy of its
+        packed inputs from pinned memory, the forward pass, the choice of the
+        tokens and their copy to pinned memory, so that one graph launch and one
+        wait are all the host does.  With ``follow`` the step takes its token
+        ids from the step before it on the device and everything else from
+        ``follow``'s pinned buffer.  With ``sampling`` the tokens are drawn with
         the rows' parameters in the static buffer (temperature 0: greedy)
         instead of the plain argmax.
 
@@ -425,6 +411,8 @@ class ModelRunner:
         def body():
             if follow is not None:
                 static.dev[B:].copy_(follow.host_in[B:], non_blocking=True)
+            else:
+                static.dev.copy_(static.host, non_blocking=True)
             # a following step reads its token ids where the step before left its greedy tokens
             batch = static.batch if follow is None else dataclasses.replace(static.batch, token_ids=static.sampled)
             logits = self.model.forward(batch, self.views)
@@ -473,11 +461,10 @@ class ModelRunner:
         ctx = max(self._ctx_hint + 1, 1)
         while True:
             static = self._static_for(R, ctx)
-            k = static.next_buffer()
-            host_np = static.hosts_np[k]
+            static.wait_until_reusable()
             try:
-                sampled = self.alloc.pack_decode(ids, static.B, static.MB, host_np[static.B:],
-                                                 sampling=host_np[static.sampling_off:])
+                sampled = self.alloc.pack_decode(ids, static.B, static.MB, static.host_np[static.B:],
+                                                 sampling=static.host_np[static.sampling_off:])
                 break
             except CacheError as e:
                 if "bad argument" in str(e) and ctx < self.model.spec.max_position:
@@ -485,21 +472,20 @@ class ModelRunner:
                     continue
                 raise
         B = static.B
-        self._ctx_hint = int(host_np[2 * B:2 * B + R].max())
+        self._ctx_hint = int(static.host_np[2 * B:2 * B + R].max())
         if self._ctx_hint > self.model.spec.max_position:
             raise BatchError(f"position {self._ctx_hint - 1} is beyond the model's max_position_embeddings "
                              f"{self.model.spec.max_position}")
-        host_np[:R] = tokens
-        host_np[R:B] = 0
-        static.upload(k)
-        self.last_h2d_bytes = static.dev.numel() * 4
+        static.host_np[:R] = tokens
+        static.host_np[R:B] = 0
+        self.last_h2d_bytes = static.host.numel() * 4
         key = sampled
         logits = None
         if key not in static.step_graphs:
             static.step_graphs[key], logits = self._capture(static, sampling=key)   # runs this step and captures it
         cap = static.step_graphs[key]
         if logits is None:
-            cap.graph.replay()                              # the step, greedy tokens back to pinned memory
+            cap.graph.replay()                              # upload, the step, greedy tokens back to pinned memory
             ops.launch_counter().value += cap.launches
             logits = cap.logits
         if static.in_flight is None:
@@ -562,6 +548,6 @@ class ModelRunner:
             f.captured[key].graph.replay()
             ops.launch_counter().value += f.captured[key].launches
         f.done.record()
-        self.last_h2d_bytes = (static.dev.numel() - B) * 4
+        self.last_h2d_bytes = (static.host.numel() - B) * 4
         f.ids = ids.copy()
         return f
