@@ -277,18 +277,19 @@ __device__ __forceinline__ void group_sync(int group) {
 }
 
 // Stages.  Split products of up to 64 tokens leave room for a second CTA on the SM (four stages of 24 KB), so that the next
-// kernel's can fetch its weights while this one's still run; split products' partial sums take the stages' place.
+// kernel's can fetch its weights while this one's still run, unless a CTA's share of K is long (SPLIT 2: eight stages);
+// split products' partial sums take the stages' place.
 __host__ __device__ constexpr int ts_groups(int tok) { return tok > 64 ? 2 : 1; }
 __host__ __device__ constexpr int ts_threads(int tok) { return tok > 64 ? 384 : 192; }
-__host__ __device__ constexpr int ts_stages(bool split, int tok) {
-    return tok == 64 ? (split ? 4 : 6) : tok == 128 ? (split ? 6 : 4) : (split ? 4 : 3);
+__host__ __device__ constexpr int ts_stages(int split, int tok) {
+    return tok == 64 ? (split == 2 ? 8 : split == 1 ? 4 : 6) : tok == 128 ? (split ? 6 : 4) : (split ? 4 : 3);
 }
-__host__ __device__ constexpr size_t ts_smem(bool split, int tok) {
+__host__ __device__ constexpr size_t ts_smem(int split, int tok) {
     return (size_t)ts_stages(split, tok) * (TS_ROWS + tok) * TS_BK * 2 + (split ? 0 : ts_groups(tok) * TS_CHUNK * TS_ROWS * 4) +
            8 * (2 * ts_stages(split, tok) + 4) + 1024;
 }
 
-template <bool SPLIT, int TOK, int EPI, int PRO, typename OUT>
+template <int SPLIT, int TOK, int EPI, int PRO, typename OUT>
 __global__ void __launch_bounds__(ts_threads(TOK))
 tc_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                  OUT* __restrict__ out, int ldo, int M, int N, int K, int splits, int* err, const StreamFusion fu) {
@@ -490,7 +491,7 @@ static int ts_num_sms() {
     return num_sms;
 }
 
-template <bool SPLIT, int TOK, int EPI, int PRO, typename OUT>
+template <int SPLIT, int TOK, int EPI, int PRO, typename OUT>
 static int launch_ts(const CUtensorMap& mw, const CUtensorMap& mx, OUT* out, int ldo, int M, int N, int K, int splits, int* err,
                      const StreamFusion& fu, cudaStream_t s) {
     constexpr size_t smem = ts_smem(SPLIT, TOK);
@@ -526,8 +527,15 @@ static int dispatch_ts_tok(const void* x, int ldx, const CUtensorMap& mw, OUT* o
     CUtensorMap mx;
     const int e = rg_make_map(&mx, x, M, K, ldx, TOK);
     if (e) return e;
-    return splits == 1 ? launch_ts<false, TOK, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, 1, err, fu, s)
-                       : launch_ts<true, TOK, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, splits, err, fu, s);
+    if constexpr (TOK == 64) {
+        // More than 16 boxes of K a CTA: copies in flight count for more than room for the next kernel's CTA.  64 rows of four
+        // 8B-sized layers at 4,096 tokens (down: 56 boxes): 1,442 us with four stages, 1,422 with eight; 64 rows of a
+        // 1B-sized model at 1,024 (down: 16 boxes) 1,290 and 1,396.
+        if (splits > 1 && (K + TS_BK - 1) / TS_BK > 16 * splits)
+            return launch_ts<2, TOK, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, splits, err, fu, s);
+    }
+    return splits == 1 ? launch_ts<0, TOK, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, 1, err, fu, s)
+                       : launch_ts<1, TOK, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, splits, err, fu, s);
 }
 
 template <int EPI, int PRO, typename OUT>
