@@ -7,18 +7,25 @@
 //   S = Q K^T            tcgen05.mma, M 128 x N 128 keys x K 128, into 128 TMEM columns
 //   softmax              128 threads, one query row each, 64 keys at a time as in attention_tcgen05.cu: one pass with a
 //                        reference maximum that is raised only when the 64 weights sum to more than 2^8
-//   O += P V             tcgen05.mma, M 128 x N 128 x K 64 per half stage, P from TMEM (bfloat16 over the columns of the
-//                        scores it was made from), O in 128 TMEM columns
+//   O += P V             tcgen05.mma, M 128 x N 128 x K 64 per half stage and twice: P is the sum of two bfloat16 numbers, in
+//                        TMEM over the columns of the scores it was made from; O in 128 TMEM columns
 // Two groups use all 512 columns.  A group's chain (scores, exponentials, product) is serial but for the product of a
 // stage's first 64 keys, which runs under the second 64 keys' exponentials; the other group's exponentials run under
 // its products and the other way round.
 //
-// What bounds it: per 64 keys and row tile the exponentials take 512 cycles of an SM's 16 lanes, the products 520 of its
+// What bounds it: per 64 keys and row tile the exponentials take 512 cycles of an SM's 16 lanes, the products 780 of its
 // tensor core (N 128 is the narrowest shape at full rate: 65 cycles for 16 of K, N 64 takes 49), on different units.
-// Measured (32 heads on 8, this kernel against attention_mma.cu's): 59 against 208 us for a prompt of 2,048 tokens (578
-// against 165 TFLOP/s), 139 against 631 us for 2,048 tokens behind 2,048, 644 against 2,988 us for 8,192 (853 TFLOP/s);
-// 16 heads on 2, a window of 512 that keeps 4: 31 against 75 us.  Shared memory (64 KB of queries, 160 KB of stages) and
-// tensor memory allow one block per SM.
+// Measured (32 heads on 8, this kernel against attention_mma.cu's): 68 against 209 us for a prompt of 2,048 tokens (505
+// against 164 TFLOP/s of the QK and PV that are needed), 154 against 631 us for 2,048 tokens behind 2,048, 680 against
+// 2,989 us for 8,192 (808 TFLOP/s); 16 heads on 2, a window of 512: 36 against 71 us.  Shared memory (64 KB of queries,
+// 160 KB of stages) and tensor memory allow one block per SM.
+//
+// Why two numbers a weight: under a reference that is the row's maximum the largest weight is 1, which bfloat16 holds; under
+// one that is seldom raised it is any number up to 2^8 and loses 2^-9 like the others.  In the 2-norm against 64 bits
+// (2,048 tokens, queries times 0.3 / 1 / 3): one number 2.07e-3 / 2.07e-3 / 2.14e-3, attention_mma.cu 2.07e-3 / 2.02e-3 /
+// 1.76e-3, two numbers 1.56e-3 / 1.61e-3 / 1.65e-3, which is the rounding of the output.  The second product costs 4 to 12 %
+// (2,048 tokens 61 to 68 us, 8,192 651 to 680); raising the reference for every new maximum would read and write O in
+// nearly every pass, since one row of a warp's 32 has one.
 //
 // P is stored only once the 64 weights' sum is known to be small enough, because the scores under it are needed again
 // otherwise.  Masks, sink, gate and the formulas are those of attention_mma.cu's prefill kernel (without pooled
@@ -33,6 +40,7 @@
 #define FW_STAGE 128               // keys per K or V stage
 #define FW_K_STAGES 3
 #define FW_V_STAGES 2
+#define FW_LOW 0x1p-17f             // see `consume`
 #define FW_THREADS 352             // warps 0-3, 4-7: softmax of group 0, 1; 8: TMA; 9, 10: MMA issue of group 0, 1
 
 // tiles: [NT][3] = first token row, rows (<= 128), request.  q_map: rows of queries, head h at column h * 128; kv_map:
@@ -184,10 +192,12 @@ fa_wide_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
             tc_fence_after();
             if (issuer) {
 #pragma unroll
-                for (int k = 0; k < FW_BN / 16; ++k)                         // 16 keys: 16 rows of V, 8 cells of P
-                    tc_mma_a_tmem(tmem_o, tmem_s + (uint32_t)(half * FW_BN + k * 8),
-                                  desc_mn_major(sV0 + s * STAGE_BYTES + half * SUB + (uint32_t)k * 2048u, KV_HALF), idesc_o,
-                                  (j > 0 || k > 0) ? 1u : 0u);
+                for (int k = 0; k < FW_BN / 16; ++k) {                       // 16 keys: 16 rows of V, 8 cells of P's halves each
+                    const uint64_t vd = desc_mn_major(sV0 + s * STAGE_BYTES + half * SUB + (uint32_t)k * 2048u, KV_HALF);
+                    const uint32_t pc = tmem_s + (uint32_t)(half * FW_BN + k * 8);
+                    tc_mma_a_tmem(tmem_o, pc, vd, idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+                    tc_mma_a_tmem(tmem_o, pc + FW_BN / 2, vd, idesc_o, 1u);
+                }
                 tc_commit(p_free0 + 16 * g + 8 * half);
                 if (half == 1 || j == n_kt - 1) tc_commit(v_empty0 + 8 * s);
             }
@@ -217,8 +227,8 @@ fa_wide_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
             const bool edge = key_base + FW_BN - 1 > p0 || (key_base < lo_last && key_base + FW_BN > (window > 0 ? keep_first : 0));
             const int k_hi = prow - key_base, k_lo = seen0 - key_base, k_keep = window > 0 ? keep_first - key_base : 0;
             auto sees = [&](int col) -> bool { return col <= k_hi && (col >= k_lo || col < k_keep); };
-            uint32_t pk[FW_BN / 2];
-            // One pass: p = 2^(s scale - reference), packed as bfloat16 into pk; returns the row sum.
+            uint32_t pk[FW_BN / 2], lo[FW_BN / 2];
+            // One pass: p = 2^(s scale - reference), as two bfloat16 numbers each into pk and lo; returns the row sum.
             auto exp_pass = [&](auto edge_c, float ms) -> float {
                 constexpr bool EDGE = decltype(edge_c)::value;
                 uint64_t rs2[4] = {0ull, 0ull, 0ull, 0ull};
@@ -244,11 +254,20 @@ fa_wide_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
                         p[c & 1][i + 1] = ex2_in_order(t1);
                     }
                 };
+                // p = high + low: its upper 16 bits, and the rest rounded.  FW_LOW p is added to the rest, so that it is 0
+                // only where p is (an infinity in a row of V that is seen stays one); the division at the end takes it out.
+                const uint64_t one2 = pack2(1.f + FW_LOW, 1.f + FW_LOW);
                 auto consume = [&](int c) {
 #pragma unroll
                     for (int i = 0; i < 16; i += 2) {
-                        rs2[(i >> 1) & 3] = add2_in_order(rs2[(i >> 1) & 3], pack2(p[c & 1][i], p[c & 1][i + 1]));
-                        pk[c * 8 + (i >> 1)] = bf16x2_in_order(p[c & 1][i], p[c & 1][i + 1]);
+                        const float p0 = p[c & 1][i], p1 = p[c & 1][i + 1];
+                        const uint32_t b0 = __float_as_uint(p0), b1 = __float_as_uint(p1);
+                        rs2[(i >> 1) & 3] = add2_in_order(rs2[(i >> 1) & 3], pack2(p0, p1));
+                        pk[c * 8 + (i >> 1)] = __byte_perm(b0, b1, 0x7632);
+                        float l0, l1;
+                        unpack2(fma2(pack2(p0, p1), one2, pack2(__uint_as_float((b0 & 0xffff0000u) | 0x80000000u),
+                                                                __uint_as_float((b1 & 0xffff0000u) | 0x80000000u))), l0, l1);
+                        lo[c * 8 + (i >> 1)] = bf16x2_in_order(l0, l1);
                     }
                 };
                 exps(0);
@@ -309,6 +328,7 @@ fa_wide_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
             }
             l_run += row_sum;
             tc_st32(tmem_s, pk);
+            tc_st32(tmem_s + FW_BN / 2, lo);
             tc_st_wait();
             tc_fence_before();
             mbar_arrive(p_full + 8 * half);                                   // this row's scores have been read, its weights written
@@ -323,7 +343,7 @@ fa_wide_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
                 f *= a;
             }
             if (gate && row < nrows) f *= 1.f / (1.f + __expf(-__bfloat162float(gate[(size_t)(row0 + row) * gate_ld + h])));
-            const float inv = l_run > 0.f ? f / l_run : 0.f;
+            const float inv = l_run > 0.f ? f / (l_run * (1.f + FW_LOW)) : 0.f;
             bf16* dst = out + (size_t)(row0 + row) * out_ld + h * FW_D;
 #pragma unroll
             for (int c = 0; c < FW_D / 32; ++c) {
