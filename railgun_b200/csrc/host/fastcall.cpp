@@ -25,7 +25,7 @@ typedef int (*Launcher)(u64, u64, u64, u64, u64, u64, u64, u64, u64, u64, u64, u
 
 static PyObject *s_data_ptr, *s_is_cuda, *s_is_contiguous, *s_dtype;
 
-// call(address, arguments..): integers (pointers among them), None (a null pointer) and floats
+// call(address, arguments..): what `integer`, `pointer`, `ptr` and `real` give (None: a null pointer)
 static PyObject* fc_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
     u64 v[MAX_INTS] = {0};
     float f[MAX_FLOATS] = {0};
@@ -78,12 +78,23 @@ static PyObject* fc_ptr(PyObject*, PyObject* t) {
     return PyObject_CallMethodNoArgs(t, s_data_ptr);
 }
 
-// same(x) is x; real(x) a float of it
-static PyObject* fc_same(PyObject*, PyObject* x) {
+// The kinds of arguments, each as ctypes takes it: `call` tells floats from the others by their type alone, so that a float
+// in an integer's place, or a text, must not get there.
+static PyObject* fc_integer(PyObject*, PyObject* x) { return PyNumber_Index(x); }      // no float, no None
+static PyObject* fc_pointer(PyObject*, PyObject* x) {
+    if (x == Py_None) return PyLong_FromLong(0);
+    if (!PyLong_Check(x)) {
+        PyErr_Format(PyExc_TypeError, "a pointer is an integer or None, not %.100s", Py_TYPE(x)->tp_name);
+        return nullptr;
+    }
     Py_INCREF(x);
     return x;
 }
-static PyObject* fc_real(PyObject*, PyObject* x) { return PyNumber_Float(x); }
+static PyObject* fc_real(PyObject*, PyObject* x) {
+    const double v = PyFloat_AsDouble(x);                                             // no text
+    if (v == -1.0 && PyErr_Occurred()) return nullptr;
+    return PyFloat_FromDouble(v);
+}
 
 // fits(tensor, dtype or None): a contiguous CUDA tensor of this type?
 static PyObject* fc_fits(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -113,8 +124,9 @@ static PyObject* fc_fits(PyObject*, PyObject* const* a, Py_ssize_t n) {
 static PyMethodDef methods[] = {
     {"call", (PyCFunction)(void (*)(void))fc_call, METH_FASTCALL, "call(address, *numbers) -> int"},
     {"ptr", fc_ptr, METH_O, "the address of a tensor's first element; 0 for None"},
-    {"same", fc_same, METH_O, "its argument"},
-    {"real", fc_real, METH_O, "its argument as a float"},
+    {"integer", fc_integer, METH_O, "its argument as an integer; TypeError where it is none"},
+    {"pointer", fc_pointer, METH_O, "its argument, an address; 0 for None"},
+    {"real", fc_real, METH_O, "its argument, a number, as a float"},
     {"fits", (PyCFunction)(void (*)(void))fc_fits, METH_FASTCALL, "is it a contiguous CUDA tensor of this type (None: any)?"},
     {nullptr, nullptr, 0, nullptr}};
 

@@ -38,8 +38,8 @@ try:
 except native.NativeBuildError:
     _fast = None
 if _fast is not None:
-    c_int = c_longlong = c_void_p = _fast.same
-    c_float, _ptr = _fast.real, _fast.ptr
+    c_int = c_longlong = _fast.integer
+    c_void_p, c_float, _ptr = _fast.pointer, _fast.real, _fast.ptr
 else:
     from ctypes import c_int, c_float, c_void_p, c_longlong
 
