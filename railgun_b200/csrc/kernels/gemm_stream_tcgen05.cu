@@ -6,7 +6,8 @@
 // CTAs of a thread-block cluster: every CTA accumulates its K range of the cluster's tile, leaves the partial sums
 // in its shared memory (over the stages, which are done with by then), and the cluster's CTAs add them, each for its
 // share of the tokens, reading the others' through distributed shared memory in rank order: one fixed order, no
-// atomics, a token's result does not depend on the batch.  Products with many tiles (gate|up, the head) run unsplit
+// atomics: with a given number of splits a token's result does not depend on the other tokens, and the number that the
+// launcher picks is one for all steps of up to 64 tokens and one for all above.  Products with many tiles (gate|up, the head) run unsplit
 // and persistent: a CTA takes tile after tile with two accumulators in tensor memory, so that a tile's epilogue
 // overlaps the next tile's loads.
 //
@@ -71,12 +72,13 @@ __device__ __forceinline__ float4 ts_ld_remote4(uint32_t addr) {
 // up, rotation pairs), and goes from token to token.  What it reads from global memory for the next four tokens (residual;
 // angles, cache slots) is requested ahead: for the first four before the tile's product is there, else every token would
 // wait for HBM or L2 once.  (The residual product of 64 rows by 2,048 x 8,192 unsplit, where one CTA writes a tile's 64
-// tokens: 48.2 us before, 41.1 after; in eight splits 13.4 and 12.6.)
-template <int EPI>
+// tokens: 48.2 us before, 41.1 after; in eight splits 13.4 and 12.6.)  AHEAD tokens at a time: four, but one of eight
+// splits and two of fewer up to 64 rows, where a thread has one to eight and what counts is how much code runs once (see
+// `FEW`).
+template <int EPI, int AHEAD>
 struct TileEpilogue {
     static constexpr bool PAIRS = EPI == TS_EPI_SILU_MUL || EPI == TS_EPI_ROPE_CACHE;
     static constexpr int STEP = PAIRS ? 8 : 4;                               // from a thread's token to its next
-    static constexpr int AHEAD = 4;
     int row, m_off;                                                          // first row of W within the tile; place of the first token
     float4 resid[EPI == TS_EPI_RESIDUAL ? AHEAD : 1];
     float4 cosv[EPI == TS_EPI_ROPE_CACHE ? AHEAD : 1], sinv[EPI == TS_EPI_ROPE_CACHE ? AHEAD : 1];
@@ -155,27 +157,28 @@ struct TileEpilogue {
     }
     // load4(r, i): partial sums i .. i + 3 of CTA r's [token][row] array; they are added in rank order, and all are requested
     // before the first is used.  inv: 1 / rms per token (TS_PRO_SCALED).
-    template <bool SPLIT, bool FEW, int PRO, typename OUT, typename Load>
+    template <bool SPLIT, int FEW, int PRO, typename OUT, typename Load>
     __device__ __forceinline__ void write(Load load4, int splits, OUT* __restrict__ out, int ldo, int N, int n0, int tile,
                                           int m_lo, int m_hi, bool vec, const float* inv, const StreamFusion& fu) {
-        // Four tokens' sums at row `at` of the tile.  A few tokens a thread (FEW): all CTAs' partial sums of one token in
+        // AHEAD tokens' sums at row `at` of the tile.  A few tokens a thread (FEW): all CTAs' partial sums of one token in
         // flight at a time; else three CTAs' of all four tokens (two at a time took o's eight splits of 64 rows from 6.8 to
-        // 10.1 us).
+        // 10.1 us).  FEW is the number of splits, so that nothing is skipped at run time: this code runs once in a block,
+        // and twice as much of it for up to eight of them and four tokens cost a layer's products of 64 rows 2 to 6 %
+        // (in a chain, 1B / 3B / 8B-sized: 46.8 / 66.0 / 107.7 us, now 45.4 / 62.5 / 102.8).
         auto sums = [&](float4 (&v)[AHEAD], int mb, int at) {
             auto place = [&](int u) { return min(mb + u * STEP, m_hi - 1) * TS_ROWS + at; };
             auto add = [](float4& a, const float4& b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; };
-            if (!SPLIT || FEW) {
-                constexpr int MAXS = SPLIT ? TS_MAX_SPLITS : 1;
+            if constexpr (!SPLIT || FEW > 0) {
+                constexpr int MAXS = SPLIT ? FEW : 1;
 #pragma unroll
                 for (int u = 0; u < AHEAD; ++u) {
                     if (mb + u * STEP >= m_hi) break;
                     float4 p[MAXS];
 #pragma unroll
-                    for (int r = 0; r < MAXS; ++r) p[r] = r < splits ? load4(r, place(u)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int r = 0; r < MAXS; ++r) p[r] = load4(r, place(u));
                     v[u] = p[0];
 #pragma unroll
-                    for (int r = 1; r < MAXS; ++r)
-                        if (r < splits) add(v[u], p[r]);
+                    for (int r = 1; r < MAXS; ++r) add(v[u], p[r]);
                 }
             } else {
 #pragma unroll
@@ -276,26 +279,30 @@ __device__ __forceinline__ void group_sync(int group) {
     else asm volatile("bar.sync 1, 128;" ::: "memory");
 }
 
-// Stages.  Split products of up to 64 tokens leave room for a second CTA on the SM (four stages of 24 KB), so that the next
-// kernel's can fetch its weights while this one's still run, unless a CTA's share of K is long (SPLIT 2: eight stages);
-// split products' partial sums take the stages' place.
+// Stages.  Eight splits of up to 64 tokens leave room for a second CTA on the SM (four stages of 24 KB): a cluster of eight
+// large CTAs starts late, and the next kernel's can fetch its weights while this one's still run (a step of 64 rows of a
+// 1B-sized model: 966 us, 1,177 with six; 17 rows by 2,048 x 16,384: 17.1 us, 26.5 with eight).  Two and four splits take
+// six: 17 rows of 8B-sized o 10.9 us with four, 10.2 with six, a step of 17 rows of six 3B-sized layers 522 and 516.  Where
+// a CTA's share of K is long (SPLIT 2) they take eight.
+// Split products' partial sums take the stages' place.  few: the number of splits of up to 64 tokens.
 __host__ __device__ constexpr int ts_groups(int tok) { return tok > 64 ? 2 : 1; }
 __host__ __device__ constexpr int ts_threads(int tok) { return tok > 64 ? 384 : 192; }
-__host__ __device__ constexpr int ts_stages(int split, int tok) {
-    return tok == 64 ? (split == 2 ? 8 : split == 1 ? 4 : 6) : tok == 128 ? (split ? 6 : 4) : (split ? 4 : 3);
+__host__ __device__ constexpr int ts_stages(int split, int tok, int few) {
+    return tok == 64 ? (split == 2 ? 8 : few == 8 ? 4 : 6) : tok == 128 ? (split ? 6 : 4) : (split ? 4 : 3);
 }
-__host__ __device__ constexpr size_t ts_smem(int split, int tok) {
-    return (size_t)ts_stages(split, tok) * (TS_ROWS + tok) * TS_BK * 2 + (split ? 0 : ts_groups(tok) * TS_CHUNK * TS_ROWS * 4) +
-           8 * (2 * ts_stages(split, tok) + 4) + 1024;
+__host__ __device__ constexpr size_t ts_smem(int split, int tok, int few) {
+    return (size_t)ts_stages(split, tok, few) * (TS_ROWS + tok) * TS_BK * 2 + (split ? 0 : ts_groups(tok) * TS_CHUNK * TS_ROWS * 4) +
+           8 * (2 * ts_stages(split, tok, few) + 4) + 1024;
 }
 
-template <int SPLIT, int TOK, int EPI, int PRO, typename OUT>
+// FEW: the number of splits, or 0 where it is known at run time only (and of unsplit products).
+template <int SPLIT, int FEW, int TOK, int EPI, int PRO, typename OUT>
 __global__ void __launch_bounds__(ts_threads(TOK))
 tc_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                  OUT* __restrict__ out, int ldo, int M, int N, int K, int splits, int* err, const StreamFusion fu) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ float inv_rms[TOK];
-    constexpr int STAGES = ts_stages(SPLIT, TOK), GROUPS = ts_groups(TOK);
+    constexpr int STAGES = ts_stages(SPLIT, TOK, FEW), GROUPS = ts_groups(TOK);
     constexpr uint32_t W_BYTES = TS_ROWS * TS_BK * 2, X_BYTES = TOK * TS_BK * 2, STAGE_BYTES = W_BYTES + X_BYTES;
     static_assert(!SPLIT || (uint32_t)TOK * TS_ROWS * 4 <= STAGES * STAGE_BYTES, "the partial sums take the stages' place");
     const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;          // swizzled tiles need 1024-byte alignment
@@ -328,7 +335,7 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     const int m_hi = SPLIT ? cta_lo + (cta_hi - cta_lo) * (group + 1) / GROUPS : min(M, (group + 1) * TS_CHUNK);
     // four numbers of the output at a time
     const bool vec = ldo % 4 == 0 && ((uintptr_t)out & (4 * sizeof(OUT) - 1)) == 0 && (((uintptr_t)fu.scaled_out | (uintptr_t)fu.kv_cache) & 7) == 0;
-    TileEpilogue<EPI> epilogue((int)threadIdx.x & 127);
+    TileEpilogue<EPI, FEW == 8 ? 1 : FEW ? 2 : 4> epilogue((int)threadIdx.x & 127);
 
     if (threadIdx.x == 0) {
         abort_flag = 0;
@@ -448,7 +455,7 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                     const int m1 = min(M, m0 + TS_CHUNK);
                     if (m0 >= GROUPS * TS_CHUNK) epilogue.fetch(m0 + epilogue.m_off, m1, t * TS_ROWS, N, out, ldo, vec, fu);
                     auto load4 = [&](int, int i) { return *reinterpret_cast<const float4*>(mine + i - m0 * TS_ROWS); };
-                    epilogue.template write<false, false, PRO>(load4, 1, out, ldo, N, t * TS_ROWS, t, m0, m1, vec, inv_rms, fu);
+                    epilogue.template write<false, 0, PRO>(load4, 1, out, ldo, N, t * TS_ROWS, t, m0, m1, vec, inv_rms, fu);
                 }
             }
             tc_fence_before();
@@ -466,7 +473,7 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             const uint32_t mine = smem_addr(part);
             auto load4 = [&](int r, int i) { return ts_ld_remote4(mapa_shared(mine, (uint32_t)r) + (uint32_t)i * 4u); };
             if ((warp & 7) < 4)
-                epilogue.template write<true, TOK == 64, PRO>(load4, splits, out, ldo, N, n0, first_tile, m_lo, m_hi, vec, inv_rms, fu);
+                epilogue.template write<true, FEW, PRO>(load4, splits, out, ldo, N, n0, first_tile, m_lo, m_hi, vec, inv_rms, fu);
         }
         cluster_sync_all();                                                 // nobody leaves while its partial sums are being read
     }
@@ -491,12 +498,12 @@ static int ts_num_sms() {
     return num_sms;
 }
 
-template <int SPLIT, int TOK, int EPI, int PRO, typename OUT>
+template <int SPLIT, int FEW, int TOK, int EPI, int PRO, typename OUT>
 static int launch_ts(const CUtensorMap& mw, const CUtensorMap& mx, OUT* out, int ldo, int M, int N, int K, int splits, int* err,
                      const StreamFusion& fu, cudaStream_t s) {
-    constexpr size_t smem = ts_smem(SPLIT, TOK);
+    constexpr size_t smem = ts_smem(SPLIT, TOK, FEW);
     static_assert(smem <= 227 * 1024, "shared memory of a block");
-    auto kernel = tc_stream_kernel<SPLIT, TOK, EPI, PRO, OUT>;
+    auto kernel = tc_stream_kernel<SPLIT, FEW, TOK, EPI, PRO, OUT>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     const int n_tiles = (N + TS_ROWS - 1) / TS_ROWS;
@@ -508,7 +515,7 @@ static int launch_ts(const CUtensorMap& mw, const CUtensorMap& mx, OUT* out, int
 static int ts_pick_splits(int splits, int N, int K, int M) {
     const int n_tiles = (N + TS_ROWS - 1) / TS_ROWS, kt = (K + TS_BK - 1) / TS_BK;
     if (splits == 0) {
-        // As many CTAs per tile as keep the whole product in one wave of one CTA per SM, with at least four boxes of K each.
+        // As many CTAs per tile as keep the whole product in one wave of one CTA per SM, with at least two boxes of K each.
         // 64 rows by 2,048 x 2,048 / 2,048 x 8,192: 7.8 / 15.5 us with 4, 6.8 / 12.6 with 8; a second CTA per SM from one
         // product (16 splits' worth) only delays the product behind it (a 64-row step 1,281 against 1,333 us).
         splits = 1;
@@ -528,14 +535,19 @@ static int dispatch_ts_tok(const void* x, int ldx, const CUtensorMap& mw, OUT* o
     const int e = rg_make_map(&mx, x, M, K, ldx, TOK);
     if (e) return e;
     if constexpr (TOK == 64) {
-        // More than 16 boxes of K a CTA: copies in flight count for more than room for the next kernel's CTA.  64 rows of four
-        // 8B-sized layers at 4,096 tokens (down: 56 boxes): 1,442 us with four stages, 1,422 with eight; 64 rows of a
-        // 1B-sized model at 1,024 (down: 16 boxes) 1,290 and 1,396.
-        if (splits > 1 && (K + TS_BK - 1) / TS_BK > 16 * splits)
-            return launch_ts<2, TOK, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, splits, err, fu, s);
+        // Many boxes of K a CTA: more copies in flight.  down with six / eight stages: 32 boxes (17 rows by 3,072 x 8,192) 14.16
+        // / 14.18 us, 56 boxes (17 rows by 4,096 x 14,336) 24.8 / 24.3, 64 rows of it 26.8 / 26.2.
+        const bool many = (K + TS_BK - 1) / TS_BK > 32 * splits;
+#define TS_SPLITS(S_) (many ? launch_ts<2, S_, TOK, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, S_, err, fu, s) \
+                            : launch_ts<1, S_, TOK, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, S_, err, fu, s))
+        if (splits == 8) return launch_ts<1, 8, TOK, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, 8, err, fu, s);
+        if (splits > 1) return splits == 2 ? TS_SPLITS(2) : TS_SPLITS(4);
+#undef TS_SPLITS
     }
-    return splits == 1 ? launch_ts<0, TOK, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, 1, err, fu, s)
-                       : launch_ts<1, TOK, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, splits, err, fu, s);
+    if constexpr (TOK > 64) {
+        if (splits > 1) return launch_ts<1, 0, TOK, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, splits, err, fu, s);
+    }
+    return launch_ts<0, 0, TOK, EPI, PRO, OUT>(mw, mx, out, ldo, M, N, K, 1, err, fu, s);
 }
 
 template <int EPI, int PRO, typename OUT>

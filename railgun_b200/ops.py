@@ -2200,13 +2200,14 @@ def tc_stream_ok(x: torch.Tensor, weight: torch.Tensor, max_rows: int = TC_STREA
 
 def tc_stream_gemm(x, weight: torch.Tensor, out_dtype=None, silu_mul: bool = False, splits: int = 0,
                    check: bool = False, max_rows: int = TC_STREAM_MAX_ROWS) -> torch.Tensor:
-    """y = x W^T for up to ``max_rows`` (at most 256) rows of x on the tcgen05 tensor cores with the operands swapped: 128 rows of W per
-    tile stream through once, the rows of x are the narrow side.  ``silu_mul``: W is interleaved gate|up storage
-    and y = silu(gate) * up.  ``splits``: 1, 2, 4 or 8 CTAs of a cluster share a tile's K and add their partial
-    sums in rank order (0: as many as keep the product in one wave).  A row's result does not depend on the other
-    rows.  ``x`` may be a ``NormedRows`` (an RMSNorm not finished yet): the product runs over its scaled rows and
-    multiplies the 32-bit sums by 1 / rms.  The kernel's waits are bounded; ``tc_gemm_check()`` (or ``check=True``)
-    raises if one gave up."""
+    """y = x W^T for up to ``max_rows`` (at most 256) rows of x on the tcgen05 tensor cores with the operands
+    swapped: 128 rows of W per tile stream through once, the rows of x are the narrow side.  ``silu_mul``: W is
+    interleaved gate|up storage and y = silu(gate) * up.  ``splits``: 1, 2, 4 or 8 CTAs of a cluster share a
+    tile's K and add their partial sums in rank order (0: as many as keep the product in one wave; up to 8 for up
+    to 64 rows, up to 4 above).  With one number of splits a row's result does not depend on the other rows.  ``x``
+    may be a ``NormedRows`` (an RMSNorm not finished yet): the product runs over its scaled rows and multiplies the
+    32-bit sums by 1 / rms.  The kernel's waits are bounded; ``tc_gemm_check()`` (or ``check=True``) raises if one
+    gave up."""
     rows = x if isinstance(x, NormedRows) else None
     if rows is not None:
         x = rows.scaled

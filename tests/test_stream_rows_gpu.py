@@ -32,9 +32,11 @@ def test_residual_then_scaled(M, H, K, splits):
     assert rel_err(resid, ref) < F32
     assert torch.equal(rows.scaled, (resid * nw).to(torch.bfloat16))           # one rounding, of the 32-bit product
     assert rel_err(rows.partials[:rows.blocks, :M].double().sum(0), (resid.double() ** 2).sum(1)) < 1e-6
-    alone = resid0[M - 1:].clone()                                              # a row does not depend on its batch
-    ops.tc_stream_gemm_residual(x[M - 1:].contiguous(), w, alone, nw, 1e-3, splits=splits)
-    assert splits == 0 or torch.equal(alone[0], resid[M - 1])                   # (the choice of splits may follow the rows)
+    # a row does not depend on its batch: alone, or (where the launcher picks the splits) last of any other batch above 64 rows
+    first = M - 1 if splits else M - 65
+    again = resid0[first:].clone()
+    ops.tc_stream_gemm_residual(x[first:].contiguous(), w, again, nw, 1e-3, splits=splits)
+    assert torch.equal(again[-1], resid[M - 1])
     for N2, silu in ((136, False), (1008, True), (3072, False)):
         w2 = (torch.randn(N2, H, generator=g) / H ** 0.5).to(torch.bfloat16).to(DEV)
         assert ops.tc_stream_scaled_ok(rows, w2) == (M < 256)
@@ -47,6 +49,24 @@ def test_residual_then_scaled(M, H, K, splits):
         assert rel_err(y, z) < BF16
         if not silu and M < 256:
             assert rel_err(ops.linear(rows, w2), z) < BF16
+
+
+@pytest.mark.parametrize("splits", [2, 4, 8])
+@pytest.mark.parametrize("M,boxes,rest", [(17, 3, 0), (33, 16, 0), (64, 32, 0), (63, 32, 8), (19, 40, 24)])
+def test_up_to_64_rows_in_splits(M, boxes, rest, splits):
+    """Shares of K up to, at and above 32 boxes of 64 a split, where the number of stages changes; M tokens in `splits` shares."""
+    from railgun_b200 import ops
+    H, K = 200, 64 * boxes * splits + rest
+    _, x, w, resid0, nw, resid, rows, ref, _ = rows_of(M, H, K, splits, M + K)
+    assert rel_err(resid, ref) < F32
+    assert torch.equal(rows.scaled, (resid * nw).to(torch.bfloat16))
+    for first, n in ((M - 1, splits), (M - 2, 0)):
+        again, whole = resid0[first:].clone(), resid
+        if n == 0:
+            whole = resid0.clone()
+            ops.tc_stream_gemm_residual(x, w, whole, nw, 1e-3)
+        ops.tc_stream_gemm_residual(x[first:].contiguous(), w, again, nw, 1e-3, splits=n)
+        assert torch.equal(again[-1], whole[M - 1])
 
 
 @pytest.mark.parametrize("M", [17, 65, 130, 256])
