@@ -2510,9 +2510,21 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k, top_p, seed: 
 SMALL_F32_ROWS, SMALL_F32_K, SMALL_F32_RESULTS = 256, 512, 128 * 1024
 
 
+def _by_address(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """May a launcher take these by their addresses where the library would take them as tensors?  Both are on the current
+    device, and their product is neither differentiated (either way), mapped nor traced."""
+    return (type(x) in _PLAIN_TYPES and type(weight) in _PLAIN_TYPES and x.is_cuda and x.device == weight.device
+            and x.device.index == _current_device()
+            and not ((x.requires_grad or weight.requires_grad) and torch.is_grad_enabled())
+            and torch.autograd.forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None)
+
+
+_PLAIN_TYPES = (torch.Tensor, torch.nn.Parameter)
+
+
 def small_gemm_f32_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """Is this a 32-bit product of a few rows by a small matrix?"""
-    if x.dtype != torch.float32 or weight.dtype != torch.float32 or x.dim() != 2:
+    if x.dtype != torch.float32 or weight.dtype != torch.float32 or x.dim() != 2 or not _by_address(x, weight):
         return False
     (M, K), N = x.shape, weight.shape[0]
     return (0 < M <= SMALL_F32_ROWS and 0 < K <= SMALL_F32_K and (K <= 128 or M >= 16) and M * N <= SMALL_F32_RESULTS

@@ -34,3 +34,24 @@ def test_what_it_refuses():
     assert not ops.small_gemm_f32_ok(torch.zeros(8, 256, device=DEV), torch.zeros(64, 256, device=DEV))    # the library's is faster
     with pytest.raises(ops.KernelError):
         ops.small_gemm_f32(x, torch.zeros(8, 63, device=DEV))
+
+
+def test_what_stays_the_librarys():
+    """A matrix elsewhere is refused as before; derivatives and maps go through the product as before."""
+    from railgun_b200 import ops
+    x, w = torch.randn(20, 64, device=DEV), torch.randn(8, 64, device=DEV)
+    y = x @ w.t()
+    with pytest.raises(RuntimeError):
+        ops.linear(x, w.cpu())
+    xg = x.clone().requires_grad_()
+    ops.linear(xg, w).sum().backward()
+    assert torch.allclose(xg.grad, w.sum(0).expand_as(x), atol=1e-5)
+    wp = torch.nn.Parameter(w.clone())
+    ops.linear(x, wp).sum().backward()
+    assert torch.allclose(wp.grad, x.sum(0).expand_as(w), atol=1e-4)
+    with torch.no_grad():
+        assert ops.small_gemm_f32_ok(x, wp)
+    value, moved = torch.func.jvp(lambda a: ops.linear(a, w), (x,), (torch.ones_like(x),))
+    assert torch.allclose(value, y, atol=1e-4) and torch.allclose(moved, w.sum(1).expand(20, 8), atol=1e-4)
+    maps = torch.vmap(lambda m: ops.linear(x, m))(torch.stack([w, 2 * w]))
+    assert torch.allclose(maps, torch.stack([y, 2 * y]), atol=1e-4)
