@@ -7,7 +7,8 @@
 // operands are read along their rows into shared memory (pitch 36: eight neighbouring rows' 16-byte pieces lie in different
 // banks), 32 numbers of k at a time, the next ones on their way in registers; W's first do not wait for the kernel before.
 // Measured on the GPU (this kernel against the library's): 67 rows by 96 x 512 2.6 / 4.0 us, by 256 x 1,024 5.4 / 6.5; 5 rows
-// by 96 x 512 2.5 / 2.5, by 256 x 1,024 5.1 / 3.6 (a step of 32 numbers of k is a chain of 0.5 us), 256 by 256 x 1,024 8.7 / 7.2.
+// by 96 x 512 2.5 / 2.5, by 256 x 1,024 5.1 / 3.6 (a step of 32 numbers of k is a chain of 0.5 us), 256 by 256 x 1,024 8.7 / 7.2;
+// 16 rows by 512 x 256 9.6 / 6.5.  ops.py takes it where it is no slower.
 #include "common.cuh"
 
 #define SG_T 32

@@ -2504,39 +2504,49 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k, top_p, seed: 
     return out
 
 
-# 32-bit products that run in this package's kernel instead of the library's: host time is what it saves (7 against 15 us), so
-# only where it is no slower on the GPU either (measured in gemm_small_f32.cu): few rows by short rows, or rows enough to
-# fill the library's tiles too.
-SMALL_F32_ROWS, SMALL_F32_K, SMALL_F32_RESULTS = 256, 512, 128 * 1024
+# 32-bit products that run in this package's kernel instead of the library's.  What it saves is host time (7 against 15 us),
+# which counts for nothing where a step is replayed from a graph, so only where it is no slower on the GPU either.  Its time
+# over the library's, over 1 to 40 rows, K 64 to 512 and N 96 to 3,000: up to 16 rows the library takes products with a
+# kernel for few rows: 0.67 to 1.01 on average (1.09 at most) up to K 96 and N 8,192, from K 97 on 0.99 to 1.15, from K 192
+# 1.2 to 3.4; from 17 rows 0.61 to 0.93 up to K 448, 512 is 0.94 from 31 rows and 1.04 to 1.08 below, and more 32 x 32 tiles
+# than SMs are up to 1.33 (33 rows by 3,000).
+SMALL_F32_ROWS = 256
+SMALL_F32_LIMITS = ((96, 256), (448, 148), (512, 148))      # numbers of a row and tiles: up to 16 rows, up to 30, above
+
+_PLAIN_TYPES = (torch.Tensor, torch.nn.Parameter)
+_forward_ad, _transforms = torch.autograd.forward_ad, torch._C._functorch.peek_interpreter_stack
 
 
 def _by_address(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """May a launcher take these by their addresses where the library would take them as tensors?  Both are on the current
     device, and their product is neither differentiated (either way), mapped nor traced."""
-    return (type(x) in _PLAIN_TYPES and type(weight) in _PLAIN_TYPES and x.is_cuda and x.device == weight.device
-            and x.device.index == _current_device()
+    return (type(x) in _PLAIN_TYPES and type(weight) in _PLAIN_TYPES and x.is_cuda
+            and x.get_device() == weight.get_device() == _current_device()
             and not ((x.requires_grad or weight.requires_grad) and torch.is_grad_enabled())
-            and torch.autograd.forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None)
-
-
-_PLAIN_TYPES = (torch.Tensor, torch.nn.Parameter)
+            and _forward_ad._current_level < 0 and _transforms() is None)
 
 
 def small_gemm_f32_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """Is this a 32-bit product of a few rows by a small matrix?"""
-    if x.dtype != torch.float32 or weight.dtype != torch.float32 or x.dim() != 2 or not _by_address(x, weight):
+    if x.dtype != torch.float32 or weight.dtype != torch.float32 or x.dim() != 2:
         return False
-    (M, K), N = x.shape, weight.shape[0]
-    return (0 < M <= SMALL_F32_ROWS and 0 < K <= SMALL_F32_K and (K <= 128 or M >= 16) and M * N <= SMALL_F32_RESULTS
-            and weight.shape[1] == K and x.stride(1) == 1 and x.stride(0) >= K and weight.is_contiguous())
+    (M, K), (N, Kw) = x.shape, weight.shape
+    most_k, most_tiles = SMALL_F32_LIMITS[0] if M <= 16 else SMALL_F32_LIMITS[1] if M <= 30 else SMALL_F32_LIMITS[2]
+    if not (0 < M <= SMALL_F32_ROWS and 0 < K <= most_k and Kw == K and -(-M // 32) * -(-N // 32) <= most_tiles):
+        return False
+    row, number = x.stride()
+    return number == 1 and row >= K and weight.is_contiguous() and _by_address(x, weight)
 
 
 def small_gemm_f32(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """y = x W^T in 32-bit for a few rows by a small matrix."""
     if not small_gemm_f32_ok(x, weight):
         raise KernelError(f"small_gemm_f32 refuses x {tuple(x.shape)} {x.dtype}, W {tuple(weight.shape)} {weight.dtype}")
-    M, K = x.shape
-    N = weight.shape[0]
+    return _small_gemm_f32(x, weight)
+
+
+def _small_gemm_f32(x, weight):
+    (M, K), N = x.shape, weight.shape[0]
     out = torch.empty((M, N), dtype=torch.float32, device=x.device)
     _ok(_fn("gemm_small_f32", "rg_small_gemm_f32")(_ptr(x), c_int(x.stride(0)), _ptr(weight), _ptr(out), c_int(N), c_int(M),
                                                    c_int(N), c_int(K), _stream()), "small_gemm_f32")
@@ -2567,7 +2577,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, bias: torch.Te
     if x.shape[0] <= SKINNY_AUTO_ROWS and skinny_gemm_ok(x, weight):
         return skinny_gemm(x, weight, out_dtype)             # small decode batches: stream the weights once
     if (out_dtype is None or out_dtype == torch.float32) and small_gemm_f32_ok(x, weight):
-        return small_gemm_f32(x, weight)
+        return _small_gemm_f32(x, weight)
     if out_dtype is not None and out_dtype != x.dtype:
         return torch.mm(x, weight.t(), out_dtype=out_dtype)
     return torch.mm(x, weight.t())

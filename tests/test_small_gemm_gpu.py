@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 1, 1), (1, 500, 96), (67, 160, 96), (32, 32, 32), (33, 33, 33), (31, 65, 511), (128, 1024, 512),
-                                   (16, 96, 256), (2, 7, 4)])
+                                   (17, 96, 256), (2, 7, 4)])
 def test_against_64_bits(M, N, K):
     from railgun_b200 import ops
     g = torch.Generator().manual_seed(M + N + K)
@@ -19,7 +19,7 @@ def test_against_64_bits(M, N, K):
     # chains of eight products and of at most sixteen of their sums: some 25 x 2^-24 of the largest, 1.5e-6
     assert y.dtype == torch.float32 and rel_err(y, ref) < 2e-6
     assert torch.equal(ops.linear(x, w), y)
-    if K <= 128:
+    if K <= 96:
         assert torch.equal(ops.small_gemm_f32(x[M // 2:M // 2 + 1], w)[0], y[M // 2])  # a row on its own
     wide = torch.full((M, K + 3), float("nan"), device=DEV)                            # rows off 16-byte boundaries
     wide[:, 1:K + 1] = x
@@ -34,6 +34,16 @@ def test_what_it_refuses():
     assert not ops.small_gemm_f32_ok(torch.zeros(8, 256, device=DEV), torch.zeros(64, 256, device=DEV))    # the library's is faster
     with pytest.raises(ops.KernelError):
         ops.small_gemm_f32(x, torch.zeros(8, 63, device=DEV))
+
+
+@pytest.mark.parametrize("M,N,K,own", [(16, 64, 96, True), (16, 64, 97, False), (1, 8192, 128, False), (1, 8192, 96, True),
+                                       (1, 8193, 96, False), (17, 64, 97, True),
+                                       (17, 64, 448, True), (30, 64, 449, False), (31, 64, 512, True), (31, 64, 513, False),
+                                       (32, 4736, 64, True), (32, 4737, 64, False), (33, 3000, 64, False), (256, 592, 64, False),
+                                       (256, 576, 64, True), (257, 8, 64, False)])
+def test_the_rules_edges(M, N, K, own):
+    from railgun_b200 import ops
+    assert ops.small_gemm_f32_ok(torch.zeros(M, K, device=DEV), torch.zeros(N, K, device=DEV)) == own
 
 
 def test_what_stays_the_librarys():
