@@ -21,7 +21,7 @@ __global__ void channel_rows_kernel(const float* __restrict__ r, int r_ld, const
     pdl_wait();
     pdl_trigger();
     int rq, lo, len;
-    if (!find_chunk(cu, R, blockIdx.x, rq, lo, len)) return;
+    if (!find_chunk(cu, R, blockIdx.x, 0, rq, lo, len)) return;
     const int c = blockIdx.y * blockDim.x + threadIdx.x;
     if (c >= n) return;
     float p = 1.f;
@@ -66,7 +66,7 @@ channel_dots_kernel(const float* __restrict__ r, int r_ld, const float* __restri
     pdl_wait();
     pdl_trigger();
     int rq, lo, n;
-    if (!find_chunk(cu, R, blockIdx.x, rq, lo, n)) return;
+    if (!find_chunk(cu, R, blockIdx.x, 0, rq, lo, n)) return;
     const int h = blockIdx.y, lane = threadIdx.x & 31, first = blockIdx.z * (DOT_THREADS / 32) + (threadIdx.x >> 5);
     float* out = dots + ((size_t)blockIdx.x * H + h) * CH * CH + (lane >> 3) * CH;
     const bool writes = (lane & 7) == 0;
@@ -136,7 +136,7 @@ channel_states_kernel(const float* __restrict__ kd, const float* __restrict__ v,
     pdl_wait();
     pdl_trigger();
     int rq, lo, n;
-    if (!find_chunk(cu, R, blockIdx.x, rq, lo, n)) return;
+    if (!find_chunk(cu, R, blockIdx.x, 0, rq, lo, n)) return;
     const int h = blockIdx.y;
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
     const int j0 = (blockIdx.z / ntiles) * TILE, n0 = (blockIdx.z % ntiles) * TILE * W;
@@ -185,7 +185,7 @@ channel_outputs_kernel(const float* __restrict__ qd, const float* __restrict__ v
     pdl_wait();
     pdl_trigger();
     int rq, lo, n;
-    if (!find_chunk(cu, R, blockIdx.x, rq, lo, n)) return;
+    if (!find_chunk(cu, R, blockIdx.x, 0, rq, lo, n)) return;
     const int h = blockIdx.y, j0 = blockIdx.z * TILE;
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
     const float* m = dots + ((size_t)blockIdx.x * H + h) * CH * CH;
@@ -260,9 +260,9 @@ extern "C" int rg_channel_chunk_scan(const float* r, int r_ld, const float* k, i
     const long long work = vec ? (long long)H * M / 4 : (long long)H * M;
     dim3 g2((unsigned)((work + 255) / 256), R);
     e = vec ? rg_launch(chunk_pass_kernel<4, true>, g2, dim3(256), 0, s, 1, sums, (const float*)decays, state, cu_seqlens,
-                        start_pos, slots, H, M, d)
+                        start_pos, slots, H, M, d, 0)
             : rg_launch(chunk_pass_kernel<1, true>, g2, dim3(256), 0, s, 1, sums, (const float*)decays, state, cu_seqlens,
-                        start_pos, slots, H, M, d);
+                        start_pos, slots, H, M, d, 0);
     if (e) return e;
     dim3 g3(chunks, H, jt);
     return rg_launch(channel_outputs_kernel, g3, dim3(NTH), 0, s, 1, (const float*)qd, v, v_ld, cu_seqlens, R,

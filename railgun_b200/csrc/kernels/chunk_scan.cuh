@@ -9,10 +9,13 @@
 #define PITCH (TILE + 4)
 #define NTH 256
 
+// Chunks of a request that brings `len` tokens: none where it brings fewer than `least` (those are state_scan's).
+__device__ __forceinline__ int chunks_of(int len, int least) { return len < least ? 0 : (len + CH - 1) / CH; }
+
 // Chunk number c of the step: its request, first token and number of tokens; false beyond the last one.
-__device__ __forceinline__ bool find_chunk(const int* __restrict__ cu, int R, int c, int& r, int& lo, int& n) {
+__device__ __forceinline__ bool find_chunk(const int* __restrict__ cu, int R, int c, int least, int& r, int& lo, int& n) {
     for (r = 0; r < R; ++r) {
-        const int len = cu[r + 1] - cu[r], k = (len + CH - 1) / CH;
+        const int len = cu[r + 1] - cu[r], k = chunks_of(len, least);
         if (c < k) {
             lo = cu[r] + c * CH;
             n = min(CH, len - c * CH);
@@ -197,16 +200,17 @@ __device__ __forceinline__ float4 values4(const V* __restrict__ src, size_t ld, 
 template <int V, bool CHANNEL>
 __global__ void chunk_pass_kernel(float* __restrict__ sums, const float* __restrict__ decays, float* __restrict__ state,
                                   const int* __restrict__ cu, const int* __restrict__ start_pos,
-                                  const int* __restrict__ slots, int H, int M, int d) {
+                                  const int* __restrict__ slots, int H, int M, int d, int least) {
     pdl_wait();
     pdl_trigger();
     const int r = blockIdx.y;
+    if (cu[r + 1] - cu[r] < least) return;
     const long long e = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * V;
     if (e >= (long long)H * M) return;
     const int h = (int)(e / M);
     int c0 = 0;
-    for (int q = 0; q < r; ++q) c0 += (cu[q + 1] - cu[q] + CH - 1) / CH;
-    const int nc = (cu[r + 1] - cu[r] + CH - 1) / CH;
+    for (int q = 0; q < r; ++q) c0 += chunks_of(cu[q + 1] - cu[q], least);
+    const int nc = chunks_of(cu[r + 1] - cu[r], least);
     const int slot = slots[r];
     float S[V];
 #pragma unroll

@@ -45,7 +45,7 @@ template <bool VEC, typename V>
 __global__ void __launch_bounds__(MTH, 4)
 delta_solve_kernel(const float* __restrict__ q, int q_ld, const float* __restrict__ k, int k_ld, const V* __restrict__ v,
                    int v_ld, const float* __restrict__ beta, const float* __restrict__ loga, const int* __restrict__ cu,
-                   int R, float* __restrict__ x_out, float* __restrict__ w_out, float* __restrict__ factors,
+                   int R, int least, float* __restrict__ x_out, float* __restrict__ w_out, float* __restrict__ factors,
                    float* __restrict__ decays, float* __restrict__ dots, int H, int Hqk, int d, int dv) {
     extern __shared__ __align__(16) float sm[];
     __shared__ double cum[CH];
@@ -53,7 +53,7 @@ delta_solve_kernel(const float* __restrict__ q, int q_ld, const float* __restric
     pdl_wait();
     pdl_trigger();
     int r, lo, n;
-    if (!find_chunk(cu, R, blockIdx.x, r, lo, n)) return;
+    if (!find_chunk(cu, R, blockIdx.x, least, r, lo, n)) return;
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
     const bool system = (int)blockIdx.y < H;
     const int h = blockIdx.y, hq = system ? h / (H / Hqk) : h - H;
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(NTH)
 delta_states_kernel(const float* __restrict__ k, int k_ld, const float* __restrict__ w, const float* __restrict__ factors,
                     const float* __restrict__ decays, float* __restrict__ u, float* __restrict__ before,
                     float* __restrict__ state, const int* __restrict__ cu, const int* __restrict__ start_pos,
-                    const int* __restrict__ slots, int H, int Hqk, int d, int dv) {
+                    const int* __restrict__ slots, int least, int H, int Hqk, int d, int dv) {
     extern __shared__ __align__(16) float sm[];
     const int KP = d + 16;                              // pitch of K's rows: two neighbouring tokens lie 16 banks apart
     const int stage_floats = d * DC_WP + CH * KP + CH * DC_CB + CH;
@@ -243,10 +243,10 @@ delta_states_kernel(const float* __restrict__ k, int k_ld, const float* __restri
     pdl_trigger();
     const int r = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * DC_CB, hq = h / (H / Hqk);
     const int first = cu[r], last = cu[r + 1];
-    if (last <= first) return;
+    const int nc = chunks_of(last - first, least);
+    if (nc < 1) return;
     int c0 = 0;
-    for (int x = 0; x < r; ++x) c0 += (cu[x + 1] - cu[x] + CH - 1) / CH;
-    const int nc = (last - first + CH - 1) / CH;
+    for (int x = 0; x < r; ++x) c0 += chunks_of(cu[x + 1] - cu[x], least);
     const int cols = min(DC_CB, dv - j0);               // a multiple of 4
     const int d4 = d / 4;
     auto issue = [&](int c) {
@@ -390,28 +390,28 @@ delta_states_kernel(const float* __restrict__ k, int k_ld, const float* __restri
 }
 
 // q, k [T, Hqk * d] float rows q_ld, k_ld apart; v [T, H * dv] float or bfloat16, rows v_ld apart; beta, loga [T, H];
-// state [slots, H, dv, d].  Results and scratch of the caller (chunks at least T / 64 + R, rounded down): u [T, H, dv],
+// state [slots, H, dv, d].  chunks, least: as ssd_chunk.cu's.  Results and scratch of the caller: u [T, H, dv],
 // before [chunks, H, dv, d], dots [chunks, Hqk, 64, 64]; w [chunks, H, d, 64], factors [chunks, H, 64], decays [chunks, H].
 // Takes d and dv in multiples of 4, d up to 128, rows of k and the state on 16-byte boundaries.
 extern "C" int rg_delta_chunk(const float* q, int q_ld, const float* k, int k_ld, const void* v, int v_dtype, int v_ld,
                               const float* beta, const float* loga, float* state, const int* cu_seqlens, const int* start_pos,
                               const int* slots, float* u, float* before, float* dots, float* w, float* factors, float* decays,
-                              int T, int R, int H, int Hqk, int d, int dv, void* stream) {
-    if (T <= 0 || R <= 0) return 0;
+                              int chunks, int R, int least, int H, int Hqk, int d, int dv, void* stream) {
+    if (chunks <= 0 || R <= 0) return 0;
     if (H < 1 || Hqk < 1 || H % Hqk || d < 4 || d % 4 || d > DC_MAX_D || dv < 4 || dv % 4 || H + Hqk > 65535 || k_ld % 4 ||
         ((uintptr_t)k & 15) || ((uintptr_t)state & 15) || ((uintptr_t)u & 15) || ((uintptr_t)before & 15))
         return RG_ERR_UNSUPPORTED;
     const int groups = (dv + DC_CB - 1) / DC_CB;
     if (groups > 65535) return RG_ERR_UNSUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
-    dim3 g1(T / CH + R, H + Hqk);
+    dim3 g1(chunks, H + Hqk);
     int e;
     const bool q4 = q_ld % 4 == 0 && ((uintptr_t)q & 15) == 0 && v_ld % 4 == 0;
 #define DC_SOLVE(VEC_, V_) { \
         const cudaError_t ce = cudaFuncSetAttribute(delta_solve_kernel<VEC_, V_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ds_smem()); \
         if (ce != cudaSuccess) return (int)ce; \
         e = rg_launch(delta_solve_kernel<VEC_, V_>, g1, dim3(MTH), ds_smem(), s, 1, q, q_ld, k, k_ld, (const V_*)v, v_ld, beta, loga, \
-                      cu_seqlens, R, u, w, factors, decays, dots, H, Hqk, d, dv); }
+                      cu_seqlens, R, least, u, w, factors, decays, dots, H, Hqk, d, dv); }
     if (v_dtype == RG_DTYPE_F32) {
         if (q4 && ((uintptr_t)v & 15) == 0) DC_SOLVE(true, float) else DC_SOLVE(false, float)
     } else if (v_dtype == RG_DTYPE_BF16) {
@@ -425,5 +425,6 @@ extern "C" int rg_delta_chunk(const float* q, int q_ld, const float* k, int k_ld
     cudaError_t ce = cudaFuncSetAttribute(delta_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (ce != cudaSuccess) return (int)ce;
     return rg_launch(delta_states_kernel, dim3(R, H, groups), dim3(NTH), smem, s, 1, k, k_ld, (const float*)w,
-                     (const float*)factors, (const float*)decays, u, before, state, cu_seqlens, start_pos, slots, H, Hqk, d, dv);
+                     (const float*)factors, (const float*)decays, u, before, state, cu_seqlens, start_pos, slots, least, H, Hqk,
+                     d, dv);
 }

@@ -48,7 +48,7 @@ template <int W, bool VEC, typename V>
 __global__ void __launch_bounds__(MTH, 4)
 chunk_states_kernel(const V* __restrict__ x, int x_ld, const float* __restrict__ B, int B_ld, const float* __restrict__ C,
                     int C_ld, const float* __restrict__ dt, const float* __restrict__ loga, const float* __restrict__ A_log,
-                    const double* __restrict__ fixed, const int* __restrict__ cu, int R, float* __restrict__ sums,
+                    const double* __restrict__ fixed, const int* __restrict__ cu, int R, int least, float* __restrict__ sums,
                     float* __restrict__ decays, float* __restrict__ dots, int H, int G, int N, int dv, int ntiles, int ones) {
     extern __shared__ __align__(16) float sm[];
     __shared__ double cum[CH];
@@ -56,7 +56,7 @@ chunk_states_kernel(const V* __restrict__ x, int x_ld, const float* __restrict__
     pdl_wait();
     pdl_trigger();
     int r, lo, n;
-    if (!find_chunk(cu, R, blockIdx.x, r, lo, n)) return;
+    if (!find_chunk(cu, R, blockIdx.x, least, r, lo, n)) return;
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
     if ((int)blockIdx.y >= H) {
         if (blockIdx.z > 0) return;
@@ -176,7 +176,7 @@ template <int W, bool VEC, typename V>
 __global__ void __launch_bounds__(MTH, 4)
 chunk_outputs_kernel(const V* __restrict__ x, int x_ld, const float* __restrict__ C, int C_ld, const float* __restrict__ dt,
                      const float* __restrict__ loga, const float* __restrict__ A_log, const double* __restrict__ fixed,
-                     const float* __restrict__ D, const int* __restrict__ cu, int R, const float* __restrict__ before,
+                     const float* __restrict__ D, const int* __restrict__ cu, int R, int least, const float* __restrict__ before,
                      const float* __restrict__ dots, float* __restrict__ o, int H, int G, int N, int dv, int ones) {
     extern __shared__ __align__(16) float sm[];
     __shared__ double cum[CH];
@@ -184,7 +184,7 @@ chunk_outputs_kernel(const V* __restrict__ x, int x_ld, const float* __restrict_
     pdl_wait();
     pdl_trigger();
     int r, lo, n;
-    if (!find_chunk(cu, R, blockIdx.x, r, lo, n)) return;
+    if (!find_chunk(cu, R, blockIdx.x, least, r, lo, n)) return;
     const int h = blockIdx.y, grp = h / (H / G), j0 = blockIdx.z * TILE * W;
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
     const float* dd = dots + ((size_t)blockIdx.x * G + grp) * CH * CH;
@@ -282,31 +282,31 @@ static int allow(K kernel, size_t smem) {
 template <typename V>
 static int launch_outputs(const V* x, int x_ld, const float* C, int C_ld, const float* dt, const float* loga, const float* A_log,
                           const double* fixed, const float* D, const int* cu_seqlens, const float* before, const float* dots,
-                          float* o, int T, int R, int H, int G, int N, int dv, int ones, cudaStream_t s) {
+                          float* o, int chunks, int R, int least, int H, int G, int N, int dv, int ones, cudaStream_t s) {
     // 128 columns a block where that leaves three blocks an SM (2,048 tokens, 16 heads: 55 us), else 64: 30 chunks of 8 heads
     // take 52 us with 128
-    const int wide = dv > TILE && (long long)(T / CH + R) * H * ((dv + 2 * TILE - 1) / (2 * TILE)) >= 3 * 148 ? 2 : 1;
+    const int wide = dv > TILE && (long long)chunks * H * ((dv + 2 * TILE - 1) / (2 * TILE)) >= 3 * 148 ? 2 : 1;
     const bool vec = by_fours(x, x_ld, before, 0, C, C_ld, N, dv);
     auto kernel = wide == 2 ? (vec ? chunk_outputs_kernel<2, true, V> : chunk_outputs_kernel<2, false, V>)
                             : (vec ? chunk_outputs_kernel<1, true, V> : chunk_outputs_kernel<1, false, V>);
     const size_t smem = outputs_smem(wide);
     const int e = allow(kernel, smem);
     if (e) return e;
-    return rg_launch(kernel, dim3(T / CH + R, H, (dv + TILE * wide - 1) / (TILE * wide) + ones), dim3(MTH), smem, s, 1, x, x_ld, C,
-                     C_ld, dt, loga, A_log, fixed, D, cu_seqlens, R, before, dots, o, H, G, N, dv, ones);
+    return rg_launch(kernel, dim3(chunks, H, (dv + TILE * wide - 1) / (TILE * wide) + ones), dim3(MTH), smem, s, 1, x, x_ld, C,
+                     C_ld, dt, loga, A_log, fixed, D, cu_seqlens, R, least, before, dots, o, H, G, N, dv, ones);
 }
 
 // x [T, H * dv] float or bfloat16, rows x_ld apart; B, C [T, G * N] float, rows B_ld, C_ld apart.  dt [T, H], or null: 1.
 // The decays: loga [T, H], or fixed [H] (logarithms, the same for every token), or A_log [H] with dt.  D [H] or null.
 // state [slots, H, dv + ones, N].
-// Scratch of the caller: sums [chunks, H, dv + ones, N], decays [chunks, H], dots [chunks, G, 64, 64], with chunks at least
-// T / 64 + R (rounded down).
+// Requests that bring fewer than `least` tokens are left alone, rows of o and state.  chunks: at least the number of chunks of
+// the others (T / 64 + R, rounded down, is enough).  Scratch of the caller: sums [chunks, H, dv + ones, N], decays [chunks, H],
+// dots [chunks, G, 64, 64].
 template <typename V>
 static int chunk_scan(const V* x, int x_ld, const float* B, int B_ld, const float* C, int C_ld, const float* dt,
                       const float* loga, const float* A_log, const double* fixed, const float* D, float* state,
                       const int* cu_seqlens, const int* start_pos, const int* slots, float* sums, float* decays, float* dots,
-                      float* o, int T, int R, int H, int G, int N, int dv, int ones, cudaStream_t s) {
-    const int chunks = T / CH + R;
+                      float* o, int chunks, int R, int least, int H, int G, int N, int dv, int ones, cudaStream_t s) {
     const int wide = N > TILE ? 2 : 1;
     const int jt = (dv + TILE - 1) / TILE, nt = (N + TILE * wide - 1) / (TILE * wide);
     if (jt * nt > 65535) return RG_ERR_UNSUPPORTED;
@@ -317,45 +317,45 @@ static int chunk_scan(const V* x, int x_ld, const float* B, int B_ld, const floa
     const size_t smem = states_smem(wide);
     int e = allow(states, smem);
     if (e) return e;
-    e = rg_launch(states, g1, dim3(MTH), smem, s, 1, x, x_ld, B, B_ld, C, C_ld, dt, loga, A_log, fixed, cu_seqlens, R, sums,
+    e = rg_launch(states, g1, dim3(MTH), smem, s, 1, x, x_ld, B, B_ld, C, C_ld, dt, loga, A_log, fixed, cu_seqlens, R, least, sums,
                   decays, dots, H, G, N, dv, nt, ones);
     if (e) return e;
     const int M = (dv + ones) * N;
     const bool vec = M % 4 == 0 && ((uintptr_t)state & 15) == 0;
     const long long work = vec ? (long long)H * M / 4 : (long long)H * M;
     dim3 g2((unsigned)((work + 255) / 256), R);
-    e = vec ? rg_launch(chunk_pass_kernel<4, false>, g2, dim3(256), 0, s, 1, sums, (const float*)decays, state, cu_seqlens, start_pos, slots, H, M, N)
-            : rg_launch(chunk_pass_kernel<1, false>, g2, dim3(256), 0, s, 1, sums, (const float*)decays, state, cu_seqlens, start_pos, slots, H, M, N);
+    e = vec ? rg_launch(chunk_pass_kernel<4, false>, g2, dim3(256), 0, s, 1, sums, (const float*)decays, state, cu_seqlens, start_pos, slots, H, M, N, least)
+            : rg_launch(chunk_pass_kernel<1, false>, g2, dim3(256), 0, s, 1, sums, (const float*)decays, state, cu_seqlens, start_pos, slots, H, M, N, least);
     if (e) return e;
-    return launch_outputs(x, x_ld, C, C_ld, dt, loga, A_log, fixed, D, cu_seqlens, (const float*)sums, (const float*)dots, o, T, R,
-                          H, G, N, dv, ones, s);
+    return launch_outputs(x, x_ld, C, C_ld, dt, loga, A_log, fixed, D, cu_seqlens, (const float*)sums, (const float*)dots, o, chunks,
+                          R, least, H, G, N, dv, ones, s);
 }
 
 extern "C" int rg_ssd_chunk_scan(const void* x, int x_dtype, int x_ld, const float* B, int B_ld, const float* C, int C_ld,
                                  const float* dt, const float* loga, const float* A_log, const double* fixed, const float* D,
                                  float* state, const int* cu_seqlens, const int* start_pos, const int* slots, float* sums,
-                                 float* decays, float* dots, float* o, int T, int R, int H, int G, int N, int dv, int ones,
-                                 void* stream) {
-    if (T <= 0 || R <= 0) return 0;
+                                 float* decays, float* dots, float* o, int chunks, int R, int least, int H, int G, int N,
+                                 int dv, int ones, void* stream) {
+    if (chunks <= 0 || R <= 0) return 0;
     if ((!loga && !fixed && !(A_log && dt)) || ones < 0 || ones > 1) return RG_ERR_UNSUPPORTED;
     if (H < 1 || G < 1 || H % G || N < 1 || dv < 1 || H + G > 65535 || R > 65535) return RG_ERR_UNSUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
     if (x_dtype == RG_DTYPE_F32)
         return chunk_scan((const float*)x, x_ld, B, B_ld, C, C_ld, dt, loga, A_log, fixed, D, state, cu_seqlens, start_pos, slots,
-                          sums, decays, dots, o, T, R, H, G, N, dv, ones, s);
+                          sums, decays, dots, o, chunks, R, least, H, G, N, dv, ones, s);
     if (x_dtype == RG_DTYPE_BF16)
         return chunk_scan((const bf16*)x, x_ld, B, B_ld, C, C_ld, dt, loga, A_log, fixed, D, state, cu_seqlens, start_pos, slots,
-                          sums, decays, dots, o, T, R, H, G, N, dv, ones, s);
+                          sums, decays, dots, o, chunks, R, least, H, G, N, dv, ones, s);
     return RG_ERR_UNSUPPORTED;
 }
 
 // The last of the three kernels alone, for a recurrence whose states and dots come from elsewhere (delta_chunk.cu): x float
 // [T, H * dv], loga [T, H], before [chunks, H, dv, N].
 extern "C" int rg_chunk_outputs(const float* x, int x_ld, const float* C, int C_ld, const float* loga, const int* cu_seqlens,
-                                const float* before, const float* dots, float* o, int T, int R, int H, int G, int N, int dv,
-                                void* stream) {
-    if (T <= 0 || R <= 0) return 0;
+                                const float* before, const float* dots, float* o, int chunks, int R, int least, int H, int G,
+                                int N, int dv, void* stream) {
+    if (chunks <= 0 || R <= 0) return 0;
     if (H < 1 || G < 1 || H % G || N < 1 || dv < 1 || H > 65535 || (dv + TILE - 1) / TILE > 65535) return RG_ERR_UNSUPPORTED;
     return launch_outputs(x, x_ld, C, C_ld, (const float*)nullptr, loga, (const float*)nullptr, (const double*)nullptr,
-                          (const float*)nullptr, cu_seqlens, before, dots, o, T, R, H, G, N, dv, 0, (cudaStream_t)stream);
+                          (const float*)nullptr, cu_seqlens, before, dots, o, chunks, R, least, H, G, N, dv, 0, (cudaStream_t)stream);
 }

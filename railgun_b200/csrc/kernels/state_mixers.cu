@@ -22,7 +22,7 @@
 // The step's tokens are packed request by request (cu_seqlens); a request whose start position is 0 begins
 // from zeros whatever its slot holds; a row whose request has slot -1 (padding of a static batch) reads zeros
 // and writes no state.  A token's result depends on its request's earlier tokens only through the state, which
-// is carried in 32-bit, so cutting a prompt into portions changes no bit here (portions of 128 tokens and more run in
+// is carried in 32-bit, so cutting a prompt into portions changes no bit here (long portions run in
 // chunks, ssd_chunk.cu, delta_chunk.cu and channel_chunk.cu, where a cut moves the order of 32-bit sums).
 #include "common.cuh"
 
@@ -354,12 +354,12 @@ extern "C" int rg_retention_prepare(const void* proj, int dtype, int ld, int q_o
 }
 
 // qk [T, ld] float: q heads (G of d) at column 0, k heads at column G d, in place.  ab: rows ab_ld apart (type A),
-// the H numbers b at b_off and the H numbers a at a_off.  beta, g (log_g 1: its logarithm) [T, H] float.
+// the H numbers b at b_off and the H numbers a at a_off.  beta, g and (unless null) g's logarithm [T, H] float.
 template <typename A>
 __global__ void delta_prepare_kernel(float* __restrict__ qk, int ld, int G, int d, float q_scale, float unit_eps,
                                      const A* __restrict__ ab, int ab_ld, int b_off, int a_off,
                                      const float* __restrict__ A_log, const float* __restrict__ dt_bias,
-                                     float* __restrict__ beta, float* __restrict__ g, int log_g, int H) {
+                                     float* __restrict__ beta, float* __restrict__ g, float* __restrict__ log_g, int H) {
     pdl_wait();
     pdl_trigger();
     const int t = blockIdx.x;
@@ -378,13 +378,14 @@ __global__ void delta_prepare_kernel(float* __restrict__ qk, int ld, int G, int 
         const float az = to_f32(ab[(size_t)t * ab_ld + a_off + h]) + dt_bias[h];
         beta[(size_t)t * H + h] = sm_sigmoid(bz);
         const float a = -expf(A_log[h]) * sm_softplus(az);
-        g[(size_t)t * H + h] = log_g ? a : expf(a);
+        g[(size_t)t * H + h] = expf(a);
+        if (log_g) log_g[(size_t)t * H + h] = a;
     }
 }
 
 extern "C" int rg_delta_prepare(float* qk, int ld, int G, int d, float q_scale, float unit_eps, const void* ab,
                                 int ab_dtype, int ab_ld, int b_off, int a_off, const float* A_log, const float* dt_bias,
-                                float* beta, float* g, int log_g, int T, int H, void* stream) {
+                                float* beta, float* g, float* log_g, int T, int H, void* stream) {
     if (T <= 0) return 0;
     if (G < 1 || d < 1 || H < 1) return RG_ERR_UNSUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
@@ -440,7 +441,7 @@ state_scan_kernel(const float* __restrict__ q, int q_ld, const float* __restrict
                   const float* __restrict__ w, int w_ld, const float* __restrict__ bonus,
                   float* __restrict__ state, const int* __restrict__ cu_seqlens,
                   const int* __restrict__ start_pos, const int* __restrict__ slots,
-                  float* __restrict__ o, int H, int Hqk, int d, int dv, int CB, int chunk, int vec, int ones) {
+                  float* __restrict__ o, int H, int Hqk, int d, int dv, int CB, int chunk, int vec, int ones, int below) {
     extern __shared__ __align__(16) float sm[];
     constexpr int parts = PARTS;
     constexpr int DP = PARTS * DPER;                 // padded length of a q or k row
@@ -453,7 +454,7 @@ state_scan_kernel(const float* __restrict__ q, int q_ld, const float* __restrict
     const int r = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * CB;
     const int hq = h / (H / Hqk);
     const int lo = cu_seqlens[r], hi = cu_seqlens[r + 1];
-    if (hi <= lo) return;
+    if (hi <= lo || (below > 0 && hi - lo >= below)) return;
     const int slot = slots[r];
     const bool has_past = slot >= 0 && start_pos[r] > 0;
     const int jl = threadIdx.x / parts, part = threadIdx.x - jl * parts;
@@ -670,11 +671,12 @@ state_scan_kernel(const float* __restrict__ q, int q_ld, const float* __restrict
 static int rg_scan_rows_override = 0;
 extern "C" void rg_state_scan_rows(int rows) { rg_scan_rows_override = rows; }
 
+// below > 0: only requests that bring fewer tokens (the others run in chunks); their rows of o and their state alone.
 extern "C" int rg_state_scan(const float* q, int q_ld, const float* k, int k_ld, const void* v, int v_dtype, int v_ld,
                              const float* decay, const float* g, const float* beta, const float* skip,
                              const float* w, int w_ld, const float* bonus, int rule, float* state,
                              const int* cu_seqlens, const int* start_pos, const int* slots, float* o, int R, int H,
-                             int Hqk, int d, int dv, int ones, void* stream) {
+                             int Hqk, int d, int dv, int ones, int below, void* stream) {
     if (R <= 0) return 0;
     if (ones < 0 || ones > 1 || (ones && dv < 2)) return RG_ERR_UNSUPPORTED;
     if (H < 1 || Hqk < 1 || H % Hqk || d < 1 || dv < 1 || d > 256 || rule < SCAN_SCALAR || rule > SCAN_CHANNEL)
@@ -727,7 +729,7 @@ extern "C" int rg_state_scan(const float* q, int q_ld, const float* k, int k_ld,
     dim3 grid(R, H, col_blocks);
 #define SM_SCAN(DP_, PA_, DE_, V) return rg_launch(state_scan_kernel<DP_, PA_, DE_, V>, grid, dim3(threads), smem, s, 1, \
         q, q_ld, k, k_ld, (const V*)v, v_ld, decay, g, beta, skip, w, w_ld, bonus, state, cu_seqlens, start_pos, slots, o, H, Hqk, d, dv, CB, \
-        chunk, vec, ones)
+        chunk, vec, ones, below)
 #define SM_SCAN_RULE(DP_, PA_, V) { if (rule == SCAN_DELTA) SM_SCAN(DP_, PA_, SCAN_DELTA, V); \
         if (rule == SCAN_CHANNEL) SM_SCAN(DP_, PA_, SCAN_CHANNEL, V); SM_SCAN(DP_, PA_, SCAN_SCALAR, V); }
 #define SM_SCAN_PARTS(DP_, V) switch (parts) { \

@@ -1064,7 +1064,7 @@ def delta_prepare(qkv: torch.Tensor, G: int, d: int, q_scale: float, unit_eps: f
     """In place on ``qkv`` [T, >= 2 G d] float32: the G query heads (from column 0) and the G key heads (from
     column G d) become unit vectors, x / sqrt(sum(x^2) + ``unit_eps``), the queries times ``q_scale``.  Returns
     beta = sigmoid(ab[:, b_off:b_off + H]) and g = exp(-exp(A_log) softplus(ab[:, a_off:a_off + H] + dt_bias)),
-    both [T, H] float32 (``log_g``: the logarithm of g in its place)."""
+    both [T, H] float32, and with ``log_g`` the logarithm of g behind them."""
     _check_rows(qkv, "qkv", torch.float32)
     _check_rows(ab, "ab")
     _check(A_log, "A_log", torch.float32)
@@ -1075,11 +1075,12 @@ def delta_prepare(qkv: torch.Tensor, G: int, d: int, q_scale: float, unit_eps: f
         raise KernelError("delta_prepare: sizes do not match")
     beta = torch.empty((T, H), dtype=torch.float32, device=qkv.device)
     g = torch.empty((T, H), dtype=torch.float32, device=qkv.device)
+    logs = torch.empty_like(g) if log_g else None
     _ok(_fn("state_mixers", "rg_delta_prepare")(
         _ptr(qkv), c_int(qkv.stride(0)), c_int(G), c_int(d), c_float(q_scale), c_float(unit_eps), _ptr(ab),
         c_int(_dtype_code(ab)), c_int(ab.stride(0)), c_int(b_off), c_int(a_off), _ptr(A_log), _ptr(dt_bias), _ptr(beta),
-        _ptr(g), c_int(1 if log_g else 0), c_int(T), c_int(H), _stream()), "delta_prepare")
-    return beta, g
+        _ptr(g), _ptr(logs), c_int(T), c_int(H), _stream()), "delta_prepare")
+    return (beta, g, logs) if log_g else (beta, g)
 
 
 SCAN_RULES = {"scalar": 0, "delta": 1, "channel": 2}
@@ -1088,7 +1089,8 @@ SCAN_RULES = {"scalar": 0, "delta": 1, "channel": 2}
 def state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, batch, H: int, d: int, dv: int,
                decay: torch.Tensor | None = None, g: torch.Tensor | None = None,
                beta: torch.Tensor | None = None, rule: str | None = None, skip: torch.Tensor | None = None,
-               w: torch.Tensor | None = None, bonus: torch.Tensor | None = None, ones: bool = False) -> torch.Tensor:
+               w: torch.Tensor | None = None, bonus: torch.Tensor | None = None, ones: bool = False,
+               below: int = 0) -> torch.Tensor:
     """A matrix S [d, dv] per head carried along each request's tokens, 32-bit, from the request's slot of ``state``
     [slots, H, dv, d] (S transposed; zeros at position 0) and left there.  ``rule``:
       "scalar"   S <- g S + beta k v^T, o = S^T q + skip_h v, with ``decay`` [H] or ``g`` [T, H], ``beta`` [T, H]
@@ -1099,7 +1101,8 @@ def state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
     By default "delta" when ``beta`` is given, else "scalar".
     ``q``, ``k``: float32 [T, Hqk * d] views (head h reads head h / (H / Hqk)); ``v``: [T, H * dv] view, float32 or
     bfloat16.  ``ones``: the last of the ``dv`` columns is that of a value that is always 1 and has no place in ``v``
-    [T, H * (dv - 1)] (its column of S is the sum of the keys with the same decays).
+    [T, H * (dv - 1)] (its column of S is the sum of the keys with the same decays).  ``below`` > 0: only requests that
+    bring fewer tokens; the others' rows of o and states are left as they are.
     Returns o [T, H, dv] float32."""
     rule = rule or ("delta" if beta is not None else "scalar")
     if rule not in SCAN_RULES:
@@ -1135,8 +1138,8 @@ def state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
         _ptr(decay), _ptr(g),
         _ptr(beta), _ptr(skip), _ptr(w), c_int(w.stride(0) if w is not None else 0), _ptr(bonus),
         c_int(SCAN_RULES[rule]), _ptr(state), _ptr(batch.cu_seqlens), _ptr(batch.start_pos), _ptr(batch.state_slots),
-        _ptr(o), c_int(batch.num_requests), c_int(H), c_int(Hqk), c_int(d), c_int(dv), c_int(1 if ones else 0), _stream()),
-        "state_scan")
+        _ptr(o), c_int(batch.num_requests), c_int(H), c_int(Hqk), c_int(d), c_int(dv), c_int(1 if ones else 0),
+        c_int(below), _stream()), "state_scan")
     return o
 
 
@@ -1276,6 +1279,21 @@ def ssd_prepare(raw: torch.Tensor, dt_bias: torch.Tensor, A_log: torch.Tensor):
 SCAN_CHUNK = 64
 # Steps whose longest portion has at least this many tokens run these recurrences in chunks side by side.
 SCAN_CHUNKED_MIN_TOKENS = 128
+# Retention's and the delta rule's go by each request's own portion: from so many tokens on in chunks, below (decoding requests
+# among them, each of which would be a whole chunk's work: 32 beside a portion of 512 and 16 heads of 128 x 128 take 182 us in
+# chunks, 189 token by token, 60 each in its own way) token by token.  What chunks add to a step of a model with one layer
+# of each, in us: a fixed decay, one portion of 256 / 512 / 768 tokens -55 / -129 / -243, 2 / 4 / 8 of 128 -13 / -14 / -38;
+# the delta rule -17 / -114 / -212 and +24 / +47 / +42, 2 / 4 / 8 of 256 -28 / +8 / +15.
+DECAY_CHUNK_MIN_TOKENS = 128
+DELTA_CHUNK_MIN_TOKENS = 256
+
+
+def scan_split(batch, least: int) -> tuple:
+    """(chunks of the step's requests that bring at least ``least`` tokens, whether there are others)."""
+    if batch.max_query_len < least:
+        return 0, True
+    counts = batch.layout[0]
+    return sum(-(-n // SCAN_CHUNK) for n in counts if n >= least), min(counts) < least
 
 
 def ssd_chunk_scan(xbc: torch.Tensor, dt: torch.Tensor, A_log: torch.Tensor, D: torch.Tensor, state: torch.Tensor, batch,
@@ -1296,23 +1314,24 @@ def ssd_chunk_scan(xbc: torch.Tensor, dt: torch.Tensor, A_log: torch.Tensor, D: 
                        T, H, G, N, dv, 0, "ssd_chunk_scan")
 
 
-def _chunk_scan(x, B, C, dt, loga, A_log, fixed, D, state, batch, T, H, G, N, dv, ones, what):
+def _chunk_scan(x, B, C, dt, loga, A_log, fixed, D, state, batch, T, H, G, N, dv, ones, what, least=0, o=None):
     """The three kernels of csrc/kernels/ssd_chunk.cu.  ``x``: (pointer, type code, row step), ``B``, ``C``: (pointer, row
-    step).  Returns o [T, H, dv + ones] float32."""
+    step); ``least``, ``o``: see ``decay_chunk_scan``.  Returns o [T, H, dv + ones] float32."""
     R, M = batch.num_requests, dv + ones
-    chunks = T // SCAN_CHUNK + R
+    chunks = scan_split(batch, least)[0] if least else T // SCAN_CHUNK + R
     new = lambda *shape: torch.empty(shape, dtype=torch.float32, device=state.device)
-    sums, decays, dots, o = new(chunks, H, M, N), new(chunks, H), new(chunks, G, SCAN_CHUNK, SCAN_CHUNK), new(T, H, M)
+    sums, decays, dots = new(chunks, H, M, N), new(chunks, H), new(chunks, G, SCAN_CHUNK, SCAN_CHUNK)
+    o = new(T, H, M) if o is None else o
     _COUNTER.value += 2                              # the launcher runs three kernels
     _ok(_fn("ssd_chunk", "rg_ssd_chunk_scan")(
         *x, *B, *C, _ptr(dt), _ptr(loga), _ptr(A_log), _ptr(fixed), _ptr(D), _ptr(state), _ptr(batch.cu_seqlens),
-        _ptr(batch.start_pos), _ptr(batch.state_slots), _ptr(sums), _ptr(decays), _ptr(dots), _ptr(o), c_int(T), c_int(R),
-        c_int(H), c_int(G), c_int(N), c_int(dv), c_int(ones), _stream()), what)
+        _ptr(batch.start_pos), _ptr(batch.state_slots), _ptr(sums), _ptr(decays), _ptr(dots), _ptr(o), c_int(chunks), c_int(R),
+        c_int(least), c_int(H), c_int(G), c_int(N), c_int(dv), c_int(ones), _stream()), what)
     return o
 
 
-def _check_scan_rows(q, k, v, state, H: int, d: int, dv: int, what: str) -> int:
-    """Checks of q, k, v and the state of a recurrence in chunks; the number of query/key heads."""
+def _check_scan_rows(q, k, v, state, H: int, d: int, dv: int, what: str, o=None) -> int:
+    """Checks of q, k, v, the state and the output of a recurrence in chunks; the number of query/key heads."""
     for t, name in ((q, "q"), (k, "k")):
         _check_rows(t, name, torch.float32)
     _check_rows(v, "v")
@@ -1322,21 +1341,27 @@ def _check_scan_rows(q, k, v, state, H: int, d: int, dv: int, what: str) -> int:
             or tuple(state.shape[1:]) != (H, dv, d):
         raise KernelError(f"{what}: q {tuple(q.shape)}, k {tuple(k.shape)}, v {tuple(v.shape)}, state {tuple(state.shape)} do "
                           f"not match {H} heads of {d} x {dv}")
+    if o is not None:
+        _check(o, "o", torch.float32)
+        if tuple(o.shape) != (T, H, dv):
+            raise KernelError(f"{what}: o {tuple(o.shape)} is not [{T}, {H}, {dv}]")
     return Hqk
 
 
 def decay_chunk_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, batch, H: int, d: int, dv: int,
-                     log_decay: torch.Tensor) -> torch.Tensor:
+                     log_decay: torch.Tensor, least: int = 0, o=None) -> torch.Tensor:
     """S <- decay_h S + k v^T, o = S^T q per head along each request's tokens, as ``state_scan`` with a fixed decay per head
     computes it token by token, in chunks of 64 tokens side by side.  ``log_decay``: float64 [H], the decays' logarithms
-    (minus infinity: nothing is kept).  q, k, v, state and the result as ``state_scan``'s."""
-    Hqk = _check_scan_rows(q, k, v, state, H, d, dv, "decay_chunk_scan")
+    (minus infinity: nothing is kept).  q, k, v, state and the result as ``state_scan``'s.  ``least``: only requests that
+    bring as many tokens; rows of ``o`` (an output of ``state_scan``, say) and states of the others are left as they
+    are."""
+    Hqk = _check_scan_rows(q, k, v, state, H, d, dv, "decay_chunk_scan", o)
     _check(log_decay, "log_decay", torch.float64)
     if log_decay.numel() != H:
         raise KernelError(f"decay_chunk_scan: {log_decay.numel()} decays for {H} heads")
     return _chunk_scan((_ptr(v), c_int(_dtype_code(v)), c_int(v.stride(0))), (_ptr(k), c_int(k.stride(0))),
                        (_ptr(q), c_int(q.stride(0))), None, None, None, log_decay, None, state, batch, q.shape[0], H, Hqk, d, dv,
-                       0, "decay_chunk_scan")
+                       0, "decay_chunk_scan", least, o)
 
 
 def delta_chunk_ok(k: torch.Tensor, state: torch.Tensor, d: int, dv: int) -> bool:
@@ -1346,11 +1371,12 @@ def delta_chunk_ok(k: torch.Tensor, state: torch.Tensor, d: int, dv: int) -> boo
 
 
 def delta_chunk_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, batch, H: int, d: int, dv: int,
-                     loga: torch.Tensor, beta: torch.Tensor) -> torch.Tensor:
+                     loga: torch.Tensor, beta: torch.Tensor, least: int = 0, o=None) -> torch.Tensor:
     """S <- exp(loga) S, u = beta (v - S^T k), S <- S + k u^T, o = S^T q per head along each request's tokens, as
     ``state_scan`` with the delta rule computes it token by token, in chunks of 64 tokens (csrc/kernels/delta_chunk.cu).
-    ``loga``, ``beta``: float32 [T, H]; q, k, v, state and the result as ``state_scan``'s."""
-    Hqk = _check_scan_rows(q, k, v, state, H, d, dv, "delta_chunk_scan")
+    ``loga``, ``beta``: float32 [T, H]; q, k, v, state and the result as ``state_scan``'s; ``least`` and ``o`` as
+    ``decay_chunk_scan``'s."""
+    Hqk = _check_scan_rows(q, k, v, state, H, d, dv, "delta_chunk_scan", o)
     T, R = q.shape[0], batch.num_requests
     for t, name in ((loga, "loga"), (beta, "beta")):
         _check(t, name, torch.float32)
@@ -1358,19 +1384,20 @@ def delta_chunk_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: t
             raise KernelError(f"delta_chunk_scan: {name} has {t.numel()} elements, expected {T * H}")
     if not delta_chunk_ok(k, state, d, dv):
         raise KernelError("delta_chunk_scan: heads of up to 128 in multiples of 4, rows on 16-byte boundaries")
-    chunks = T // SCAN_CHUNK + R
+    chunks = scan_split(batch, least)[0] if least else T // SCAN_CHUNK + R
     new = lambda *shape: torch.empty(shape, dtype=torch.float32, device=state.device)
-    u, before, dots, o = new(T, H, dv), new(chunks, H, dv, d), new(chunks, Hqk, SCAN_CHUNK, SCAN_CHUNK), new(T, H, dv)
+    u, before, dots = new(T, H, dv), new(chunks, H, dv, d), new(chunks, Hqk, SCAN_CHUNK, SCAN_CHUNK)
+    o = new(T, H, dv) if o is None else o
     w, factors, decays = new(chunks, H, d, SCAN_CHUNK), new(chunks, H, SCAN_CHUNK), new(chunks, H)
     _COUNTER.value += 1                              # the launcher runs two kernels
     _ok(_fn("delta_chunk", "rg_delta_chunk")(
         _ptr(q), c_int(q.stride(0)), _ptr(k), c_int(k.stride(0)), _ptr(v), c_int(_dtype_code(v)), c_int(v.stride(0)), _ptr(beta),
         _ptr(loga), _ptr(state), _ptr(batch.cu_seqlens), _ptr(batch.start_pos), _ptr(batch.state_slots), _ptr(u), _ptr(before),
-        _ptr(dots), _ptr(w), _ptr(factors), _ptr(decays), c_int(T), c_int(R), c_int(H), c_int(Hqk), c_int(d), c_int(dv),
-        _stream()), "delta_chunk_scan")
+        _ptr(dots), _ptr(w), _ptr(factors), _ptr(decays), c_int(chunks), c_int(R), c_int(least), c_int(H), c_int(Hqk), c_int(d),
+        c_int(dv), _stream()), "delta_chunk_scan")
     _ok(_fn("ssd_chunk", "rg_chunk_outputs")(
         _ptr(u), c_int(H * dv), _ptr(q), c_int(q.stride(0)), _ptr(loga), _ptr(batch.cu_seqlens), _ptr(before), _ptr(dots),
-        _ptr(o), c_int(T), c_int(R), c_int(H), c_int(Hqk), c_int(d), c_int(dv), _stream()), "delta_chunk_scan")
+        _ptr(o), c_int(chunks), c_int(R), c_int(least), c_int(H), c_int(Hqk), c_int(d), c_int(dv), _stream()), "delta_chunk_scan")
     return o
 
 

@@ -24,8 +24,8 @@ Between steps a request keeps, in its state slot and in 32-bit: S of every
 head (transposed, [dv, d]), and the last taps - 1 inputs of every
 convolution.  Everything from the projections' outputs to the rounding
 before the output product is 32-bit.  The recurrences of retention and of the
-delta rule run token by token, or in chunks of 64 tokens side by side once a
-portion is long (the delta rule's where its sizes allow it).
+delta rule run token by token, or for requests whose portion is long in chunks
+of 64 tokens side by side (the delta rule's where its sizes allow it).
 """
 from __future__ import annotations
 
@@ -109,10 +109,12 @@ class Retention(Mixer):
         else:
             q, k = ops.retention_prepare(proj, 0, H * d, self.freq, self.rot_dims, batch.positions, H, d, self.k_scale)
             v = proj[:, 2 * H * d:2 * H * d + H * dv]
-        if self.log_decay is not None and batch.max_query_len >= ops.SCAN_CHUNKED_MIN_TOKENS:
-            o = ops.decay_chunk_scan(q.view(-1, H * d), k.view(-1, H * d), v, cache.state, batch, H, d, dv, self.log_decay)
-        else:
-            o = ops.state_scan(q.view(-1, H * d), k.view(-1, H * d), v, cache.state, batch, H, d, dv, decay=self.decay)
+        q, k, o, least = q.view(-1, H * d), k.view(-1, H * d), None, ops.DECAY_CHUNK_MIN_TOKENS
+        chunks, others = ops.scan_split(batch, least) if self.log_decay is not None else (0, True)
+        if others:
+            o = ops.state_scan(q, k, v, cache.state, batch, H, d, dv, decay=self.decay, below=least if chunks else 0)
+        if chunks:
+            o = ops.decay_chunk_scan(q, k, v, cache.state, batch, H, d, dv, self.log_decay, least, o)
         z = ops.head_norm_gate(o, proj[:, 2 * H * d + H * dv:], self.norm, self.eps, self.env.dtype, whole=self.whole,
                                gate_kind=self.gate)
         return ops.linear(z, self.w_o)
@@ -171,13 +173,14 @@ class GatedDelta(Mixer):
         if writes and conv_state is not None:
             ops.conv_state_update(proj, 0, conv_state, batch)
         q, k, v, state = qkv[:, :G * d], qkv[:, G * d:2 * G * d], qkv[:, 2 * G * d:], cache.parts[0].state
-        chunked = batch.max_query_len >= ops.SCAN_CHUNKED_MIN_TOKENS and ops.delta_chunk_ok(k, state, d, dv)
-        beta, g = ops.delta_prepare(qkv, G, d, self.q_scale, self.unit_eps, ba, 0, H, self.A_log, self.dt_bias, H,
-                                    log_g=chunked)
-        if chunked:
-            o = ops.delta_chunk_scan(q, k, v, state, batch, H, d, dv, g, beta)
-        else:
-            o = ops.state_scan(q, k, v, state, batch, H, d, dv, g=g, beta=beta)
+        o, least = None, ops.DELTA_CHUNK_MIN_TOKENS
+        chunks, others = ops.scan_split(batch, least) if ops.delta_chunk_ok(k, state, d, dv) else (0, True)
+        beta, g, *loga = ops.delta_prepare(qkv, G, d, self.q_scale, self.unit_eps, ba, 0, H, self.A_log, self.dt_bias, H,
+                                           log_g=chunks > 0)
+        if others:
+            o = ops.state_scan(q, k, v, state, batch, H, d, dv, g=g, beta=beta, below=least if chunks else 0)
+        if chunks:
+            o = ops.delta_chunk_scan(q, k, v, state, batch, H, d, dv, *loga, beta, least, o)
         z = ops.head_norm_gate(o, proj[:, C:], self.norm, self.eps, self.env.dtype)
         return ops.linear(z, self.w_o)
 

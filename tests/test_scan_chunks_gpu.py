@@ -1,6 +1,8 @@
 """Retention's and the delta rule's recurrences in chunks against the token-by-token loop in 64 bits, where they can go
 wrong: portions of one token to several chunks, chunks of one token, requests that continue or have no slot, heads that share
 keys, sizes that fill no tile, decays of 0 and 1, keys that point the same way."""
+from types import SimpleNamespace
+
 import numpy as np
 import pytest
 import torch
@@ -106,3 +108,52 @@ def test_what_it_refuses():
     assert not ops.delta_chunk_ok(torch.zeros(2, 6, device="cuda"), state, 6, 4)
     assert not ops.delta_chunk_ok(torch.zeros(2, 132, device="cuda"), torch.zeros(1, 1, 4, 132, device="cuda"), 132, 4)
     assert not ops.delta_chunk_ok(torch.zeros(2, 9, device="cuda")[:, 1:], torch.zeros(1, 1, 4, 8, device="cuda"), 8, 4)
+
+
+@pytest.mark.parametrize("rule", ["retention", "delta"])
+def test_each_request_by_its_own_length(rule):
+    """Long portions run in chunks and the others token by token, as they would in a step of their own."""
+    from railgun_b200 import ops
+    least = ops.DECAY_CHUNK_MIN_TOKENS if rule == "retention" else ops.DELTA_CHUNK_MIN_TOKENS
+    lengths = [1, least + 70, least - 1, 1, least, 3]
+    starts, slots = [9, 0, 4, 0, 7, 2], [2, 0, 5, 1, -1, 4]
+    H, d, dv, T = 4, 64, 32, sum(lengths)
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    q, k, v = (0.2 * torch.randn(T, H * n, device="cuda", generator=gen) for n in (d, d, dv))
+    k = torch.nn.functional.normalize(k.view(T, H, d), dim=-1).reshape(T, H * d)
+    loga, beta = -torch.rand(T, H, device="cuda", generator=gen), torch.rand(T, H, device="cuda", generator=gen)
+    decay = torch.tensor([0.5, 0.9, 0.99, 1.0], device="cuda")
+    state0 = torch.randn(6, H, dv, d, device="cuda", generator=gen)
+
+    def step(part, lengths, starts, slots, scan, chunks):
+        batch, state = step_batch(lengths, starts, slots), state0.clone()
+        batch.max_query_len, batch.layout = max(lengths), (tuple(lengths),)
+        a, b, more = loga[part].contiguous(), beta[part].contiguous(), scan and chunks
+        args, o = (q[part], k[part], v[part], state, batch, H, d, dv), None
+        if scan:
+            below = least if more else 0
+            o = ops.state_scan(*args, decay=decay, below=below) if rule == "retention" else \
+                ops.state_scan(*args, g=a.exp(), beta=b, below=below)
+        if chunks:
+            own = dict(least=least, o=o) if more else {}
+            o = ops.decay_chunk_scan(*args, decay.double().log(), **own) if rule == "retention" else \
+                ops.delta_chunk_scan(*args, a, b, **own)
+        return o, state
+
+    whole = slice(0, T)
+    assert ops.scan_split(SimpleNamespace(max_query_len=max(lengths), layout=(tuple(lengths),)), least) == (
+        -(-(least + 70) // 64) + -(-least // 64), True)
+    got, state = step(whole, lengths, starts, slots, True, True)
+    want, scanned = step(whole, lengths, starts, slots, True, False)
+    lo = 0
+    for r, n in enumerate(lengths):
+        part = slice(lo, lo + n)
+        if n >= least:
+            alone, after = step(part, [n], starts[r:r + 1], slots[r:r + 1], False, True)
+        else:
+            alone, after = want[part], scanned
+        assert torch.equal(got[part], alone), r
+        if slots[r] >= 0:
+            assert torch.equal(state[slots[r]], after[slots[r]]), r
+        lo += n
+    assert torch.equal(state[3], state0[3])                             # nobody's slot
