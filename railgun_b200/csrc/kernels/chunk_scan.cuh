@@ -103,7 +103,12 @@ __device__ __forceinline__ void multiply(float (&acc)[4][4 * W], const float (*_
 #define MK 32                 // of the contraction at a time
 #define MP (MK + 4)           // pitch of its rows: eight neighbouring rows' 16-byte pieces lie in different banks
 
-// acc[i][q] += sum over k in [k_lo, k_hi) of A[8 ty + i][k] B[tx + 16 q][k], four k at a time; rows PA and PB apart.
+// acc[i][q] += sum over k in [k_lo, k_hi) of A[8 ty + i][k] B[tx + 16 q][k], four k at a time; rows PA and PB apart.  Four
+// products are added up before they join the sum: a chain of 128 ends up twice as far from it as one of 32, and the forms
+// in chunks are to be no further from 64 bits than the token-by-token kernel, which adds a column up in shares.  Output of
+// 2,048 tokens in the 2-norm, in 1e-7, token by token / in chunks with one chain / with fours (and sixteens in the dots): 16
+// heads of decays 1 - 2^-5 .. 2^-11 4.62 / 3.67 / 3.05, 8 heads 2.21 / 2.66 / 1.78; the delta rule with logarithms to -0.01
+// 3.31 / 2.99 / 1.97, to -2 0.94 / 2.09 / 0.93.  It costs a fifth multiply-add slot: 16 heads 124 to 133 us, 258 to 269.
 template <int Q, int PA, int PB>
 __device__ __forceinline__ void multiply_rows(float (&acc)[8][Q], const float* __restrict__ A, const float* __restrict__ B, int k_lo,
                                               int k_hi, int ty, int tx) {
@@ -117,13 +122,17 @@ __device__ __forceinline__ void multiply_rows(float (&acc)[8][Q], const float* _
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
             const float4 b = *reinterpret_cast<const float4*>(b0 + 16 * q * PB + k);
+            float t[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                acc[i][q] += a[i].x * b.x;
-                acc[i][q] += a[i].y * b.y;
-                acc[i][q] += a[i].z * b.z;
-                acc[i][q] += a[i].w * b.w;
-            }
+            for (int i = 0; i < 8; ++i) t[i] = a[i].x * b.x;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) t[i] += a[i].y * b.y;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) t[i] += a[i].z * b.z;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) t[i] += a[i].w * b.w;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[i][q] += t[i];
         }
     }
 }
@@ -151,8 +160,9 @@ __device__ __forceinline__ void fetch_rows(float* __restrict__ dst, const float*
 }
 
 // acc += A B^T over all N numbers of their rows: A has 64 rows (na there), B 16 Q (nb there); two stages of MK numbers in
-// `sm` [2][64 + 16 Q][MP], the next on its way while one is multiplied.
-template <int Q, bool VEC>
+// `sm` [2][64 + 16 Q][MP], the next on its way while one is multiplied.  RUN > 0: sums of RUN products are made first and
+// then added.
+template <int Q, bool VEC, int RUN = 0>
 __device__ __forceinline__ void product_of_rows(float (&acc)[8][Q], float* __restrict__ sm, const float* __restrict__ A, size_t lda,
                                                 int na, const float* __restrict__ B, size_t ldb, int nb, int N, int ty, int tx) {
     constexpr int STAGE = (64 + 16 * Q) * MP;
@@ -173,7 +183,19 @@ __device__ __forceinline__ void product_of_rows(float (&acc)[8][Q], float* __res
         }
         __syncthreads();
         const float* st = sm + (it & 1) * STAGE;
-        multiply_rows<Q, MP, MP>(acc, st, st + 64 * MP, 0, MK, ty, tx);
+        if constexpr (RUN > 0) {
+#pragma unroll 1
+            for (int k = 0; k < MK; k += RUN) {
+                float part[8][Q] = {};
+                multiply_rows<Q, MP, MP>(part, st, st + 64 * MP, k, k + RUN, ty, tx);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int q = 0; q < Q; ++q) acc[i][q] += part[i][q];
+            }
+        } else {
+            multiply_rows<Q, MP, MP>(acc, st, st + 64 * MP, 0, MK, ty, tx);
+        }
         __syncthreads();
     }
 }

@@ -65,8 +65,8 @@ delta_solve_kernel(const float* __restrict__ q, int q_ld, const float* __restric
         for (int i = 0; i < 8; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-        if (system) product_of_rows<4, true>(acc, sm, kh, k_ld, n, kh, k_ld, n, d, ty, tx);
-        else product_of_rows<4, VEC>(acc, sm, q + (size_t)lo * q_ld + (size_t)hq * d, q_ld, n, kh, k_ld, n, d, ty, tx);
+        if (system) product_of_rows<4, true, 16>(acc, sm, kh, k_ld, n, kh, k_ld, n, d, ty, tx);
+        else product_of_rows<4, VEC, 16>(acc, sm, q + (size_t)lo * q_ld + (size_t)hq * d, q_ld, n, kh, k_ld, n, d, ty, tx);
         if (!system) {
             float* out = dots + ((size_t)blockIdx.x * Hqk + hq) * CH * CH;
 #pragma unroll

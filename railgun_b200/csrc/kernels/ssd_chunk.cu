@@ -66,7 +66,7 @@ chunk_states_kernel(const V* __restrict__ x, int x_ld, const float* __restrict__
         for (int i = 0; i < 8; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) a1[i][j] = 0.f;
-        product_of_rows<4, VEC>(a1, sm, C + (size_t)lo * C_ld + (size_t)g * N, C_ld, n, B + (size_t)lo * B_ld + (size_t)g * N,
+        product_of_rows<4, VEC, 16>(a1, sm, C + (size_t)lo * C_ld + (size_t)g * N, C_ld, n, B + (size_t)lo * B_ld + (size_t)g * N,
                                 B_ld, n, N, ty, tx);
         float* out = dots + ((size_t)blockIdx.x * G + g) * CH * CH;
 #pragma unroll

@@ -157,3 +157,32 @@ def test_each_request_by_its_own_length(rule):
             assert torch.equal(state[slots[r]], after[slots[r]]), r
         lo += n
     assert torch.equal(state[3], state0[3])                             # nobody's slot
+
+
+@pytest.mark.parametrize("rule", ["retention", "delta", "delta that forgets"])
+def test_no_further_off_than_token_by_token(rule):
+    """Both forms against 64 bits, over the decays that models have: sums of 128 products in one chain, as the chunks once made
+    them, were 1.4 to 2.2 times as far off as the token-by-token kernel; sums of fours are 0.6 to 0.99 times."""
+    from railgun_b200 import ops
+    H, d, T = 4, 128, 400
+    rng = np.random.default_rng(11)
+    unit = lambda a: a / np.linalg.norm(a, axis=-1, keepdims=True)   # noqa: E731
+    q, k, v = unit(rng.normal(size=(T, H, d))), unit(rng.normal(size=(T, H, d))), rng.normal(size=(T, H, d))
+    q, k, v = (a.astype(np.float32) for a in (q, k, v))
+    loga = (rng.uniform(size=(T, H)) * (-2.0 if rule == "delta that forgets" else -0.01)).astype(np.float32)
+    beta = rng.uniform(size=(T, H)).astype(np.float32)
+    decay = np.array([1.0 - 2.0 ** (-5 - 0.8 * i) for i in range(H)], dtype=np.float32)
+    batch, rows = step_batch([T], [0], [0]), [dev(a.reshape(T, -1)) for a in (q, k, v)]
+    state = lambda: torch.zeros(1, H, d, d, device="cuda")           # noqa: E731
+    if rule == "retention":
+        scan = ops.state_scan(*rows, state(), batch, H, d, d, decay=dev(decay))
+        chunks = ops.decay_chunk_scan(*rows, state(), batch, H, d, d, dev(decay).double().log())
+        g = np.broadcast_to(decay.astype(np.float64), (T, H))
+    else:
+        scan = ops.state_scan(*rows, state(), batch, H, d, d, g=dev(loga).exp(), beta=dev(beta))
+        chunks = ops.delta_chunk_scan(*rows, state(), batch, H, d, d, dev(loga), dev(beta))
+        g = np.exp(loga.astype(np.float64))
+    ref = np.stack([loop(*(a[:, h].astype(np.float64) for a in (q, k, v)), np.zeros((d, d)), g[:, h],
+                         None if rule == "retention" else beta[:, h].astype(np.float64)) for h in range(H)], 1)
+    off = lambda a: np.linalg.norm(a.cpu().double().numpy() - ref)    # noqa: E731
+    assert off(chunks) < 1.05 * off(scan)
