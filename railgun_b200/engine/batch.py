@@ -20,6 +20,9 @@ import torch
 
 
 ATTENTION_TILE_ROWS = 64      # query rows per tile of the prefill attention kernel
+# Contexts of portions at which parts choose another attention kernel.  A captured step keeps its choice, so steps on
+# different sides of one are different graphs: what a step computes never depends on which one was captured first.
+PORTION_CONTEXTS = (128, 256)
 
 
 class BatchError(ValueError):
@@ -93,6 +96,8 @@ class StepBatch:
     num_decode_rows: int = 0
     prefill_tiles128: torch.Tensor | None = None     # the same requests in tiles of up to 128 positions
     num_prefill_tiles128: int = 0
+    max_portion_context: int = 0     # the longest context among those requests (of several tokens)
+    graph_key: tuple = ()            # the layout and what else decides which kernels the step takes: see build_step_batch
 
 
 def build_step_batch(entries, alloc, page_sizes, vocab_size: int, max_position: int, device,
@@ -104,7 +109,9 @@ def build_step_batch(entries, alloc, page_sizes, vocab_size: int, max_position: 
     Nothing is launched and nothing is reserved if any entry is invalid.
     Block tables are as wide as the longest one rounded up to a power of two,
     so that steps of the same token counts have the same layout.  ``into``:
-    called with the layout (token counts, wanted places, block-table widths)
+    called with the graph key (the layout, that is token counts, wanted places
+    and block-table widths; and whether the longest context of a portion is
+    above each of ``PORTION_CONTEXTS``, at which the attention kernels change)
     once it is known; if it returns a device int32 buffer (of exactly the
     layout's size) the step is copied into that buffer, whose address is what a
     captured graph reads, and the batch's tensors are views of it."""
@@ -160,7 +167,9 @@ def build_step_batch(entries, alloc, page_sizes, vocab_size: int, max_position: 
     cu = host[offs[4]:offs[5]].copy()
     slots = host[offs[7]:offs[8]].copy()
     layout = (tuple(count_list), W, max_blocks_t)
-    static = into(layout) if into is not None else None
+    portion_context = max((a + b for a, b in zip(start_list, count_list) if b > 1), default=0)
+    key = (layout, tuple(portion_context > n for n in PORTION_CONTEXTS))
+    static = into(key) if into is not None else None
     if static is not None:
         if static.numel() != buf.numel():
             raise BatchError(f"the step packs {buf.numel()} ints, the buffer to copy into holds {static.numel()}")
@@ -184,4 +193,5 @@ def build_step_batch(entries, alloc, page_sizes, vocab_size: int, max_position: 
         prefill_tiles=d(8 + 2 * G).view(-1, 3) if n_tiles else None, num_prefill_tiles=n_tiles,
         decode_rows=d(9 + 2 * G) if n_dec else None, num_decode_rows=n_dec,
         prefill_tiles128=d(10 + 2 * G).view(-1, 3) if n_tiles128 else None, num_prefill_tiles128=n_tiles128,
+        max_portion_context=portion_context, graph_key=key,
     )

@@ -260,7 +260,7 @@ class ModelRunner:
         # static and the rows' slots are data of the step (-1 in a padding row).
         self.use_graphs = bool(use_graphs) and self.model.graph_safe
         self._static: dict = {}
-        self._shape_steps: dict = {}       # layout -> ShapeGraph: steps of a layout seen before replay a captured graph
+        self._shape_steps: dict = {}       # graph key -> ShapeGraph: steps seen before replay a captured graph
         self._shape_seen: dict = {}
         self.shape_graph_min_tokens = SHAPE_GRAPH_MIN_TOKENS
         self._graph_pool = None
@@ -313,10 +313,10 @@ class ModelRunner:
         (the portions a scheduler cuts are mostly of one size) are kept."""
         build = lambda into: build_step_batch(entries, self.alloc, self.page_sizes, self.model.vocab_size,
                                               self.model.spec.max_position, self.device, self.err_flag, into=into)
-        known = lambda layout: self._shape_steps[layout].dev if layout in self._shape_steps else None
+        known = lambda key: self._shape_steps[key].dev if key in self._shape_steps else None
         batch = build(known)
         self.last_h2d_bytes = batch.h2d_bytes
-        key = batch.layout
+        key = batch.graph_key
         shape = self._shape_steps.get(key)
         if shape is not None:
             # the step was packed straight into the graph's buffer: launch
@@ -338,7 +338,7 @@ class ModelRunner:
         if len(self._shape_steps) >= SHAPE_GRAPHS_KEPT:
             self._shape_steps.pop(next(iter(self._shape_steps)))
         dev = torch.empty(batch.host_buffer.numel(), dtype=torch.int32, device=self.device)
-        batch = build(lambda layout: dev)
+        batch = build(lambda key: dev)
         side = torch.cuda.Stream(device=self.device)
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):

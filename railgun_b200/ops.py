@@ -2145,13 +2145,18 @@ def _sm_pairs(device_index: int) -> int:
     return torch.cuda.get_device_properties(device_index).multi_processor_count // 2
 
 
+def num_sms(device) -> int:
+    """SMs of a device (of its whole pairs)."""
+    return 2 * _sm_pairs(device.index if device.index is not None else torch.cuda.current_device())
+
+
 def tc_pair_tile(M: int, N: int, device) -> str:
     """The tile for a product on CTA pairs: 256 x 256, or a narrower one where that leaves the GPU's pairs idle less.  Tiles
     are worked off in rounds of one per pair, and a round takes about as long as its tiles are wide (and 8 columns more).
     A narrower tile has to save a twelfth of that: it moves more of x per result, and where nearly every pair is busy the
     power limit, not the rounds, is the bound.  Back to back with SiLU-mul, 256 / 224 / 192 columns: 1,056 rows by 3,072 x
     16,384 150 / 135 / 140 us, 1,701 by 2,048 x 16,384 195 / 165 / 172, 2,048 by 4,096 x 28,672 417 / 448 / 473."""
-    pairs = _sm_pairs(device.index if device.index is not None else torch.cuda.current_device())
+    pairs = num_sms(device) // 2
     m_tiles = -(-M // 256)
     cost = {n: -(-(m_tiles * -(-N // n)) // pairs) * (n + 8) for n in (256, 224, 192)}
     best = min(cost, key=lambda n: (cost[n], -n))

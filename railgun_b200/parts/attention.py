@@ -19,6 +19,7 @@ from ..weights.loader import TensorSpec
 from .base import Mixer
 from .latent_attention import rotary_frequencies
 from .registry import register_mixer, POSITION_ENCODINGS
+from ..engine.batch import PORTION_CONTEXTS
 
 
 # The tcgen05 flash kernel takes portions of prompts when the head size is 64 and pages hold 8..128 tokens;
@@ -26,12 +27,27 @@ from .registry import register_mixer, POSITION_ENCODINGS
 USE_TC_ATTENTION = os.environ.get("RAILGUN_B200_TC_ATTENTION", "1") != "0"
 
 
-def use_wide_attention(q, out, batch, cache, d: int) -> bool:
-    """Whether portions of prompts take the tcgen05 kernel for head size 128 (where it can).  It pays for its set-up
-    from contexts of about two of its 128-key stages: one prompt of 100 tokens takes 11.5 us against 9.5 on the mma.sync
-    kernel (32 heads on 8), of 200 13.6 against 14.2, of 400 17.7 against 25.9, of 2,048 59 against 208; 16 tokens
-    behind 1,024 28.0 against 49.7."""
-    return (USE_TC_ATTENTION and batch.num_prefill_tiles128 > 0 and batch.max_context_len > 128
+def wide_attention_pays(context: int, tiles: int, tiles128: int, nh: int, nkv: int, sms: int) -> bool:
+    """Is the tcgen05 kernel for head size 128 the faster one for portions whose longest context is ``context`` (decoding
+    requests of the step do not count), in ``tiles`` tiles of 64 rows and ``tiles128`` of 128?  It has one block an SM, with
+    two heads of a key/value head where there are two; the mma.sync kernel several, of one head and 64 rows.  This kernel's
+    time over the other's (750 shapes, 6 to 128 heads, contexts to 3,000):
+      two heads and more to a key/value head: one prompt of 129 / 160 / 200 / 256 tokens 1.05 to 1.22 / 1.17 / 1.1 / 1.0, from
+      257 on 0.9 down to 0.25; as soon as the mma.sync kernel's blocks are more than the SMs, 129 tokens 0.6 to 1.0 (three
+      heads: up to 1.09);
+      one head: 129 tokens 0.85, but more blocks than SMs are a second round: 129 / 200 tokens up to 1.39 / 1.25, from 257 on
+      up to 1.12 and mostly below 0.9."""
+    short, long = PORTION_CONTEXTS
+    if nh // nkv >= 2:
+        return context > long or (context > short and tiles * nh > sms)
+    return context > (short if tiles128 * nkv <= sms else long)
+
+
+def use_wide_attention(q, out, batch, cache, nh: int, nkv: int, d: int) -> bool:
+    """Whether portions of prompts take the tcgen05 kernel for head size 128: where it can and pays."""
+    return (USE_TC_ATTENTION and batch.num_prefill_tiles128 > 0 and d == 128
+            and wide_attention_pays(batch.max_portion_context, batch.num_prefill_tiles, batch.num_prefill_tiles128, nh, nkv,
+                                    ops.num_sms(q.device))
             and ops.prefill_attention_wide_ok(q, out, cache.kv, d, cache.page_size))
 
 
@@ -136,7 +152,7 @@ class PagedAttention(Mixer):
                     qkv, cache.kv, d, cache.page_size):
                 ops.prefill_attention_tc(qkv, out, cache.kv, table, batch.prefill_tiles128, batch.positions,
                                          nh, nkv, d, self.window, self.scale)
-            elif use_wide_attention(qkv, out, batch, cache, d):
+            elif use_wide_attention(qkv, out, batch, cache, nh, nkv, d):
                 ops.prefill_attention_wide(qkv, out, cache.kv, table, batch.prefill_tiles128, batch.positions,
                                            nh, nkv, d, self.window, self.scale)
             else:
@@ -405,7 +421,7 @@ class NormedAttention(Mixer):
         if self.chunk:
             reach = min(reach, self.chunk)
         if batch.num_prefill_tiles:
-            if pooled is None and use_wide_attention(q, out, batch, cache, D):
+            if pooled is None and use_wide_attention(q, out, batch, cache, H, G, D):
                 ops.prefill_attention_wide(q, out, cache.kv, table, batch.prefill_tiles128, batch.positions, H, G, D,
                                            self.window, 1.0, self.keep_first, sink=self.sink, gate=gate,
                                            out_scale=out_scale, chunk=self.chunk)

@@ -77,6 +77,8 @@ def test_fields_of_random_steps(seed):
         assert b.decode_only == all(len(e.tokens) == 1 for e in entries)
         assert b.layout == (tuple(len(e.tokens) for e in entries), len(exp["want_rows"]),
                             tuple(t.shape[1] for t in b.block_table))
+        portion = max((c for c, e in zip(exp["ctx"], entries) if len(e.tokens) > 1), default=0)
+        assert b.max_portion_context == portion and b.graph_key == (b.layout, (portion > 128, portion > 256))
         alloc.commit_many(b.host_request_ids, b.host_context_lens)
         for e, s in zip(entries, starts):
             assert alloc.num_computed(e.request_id) == s + len(e.tokens)
