@@ -46,6 +46,10 @@ class NativeBuildError(RuntimeError):
     """A native library could not be compiled or loaded."""
 
 
+class NativeToolMissing(NativeBuildError):
+    """What a build needs (a compiler, Python's headers, a folder to write into) is not on this machine."""
+
+
 _lock = threading.Lock()
 _loaded: dict = {}
 
@@ -64,7 +68,7 @@ def _find(tool: str, extra: list[str]) -> str:
     for p in extra:
         if os.path.exists(p):
             return p
-    raise NativeBuildError(f"{tool} not found; it is needed to build the native libraries")
+    raise NativeToolMissing(f"{tool} not found; it is needed to build the native libraries")
 
 
 _build_dir_cache: list = []
@@ -89,7 +93,7 @@ def _build_dir() -> Path:
             return c
         except OSError:
             continue
-    raise NativeBuildError("no writable folder for the native libraries: tried " + ", ".join(map(str, candidates)))
+    raise NativeToolMissing("no writable folder for the native libraries: tried " + ", ".join(map(str, candidates)))
 
 
 def _source_digest(src: Path, flags: list[str]) -> str:
@@ -143,6 +147,8 @@ def build(name: str, kind: str = "kernel") -> Path:
     if compiler == "nvcc":
         exe = _find("nvcc", ["/usr/local/cuda/bin/nvcc"])
     else:
+        if kind == "host" and name in PYTHON_MODULES and not python_headers():
+            raise NativeToolMissing(f"{src.name} needs Python's headers (Python.h in {sysconfig.get_paths()['include']})")
         exe = _find("g++", ["/usr/bin/g++"])
     tmp = out.with_suffix(f".tmp{os.getpid()}.so")
     cmd = [exe, *flags, "-o", str(tmp), str(src)]
@@ -172,8 +178,14 @@ def load(name: str, kind: str = "kernel") -> ctypes.CDLL:
         return lib
 
 
+def python_headers() -> bool:
+    """Are the headers that Python extension modules are built with on this machine?"""
+    return os.path.exists(os.path.join(sysconfig.get_paths()["include"], "Python.h"))
+
+
 def load_module(name: str):
-    """A Python extension module among the host sources, built first if need be.  Raises, never falls back."""
+    """A Python extension module among the host sources, built first if need be.  Raises, never falls back
+    (``NativeToolMissing`` where this machine cannot build it)."""
     key = f"module:{name}"
     with _lock:
         mod = _loaded.get(key)
@@ -198,8 +210,12 @@ def host_sources() -> list[str]:
 
 
 def build_all() -> list[Path]:
-    """Compile every library (the check that everything builds for sm_100a)."""
+    """Compile every library (the check that everything builds for sm_100a).  Without Python's headers the extension
+    modules, whose users have another way, are left out."""
     from concurrent.futures import ThreadPoolExecutor
-    jobs = [(n, "kernel") for n in kernel_sources()] + [(n, "host") for n in host_sources()]
+    left_out = () if python_headers() else PYTHON_MODULES
+    for n in left_out:
+        _say(f"{n}.cpp is left out: no Python headers")
+    jobs = [(n, "kernel") for n in kernel_sources()] + [(n, "host") for n in host_sources() if n not in left_out]
     with ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)))) as ex:
         return list(ex.map(lambda j: build(*j), jobs))

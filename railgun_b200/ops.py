@@ -13,7 +13,7 @@ import os
 
 import torch
 
-from . import native
+from . import log, native
 
 F32, BF16 = 0, 1
 
@@ -31,11 +31,12 @@ def _dtype_code(t: torch.Tensor) -> int:
 
 
 # How a launcher (a C function of integers, pointers and floats) is called: through an extension module with plain numbers
-# (csrc/host/fastcall.cpp), or, where that cannot be built (no Python headers), through ctypes.  Either way an argument is
-# written as the C type it has.
+# (csrc/host/fastcall.cpp), or, on a machine that cannot build it (no compiler, no Python headers), through ctypes, with a word
+# about it.  A module that does not compile or load is an error.  Either way an argument is written as the C type it has.
 try:
     _fast = native.load_module("fastcall")
-except native.NativeBuildError:
+except native.NativeToolMissing as e:
+    log.warning("kernels are called through ctypes, which takes some 2 us a launch longer: %s", e)
     _fast = None
 if _fast is not None:
     c_int = c_longlong = _fast.integer

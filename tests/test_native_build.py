@@ -2,6 +2,9 @@
 the host library: names carry a digest of the source and its headers, a missing
 source or a failing compiler is one clear error, the build folder can be moved."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import pytest
 
@@ -32,3 +35,33 @@ def test_the_build_folder_can_be_moved(tmp_path, monkeypatch):
     lib = ctypes.CDLL(str(path))
     assert hasattr(lib, "rg_cache_create") and hasattr(lib, "rg_sched_schedule")
     assert native.build("runtime", "host") == path                       # built once
+
+
+def _import_ops(tmp_path, before):
+    """A process of its own that runs ``before`` (with railgun_b200.native as n), imports ops without anything built and says how
+    launchers are called there."""
+    code = f"import railgun_b200.native as n\n{before}\nimport railgun_b200.ops as o, ctypes\nprint('ctypes', o.c_int is ctypes.c_int)"
+    env = dict(os.environ, RAILGUN_B200_BUILD_DIR=str(tmp_path))
+    return subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
+
+
+def test_without_pythons_headers_launchers_go_through_ctypes_and_it_is_said(tmp_path):
+    done = _import_ops(tmp_path, "n.python_headers = lambda: False")
+    assert done.returncode == 0 and done.stdout.strip() == "ctypes True"
+    assert "through ctypes" in done.stderr and "Python's headers" in done.stderr
+
+
+def test_an_extension_module_that_does_not_compile_is_an_error(tmp_path):
+    done = _import_ops(tmp_path, "n.GXX_FLAGS.append('-fno-such-option')")
+    assert done.returncode != 0 and "NativeBuildError" in done.stderr and "fastcall.cpp" in done.stderr
+
+
+def test_everything_builds_without_pythons_headers(monkeypatch):
+    built = []
+    monkeypatch.setattr(native, "build", lambda name, kind: built.append((name, kind)) or name)
+    monkeypatch.setattr(native, "python_headers", lambda: False)
+    native.build_all()
+    assert set(built) == {(n, "kernel") for n in native.kernel_sources()} | {("runtime", "host")}
+    monkeypatch.setattr(native, "python_headers", lambda: True)
+    native.build_all()
+    assert ("fastcall", "host") in built
