@@ -107,7 +107,8 @@ __device__ __forceinline__ int first_seen(int p, int window) {
 // Programmatic dependent launch.  A kernel launched with the attribute may start while the kernel before it
 // in the stream is still running; it must not touch anything that kernel (or an earlier one) reads or writes
 // before pdl_wait(), which returns once the previous kernel has completed and its writes are visible.  Only
-// constants (weights) may be read earlier.  pdl_trigger() lets the next kernel start launching.  Without the
+// constants (weights) and the step's description (positions, slots, tiles, block tables: copied from the host before the
+// step's first kernel, never written by a kernel) may be read earlier.  pdl_trigger() lets the next kernel start launching.  Without the
 // attribute both are no-ops.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

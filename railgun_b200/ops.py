@@ -2274,13 +2274,14 @@ def tc_stream_gemm(x, weight: torch.Tensor, out_dtype=None, silu_mul: bool = Fal
 
 
 def tc_stream_rope_ok(x, weight: torch.Tensor, d: int, max_rows: int | None = None) -> bool:
-    """Can the q|k|v projection of these rows (17 to ``max_rows`` of them, default ``TC_STREAM_AUTO_ROWS``) rotate and write the cache in the streaming
-    tcgen05 product's own kernel?"""
+    """Can the q|k|v projection of these rows (17 to ``max_rows`` of them, default ``TC_STREAM_AUTO_ROWS``) rotate and
+    write the cache in the streaming tcgen05 product's own kernel?"""
     if d % 16:
         return False
     if isinstance(x, NormedRows):
         return tc_stream_scaled_ok(x, weight)
-    return SKINNY_AUTO_ROWS < x.shape[0] <= (max_rows or TC_STREAM_AUTO_ROWS) and tc_stream_ok(x, weight, TC_STREAM_STEP_ROWS)
+    return (SKINNY_AUTO_ROWS < x.shape[0] <= (max_rows or TC_STREAM_AUTO_ROWS)
+            and tc_stream_ok(x, weight, TC_STREAM_STEP_ROWS))
 
 
 def tc_stream_gemm_rope_cache(x, weight: torch.Tensor, table: torch.Tensor, positions: torch.Tensor, slots, kv_cache,
@@ -2345,7 +2346,8 @@ def tc_stream_gemm_residual(x: torch.Tensor, weight: torch.Tensor, resid: torch.
     if weight.shape[1] != K or resid.shape != (M, N) or norm_weight.numel() != N:
         raise KernelError(f"tc_stream_gemm_residual: x {tuple(x.shape)}, W {tuple(weight.shape)}, residual "
                           f"{tuple(resid.shape)}, norm weight {norm_weight.numel()}")
-    partials = torch.empty((-(-N // 128), TC_STREAM_MAX_ROWS if M <= TC_STREAM_MAX_ROWS else TC_STREAM_STEP_ROWS), dtype=torch.float32, device=x.device)
+    ld = TC_STREAM_MAX_ROWS if M <= TC_STREAM_MAX_ROWS else TC_STREAM_STEP_ROWS
+    partials = torch.empty((-(-N // 128), ld), dtype=torch.float32, device=x.device)
     scaled = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
     err = _tc_err.get(x.device)
     if err is None:

@@ -186,3 +186,24 @@ def test_no_further_off_than_token_by_token(rule):
                          None if rule == "retention" else beta[:, h].astype(np.float64)) for h in range(H)], 1)
     off = lambda a: np.linalg.norm(a.cpu().double().numpy() - ref)    # noqa: E731
     assert off(chunks) < 1.05 * off(scan)
+
+
+@pytest.mark.parametrize("rule", ["retention", "delta"])
+@pytest.mark.parametrize("at", [3, 37, 64, 130])
+def test_a_later_tokens_infinity_stays_out_of_earlier_outputs(rule, at):
+    """Within a chunk a token's weight for a later one is left out, not multiplied by zero."""
+    from railgun_b200 import ops
+    H, d, dv, T = 2, 32, 36, 200
+    gen = torch.Generator(device="cuda").manual_seed(at)
+    q, k, v = (0.2 * torch.randn(T, H * n, device="cuda", generator=gen) for n in (d, d, dv))
+    loga, beta = -torch.rand(T, H, device="cuda", generator=gen) * 0.1, torch.rand(T, H, device="cuda", generator=gen) + 0.1
+    log_decay, batch = torch.tensor([-0.01, -0.2], dtype=torch.float64, device="cuda"), step_batch([T], [0], [0])
+
+    def run(v):
+        args = (q, k, v, torch.zeros(1, H, dv, d, device="cuda"), batch, H, d, dv)
+        return ops.delta_chunk_scan(*args, loga, beta) if rule == "delta" else ops.decay_chunk_scan(*args, log_decay)
+
+    want = run(v)
+    v[at, 5] = float("inf")
+    got = run(v)
+    assert torch.equal(got[:at], want[:at]) and not torch.isfinite(got[at, 0, 5])
