@@ -162,7 +162,11 @@ class StaticDecodeBatch:
         self.sampled = self.out_dev[:B]                                         # the tokens the last step chose
         self.step_graphs = {}          # with sampling parameters or greedy -> CapturedStep
         self.follow = [None, None]     # FollowStep: the same step fed with ``sampled`` instead of host tokens
-        self.in_flight = None          # an event after the last replay that reads ``host`` and writes ``host_out``
+        self.in_flight = None          # an event after the last replay, which writes ``host_out``
+        # the number of the step last packed into ``host`` and of the one whose step has read it (written by that step)
+        self.seq = torch.zeros(2, dtype=torch.int32, pin_memory=True)
+        self.seq_np = self.seq.numpy()
+        self.blocks_done = torch.zeros(2, dtype=torch.int32, device=dev)
 
     def raise_if_flagged(self, host_out_np) -> None:
         code = int(host_out_np[self.B])
@@ -172,13 +176,15 @@ class StaticDecodeBatch:
             raise_device_error(code)
 
     def wait_until_reusable(self) -> None:
-        """The pinned buffers may be written again once the last replay that copies them has run."""
-        if self.in_flight is not None and not self.in_flight.query():
-            self.in_flight.synchronize()
+        """``host`` may be written again once the last step packed into it has read it: its first kernel says so, while
+        the rest of the step still runs."""
+        while self.in_flight is not None and self.seq_np[1] != self.seq_np[0]:
+            if self.in_flight.query():                       # the step is over (raises if it failed)
+                break
 
-    def upload(self) -> int:
-        self.dev.copy_(self.host, non_blocking=True)
-        return self.host.numel() * 4
+    def packed(self) -> None:
+        """``host`` holds another step: number it, for ``wait_until_reusable``."""
+        self.seq_np[0] = (int(self.seq_np[0]) + 1) & 0x7fffffff
 
 
 def sampling_views(buf, off: int, B: int) -> dict:
@@ -410,9 +416,9 @@ class ModelRunner:
 
         def body():
             if follow is not None:
-                static.dev[B:].copy_(follow.host_in[B:], non_blocking=True)
+                ops.step_in(follow.host_in, static.dev, first=B)
             else:
-                static.dev.copy_(static.host, non_blocking=True)
+                ops.step_in(static.host, static.dev, seq=static.seq, done=static.blocks_done)
             # a following step reads its token ids where the step before left its greedy tokens
             batch = static.batch if follow is None else dataclasses.replace(static.batch, token_ids=static.sampled)
             logits = self.model.forward(batch, self.views)
@@ -422,7 +428,7 @@ class ModelRunner:
                                      sp["counter"], out=static.sampled)
             else:
                 sampled = ops.argmax(logits, out=static.sampled)
-            (follow or static).host_out.copy_(static.out_dev, non_blocking=True)
+            ops.step_out(static.out_dev, (follow or static).host_out)
             return logits, sampled
 
         side = torch.cuda.Stream(device=self.device)
@@ -478,6 +484,7 @@ class ModelRunner:
                              f"{self.model.spec.max_position}")
         static.host_np[:R] = tokens
         static.host_np[R:B] = 0
+        static.packed()
         self.last_h2d_bytes = static.host.numel() * 4
         key = sampled
         logits = None

@@ -2500,15 +2500,33 @@ def argmax(logits: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tenso
         _check(out, "out", torch.int32)
         if out.shape != (rows,):
             raise KernelError(f"argmax: out has shape {tuple(out.shape)}, the logits have {rows} rows")
-    pieces = min(64, -(-V // 2048))            # wide rows are cut into pieces so that many blocks share a row
-    pv = pi = None
-    if pieces > 1:
-        pv = torch.empty((rows, pieces), dtype=torch.float32, device=logits.device)
-        pi = torch.empty((rows, pieces), dtype=torch.int32, device=logits.device)
-        _COUNTER.value += 1
-    _ok(_fn("sampling", "rg_argmax")(_ptr(logits), c_int(rows), c_int(V), _ptr(out), _ptr(pv), _ptr(pi),
-                                     c_int(pieces), _stream()), "argmax")
+    _ok(_fn("sampling", "rg_argmax")(_ptr(logits), c_int(rows), c_int(V), _ptr(out), _stream()), "argmax")
     return out
+
+
+def step_in(host: torch.Tensor, dev: torch.Tensor, first: int = 0, seq: torch.Tensor | None = None,
+            done: torch.Tensor | None = None) -> None:
+    """dev[first:] = host[first:] (int32, ``host`` page-locked), read by a kernel.  ``seq`` (page-locked, two numbers): the
+    kernel sets seq[1] to the seq[0] that it finds once it has read all of ``host``; ``done``: two int32 of the device, zero
+    at first, for its own use."""
+    _check(dev, "dev", torch.int32)
+    for name, t, n in (("host", host, dev.numel()), ("seq", seq, 2)):
+        if t is not None and not (t.dtype == torch.int32 and t.is_pinned() and t.is_contiguous() and t.numel() == n):
+            raise KernelError(f"step_in: {name} must be {n} page-locked int32 numbers")
+    if done is not None:
+        _check(done, "done", torch.int32)
+        if done.numel() != 2:
+            raise KernelError("step_in: done must be two numbers")
+    _ok(_fn("step_io", "rg_step_in")(c_void_p(host.data_ptr()), _ptr(dev), c_int(first), c_int(dev.numel()),
+                                     c_void_p(seq.data_ptr() if seq is not None else 0), _ptr(done), _stream()), "step_in")
+
+
+def step_out(dev: torch.Tensor, host: torch.Tensor) -> None:
+    """host = dev (int32, ``host`` page-locked), written by a kernel."""
+    _check(dev, "dev", torch.int32)
+    if not (host.dtype == torch.int32 and host.is_pinned() and host.is_contiguous() and host.numel() == dev.numel()):
+        raise KernelError(f"step_out: host must be {dev.numel()} page-locked int32 numbers")
+    _ok(_fn("step_io", "rg_step_out")(_ptr(dev), c_void_p(host.data_ptr()), c_int(dev.numel()), _stream()), "step_out")
 
 
 def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k, top_p, seed: torch.Tensor,

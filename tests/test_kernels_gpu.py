@@ -31,6 +31,19 @@ def test_embedding(dtype):
     assert out.dtype == torch.float32 and torch.equal(out, table[ids.long()].float())
 
 
+@pytest.mark.parametrize("H,shift", [(4, 0), (202, 0), (1020, 0), (2048, 0), (2048, 1), (4100, 0), (12288, 0)])
+def test_embedding_four_numbers_a_load(H, shift):
+    """Widths with and without a remainder of a block's loads; a table that starts off an 8-byte boundary; tokens outside of it."""
+    from railgun_b200 import ops
+    g = torch.Generator().manual_seed(H)
+    table = torch.randn(50 * H + shift, generator=g).to(torch.bfloat16).to(DEV)[shift:].view(50, H)
+    table[7, 0] = float("inf")
+    ids = torch.tensor([49, 0, 7, -1, 50, 7], dtype=torch.int32, device=DEV)
+    want = table.float()[ids.long().clamp(0, 49)] * 3.0
+    want[3:5] = 0.0
+    assert torch.equal(ops.embedding(ids, table, 3.0), want)
+
+
 @pytest.mark.parametrize("H", [96, 200, 2048, 5000])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_add_rmsnorm(H, dtype):
@@ -311,6 +324,48 @@ def test_argmax_with_ties(V):
     out = ops.argmax(logits.to(DEV)).cpu()
     ref = torch.tensor([int(np.argmax(r.numpy())) for r in logits], dtype=torch.int32)
     assert torch.equal(out, ref) and out[1] == 33
+
+
+@pytest.mark.parametrize("V", [4095, 4096, 4099, 32768, 128255])
+def test_argmax_shared_by_a_cluster(V):
+    """The widths where a row goes to eight blocks, in parts of 16-byte loads or of single numbers: ties across parts,
+    infinities, rows without a number."""
+    from railgun_b200 import ops
+    g = torch.Generator().manual_seed(V)
+    logits = torch.randn(7, V, generator=g)
+    logits[1, V - 1] = logits[1, V // 8] = logits[1, 3 * V // 4] = 9.0
+    logits[2, V - 1] = float("inf")
+    logits[3, 0] = logits[3, V - 2] = float("inf")
+    logits[4, :] = float("-inf")
+    logits[5, :] = float("nan")
+    logits[6, :] = float("nan")
+    logits[6, V - 3] = -2.0
+    out = ops.argmax(logits.to(DEV)).cpu().tolist()
+    assert out == [int(logits[0].argmax()), V // 8, V - 1, 0, 0, 0, V - 3]
+    assert ops.argmax(logits[:1].contiguous().to(DEV)).cpu().tolist() == out[:1]
+
+
+@pytest.mark.parametrize("n,first", [(1, 0), (3, 1), (64, 64), (67, 5), (1027, 2), (8 * 1024, 8), (300001, 64)])
+def test_a_step_comes_in_and_goes_out_by_kernels(n, first):
+    from railgun_b200 import ops
+    host = torch.arange(1, n + 1, dtype=torch.int32).pin_memory()
+    seq = torch.tensor([41, 7], dtype=torch.int32).pin_memory()
+    done = torch.zeros(2, dtype=torch.int32, device=DEV)
+    dev = torch.full((n,), -1, dtype=torch.int32, device=DEV)
+    back = torch.zeros(n, dtype=torch.int32).pin_memory()
+    ops.step_in(host, dev, first, seq, done)
+    ops.step_out(dev, back)
+    torch.cuda.synchronize()
+    want = torch.where(torch.arange(n) < first, torch.tensor(-1, dtype=torch.int32), host)
+    assert torch.equal(dev.cpu(), want) and torch.equal(back, want)
+    assert seq.tolist() == [41, 41] and done[0].item() == 0
+    host += 1
+    ops.step_in(host, dev, first)                               # without a number
+    assert torch.equal(dev.cpu(), torch.where(want < 0, want, want + 1)) and seq.tolist() == [41, 41]
+    with pytest.raises(ops.KernelError):
+        ops.step_in(torch.zeros(n, dtype=torch.int32), dev)     # pageable memory
+    with pytest.raises(ops.KernelError):
+        ops.step_in(host, dev, first, seq)                      # a number, but nothing to count the blocks with
 
 
 def _plain_interval(logits, temperature, top_k, top_p, tok):
