@@ -125,21 +125,24 @@ __device__ __forceinline__ void store4(bf16* p, const float (&v)[4]) {
     *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
 
-// The same for heads of up to 128 numbers in multiples of 4 (each head's numbers normed on their own, or not at all), where
-// rows, pages, weights and bias allow four numbers at a time: a warp holds a head in registers, four neighbouring numbers a
+// The same for heads of up to 128 numbers in multiples of 4, where
+// rows, pages, weights and bias allow four numbers at a time: a warp holds HP heads in registers, four neighbouring numbers a
 // lane, and rotation partners come by shuffles; v's heads are further warps' turns.  Such a step is a chain of latencies:
 // the position's angles, the only 64-bit work, are made before the wait for the kernel before this one (positions were
-// written before the step's first kernel), and the first head's numbers are requested before the block meets.  Measured
-// (16 heads on 2 of 128): 2,048 tokens 39.4 to 23.6 us, 6 tokens 7.7 to 5.1.
-template <typename A, typename O>
+// written before the step's first kernel), and the first heads' numbers are requested before the block meets.  Single tokens
+// have a warp per head (up to 16); where there are more tokens than SMs a warp has four heads, so that enough loads are under
+// way with fewer registers per head (16 heads on 2 of 128, 2,000 tokens: 10.2 us, with one head a warp 18.1; the form below one number at a
+// time and 2,048 39.4; 6 tokens 2.6, one number at a time 7.7).
+template <int HP, typename A, typename O>
 __global__ void attention_prepare4_kernel(const A* __restrict__ qkv, int ld, const float* __restrict__ bias,
                                           O* __restrict__ q_out, O* kv,
-                                          const float* __restrict__ q_norm, const float* __restrict__ k_norm, float eps,
-                                          const double* __restrict__ freq, int dims, int interleaved,
+                                          const float* __restrict__ q_norm, const float* __restrict__ k_norm,
+                                          int norm_whole, float eps, const double* __restrict__ freq, int dims, int interleaved,
                                           const int* __restrict__ positions, const int* __restrict__ slots,
                                           const float* __restrict__ factor, float temp_coef, int temp_every,
                                           int H, int G, int d, int dv, int D, int page_size, PooledWrite pw) {
     __shared__ float cs[128];                        // cos | sin of the token's dims / 2 angles
+    __shared__ float whole[2][33];
     const int t = blockIdx.x;
     const int half = dims >> 1;
     const int ipos = positions[t];
@@ -153,35 +156,57 @@ __global__ void attention_prepare4_kernel(const A* __restrict__ qkv, int ld, con
     const A* row = qkv + (size_t)t * ld;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     const int i0 = 4 * lane, last = slot < 0 ? H : H + 2 * G;         // k and v are the cache's alone
-    float x[4];
-    auto fetch = [&](int hh) {
-        const int n = hh < H + G ? d : dv, at = hh < H + G ? hh * d : (H + G) * d + (hh - H - G) * dv;
+    float x[HP][4];
+    auto fetch = [&](int h0) {                       // heads h0, h0 + nwarp, .. of this warp
 #pragma unroll
-        for (int j = 0; j < 4; ++j) x[j] = 0.f;
-        if (hh < last && i0 < n) {
-            load4(row + at + i0, x);
-            if (bias) {
-                float b[4];
-                load4(bias + at + i0, b);
+        for (int p = 0; p < HP; ++p) {
+            const int hh = h0 + p * nwarp;
+            const int n = hh < H + G ? d : dv, at = hh < H + G ? hh * d : (H + G) * d + (hh - H - G) * dv;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) x[j] += b[j];
+            for (int j = 0; j < 4; ++j) x[p][j] = 0.f;
+            if (hh < last && i0 < n) {
+                load4(row + at + i0, x[p]);
+                if (bias) {
+                    float b[4];
+                    load4(bias + at + i0, b);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) x[p][j] += b[j];
+                }
             }
         }
     };
-    fetch(warp);
+    auto squares = [&](int p) { return x[p][0] * x[p][0] + x[p][1] * x[p][1] + x[p][2] * x[p][2] + x[p][3] * x[p][3]; };
+    float inv_q = 1.f, inv_k = 1.f;
+    if (norm_whole && q_norm) {                      // last heads first: the first ones' numbers stay in registers
+        float sq = 0.f, sk = 0.f;
+        int h0 = warp;
+        while (h0 + HP * nwarp < last) h0 += HP * nwarp;
+        for (; h0 >= 0; h0 -= HP * nwarp) {
+            fetch(h0);
+#pragma unroll
+            for (int p = 0; p < HP; ++p) {
+                if (h0 + p * nwarp < H) sq += squares(p);
+                else if (h0 + p * nwarp < H + G) sk += squares(p);
+            }
+        }
+        inv_q = rsqrtf(block_sum(sq, whole[0]) / (float)(H * d) + eps);
+        inv_k = rsqrtf(block_sum(sk, whole[1]) / (float)(G * d) + eps);
+    } else {
+        fetch(warp);
+    }
     __syncthreads();
-    for (int hh = warp; hh < last; hh += nwarp) {
-        if (hh != warp) fetch(hh);
+    auto finish = [&](int hh, float (&v)[4]) {
         const bool is_q = hh < H, is_v = hh >= H + G;
         if (!is_v) {
             const float* w = is_q ? q_norm : k_norm;
             if (w) {
-                const float ss = warp_sum(x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3]);
-                const float inv = rsqrtf(ss / (float)d + eps);
+                float inv = is_q ? inv_q : inv_k;
+                if (norm_whole) w += (size_t)(is_q ? hh : hh - H) * d;
+                else inv = rsqrtf(warp_sum(v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3]) / (float)d + eps);
                 float g[4] = {0.f, 0.f, 0.f, 0.f};
                 if (i0 < d) load4(w + i0, g);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) x[j] = x[j] * inv * g[j];
+                for (int j = 0; j < 4; ++j) v[j] = v[j] * inv * g[j];
             }
             if (dims > 0) {
                 if (interleaved) {
@@ -189,9 +214,9 @@ __global__ void attention_prepare4_kernel(const A* __restrict__ qkv, int ld, con
 #pragma unroll
                         for (int j = 0; j < 4; j += 2) {
                             const int a = (i0 + j) >> 1;
-                            const float u = x[j], v = x[j + 1];
-                            x[j] = u * cs[a] - v * cs[half + a];
-                            x[j + 1] = v * cs[a] + u * cs[half + a];
+                            const float u = v[j], m = v[j + 1];
+                            v[j] = u * cs[a] - m * cs[half + a];
+                            v[j + 1] = m * cs[a] + u * cs[half + a];
                         }
                     }
                 } else {
@@ -199,12 +224,12 @@ __global__ void attention_prepare4_kernel(const A* __restrict__ qkv, int ld, con
                     const int mate = i0 < dims ? (first ? lane + (half >> 2) : lane - (half >> 2)) : lane;
                     float m[4];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) m[j] = __shfl_sync(0xffffffffu, x[j], mate);
+                    for (int j = 0; j < 4; ++j) m[j] = __shfl_sync(0xffffffffu, v[j], mate);
                     if (i0 < dims) {
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
                             const int a = (first ? i0 : i0 - half) + j;
-                            x[j] = first ? x[j] * cs[a] - m[j] * cs[half + a] : x[j] * cs[a] + m[j] * cs[half + a];
+                            v[j] = first ? v[j] * cs[a] - m[j] * cs[half + a] : v[j] * cs[a] + m[j] * cs[half + a];
                         }
                     }
                 }
@@ -212,12 +237,18 @@ __global__ void attention_prepare4_kernel(const A* __restrict__ qkv, int ld, con
             if (is_q) {
                 const float f = (factor ? factor[hh] : 1.f) * temp;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) x[j] *= f;
+                for (int j = 0; j < 4; ++j) v[j] *= f;
             }
         }
         if (i0 < D)
             store4((is_q ? q_out + ((size_t)t * H + hh) * D
-                         : kpage + (is_v ? (size_t)G * page_size * D : 0) + ((size_t)(is_v ? hh - H - G : hh - H) * page_size + off) * D) + i0, x);
+                         : kpage + (is_v ? (size_t)G * page_size * D : 0) + ((size_t)(is_v ? hh - H - G : hh - H) * page_size + off) * D) + i0, v);
+    };
+    for (int h0 = warp; h0 < last; h0 += HP * nwarp) {
+        if (h0 != warp) fetch(h0);
+#pragma unroll
+        for (int p = 0; p < HP; ++p)
+            if (h0 + p * nwarp < last) finish(h0 + p * nwarp, x[p]);
     }
     if (slot >= 0 && pw.pool > 0 && (ipos + 1) % pw.pool == 0) {
         __syncthreads();                                            // the token's own key and value are in place
@@ -250,18 +281,21 @@ extern "C" int rg_attention_prepare(const void* qkv, int dtype, int ld, const fl
     // four numbers at a time: sizes, pitches and addresses in multiples of four numbers of their types
     auto aligned = [](const void* p, int bytes) { return ((uintptr_t)p & (uintptr_t)(bytes - 1)) == 0; };
     const int in = dtype == RG_DTYPE_F32 ? 16 : 8, outb = out_dtype == RG_DTYPE_F32 ? 16 : 8;
-    if (!(norm_whole && q_norm) && D <= 128 && d % 4 == 0 && dv % 4 == 0 && D % 4 == 0 && dims % 8 == 0 && ld % 4 == 0 &&
+    if (D <= 128 && d % 4 == 0 && dv % 4 == 0 && D % 4 == 0 && dims % 8 == 0 && ld % 4 == 0 &&
         aligned(qkv, in) && aligned(q_out, outb) && aligned(kv, outb) && aligned(bias, 16) && aligned(q_norm, 16) &&
         aligned(k_norm, 16)) {
-        int nw = H + 2 * G < 16 ? H + 2 * G : 16;
-        if (nw < 4) nw = 4;
-#define RG_PREPARE4(A, O) return rg_launch(attention_prepare4_kernel<A, O>, dim3(T), dim3(32 * nw), 0, s, 1, \
-        (const A*)qkv, ld, bias, (O*)q_out, (O*)kv, q_norm, k_norm, eps, freq, dims, interleaved, positions, slots, \
+        const bool many = T > 148;
+        int nw = many ? (H + 2 * G + 3) / 4 : H + 2 * G;
+        nw = nw < (many ? 2 : 4) ? (many ? 2 : 4) : nw > 16 ? 16 : nw;
+#define RG_PREPARE4_(HP, A, O) return rg_launch(attention_prepare4_kernel<HP, A, O>, dim3(T), dim3(32 * nw), 0, s, 1, \
+        (const A*)qkv, ld, bias, (O*)q_out, (O*)kv, q_norm, k_norm, norm_whole, eps, freq, dims, interleaved, positions, slots, \
         factor, temp_coef, temp_every, H, G, d, dv, D, page_size, pw)
-        if (dtype == RG_DTYPE_BF16 && out_dtype == RG_DTYPE_BF16) RG_PREPARE4(bf16, bf16);
-        if (dtype == RG_DTYPE_F32 && out_dtype == RG_DTYPE_F32) RG_PREPARE4(float, float);
-        if (dtype == RG_DTYPE_F32 && out_dtype == RG_DTYPE_BF16) RG_PREPARE4(float, bf16);
+#define RG_PREPARE4(A, O) { if (many) RG_PREPARE4_(4, A, O); RG_PREPARE4_(1, A, O); }
+        if (dtype == RG_DTYPE_BF16 && out_dtype == RG_DTYPE_BF16) RG_PREPARE4(bf16, bf16)
+        if (dtype == RG_DTYPE_F32 && out_dtype == RG_DTYPE_F32) RG_PREPARE4(float, float)
+        if (dtype == RG_DTYPE_F32 && out_dtype == RG_DTYPE_BF16) RG_PREPARE4(float, bf16)
 #undef RG_PREPARE4
+#undef RG_PREPARE4_
     }
 #define RG_PREPARE(A, O) return rg_launch(attention_prepare_kernel<A, O>, dim3(T), dim3(32 * nwarp), smem, s, 1, \
         (const A*)qkv, ld, bias, (O*)q_out, (O*)kv, q_norm, k_norm, norm_whole, eps, freq, dims, interleaved, positions, slots, \

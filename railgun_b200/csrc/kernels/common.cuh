@@ -108,7 +108,7 @@ __device__ __forceinline__ int first_seen(int p, int window) {
 // in the stream is still running; it must not touch anything that kernel (or an earlier one) reads or writes
 // before pdl_wait(), which returns once the previous kernel has completed and its writes are visible.  Only
 // constants (weights) and the step's description (positions, slots, tiles, block tables: copied from the host before the
-// step's first kernel, never written by a kernel) may be read earlier.  pdl_trigger() lets the next kernel start launching.  Without the
+// step's first kernel, or by it in front of the embedding, which waits for it before it lets another start) may be read earlier.  pdl_trigger() lets the next kernel start launching.  Without the
 // attribute both are no-ops.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

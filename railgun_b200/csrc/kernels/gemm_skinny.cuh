@@ -56,6 +56,12 @@ struct SkinnyFusion {
     bf16* kv_cache;
     int nh, nkv, d, page_size, max_pos;
     int* err;                     // set to 1 when a position is outside the table (never read outside it)
+    // EPI_NONE: added to the 32-bit sums, in front of the one rounding [N] (nullptr: no bias)
+    const bf16* bias;
+    // EPI_NONE: several products of as many inputs in one launch.  W's rows are groups of group_rows (a multiple of 32; 0: one
+    // group); group i reads x + i group_x and writes its columns 0 .. group_rows - 1 at out + i group_out.
+    int group_rows;
+    size_t group_x, group_out;
 };
 
 __device__ __forceinline__ uint4 ld_stream16(const void* p) {
@@ -90,6 +96,8 @@ skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* __restrict__ x, int l
     const int g = lane >> 2, tq = lane & 3;
     const int rank = CS > 1 ? (int)(blockIdx.x % CS) : 0;
     const int n0 = (int)(blockIdx.x / CS) * ROWS;
+    const int group = EPI == EPI_NONE && fu.group_rows ? n0 / fu.group_rows : 0;     // a block's rows are of one group
+    x += group * fu.group_x;
     const int slice = ((K + CS * 128 - 1) / (CS * 128)) * 128;     // K slice of one block, a multiple of 128
     const int k_lo = rank * slice, k_hi = min(K, k_lo + slice);
     const bf16* w0[RT];
@@ -145,6 +153,8 @@ skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* __restrict__ x, int l
             pre_w = __ldg(fu.norm_w + n0 + row);
         }
     }
+    float pre_b = 0.f;                                 // EPI_NONE: the bias of the first element this thread will write
+    if (EPI == EPI_NONE && fu.bias && n0 + threadIdx.x % ROWS < N) pre_b = to_f32(fu.bias[n0 + threadIdx.x % ROWS]);
     bool first = true;
     for (; kb < k_hi; kb += NW * 128) {
         uint4 xq[MT][4];
@@ -292,10 +302,12 @@ skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* __restrict__ x, int l
             }
         }
     } else if (EPI == EPI_NONE) {
+        OUT* o = out + group * fu.group_out + n0 - group * fu.group_rows;
+        static_assert((NW * 32) % ROWS == 0, "a thread's elements are of one row of W");
         for (int idx = threadIdx.x; idx < ROWS * COLS; idx += NW * 32) {
             const int m = idx / ROWS, row = idx - m * ROWS;   // consecutive threads -> consecutive n: coalesced stores
             if (m < M && n0 + row < N)
-                out[(size_t)m * ldo + n0 + row] = from_f32<OUT>(fin[row * COLS + m] * (PRO == PRO_SCALED ? inv_rms(m) : 1.f));
+                o[(size_t)m * ldo + row] = from_f32<OUT>(fin[row * COLS + m] * (PRO == PRO_SCALED ? inv_rms(m) : 1.f) + pre_b);
         }
     } else {
         for (int idx = threadIdx.x; idx < (ROWS / 2) * COLS; idx += NW * 32) {

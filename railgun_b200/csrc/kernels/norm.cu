@@ -56,39 +56,80 @@ __device__ __forceinline__ void store4(bf16* p, float4 v) {
     *reinterpret_cast<uint2*>(p) = o;
 }
 
-template <typename P, typename O>
-__global__ void add_rmsnorm_vec4_kernel(float* __restrict__ resid, const P* __restrict__ pending,
+// NV > 0: a thread keeps its NV pieces of the row between the two passes, with every load of the row under way at once, and asks
+// for the norm's weight before the wait for the kernel before this one: few rows are bound by the trips to memory.  Many are
+// bound by their bytes and keep more of them under way with the registers that this would take (NV 0: the row is read again,
+// from L1).  Rows of 2,048, NV 0 and kept: 1 row 2.0 and 1.6 us, 32 2.5 and 1.9, 175 2.5 and 2.3, 1,056 4.4 and 4.9, 2,048 7.1 (50 MB)
+// and 7.3; rows of 4,096: 32 2.7 and 2.3, 1,056 7.3 and 8.0.
+template <int NV, typename P, typename O>
+__global__ void __launch_bounds__(1024) add_rmsnorm_vec4_kernel(float* __restrict__ resid, const P* __restrict__ pending,
                                         const float* __restrict__ w, float eps, O* __restrict__ out,
                                         const int* __restrict__ rows, int H) {
     __shared__ float scratch[33];
+    constexpr int KEEP = NV ? NV : 1;
+    const int orow = blockIdx.x;
+    float4 g[KEEP], v[KEEP], q[KEEP];
+    if constexpr (NV > 0) {
+#pragma unroll
+        for (int j = 0; j < KEEP; ++j) {
+            const int i = 4 * (threadIdx.x + j * blockDim.x);
+            if (i < H) g[j] = load4(w + i);
+        }
+    }
     pdl_wait();
     pdl_trigger();
-    const int orow = blockIdx.x;
     const int srow = rows ? rows[orow] : orow;
     float* r = resid + (size_t)srow * H;
     const P* p = pending ? pending + (size_t)srow * H : nullptr;
     const bool write_back = (rows == nullptr) && (p != nullptr);
     float ss = 0.f;
-    for (int i = threadIdx.x * 4; i < H; i += blockDim.x * 4) {
-        float4 v = load4(r + i);
-        if (p) {
-            const float4 q = load4(p + i);
-            v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
-            if (write_back) store4(r + i, v);
+    if constexpr (NV > 0) {
+#pragma unroll
+        for (int j = 0; j < KEEP; ++j) {
+            const int i = 4 * (threadIdx.x + j * blockDim.x);
+            v[j] = q[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (i < H) {
+                v[j] = load4(r + i);
+                if (p) q[j] = load4(p + i);
+            }
         }
-        ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+#pragma unroll
+        for (int j = 0; j < KEEP; ++j) {
+            v[j].x += q[j].x; v[j].y += q[j].y; v[j].z += q[j].z; v[j].w += q[j].w;
+            ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
+        }
+    } else {
+        for (int i = threadIdx.x * 4; i < H; i += blockDim.x * 4) {
+            float4 x = load4(r + i);
+            if (p) {
+                const float4 y = load4(p + i);
+                x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+                if (write_back) store4(r + i, x);
+            }
+            ss += x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
+        }
     }
     ss = block_sum(ss, scratch);
     const float inv = rsqrtf(ss / (float)H + eps);
     O* o = out + (size_t)orow * H;
-    for (int i = threadIdx.x * 4; i < H; i += blockDim.x * 4) {
-        float4 v = load4(r + i);
-        if (p && !write_back) {
-            const float4 q = load4(p + i);
-            v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
+    if constexpr (NV > 0) {
+#pragma unroll
+        for (int j = 0; j < KEEP; ++j) {
+            const int i = 4 * (threadIdx.x + j * blockDim.x);
+            if (i >= H) continue;
+            if (write_back) store4(r + i, v[j]);
+            store4(o + i, make_float4(v[j].x * inv * g[j].x, v[j].y * inv * g[j].y, v[j].z * inv * g[j].z, v[j].w * inv * g[j].w));
         }
-        const float4 g = load4(w + i);
-        store4(o + i, make_float4(v.x * inv * g.x, v.y * inv * g.y, v.z * inv * g.z, v.w * inv * g.w));
+    } else {
+        for (int i = threadIdx.x * 4; i < H; i += blockDim.x * 4) {
+            float4 x = load4(r + i);
+            if (p && !write_back) {
+                const float4 y = load4(p + i);
+                x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+            }
+            const float4 a = load4(w + i);
+            store4(o + i, make_float4(x.x * inv * a.x, x.y * inv * a.y, x.z * inv * a.z, x.w * inv * a.w));
+        }
     }
 }
 
@@ -101,6 +142,8 @@ __global__ void residual_add_kernel(float* __restrict__ resid, const P* __restri
     if (i < n) resid[i] += to_f32(pending[i]);
 }
 
+#define NORM_KEPT_ROWS 592
+
 extern "C" int rg_add_rmsnorm(float* resid, const void* pending, int pending_dtype, const float* w,
                               float eps, void* out, int out_dtype, const int* rows, int n_out_rows,
                               int H, void* stream) {
@@ -108,9 +151,15 @@ extern "C" int rg_add_rmsnorm(float* resid, const void* pending, int pending_dty
     cudaStream_t s = (cudaStream_t)stream;
     const bool vec = H % 4 == 0 && (uintptr_t)resid % 16 == 0 && (uintptr_t)out % 16 == 0 &&
                      (uintptr_t)pending % 16 == 0 && (uintptr_t)w % 16 == 0;
-    const int threads = vec ? (H >= 4096 ? 512 : (H >= 1024 ? 256 : 128)) : (H >= 2048 ? 512 : (H >= 512 ? 256 : 128));
-#define RG_NORM(P, O) return vec ? rg_launch(add_rmsnorm_vec4_kernel<P, O>, dim3(n_out_rows), dim3(threads), 0, s, 1, \
-        resid, (const P*)pending, w, eps, (O*)out, rows, H) \
+    // kept rows: as many as four blocks an SM hold, one piece a thread unless a block of 1,024 threads cannot hold the row so
+    const int work = (H + 3) / 4, nv = work <= 1024 ? 1 : work <= 2048 ? 2 : 4;
+    const bool kept = vec && n_out_rows <= NORM_KEPT_ROWS && work <= 4096;
+    const int threads = kept ? ((work + nv - 1) / nv + 31) / 32 * 32
+                       : vec ? (H >= 4096 ? 512 : (H >= 1024 ? 256 : 128)) : (H >= 2048 ? 512 : (H >= 512 ? 256 : 128));
+#define RG_NORM_NV(NV, P, O) rg_launch(add_rmsnorm_vec4_kernel<NV, P, O>, dim3(n_out_rows), dim3(threads), 0, s, 1, \
+        resid, (const P*)pending, w, eps, (O*)out, rows, H)
+#define RG_NORM(P, O) return kept ? (nv == 1 ? RG_NORM_NV(1, P, O) : nv == 2 ? RG_NORM_NV(2, P, O) : RG_NORM_NV(4, P, O)) \
+      : vec ? RG_NORM_NV(0, P, O) \
       : rg_launch(add_rmsnorm_kernel<P, O>, dim3(n_out_rows), dim3(threads), 0, s, 1, \
         resid, (const P*)pending, w, eps, (O*)out, rows, H)
     if (pending == nullptr) pending_dtype = out_dtype;
@@ -119,6 +168,7 @@ extern "C" int rg_add_rmsnorm(float* resid, const void* pending, int pending_dty
     if (pending_dtype == RG_DTYPE_F32 && out_dtype == RG_DTYPE_BF16) RG_NORM(float, bf16);
     if (pending_dtype == RG_DTYPE_BF16 && out_dtype == RG_DTYPE_F32) RG_NORM(bf16, float);
 #undef RG_NORM
+#undef RG_NORM_NV
     return RG_ERR_UNSUPPORTED;
 }
 
@@ -286,12 +336,27 @@ __device__ __forceinline__ float4 load_any4(const void* p, int dtype, size_t i) 
     return *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p) + i);
 }
 
-template <typename O>
+// A thread keeps its NV pieces of a group between the two passes (NV 0: any number, read again: as above; four groups of rows of
+// 2,048, read again and kept: 1 row 2.6 and 2.1 us, 175 3.3 and 2.8, 2,048 9.9 and 10.5; of 4,096: 32 4.6 and 3.9, 175 4.7 and 4.4,
+// 1,056 8.8 and 14.1).
+template <int NV, typename O>
 __global__ void __launch_bounds__(256) add_group_rmsnorm4_kernel(
         float* __restrict__ resid, const void* __restrict__ p1, int p1_dtype, const void* __restrict__ p2, int p2_dtype,
         const float* __restrict__ w1, const float* __restrict__ w2, float eps, O* __restrict__ out1,
         O* __restrict__ out2, const int* __restrict__ rows, int H, int groups, int wpt) {
     __shared__ float scratch[8];
+    constexpr int KEEP = NV ? NV : 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nteams = 8 / wpt, team = warp / wpt, in_team = (warp - team * wpt) * 32 + lane, team_threads = wpt * 32;
+    const int gs = H / groups, gs4 = gs >> 2;
+    float4 a1[KEEP];                                      // the first group's weight, asked for before the wait
+    auto weights = [&](int g) {
+#pragma unroll
+        for (int j = 0; j < KEEP; ++j)
+            if (NV && g < groups && in_team + j * team_threads < gs4)
+                a1[j] = *reinterpret_cast<const float4*>(w1 + g * gs + 4 * (in_team + j * team_threads));
+    };
+    weights(team);
     pdl_wait();
     pdl_trigger();
     const int orow = blockIdx.x;
@@ -299,24 +364,50 @@ __global__ void __launch_bounds__(256) add_group_rmsnorm4_kernel(
     float* r = resid + (size_t)srow * H;
     const size_t pbase = (size_t)srow * H;
     const bool write_back = rows == nullptr && (p1 != nullptr || p2 != nullptr);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nteams = 8 / wpt, team = warp / wpt, in_team = (warp - team * wpt) * 32 + lane, team_threads = wpt * 32;
-    const int gs = H / groups, gs4 = gs >> 2;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto sum = [&](float4 v, float4 a, float4 b) {        // the row's number, then the parts in order
+        if (p1) { v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w; }
+        if (p2) { v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w; }
+        return v;
+    };
+    auto finish = [&](int i, float4 v, float inv, float4 a) {
+        v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
+        store4(out1 + (size_t)orow * H + i, make_float4(v.x * a.x, v.y * a.y, v.z * a.z, v.w * a.w));
+        if (out2) {
+            const float4 b = *reinterpret_cast<const float4*>(w2 + i);
+            store4(out2 + (size_t)orow * H + i, make_float4(v.x * b.x, v.y * b.y, v.z * b.z, v.w * b.w));
+        }
+    };
     for (int g0 = 0; g0 < groups; g0 += nteams) {
         const int g = g0 + team;
         const bool active = g < groups;
         const int lo = g * gs;
+        if (g0 > 0) weights(g);
         float ss = 0.f;
-        if (active) {
+        float4 v[KEEP], a[KEEP], b[KEEP];
+        if (NV) {
+#pragma unroll
+            for (int j = 0; j < KEEP; ++j) {
+                const int i4 = in_team + j * team_threads, i = lo + 4 * i4;
+                v[j] = a[j] = b[j] = zero;
+                if (active && i4 < gs4) {
+                    v[j] = *reinterpret_cast<const float4*>(r + i);
+                    if (p1) a[j] = load_any4(p1, p1_dtype, pbase + i);
+                    if (p2) b[j] = load_any4(p2, p2_dtype, pbase + i);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < KEEP; ++j) {
+                v[j] = sum(v[j], a[j], b[j]);
+                ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
+            }
+        } else if (active) {
             for (int i4 = in_team; i4 < gs4; i4 += team_threads) {
                 const int i = lo + 4 * i4;
-                float4 v = *reinterpret_cast<const float4*>(r + i);
-                if (p1 || p2) {
-                    if (p1) { const float4 a = load_any4(p1, p1_dtype, pbase + i); v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w; }
-                    if (p2) { const float4 a = load_any4(p2, p2_dtype, pbase + i); v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w; }
-                    if (write_back) *reinterpret_cast<float4*>(r + i) = v;
-                }
-                ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+                const float4 x = sum(*reinterpret_cast<const float4*>(r + i), p1 ? load_any4(p1, p1_dtype, pbase + i) : zero,
+                                     p2 ? load_any4(p2, p2_dtype, pbase + i) : zero);
+                if (write_back) *reinterpret_cast<float4*>(r + i) = x;
+                ss += x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
             }
         }
         ss = warp_sum(ss);
@@ -329,19 +420,21 @@ __global__ void __launch_bounds__(256) add_group_rmsnorm4_kernel(
         }
         if (!active) continue;
         const float inv = rsqrtf(ss / (float)gs + eps);
-        for (int i4 = in_team; i4 < gs4; i4 += team_threads) {
-            const int i = lo + 4 * i4;
-            float4 v = *reinterpret_cast<const float4*>(r + i);
-            if (!write_back && (p1 || p2)) {
-                if (p1) { const float4 a = load_any4(p1, p1_dtype, pbase + i); v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w; }
-                if (p2) { const float4 a = load_any4(p2, p2_dtype, pbase + i); v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w; }
+        if (NV) {
+#pragma unroll
+            for (int j = 0; j < KEEP; ++j) {
+                const int i4 = in_team + j * team_threads, i = lo + 4 * i4;
+                if (i4 >= gs4) continue;
+                if (write_back) *reinterpret_cast<float4*>(r + i) = v[j];
+                finish(i, v[j], inv, a1[j]);
             }
-            v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
-            const float4 a = *reinterpret_cast<const float4*>(w1 + i);
-            store4(out1 + (size_t)orow * H + i, make_float4(v.x * a.x, v.y * a.y, v.z * a.z, v.w * a.w));
-            if (out2) {
-                const float4 b = *reinterpret_cast<const float4*>(w2 + i);
-                store4(out2 + (size_t)orow * H + i, make_float4(v.x * b.x, v.y * b.y, v.z * b.z, v.w * b.w));
+        } else {
+            for (int i4 = in_team; i4 < gs4; i4 += team_threads) {
+                const int i = lo + 4 * i4;
+                float4 x = *reinterpret_cast<const float4*>(r + i);
+                if (!write_back)
+                    x = sum(x, p1 ? load_any4(p1, p1_dtype, pbase + i) : zero, p2 ? load_any4(p2, p2_dtype, pbase + i) : zero);
+                finish(i, x, inv, *reinterpret_cast<const float4*>(w1 + i));
             }
         }
     }
@@ -358,12 +451,15 @@ extern "C" int rg_add_group_rmsnorm(float* resid, const void* p1, int p1_dtype, 
     auto aligned = [](const void* p, int dtype) { return ((uintptr_t)p & (dtype == RG_DTYPE_BF16 ? 7 : 15)) == 0; };
     if ((H / groups) % 4 == 0 && ((uintptr_t)resid & 15) == 0 && aligned(p1, p1_dtype) && aligned(p2, p2_dtype) &&
         ((uintptr_t)w1 & 15) == 0 && ((uintptr_t)w2 & 15) == 0 && aligned(out1, out_dtype) && aligned(out2, out_dtype)) {
-        if (out_dtype == RG_DTYPE_BF16)
-            return rg_launch(add_group_rmsnorm4_kernel<bf16>, dim3(n_out_rows), dim3(256), 0, s, 1, resid, p1, p1_dtype,
-                             p2, p2_dtype, w1, w2, eps, (bf16*)out1, (bf16*)out2, rows, H, groups, wpt);
-        if (out_dtype == RG_DTYPE_F32)
-            return rg_launch(add_group_rmsnorm4_kernel<float>, dim3(n_out_rows), dim3(256), 0, s, 1, resid, p1, p1_dtype,
-                             p2, p2_dtype, w1, w2, eps, (float*)out1, (float*)out2, rows, H, groups, wpt);
+        const int per_thread = (H / groups / 4 + 32 * wpt - 1) / (32 * wpt);
+#define RG_GROUP(NV, O) return rg_launch(add_group_rmsnorm4_kernel<NV, O>, dim3(n_out_rows), dim3(256), 0, s, 1, resid, p1, p1_dtype, \
+                             p2, p2_dtype, w1, w2, eps, (O*)out1, (O*)out2, rows, H, groups, wpt)
+#define RG_GROUPS(O) { if (n_out_rows > NORM_KEPT_ROWS) RG_GROUP(0, O); if (per_thread <= 1) RG_GROUP(1, O); if (per_thread <= 2) RG_GROUP(2, O); if (per_thread <= 4) RG_GROUP(4, O); \
+                       RG_GROUP(0, O); }
+        if (out_dtype == RG_DTYPE_BF16) RG_GROUPS(bf16)
+        if (out_dtype == RG_DTYPE_F32) RG_GROUPS(float)
+#undef RG_GROUPS
+#undef RG_GROUP
     }
     if (out_dtype == RG_DTYPE_BF16)
         return rg_launch(add_group_rmsnorm_kernel<bf16>, dim3(n_out_rows), dim3(256), 0, s, 1, resid, p1, p1_dtype, p2,

@@ -43,6 +43,7 @@ extern "C" int rg_ssd_prepare(const float* raw, int raw_ld, const float* dt_bias
 // side by side, raw dt at dt_off (32-bit rows).  conv_state [slots, K - 1, C] (C = H dv + 2 G N), taps [K, C], bias [C].
 // state [slots, H, dv, N]: S transposed.  o [T, H, dv].  A warp takes one column of S at a time: N numbers side by side.
 #define SSD_THREADS 256
+#define SSD_AHEAD 4               // taps whose weights and inputs a thread asks for ahead, for its first channel
 template <bool VEC>
 __global__ void __launch_bounds__(SSD_THREADS)
 ssd_step_kernel(const float* __restrict__ proj, int ld, int x_off, int dt_off, const float* __restrict__ taps,
@@ -53,8 +54,6 @@ ssd_step_kernel(const float* __restrict__ proj, int ld, int x_off, int dt_off, c
     extern __shared__ __align__(16) float sm[];       // B [N], C [N] (padded to 4), x [cols]
     const int NP = (N + 3) & ~3;
     float *sB = sm, *sC = sm + NP, *sx = sm + 2 * NP;
-    pdl_wait();
-    pdl_trigger();
     const int t = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * cols;
     const int n = min(cols, dv - j0);
     const int r = req_of_token[t];
@@ -63,30 +62,62 @@ ssd_step_kernel(const float* __restrict__ proj, int ld, int x_off, int dt_off, c
     const int grp = h / (H / G), C = H * dv + 2 * G * N;
     const float* row = proj + (size_t)t * ld;
     const float* past = conv_state + (size_t)(slot >= 0 ? slot : 0) * (K - 1) * C;
-    for (int e = threadIdx.x; e < 2 * N + n; e += blockDim.x) {
-        const int c = e < N ? H * dv + grp * N + e : (e < 2 * N ? H * dv + G * N + grp * N + (e - N) : h * dv + j0 + (e - 2 * N));
-        float acc = bias ? bias[c] : 0.f;
-        if (has_past)
-            for (int j = 0; j < K - 1; ++j) acc += taps[(size_t)j * C + c] * past[(size_t)j * C + c];
-        acc += taps[(size_t)(K - 1) * C + c] * row[x_off + c];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float* st = state + (((size_t)(slot >= 0 ? slot : 0) * H + h) * dv + j0) * N;
+    // A step is a chain of trips to memory.  The weights are asked for in front of the wait for the kernel before this one; behind
+    // it everything else at once: the row, the convolution's past and the warp's first column of S.
+    auto channel = [&](int e) {
+        return e < N ? H * dv + grp * N + e : (e < 2 * N ? H * dv + G * N + grp * N + (e - N) : h * dv + j0 + (e - 2 * N));
+    };
+    const int e0 = threadIdx.x, c0 = e0 < 2 * N + n ? channel(e0) : 0;
+    float w0[SSD_AHEAD], b0 = bias ? bias[c0] : 0.f;
+#pragma unroll
+    for (int j = 0; j < SSD_AHEAD; ++j) w0[j] = j < K ? taps[(size_t)(K - 1 - j) * C + c0] : 0.f;      // the newest first
+    const float dtb = dt_bias[h], rate = -expf(A_log[h]), skip = D[h];
+    pdl_wait();
+    pdl_trigger();
+    const float raw = row[dt_off + h], x0 = row[x_off + c0];
+    float p0[SSD_AHEAD];
+#pragma unroll
+    for (int j = 1; j < SSD_AHEAD; ++j) p0[j] = has_past && j < K ? past[(size_t)(K - 1 - j) * C + c0] : 0.f;
+    float4 S0 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (VEC && has_past && warp < n && lane * 4 < N) S0 = *reinterpret_cast<const float4*>(st + (size_t)warp * N + lane * 4);
+    for (int e = e0; e < 2 * N + n; e += blockDim.x) {
+        float acc;
+        if (e == e0) {
+            acc = b0;
+            if (has_past) {
+                for (int j = 0; j < K - SSD_AHEAD; ++j) acc += taps[(size_t)j * C + c0] * past[(size_t)j * C + c0];
+#pragma unroll
+                for (int j = SSD_AHEAD - 1; j > 0; --j)
+                    if (j < K) acc += w0[j] * p0[j];
+            }
+            acc += w0[0] * x0;
+        } else {
+            const int c = channel(e);
+            acc = bias ? bias[c] : 0.f;
+            if (has_past)
+#pragma unroll 4
+                for (int j = 0; j < K - 1; ++j) acc += taps[(size_t)j * C + c] * past[(size_t)j * C + c];
+            acc += taps[(size_t)(K - 1) * C + c] * row[x_off + c];
+        }
         acc = ssd_silu(acc);
         if (e < N) sB[e] = acc;
         else if (e < 2 * N) sC[e - N] = acc;
         else sx[e - 2 * N] = acc;
     }
-    const float dt = ssd_softplus(row[dt_off + h] + dt_bias[h]);
-    const float g = expf(-expf(A_log[h]) * dt);
-    const float skip = D[h];
+    const float dt = ssd_softplus(raw + dtb);
+    const float g = expf(rate * dt);
     __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float* st = state + (((size_t)(slot >= 0 ? slot : 0) * H + h) * dv + j0) * N;
     for (int j = warp; j < n; j += SSD_THREADS / 32) {
         float* col = st + (size_t)j * N;
         const float u = dt * sx[j];
         float acc = 0.f;
         if (VEC) {
             for (int i = lane * 4; i < N; i += 128) {
-                float4 S = has_past ? *reinterpret_cast<const float4*>(col + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                float4 S = j == warp && i < 128 ? S0
+                           : has_past           ? *reinterpret_cast<const float4*>(col + i)
+                                                : make_float4(0.f, 0.f, 0.f, 0.f);
                 const float4 b = *reinterpret_cast<const float4*>(sB + i), c = *reinterpret_cast<const float4*>(sC + i);
                 S.x = S.x * g + b.x * u; S.y = S.y * g + b.y * u; S.z = S.z * g + b.z * u; S.w = S.w * g + b.w * u;
                 acc += S.x * c.x + S.y * c.y + S.z * c.z + S.w * c.w;
@@ -129,6 +160,7 @@ extern "C" int rg_ssd_step(const float* proj, int ld, int x_off, int dt_off, con
 // o [T, n] float; z: rows z_ld apart (type Z).  One block per (token, group of n / groups numbers); the gated numbers
 // wait in shared memory for the group's root mean square.  With `raw` (rows raw_ld apart, C numbers) further blocks of
 // the same launch move the convolution state of the token's request on by that one token (single-token steps).
+#define GGN_AHEAD 4
 template <typename Z, typename O>
 __global__ void gate_group_norm_kernel(const float* __restrict__ o, const Z* __restrict__ z, int z_ld,
                                        const float* __restrict__ weight, float eps, O* __restrict__ out, int n, int gs,
@@ -137,14 +169,14 @@ __global__ void gate_group_norm_kernel(const float* __restrict__ o, const Z* __r
                                        const int* __restrict__ start_pos, const int* __restrict__ slots, int C, int K) {
     extern __shared__ __align__(16) float y[];        // [gs]
     __shared__ float scratch[33];
-    pdl_wait();
-    pdl_trigger();
     const int t = blockIdx.x;
     if ((int)blockIdx.y >= groups) {
         const int c = (blockIdx.y - groups) * blockDim.x + threadIdx.x;
         const int r = req_of_token[t], slot = slots[r];
-        if (slot < 0 || c >= C) return;
         const bool has_past = start_pos[r] > 0;
+        pdl_wait();
+        pdl_trigger();
+        if (slot < 0 || c >= C) return;
         float* st = conv_state + (size_t)slot * (K - 1) * C + c;
         const float now = raw[(size_t)t * raw_ld + c];
         for (int j0 = 0; j0 < K - 2; j0 += 4) {       // four rows at a time, each read before the one above it is written
@@ -161,14 +193,25 @@ __global__ void gate_group_norm_kernel(const float* __restrict__ o, const Z* __r
     const int base = blockIdx.y * gs;
     const float* src = o + (size_t)t * n + base;
     const Z* zr = z + (size_t)t * z_ld + base;
+    float w[GGN_AHEAD];                               // the first weights, asked for before the wait
+#pragma unroll
+    for (int j = 0; j < GGN_AHEAD; ++j) w[j] = threadIdx.x + j * blockDim.x < gs ? weight[base + threadIdx.x + j * blockDim.x] : 0.f;
+    pdl_wait();
+    pdl_trigger();
     float ss = 0.f;
+#pragma unroll 4
     for (int i = threadIdx.x; i < gs; i += blockDim.x) {
         const float v = src[i] * ssd_silu(to_f32(zr[i]));
         y[i] = v;
         ss += v * v;
     }
     const float inv = rsqrtf(block_sum(ss, scratch) / (float)gs + eps);
-    for (int i = threadIdx.x; i < gs; i += blockDim.x)
+#pragma unroll
+    for (int j = 0; j < GGN_AHEAD; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        if (i < gs) out[(size_t)t * n + base + i] = from_f32<O>(y[i] * inv * w[j]);
+    }
+    for (int i = threadIdx.x + GGN_AHEAD * blockDim.x; i < gs; i += blockDim.x)
         out[(size_t)t * n + base + i] = from_f32<O>(y[i] * inv * weight[base + i]);
 }
 

@@ -117,6 +117,115 @@ __global__ void postnorm_shift_kernel(const float* __restrict__ x, const P* __re
     }
 }
 
+// The same for blocks of one row whose numbers fit in registers, NV pieces of four a thread: the row and the one before it are
+// asked for together, right behind the wait for the kernel before this one, and what does not depend on that kernel (the step's
+// description, the weights) in front of it.  Such a step is a chain of trips to memory: a row of 2,048 2.0 us, with the
+// rows read again in both passes 3.0.
+__device__ __forceinline__ float2 block_sum2(float a, float b, float (*scratch)[2]) {       // scratch [33][2]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+    a = warp_sum(a);
+    b = warp_sum(b);
+    __syncthreads();
+    if (lane == 0) { scratch[warp][0] = a; scratch[warp][1] = b; }
+    __syncthreads();
+    a = lane < nwarp ? scratch[lane][0] : 0.f;                  // every warp adds the warps' sums up, in the same order
+    b = lane < nwarp ? scratch[lane][1] : 0.f;
+    return make_float2(warp_sum(a), warp_sum(b));
+}
+template <int NV, typename P, typename O>
+__global__ void __launch_bounds__(1024)
+postnorm_shift_row_kernel(const float* __restrict__ x, const P* __restrict__ y, const float* __restrict__ post_w, float eps,
+                          const float* __restrict__ shift, float* __restrict__ state, const int* __restrict__ cu_seqlens,
+                          const int* __restrict__ req_of_token, const int* __restrict__ start_pos, const int* __restrict__ slots,
+                          float* __restrict__ x_out, O* __restrict__ out, int H) {
+    __shared__ float scratch[33][2];
+    const int t = blockIdx.x;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    bool first = false, has_past = false;
+    int slot = -1, last = t;
+    if (shift) {
+        const int r = req_of_token[t];
+        first = t == cu_seqlens[r];
+        last = cu_seqlens[r + 1] - 1;
+        slot = slots[r];
+        has_past = first && slot >= 0 && start_pos[r] > 0;
+    }
+    auto at = [&](int j) { return 4 * (int)(threadIdx.x + j * blockDim.x); };
+    float4 w[NV], sh[NV], v[NV], p[NV], bv[NV], bp[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        w[j] = sh[j] = zero;
+        if (at(j) < H && y && post_w) w[j] = load4(post_w + at(j));
+        if (at(j) < H && shift) sh[j] = load4(shift + at(j));
+    }
+    pdl_wait();
+    pdl_trigger();
+    float* st = state + (size_t)(slot >= 0 ? slot : 0) * H;
+    const bool inside = shift && !first;                        // the row before this one is the step's
+    auto fetch = [&](int row, float4 (&a)[NV], float4 (&b)[NV]) {
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            a[j] = b[j] = zero;
+            if (at(j) >= H) continue;
+            a[j] = load4(x + (size_t)row * H + at(j));
+            if (y) b[j] = load4(y + (size_t)row * H + at(j));
+        }
+    };
+    auto squares = [&](const float4 (&b)[NV]) {
+        float ss = 0.f;
+#pragma unroll
+        for (int j = 0; j < NV; ++j) ss += b[j].x * b[j].x + b[j].y * b[j].y + b[j].z * b[j].z + b[j].w * b[j].w;
+        return ss;
+    };
+    auto add = [&](float4 (&a)[NV], const float4 (&b)[NV], float inv) {
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            if (post_w) {
+                a[j].x += b[j].x * inv * w[j].x; a[j].y += b[j].y * inv * w[j].y;
+                a[j].z += b[j].z * inv * w[j].z; a[j].w += b[j].w * inv * w[j].w;
+            } else {
+                a[j].x += b[j].x; a[j].y += b[j].y; a[j].z += b[j].z; a[j].w += b[j].w;
+            }
+        }
+    };
+    fetch(t, v, p);
+    if (inside) {
+        fetch(t - 1, bv, bp);
+    } else {
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            bv[j] = bp[j] = zero;
+            if (has_past && at(j) < H) bv[j] = load4(st + at(j));
+        }
+    }
+    float2 inv = make_float2(1.f, 1.f);
+    if (y && post_w) {
+        const float2 ss = block_sum2(squares(p), squares(bp), scratch);
+        inv = make_float2(rsqrtf(ss.x / (float)H + eps), rsqrtf(ss.y / (float)H + eps));
+    }
+    if (y) {
+        add(v, p, inv.x);
+        if (inside) add(bv, bp, inv.y);
+    }
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        if (at(j) >= H) continue;
+        store4(x_out + (size_t)t * H + at(j), v[j]);
+        const float4 h = shift ? make_float4(v[j].x + (bv[j].x - v[j].x) * sh[j].x, v[j].y + (bv[j].y - v[j].y) * sh[j].y,
+                                             v[j].z + (bv[j].z - v[j].z) * sh[j].z, v[j].w + (bv[j].w - v[j].w) * sh[j].w)
+                               : v[j];
+        store4(out + (size_t)t * H + at(j), h);
+        if (first && last == t && slot >= 0) store4(st + at(j), v[j]);
+    }
+    if (first && last > t && slot >= 0) {                       // the slot gets the step's last row
+        fetch(last, v, p);
+        if (y) add(v, p, y && post_w ? rsqrtf(block_sum2(squares(p), 0.f, scratch).x / (float)H + eps) : 1.f);
+#pragma unroll
+        for (int j = 0; j < NV; ++j)
+            if (at(j) < H) store4(st + at(j), v[j]);
+    }
+}
+
 extern "C" int rg_postnorm_shift(const float* x, const void* y, int y_dtype, const float* post_w, float eps,
                                  const float* shift, float* state, const int* cu_seqlens, const int* req_of_token,
                                  const int* start_pos, const int* slots, float* x_out, void* out, int out_dtype, int T,
@@ -134,15 +243,22 @@ extern "C" int rg_postnorm_shift(const float* x, const void* y, int y_dtype, con
     const int threads = work >= 512 ? 512 : (work >= 256 ? 256 : 128);
     dim3 grid((T + rows_per_block - 1) / rows_per_block);
     if (!y) y_dtype = RG_DTYPE_F32;
+    // (rows that are not shifted read nothing twice that matters: many of them are faster with fewer registers a thread, 2,000 rows
+    // of 2,048 8.6 us against 12.3; shifted, 16.6 against 15.0)
+    const bool one_row = vec && (rows_per_block == 1 || T == 1) && work <= 2048 && (shift || T <= 592);
+    const int nv = work <= 1024 ? 1 : 2, row_threads = ((work + nv - 1) / nv + 31) / 32 * 32;
+#define TS_ROW(NV, P, O) return rg_launch(postnorm_shift_row_kernel<NV, P, O>, dim3(T), dim3(row_threads), 0, s, 1, x, (const P*)y, \
+        post_w, eps, shift, state, cu_seqlens, req_of_token, start_pos, slots, x_out, (O*)out, H)
 #define TS_LAUNCH(V, P, O) return rg_launch(postnorm_shift_kernel<V, P, O>, grid, dim3(threads), smem, s, 1, x, (const P*)y, \
         post_w, eps, shift, state, cu_seqlens, req_of_token, start_pos, slots, x_out, (O*)out, T, H, rows_per_block)
-#define TS_TYPES(P, O) { if (vec) TS_LAUNCH(4, P, O); TS_LAUNCH(1, P, O); }
+#define TS_TYPES(P, O) { if (one_row) { if (nv == 1) TS_ROW(1, P, O); TS_ROW(2, P, O); } if (vec) TS_LAUNCH(4, P, O); TS_LAUNCH(1, P, O); }
     if (y_dtype == RG_DTYPE_BF16 && out_dtype == RG_DTYPE_BF16) TS_TYPES(bf16, bf16)
     if (y_dtype == RG_DTYPE_F32 && out_dtype == RG_DTYPE_BF16) TS_TYPES(float, bf16)
     if (y_dtype == RG_DTYPE_F32 && out_dtype == RG_DTYPE_F32) TS_TYPES(float, float)
     if (y_dtype == RG_DTYPE_BF16 && out_dtype == RG_DTYPE_F32) TS_TYPES(bf16, float)
 #undef TS_TYPES
 #undef TS_LAUNCH
+#undef TS_ROW
     return RG_ERR_UNSUPPORTED;
 }
 

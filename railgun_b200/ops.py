@@ -989,13 +989,15 @@ def recurrent_scan(proj: torch.Tensor, y_off: int, x_off: int, yb, xb, u: torch.
 # ---- short convolutions with state, matrix-state mixers (retention, delta rule), attention's per-token work -------
 
 def causal_conv(x: torch.Tensor, x_off: int, taps: torch.Tensor, state, batch, out_dtype, residual: bool = False,
-                silu: bool = False, out: torch.Tensor | None = None, bias: torch.Tensor | None = None) -> torch.Tensor:
+                silu: bool = False, out: torch.Tensor | None = None, bias: torch.Tensor | None = None,
+                update: bool = False) -> torch.Tensor:
     """[T, C]: per channel the causal convolution of x[:, x_off:x_off + C] with ``taps`` [K, C] (tap-major: what the
     tensor files hold as [C, K], transposed once at load; last row: the
     current token's) along each request's tokens, continued from the K - 1 inputs in the request's state slot
     (``state`` [slots, K - 1, C] float32; None when K = 1) unless the request starts at position 0.  ``silu``:
     the activation on the convolution (and its ``bias`` [C], if there is one); ``residual``: x is added.  32-bit arithmetic, one rounding into
-    ``out_dtype``.  The state is not changed (``conv_state_update`` does that, afterwards)."""
+    ``out_dtype``.  The state is not changed, unless ``update`` says that the step's last inputs are to be left in it, as
+    ``conv_state_update`` does (in the same kernel where every request brings one token)."""
     _check_rows(x, "x")
     _check(taps, "taps", torch.float32)
     K, C = taps.shape
@@ -1017,7 +1019,9 @@ def causal_conv(x: torch.Tensor, x_off: int, taps: torch.Tensor, state, batch, o
         _ptr(x), c_int(_dtype_code(x)), c_int(x.stride(0)), c_int(x_off), _ptr(taps), _ptr(bias),
         _ptr(state if K > 1 else None), _ptr(batch.cu_seqlens), _ptr(batch.req_of_token), _ptr(batch.start_pos), _ptr(batch.state_slots), _ptr(out),
         c_int(_dtype_code(out)), c_int(out.stride(0)), c_int(T), c_int(C), c_int(K), c_int(1 if residual else 0),
-        c_int(1 if silu else 0), _stream()), "causal_conv")
+        c_int(1 if silu else 0), c_int(1 if update and K > 1 and batch.decode_only else 0), _stream()), "causal_conv")
+    if update and K > 1 and not batch.decode_only:
+        conv_state_update(x, x_off, state, batch)
     return out
 
 
@@ -1760,8 +1764,9 @@ def skinny_gemm_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
             and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and weight.is_contiguous())
 
 
-def skinny_gemm(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, silu_mul: bool = False) -> torch.Tensor:
-    """y = x W^T for up to 64 rows of x, reading W once at memory speed.
+def skinny_gemm(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, silu_mul: bool = False,
+                bias: torch.Tensor | None = None) -> torch.Tensor:
+    """y = x W^T (+ ``bias`` [N] bfloat16) for up to 64 rows of x, reading W once at memory speed.
     ``silu_mul``: W is interleaved gate|up storage and y = silu(gate) * up."""
     if not skinny_gemm_ok(x, weight):
         raise KernelError(f"skinny_gemm refuses x {tuple(x.shape)} {x.dtype}, W {tuple(weight.shape)} {weight.dtype}: "
@@ -1773,11 +1778,35 @@ def skinny_gemm(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, silu_mul:
     out_dtype = out_dtype or torch.bfloat16
     if silu_mul and (N % 16 or out_dtype != torch.bfloat16):
         raise KernelError("skinny_gemm: the SiLU-mul epilogue needs N % 16 == 0 and bfloat16 output")
+    if bias is not None:
+        _check(bias, "bias", torch.bfloat16)
+        if bias.numel() != N or silu_mul:
+            raise KernelError(f"skinny_gemm: a bias of {bias.numel()} numbers for {N} plain columns")
     out = torch.empty((M, N // 2 if silu_mul else N), dtype=out_dtype, device=x.device)
     _ok(_fn("gemm_skinny", "rg_skinny_gemm")(
         _ptr(weight), _ptr(x), c_int(x.stride(0)), _ptr(out), c_int(out.shape[1]), c_int(_dtype_code(out)),
-        c_int(1 if silu_mul else 0), c_int(M), c_int(N), c_int(K), _stream()), "skinny_gemm")
+        c_int(1 if silu_mul else 0), c_int(M), c_int(N), c_int(K), _ptr(bias), c_int(0), c_longlong(0), c_longlong(0),
+        _stream()), "skinny_gemm")
     return out
+
+
+def linear_groups(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    """float32 [G, M, N] = x[g] W[g]^T for ``x`` [G, M, K] and ``weight`` [G, N, K] of one type.  Up to 16 bfloat16 rows go
+    through the weight-streaming kernel, all groups in one launch (four products of one row by 1,024 x 2,048: the library's
+    batched product 7.5 us, this one 2.7); everything else through the library."""
+    G, M, K = x.shape
+    N = weight.shape[1]
+    if (x.dtype == weight.dtype == torch.bfloat16 and 0 < M <= SKINNY_AUTO_ROWS and N % 32 == 0 and K % 8 == 0
+            and x.is_cuda and x.is_contiguous() and x.data_ptr() % 16 == 0 and weight.is_contiguous()
+            and weight.shape == (G, N, K)):
+        out = torch.empty((G, M, N), dtype=torch.float32, device=x.device)
+        _ok(_fn("gemm_skinny", "rg_skinny_gemm")(
+            _ptr(weight), _ptr(x), c_int(K), _ptr(out), c_int(N), c_int(F32), c_int(0), c_int(M), c_int(G * N), c_int(K),
+            _ptr(None), c_int(N), c_longlong(M * K), c_longlong(M * N), _stream()), "linear_groups")
+        return out
+    if x.dtype == torch.float32:
+        return torch.bmm(x, weight.transpose(1, 2))
+    return torch.bmm(x, weight.transpose(1, 2), out_dtype=torch.float32)
 
 
 SKINNY_FUSED_MAX_ROWS = 16     # what the fused variants (residual epilogue, norm prologue) are compiled for
@@ -2607,7 +2636,7 @@ def _small_gemm_f32(x, weight):
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, bias: torch.Tensor | None = None) -> torch.Tensor:
-    """y = x W^T (+ ``bias``, added inside the library product), W stored [out, in].  Up to 64 bfloat16 rows go through the
+    """y = x W^T (+ ``bias``, added inside the product), W stored [out, in].  Up to 64 bfloat16 rows go through the
     weight-streaming kernel of this package; everything else through the
     library matrix product (cuBLAS), as in the reference, whose projections
     are library GEMMs (crates/vllm-models/src/llama/attention.rs:94-96,133).
@@ -2624,8 +2653,12 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, bias: torch.Te
     if x.dtype == torch.float32 and torch.backends.cuda.matmul.allow_tf32:
         raise KernelError("linear: TF32 is enabled; the 32-bit path must be true 32-bit")
     if bias is not None:
+        # (up to 16 rows by 2,576 x 2,048: the library's 6.5 us, this package's 2.5)
         if out_dtype is not None and out_dtype != x.dtype:
             raise KernelError("linear: a product with a bias comes out in its input's type")
+        if (x.shape[0] <= SKINNY_AUTO_ROWS and skinny_gemm_ok(x, weight) and bias.dtype == torch.bfloat16
+                and bias.is_contiguous() and bias.shape == weight.shape[:1]):
+            return skinny_gemm(x, weight, bias=bias)
         return torch.addmm(bias, x, weight.t())
     if x.shape[0] <= SKINNY_AUTO_ROWS and skinny_gemm_ok(x, weight):
         return skinny_gemm(x, weight, out_dtype)             # small decode batches: stream the weights once

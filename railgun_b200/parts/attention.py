@@ -382,9 +382,7 @@ class NormedAttention(Mixer):
         qkv = proj if proj.shape[1] == C else proj[:, :C]
         if self.K >= 1:
             state = cache.parts[-1].state if self.K > 1 else None
-            qkv = ops.causal_conv(qkv, 0, self.taps, state, batch, torch.float32)
-            if writes and state is not None:
-                ops.conv_state_update(proj, 0, state, batch)
+            qkv = ops.causal_conv(qkv, 0, self.taps, state, batch, torch.float32, update=writes)
         slots = batch.slot_mapping[pages.group] if writes else None
         table = batch.block_table[pages.group]
         blocks = cache.parts[1] if self.pool else None

@@ -169,9 +169,7 @@ class GatedDelta(Mixer):
         proj = ops.linear(x, self.w_in)                                      # [T, q | k | v | gate]
         ba = ops.linear(x, self.w_ba, out_dtype=torch.float32)               # [T, b | a], kept in 32-bit
         conv_state = cache.parts[1].state if self.K > 1 else None
-        qkv = ops.causal_conv(proj, 0, self.taps, conv_state, batch, torch.float32, silu=True)
-        if writes and conv_state is not None:
-            ops.conv_state_update(proj, 0, conv_state, batch)
+        qkv = ops.causal_conv(proj, 0, self.taps, conv_state, batch, torch.float32, silu=True, update=writes)
         q, k, v, state = qkv[:, :G * d], qkv[:, G * d:2 * G * d], qkv[:, 2 * G * d:], cache.parts[0].state
         o, least = None, ops.DELTA_CHUNK_MIN_TOKENS
         chunks, others = ops.scan_split(batch, least) if ops.delta_chunk_ok(k, state, d, dv) else (0, True)
@@ -219,9 +217,7 @@ class InputConv(Mixer):
 
     def forward(self, x, batch, cache, writes=True):
         state = cache.parts[0].state if self.K > 1 else None
-        h = ops.causal_conv(x, 0, self.taps, state, batch, self.env.dtype, residual=True)
-        if writes and state is not None:
-            ops.conv_state_update(x, 0, state, batch)
+        h = ops.causal_conv(x, 0, self.taps, state, batch, self.env.dtype, residual=True, update=writes)
         view = CacheView(cache.cache_id, parts=cache.parts[1:]) if self.inner_composite else cache.parts[1]
         return self.inner.forward(h, batch, view, writes)
 

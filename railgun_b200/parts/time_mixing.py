@@ -69,9 +69,7 @@ class TokenShift(Mixer):
     def forward(self, x, batch, cache, writes=True):
         # rows that come from a norm: the shift is a convolution of two taps
         taps = torch.stack([self.share, 1.0 - self.share])
-        h = ops.causal_conv(x, 0, taps, cache.parts[0].state, batch, self.env.dtype)
-        if writes:
-            ops.conv_state_update(x, 0, cache.parts[0].state, batch)
+        h = ops.causal_conv(x, 0, taps, cache.parts[0].state, batch, self.env.dtype, update=writes)
         return self.inner.forward(h, batch, self._inner_view(cache), writes)
 
     def forward_stream(self, stream, batch, cache, writes=True):
@@ -139,11 +137,7 @@ class RwkvTimeMixing(Mixer):
         product.  The state advances by the step's tokens."""
         H, d = self.H, self.d
         mixes, last = ops.shift_mixes(x, self.mu, cache.parts[1].state, batch)
-        wide = self.w_rkvg.transpose(1, 2)
-        if mixes.dtype == torch.float32:
-            r, k, v, g = torch.bmm(mixes, wide)
-        else:
-            r, k, v, g = torch.bmm(mixes, wide, out_dtype=torch.float32)
+        r, k, v, g = ops.linear_groups(mixes, self.w_rkvg)
         w = ops.lowrank_decay(ops.linear(last, self.w1, out_dtype=torch.float32), self.w2, self.w0)
         if batch.max_query_len >= ops.SCAN_CHUNKED_MIN_TOKENS:
             o = ops.channel_chunk_scan(r, k, v, w, self.u, cache.parts[0].state, batch, H, d, d)
