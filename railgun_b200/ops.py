@@ -550,6 +550,7 @@ def latent_attention_mma(qa: torch.Tensor, out: torch.Tensor, cache: torch.Tenso
 
 
 MOE_TILE_ROWS = 32
+MOE_TC_TILE_ROWS = 256     # of the grouped tcgen05 product (a CTA pair's tile)
 
 
 ROUTE_PRODUCT_MIN_ROWS = 128
@@ -649,7 +650,7 @@ def moe_grouped_gemm(a: torch.Tensor, src, src_div: int, w: torch.Tensor, tiles:
     ``plain_act`` names an activation on the product, see ``ACTIVATIONS``).  Row ``pos`` of the input is ``a[src[pos] // src_div]``
     or, without ``src``, ``a[pos]``.  Returns [places, N]; rows that belong to no
     tile are not written.  bfloat16 with rows on 16-byte boundaries runs on the
-    tensor cores (tiles of 32 places: mma.sync, weight-streaming; tiles of 128:
+    tensor cores (tiles of 32 places: mma.sync, weight-streaming; tiles of 128 or 256:
     the grouped tcgen05 product, whose bounded waits ``tc_gemm_check`` reports
     on), everything else in 32-bit arithmetic on the CUDA cores (tiles of 32)."""
     _check(a, "a")
@@ -661,11 +662,11 @@ def moe_grouped_gemm(a: torch.Tensor, src, src_div: int, w: torch.Tensor, tiles:
     N = rows_w // 2 if gated else rows_w
     if a.shape[1] != K or (gated and rows_w % 2):
         raise KernelError(f"moe_grouped_gemm: a {tuple(a.shape)} vs w {tuple(w.shape)}")
-    if tile_rows == 128:
+    if tile_rows in (128, MOE_TC_TILE_ROWS):
         if not moe_grouped_gemm_tc_ok(a.dtype, K, a.stride(0)):
-            raise KernelError("moe_grouped_gemm: tiles of 128 places are for the tensor-core path")
+            raise KernelError(f"moe_grouped_gemm: tiles of {tile_rows} places are for the tensor-core path")
         # prompts: the tcgen05 product over the tile list (its rows come through TMA, so they are gathered
-        # into expert order first); gate and up as one product, silu * up by the activation kernel
+        # into expert order first); the gated activation is its epilogue where gate rows come in whole blocks of 8
         if src is not None:
             rows = torch.empty((places, K), dtype=a.dtype, device=a.device)
             _ok(_fn("moe", "rg_moe_gather_rows")(_ptr(a), c_int(a.stride(0)), _ptr(src), c_int(src_div), _ptr(rows),
@@ -678,12 +679,18 @@ def moe_grouped_gemm(a: torch.Tensor, src, src_div: int, w: torch.Tensor, tiles:
             err = _tc_err[a.device] = torch.zeros(1, dtype=torch.int32, device=a.device)
         global _tc_unchecked
         _tc_unchecked = True
-        wide = torch.empty((places, rows_w), dtype=a.dtype, device=a.device)
-        _ok(_fn("gemm_tcgen05", "rg_tc_gemm_grouped")(
-            _ptr(a), c_int(a.stride(0)), c_int(places), _ptr(w), c_int(E), c_int(rows_w), c_int(K), _ptr(wide),
-            c_int(rows_w), _ptr(tiles), c_int(tiles.shape[0]), _ptr(err), _stream()), "tc_gemm_grouped")
+        fused = gated and N % 8 == 0
+        if fused and act not in GATED_ACTIVATIONS:
+            raise KernelError(f"unknown gated activation {act!r}; known: {sorted(GATED_ACTIVATIONS)}")
+        wide = torch.empty((places, N if fused else rows_w), dtype=a.dtype, device=a.device)
+        _ok(_fn("gemm_grouped_tcgen05", "rg_tc_gemm_grouped")(
+            _ptr(a), c_int(a.stride(0)), c_int(places), _ptr(w), c_int(E), c_int(rows_w), c_int(K), c_int(1 if fused else 0),
+            c_int(GATED_ACTIVATIONS[act] if fused else 0), c_float(limit), _ptr(wide), c_int(wide.shape[1]), _ptr(tiles),
+            c_int(tiles.shape[0]), _ptr(err), _stream()), "tc_gemm_grouped")
         if not gated:
             return activation(wide, plain_act) if plain_act else wide
+        if fused:
+            return wide
         return silu_mul(wide) if act == "silu" else gated_activation(wide, act, limit)
     if act not in GATED_ACTIVATIONS:
         raise KernelError(f"unknown gated activation {act!r}; known: {sorted(GATED_ACTIVATIONS)}")
@@ -711,10 +718,10 @@ def moe_grouped_gemm_tc_ok(dtype, K: int, lda: int) -> bool:
 
 
 def moe_tile_rows(dtype, pairs: int, num_experts: int, K1: int, K2: int) -> int:
-    """Places per tile of the grouped products: 128 (the tcgen05 product) once an expert gets 64 places on
+    """Places per tile of the grouped products: 256 (the tcgen05 product) once an expert gets 64 places on
     average (prompts: every weight row that is read serves 128 rows), else 32."""
     tc = moe_grouped_gemm_tc_ok(dtype, K1, K1) and moe_grouped_gemm_tc_ok(dtype, K2, K2)
-    return 128 if tc and pairs >= 64 * max(1, num_experts) else MOE_TILE_ROWS
+    return MOE_TC_TILE_ROWS if tc and pairs >= 64 * max(1, num_experts) else MOE_TILE_ROWS
 
 
 def moe_scaled_rows(x: torch.Tensor, sorted_pair: torch.Tensor, top: int, weights: torch.Tensor,
@@ -2228,6 +2235,30 @@ def tc_gemm(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, silu_mul: boo
         "tc_gemm")
     if check:
         tc_gemm_check(x.device)
+    return out
+
+
+def tc_gemm_gated_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Can ``tc_gemm_gated`` take these operands, and is it worth it?  From as many rows on as the SiLU-mul form."""
+    return (isinstance(x, torch.Tensor) and x.dim() == 2 and x.shape[0] >= TC_GEMM_MIN_ROWS and weight.shape[0] % 16 == 0
+            and tc_gemm_ok(x, weight))
+
+
+def tc_gemm_gated(x: torch.Tensor, weight: torch.Tensor, act: str, limit: float = 0.0) -> torch.Tensor:
+    """[M, N / 2] bfloat16 = act(gate) * up of the 32-bit sums x W^T, W [N, K] = gate rows, then as many up rows (``act``,
+    ``limit``: see ``gated_activation``), on tcgen05 CTA pairs.  Its waits are bounded; ``tc_gemm_check`` reports on them."""
+    if not tc_gemm_ok(x, weight) or weight.shape[0] % 16 or weight.shape[1] != x.shape[1] or act not in GATED_ACTIVATIONS:
+        raise KernelError(f"tc_gemm_gated refuses x {tuple(x.shape)} {x.dtype}, W {tuple(weight.shape)} {weight.dtype}, {act!r}")
+    (M, K), N = x.shape, weight.shape[0]
+    err = _tc_err.get(x.device)
+    if err is None:
+        err = _tc_err[x.device] = torch.zeros(1, dtype=torch.int32, device=x.device)
+    global _tc_unchecked
+    _tc_unchecked = True
+    out = torch.empty((M, N // 2), dtype=torch.bfloat16, device=x.device)
+    _ok(_fn("gemm_tcgen05", "rg_tc_gemm_gated")(
+        _ptr(x), c_int(x.stride(0)), _ptr(weight), _ptr(out), c_int(N // 2), c_int(GATED_ACTIVATIONS[act]), c_float(limit),
+        c_int(M), c_int(N), c_int(K), c_int(TC_TILES[tc_pair_tile(M, N, x.device)]), _ptr(err), _stream()), "tc_gemm_gated")
     return out
 
 

@@ -49,7 +49,8 @@ class SwiGLU(FeedForward):
         if self.act != "silu":
             if isinstance(x, ops.NormedRows):
                 x = x.materialize()
-            act = ops.gated_activation(ops.linear(x, self.w_gate_up), self.act)
+            act = (ops.tc_gemm_gated(x, self.w_gate_up, self.act) if ops.tc_gemm_gated_ok(x, self.w_gate_up)
+                   else ops.gated_activation(ops.linear(x, self.w_gate_up), self.act))
             return ops.PendingLinear(act, self.w_down, stream) if defer else ops.linear(act, self.w_down)
         if isinstance(x, ops.NormedRows):
             if self.interleaved and ops.skinny_scaled_ok(x, self.w_gate_up):
