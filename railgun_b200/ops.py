@@ -2666,6 +2666,70 @@ def _small_gemm_f32(x, weight):
     return out
 
 
+# Products whose rows the small product's kernel makes itself: 32-bit, of numbers that a block keeps in shared memory.
+SMALL_F32_ROWS_K = 256
+
+
+def _small_rows_ok(M: int, K: int, weight: torch.Tensor) -> bool:
+    """The small product's rule, for rows of K numbers that a kernel makes."""
+    most_k, most_tiles = SMALL_F32_LIMITS[0] if M <= 16 else SMALL_F32_LIMITS[1] if M <= 30 else SMALL_F32_LIMITS[2]
+    return (0 < M <= SMALL_F32_ROWS and 0 < K <= min(most_k, SMALL_F32_ROWS_K) and weight.dtype == torch.float32
+            and weight.dim() == 2 and weight.shape[1] == K and weight.is_contiguous()
+            and -(-M // 32) * -(-weight.shape[0] // 32) <= most_tiles)
+
+
+class FreshNorm:
+    """A 32-bit RMS norm that the product which reads it computes: of the rows ``resid`` (+ ``pending``), whose sum that
+    product leaves in ``new`` (``resid`` itself with nothing pending).  Exists only where ``linear`` of it by a matrix of
+    ``weight``'s shape is the small product (``fresh_norm``)."""
+
+    __slots__ = ("resid", "pending", "norm", "eps", "new")
+
+    def __init__(self, resid, pending, norm, eps: float):
+        self.resid, self.pending, self.norm, self.eps = resid, pending, norm, float(eps)
+        self.new = resid if pending is None else torch.empty_like(resid)
+
+    @property
+    def shape(self):
+        return self.resid.shape
+
+    dtype = torch.float32
+
+
+def fresh_norm(resid: torch.Tensor, pending, norm: torch.Tensor, eps: float, weight) -> FreshNorm | None:
+    """The norm of ``resid`` + ``pending`` for the one product by ``weight`` that reads it, if its kernel can compute it."""
+    if (resid.dtype != torch.float32 or resid.dim() != 2 or norm.dtype != torch.float32 or weight is None
+            or not (pending is None or (isinstance(pending, torch.Tensor) and pending.dtype == torch.float32
+                                        and pending.shape == resid.shape and pending.is_contiguous() and _by_address(pending, weight)))
+            or not resid.is_contiguous() or norm.numel() != resid.shape[1] or not norm.is_contiguous()
+            or not _small_rows_ok(*resid.shape, weight) or not (_by_address(resid, weight) and _by_address(norm, weight))):
+        return None
+    return FreshNorm(resid, pending, norm, eps)
+
+
+def _small_rows(x, ldx: int, pending, norm, eps: float, new, silu: bool, weight, M: int, K: int):
+    N = weight.shape[0]
+    out = torch.empty((M, N), dtype=torch.float32, device=weight.device)
+    _ok(_fn("gemm_small_f32", "rg_small_gemm_rows_f32")(
+        _ptr(x), c_int(ldx), _ptr(pending), _ptr(norm), c_float(eps), _ptr(new), c_int(1 if silu else 0), _ptr(weight), _ptr(out),
+        c_int(N), c_int(M), c_int(N), c_int(K), _stream()), "small_gemm_rows_f32")
+    return out
+
+
+def silu_linear_ok(gate_up: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Is the product of silu(gate) * up by ``weight`` one that the small product's kernel can make the rows of?"""
+    return (gate_up.dtype == torch.float32 and gate_up.dim() == 2 and gate_up.is_contiguous() and gate_up.shape[1] % 2 == 0
+            and _small_rows_ok(gate_up.shape[0], gate_up.shape[1] // 2, weight) and _by_address(gate_up, weight))
+
+
+def silu_linear(gate_up: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    """(silu(gate) * up) W^T in 32-bit, ``gate_up`` [M, 2 K] = gate | up."""
+    if not silu_linear_ok(gate_up, weight):
+        raise KernelError(f"silu_linear refuses {tuple(gate_up.shape)} {gate_up.dtype}, W {tuple(weight.shape)} {weight.dtype}")
+    M, K2 = gate_up.shape
+    return _small_rows(gate_up, K2, None, None, 0.0, None, True, weight, M, K2 // 2)
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, bias: torch.Tensor | None = None) -> torch.Tensor:
     """y = x W^T (+ ``bias``, added inside the product), W stored [out, in].  Up to 64 bfloat16 rows go through the
     weight-streaming kernel of this package; everything else through the
@@ -2673,6 +2737,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, bias: torch.Te
     are library GEMMs (crates/vllm-models/src/llama/attention.rs:94-96,133).
     32-bit inputs run in true 32-bit: the reduced-precision matrix mode is
     refused."""
+    if isinstance(x, FreshNorm):
+        return _small_rows(x.resid, x.shape[1], x.pending, x.norm, x.eps, x.new, False, weight, *x.shape)
     if isinstance(x, NormedRows):
         if (out_dtype is None or out_dtype == torch.bfloat16) and skinny_scaled_ok(x, weight):
             return skinny_gemm_scaled(x, weight)              # the norm is finished inside the product

@@ -98,6 +98,7 @@ class PagedAttention(Mixer):
 
     takes_normed_rows = True
     defers_output = True
+    first_matrix = property(lambda self: self.w_qkv)
 
     def forward(self, x, batch, cache, writes=True, defer=False):
         nh, nkv, d = self.nh, self.nkv, self.d

@@ -11,6 +11,8 @@ from __future__ import annotations
 
 from dataclasses import dataclass
 
+import torch
+
 from .. import ops
 
 
@@ -79,6 +81,15 @@ def normed_input(norm, part, stream, rows=None):
         pending = pending.materialize()
     if isinstance(pending, ops.PendingSum) and not getattr(norm, "fuses_pending_sum", False):
         pending = pending.materialize()
+    matrix = getattr(part, "first_matrix", None)
+    if rows is None and matrix is not None and getattr(norm, "plain_rms", False) and norm.env.dtype == torch.float32:
+        # a small 32-bit product computes the norm of its rows itself; what it leaves as the sum is the new stream
+        if isinstance(pending, ops.PendingLinear):
+            pending = pending.materialize()
+        h = ops.fresh_norm(stream.resid, pending, norm.weight, norm.eps, matrix)
+        if h is not None:
+            stream.resid = h.new
+            return h
     h = norm.add_norm(stream.resid, pending) if rows is None else norm.add_norm(stream.resid, pending, rows=rows)
     if isinstance(h, ops.NormedRows) and not getattr(part, "takes_normed_rows", False):
         h = h.materialize()
@@ -95,7 +106,8 @@ class Mixer(Part):
     [T, H]; ``cache`` is a ``CacheView`` of what the need asked for; ``writes``
     False means the layer reads a cache that another layer fills.
 
-    Optional, for mixers and feed-forwards alike: ``takes_normed_rows`` = True
+    Optional, for mixers and feed-forwards alike: ``first_matrix``, the matrix of the one product that reads ``x``: in 32-bit
+    ``x`` may then be an ``ops.FreshNorm``, which ``ops.linear`` takes; ``takes_normed_rows`` = True
     says that ``x`` may be an ``ops.NormedRows`` (which ``ops.linear`` takes in
     place of a tensor); ``defers_output`` = True says that ``forward`` has a
     keyword ``defer`` and, when it is True, may return its last product as an

@@ -43,6 +43,7 @@ class SwiGLU(FeedForward):
 
     takes_normed_rows = True
     defers_output = True
+    first_matrix = property(lambda self: self.w_gate_up)
 
     def forward(self, x, batch, defer=False):
         stream = ops.tc_stream_rows(batch, self.w_down.shape[0])
@@ -72,7 +73,10 @@ class SwiGLU(FeedForward):
             act = ops.tc_gemm(x, self.w_gate_up, silu_mul=True,
                               tile=ops.tc_pair_tile(x.shape[0], self.w_gate_up.shape[0], x.device))
         else:
-            act = ops.silu_mul(ops.linear(x, self.w_gate_up), interleaved=self.interleaved)
+            gate_up = ops.linear(x, self.w_gate_up)
+            if not self.interleaved and ops.silu_linear_ok(gate_up, self.w_down):
+                return ops.silu_linear(gate_up, self.w_down)                     # a small 32-bit product, SiLU-mul in front of it
+            act = ops.silu_mul(gate_up, interleaved=self.interleaved)
         return ops.PendingLinear(act, self.w_down, stream) if defer else ops.linear(act, self.w_down)
 
 

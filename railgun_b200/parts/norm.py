@@ -51,6 +51,7 @@ class RMSNorm(Norm):
     fuses_pending_linear = True
     fuses_post_norm = True
     fuses_pending_sum = True
+    plain_rms = property(lambda self: self.groups == 1)          # over the whole row, with ``weight`` and ``eps`` alone
 
     def add_norm(self, resid, pending, rows=None):
         if self.groups > 1 or isinstance(pending, ops.PendingSum):

@@ -65,3 +65,43 @@ def test_what_stays_the_librarys():
     assert torch.allclose(value, y, atol=1e-4) and torch.allclose(moved, w.sum(1).expand(20, 8), atol=1e-4)
     maps = torch.vmap(lambda m: ops.linear(x, m))(torch.stack([w, 2 * w]))
     assert torch.allclose(maps, torch.stack([y, 2 * y]), atol=1e-4)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (67, 160, 96), (33, 33, 33), (17, 96, 256), (31, 65, 255), (2, 7, 4), (256, 40, 130)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_rows_that_the_kernel_makes(M, N, K, shift):
+    """The norm of a residual with and without something pending, and SiLU-mul, in front of the product; on and off 16-byte
+    boundaries; the first row of blocks leaves the sum."""
+    from railgun_b200 import ops
+    g = torch.Generator().manual_seed(M + N + K)
+    new = lambda *shape: torch.randn(shape[0] * shape[1] + shift, generator=g).to(DEV)[shift:].view(*shape)
+    x, p, w = new(M, K), new(M, K), new(N, K)
+    norm = (torch.rand(K, generator=g) + 0.5).to(DEV)
+    for pending in (p, None):
+        total = x if pending is None else x + pending
+        unit = total.double() / (total.double().pow(2).mean(1, keepdim=True) + 1e-5).sqrt() * norm.double()
+        h = ops.fresh_norm(x, pending, norm, 1e-5, w)
+        if not ops.small_gemm_f32_ok(torch.empty(M, K, device=DEV), w):
+            assert h is None                                             # the small product's rule
+            continue
+        y = ops.linear(h, w)
+        # as above; the root mean square and its two products are four more roundings
+        assert rel_err(y, unit @ w.double().T) < 3e-6 and torch.equal(h.new, total)
+        assert (h.new is x) == (pending is None)
+    gu = new(M, 2 * K)
+    want = (torch.nn.functional.silu(gu[:, :K].double()) * gu[:, K:].double()) @ w.double().T
+    if ops.silu_linear_ok(gu, w):
+        assert rel_err(ops.silu_linear(gu, w), want) < 3e-6
+
+
+def test_what_makes_no_rows():
+    from railgun_b200 import ops
+    x, w, n = torch.zeros(40, 64, device=DEV), torch.zeros(8, 64, device=DEV), torch.ones(64, device=DEV)
+    assert ops.fresh_norm(x, None, n, 1e-5, w) is not None
+    assert ops.fresh_norm(x, x.bfloat16(), n, 1e-5, w) is None and ops.fresh_norm(x, None, n, 1e-5, None) is None
+    assert ops.fresh_norm(x, None, n, 1e-5, torch.zeros(8, 65, device=DEV)) is None
+    wide = torch.zeros(40, 288, device=DEV)
+    assert ops.fresh_norm(wide, None, torch.ones(288, device=DEV), 1e-5, torch.zeros(8, 288, device=DEV)) is None
+    assert not ops.silu_linear_ok(torch.zeros(40, 127, device=DEV), w) and not ops.silu_linear_ok(x, w)
+    grown = torch.zeros(8, 64, device=DEV, requires_grad=True)
+    assert ops.fresh_norm(x, None, n, 1e-5, grown) is None
