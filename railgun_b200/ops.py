@@ -2099,7 +2099,7 @@ _decode_counters: dict = {}
 def decode_attention(q, q_stride: int, out, kv_cache, block_table, rows, n_tokens: int, req_of_token, positions,
                      nh: int, nkv: int, d: int, window: int, scale: float, num_splits: int,
                      scratch=None, fused_reduce=None, cluster: bool = False, keep_first: int = 0, sink=None,
-                     gate=None, pooled=None, out_scale: float = 1.0, chunk: int = 0) -> None:
+                     gate=None, pooled=None, out_scale: float = 1.0, chunk: int = 0, beside: bool = False) -> None:
     """Split attention for single tokens: token rows ``rows`` (None: rows
     0..n_tokens-1) each attend their request's context.  Partial results go
     through scratch memory (allocated here unless given) and are reduced into
@@ -2116,7 +2116,9 @@ def decode_attention(q, q_stride: int, out, kv_cache, block_table, rows, n_token
     ``_sink_and_gate``; they enter where the splits are added up (not with
     ``cluster``).  ``pooled``: see ``_pooled`` (not with ``cluster``).  ``out``
     may be a view whose rows are further apart; the output is multiplied by
-    ``out_scale`` (neither with ``cluster``).  ``chunk``: see ``_reach``."""
+    ``out_scale`` (neither with ``cluster``).  ``chunk``: see ``_reach``.
+    ``beside``: the launch right before this one on this stream is the step's prompt attention over the same ``q`` and
+    cache into other rows of ``out``; the two then run side by side (not with ``cluster``)."""
     if fused_reduce is None:
         fused_reduce = num_splits == 1
     page_size = _check_paged(q, kv_cache, block_table, nkv, d)
@@ -2131,8 +2133,8 @@ def decode_attention(q, q_stride: int, out, kv_cache, block_table, rows, n_token
             raise KernelError("decode_attention: the cluster form does not keep first tokens")
         if sink is not None or gate is not None or pooled is not None or out_scale != 1.0 or not out.is_contiguous():
             raise KernelError("decode_attention: the cluster form has neither sink, gate, pooled entries nor an output view")
-        if not 2 <= num_splits <= 8:
-            raise KernelError("decode_attention: a cluster takes 2 to 8 splits")
+        if not 2 <= num_splits <= 8 or beside:
+            raise KernelError("decode_attention: a cluster takes 2 to 8 splits and runs beside nothing")
         _ok(_fn("attention_mma", "rg_decode_attention_cluster")(
             _ptr(q), c_int(q_stride), _ptr(out), _ptr(kv_cache), _ptr(block_table), c_int(block_table.shape[1]),
             _ptr(rows), c_int(n_tokens), _ptr(req_of_token), _ptr(positions), c_int(nh), c_int(nkv), c_int(d),
@@ -2152,6 +2154,7 @@ def decode_attention(q, q_stride: int, out, kv_cache, block_table, rows, n_token
         counters = _decode_counters.get(q.device)
         if counters is None or counters.numel() < need:
             counters = _decode_counters[q.device] = torch.zeros(max(need, 4096), dtype=torch.int32, device=q.device)
+            beside = False                   # the launch before this one is the one that fills them
     else:
         _COUNTER.value += 1                  # the launcher runs two kernels: partial results, then the reduction
     _ok(_fn("attention_mma", "rg_decode_attention_sink")(
@@ -2159,8 +2162,8 @@ def decode_attention(q, q_stride: int, out, kv_cache, block_table, rows, n_token
         _ptr(rows), c_int(n_tokens), _ptr(req_of_token), _ptr(positions), _ptr(part_o), _ptr(part_ml),
         _ptr(counters), c_int(nh), c_int(nkv), c_int(d), c_int(page_size), c_int(_reach(window, chunk, keep_first)),
         c_int(keep_first if window else 0), c_float(scale), c_int(num_splits), _ptr(sink), _ptr(gate), c_int(gate_ld),
-        *_pooled(pooled, kv_cache, window, keep_first), c_int(out.stride(0)), c_float(out_scale), _stream()),
-        "decode_attention")
+        *_pooled(pooled, kv_cache, window, keep_first), c_int(out.stride(0)), c_float(out_scale), c_int(1 if beside else 0),
+        _stream()), "decode_attention")
 
 
 _tc_err: dict = {}

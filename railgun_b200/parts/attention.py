@@ -163,7 +163,7 @@ class PagedAttention(Mixer):
             n = batch.num_decode_rows
             ops.decode_attention(qkv, qkv.shape[1], out, cache.kv, table, batch.decode_rows, n, batch.req_of_token,
                                  batch.positions, nh, nkv, d, self.window, self.scale,
-                                 ops.decode_splits(n, kv_tiles, batch.max_context_len))
+                                 ops.decode_splits(n, kv_tiles, batch.max_context_len), beside=batch.num_prefill_tiles > 0)
         return out
 
 
@@ -431,7 +431,8 @@ class NormedAttention(Mixer):
         if n:
             ops.decode_attention(q, q.shape[1], out, cache.kv, table, None if batch.decode_only else batch.decode_rows,
                                  n, batch.req_of_token, batch.positions, H, G, D, self.window, 1.0,
-                                 ops.decode_splits(n, kv_tiles, reach), keep_first=self.keep_first, **more)
+                                 ops.decode_splits(n, kv_tiles, reach), keep_first=self.keep_first,
+                                 beside=batch.num_prefill_tiles > 0, **more)
         return out
 
 

@@ -184,3 +184,43 @@ def test_stream_rows_and_the_shift(H, normed):
     assert rel(rows, new) < 2e-6 and rel(h, new + (before - new) * share.double()) < 2e-6 and rel(state, after) < 2e-6
     rows, h = ops.postnorm_shift(x, pending, None, None, None, torch.float32)
     assert rows is x and rel(x, new) < 2e-6 and torch.equal(h, x)
+
+
+@pytest.mark.parametrize("nh,nkv,d", [(32, 8, 64), (24, 8, 128), (4, 2, 48)])
+@pytest.mark.parametrize("splits", [1, 3])
+@pytest.mark.parametrize("portions", [1, 9])
+def test_single_tokens_beside_portions(nh, nkv, d, splits, portions):
+    """Single tokens' attention that starts beside the portions' of the same step: the bits of both in turn, many times over."""
+    from railgun_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(nh * d + portions)
+    page, tokens, singles, ctx = 16, 130, 11, 700
+    R, width = portions + singles, -(-ctx // page)
+    T = portions * tokens + singles
+    kv = torch.randn(R * width, 2, nkv, page, d, device=DEV, generator=g).bfloat16()
+    table = torch.randperm(R * width, device=DEV, generator=g).to(torch.int32).view(R, width)
+    q = torch.randn(T, (nh + 2 * nkv) * d, device=DEV, generator=g).bfloat16()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    pos = i32([j for _ in range(portions) for j in range(ctx - tokens, ctx)] + [ctx - 1 - 60 * j for j in range(singles)])
+    req = i32([r for r in range(portions) for _ in range(tokens)] + list(range(portions, R)))
+    rows = i32(list(range(portions * tokens, T)))
+
+    def tiles(size):
+        return i32([[r * tokens + a, min(size, tokens - a), r] for r in range(portions) for a in range(0, tokens, size)])
+
+    t128, t64 = tiles(128), tiles(64)
+
+    def step(beside):
+        out = torch.zeros(T, nh * d, dtype=torch.bfloat16, device=DEV)
+        if d == 64:
+            ops.prefill_attention_tc(q, out, kv, table, t128, pos, nh, nkv, d, 0, d ** -0.5)
+        elif d == 128:
+            ops.prefill_attention_wide(q, out, kv, table, t128, pos, nh, nkv, d, 0, d ** -0.5)
+        else:
+            ops.prefill_attention(q, q.shape[1], out, kv, table, t64, pos, nh, nkv, d, 0, d ** -0.5)
+        ops.decode_attention(q, q.shape[1], out, kv, table, rows, singles, req, pos, nh, nkv, d, 0, d ** -0.5, splits, beside=beside)
+        return out.clone()                                                  # behind both
+
+    want = step(False)
+    for _ in range(20):
+        assert torch.equal(step(True), want)
+    ops.tc_gemm_check()
