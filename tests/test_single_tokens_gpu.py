@@ -224,3 +224,36 @@ def test_single_tokens_beside_portions(nh, nkv, d, splits, portions):
     for _ in range(20):
         assert torch.equal(step(True), want)
     ops.tc_gemm_check()
+
+
+@pytest.mark.parametrize("nh,nkv,d", [(1, 1, 16), (32, 8, 64), (32, 8, 128), (64, 16, 128), (8, 8, 256)])
+@pytest.mark.parametrize("paired", [False, True])
+def test_rotation_and_cache_write(nh, nkv, d, paired):
+    """Rows of less and of more pieces than a block has threads; tokens without a slot, a position outside the table."""
+    from railgun_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(nh * d)
+    T, page = 7, 4
+    x = torch.randn(T, (nh + 2 * nkv) * d, device=DEV, generator=g).bfloat16()
+    angle = torch.rand(50, d // 2, device=DEV, generator=g) * 6.0
+    table = torch.cat([angle.cos(), angle.sin()], 1)
+    pos = torch.tensor([0, 49, 3, 50, 7, 8, 9], dtype=torch.int32, device=DEV)
+    slots = torch.tensor([3, 0, -1, 9, 4, 11, 6], dtype=torch.int32, device=DEV)
+    cache = torch.full((3, 2, nkv, page, d), 7.0, dtype=torch.bfloat16, device=DEV)
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+    order = ops.rope_pair_order(d).to(DEV) if paired else torch.arange(d, device=DEV)      # storage index -> feature
+    heads = x.view(T, -1, d)
+    plain = torch.empty_like(heads)
+    plain[..., order] = heads                                              # features in the model's order
+    c, s = (table[pos.long().clamp(max=49) * (pos < 50)][:, None, i * d // 2:(i + 1) * d // 2].double() for i in (0, 1))
+    u, v = plain[..., :d // 2].double(), plain[..., d // 2:].double()
+    turned = torch.cat([u * c - v * s, v * c + u * s], -1)[..., order]
+    want = torch.cat([turned[:, :nh + nkv], heads[:, nh + nkv:].double()], 1)
+    got = x.clone()
+    ops.rope_cache_write(got, table, pos, slots, cache, nh, nkv, d, page, err_flag=err, paired8=paired)
+    close = lambda a, b: (a.double() - b).abs().max() <= 2.0 ** -8 * b.abs().max()
+    assert close(got.view(T, -1, d)[:, :nh + nkv], want[:, :nh + nkv]) and err.item() == 1
+    for t, slot in enumerate(slots.tolist()):
+        if slot >= 0:
+            k, v = cache[slot // page, 0, :, slot % page], cache[slot // page, 1, :, slot % page]
+            assert close(k, want[t, nh:nh + nkv]) and torch.equal(v, heads[t, nh + nkv:])
+    assert int((cache == 7.0).all(-1).sum()) >= 2 * nkv * (12 - 6)
