@@ -10,7 +10,7 @@ crates/vllm-models/src/llama/architecture.rs:141-156).
 How a step reaches the GPU: steps of single tokens replay a CUDA graph over a
 static batch (``decode_step_flat``; the graph copies its inputs in, chooses
 the tokens and copies them out), and the step after such a step can be
-launched before its tokens are known (``decode_follow``); large steps whose
+launched before its tokens are known (``decode_follow``); other steps whose
 packed layout repeats replay a graph captured for that layout
 (``_step_shape_graph``); everything else launches its kernels one by one.
 """
@@ -38,10 +38,16 @@ _DTYPES = {"bfloat16": torch.bfloat16, "bf16": torch.bfloat16, "float32": torch.
            "f32": torch.float32}
 
 
-# Steps of at least this many tokens go through a graph captured for their layout once that layout repeats
-# (below it the launches are few and short; single tokens have their own graphs), and so many layouts are kept.
+# Steps other than single tokens' (which have graphs of their own) go through a graph captured for their layout once that
+# layout repeats: a portion's size is mostly the scheduler's, and the step of a prompt's next portion beside the same decoding
+# requests has the layout of the one before.  From SHAPE_GRAPH_MIN_TOKENS tokens on at the second step of a layout; shorter
+# steps at the SMALL_GRAPH_AT-th: what a replay saves there is host time (some 30 to 85 launches of 14 to 18 us), a capture
+# costs as much as some of them, and short prompts' layouts are many.  So many layouts of either kind are kept, the ones used last.
 SHAPE_GRAPH_MIN_TOKENS = 256
 SHAPE_GRAPHS_KEPT = 4
+SMALL_GRAPH_AT = 4
+SMALL_GRAPHS_KEPT = 8
+SHAPES_COUNTED = 64, 512           # layouts whose steps are counted: of long steps, of short ones
 
 
 @contextlib.contextmanager
@@ -268,6 +274,8 @@ class ModelRunner:
         self._static: dict = {}
         self._shape_steps: dict = {}       # graph key -> ShapeGraph: steps seen before replay a captured graph
         self._shape_seen: dict = {}
+        self._small_steps: dict = {}       # the same for steps of fewer than ``shape_graph_min_tokens`` tokens
+        self._small_seen: dict = {}
         self.shape_graph_min_tokens = SHAPE_GRAPH_MIN_TOKENS
         self._graph_pool = None
         self._ctx_hint = 0
@@ -298,7 +306,7 @@ class ModelRunner:
         if self.use_graphs and entries and all(
                 len(e.tokens) == 1 and list(e.want) == [0] and self.alloc.has(e.request_id) for e in entries):
             return self._step_decode_graph(entries)
-        if self.use_graphs and sum(len(e.tokens) for e in entries) >= self.shape_graph_min_tokens:
+        if self.use_graphs and entries:
             return self._step_shape_graph(entries)
         batch = build_step_batch(entries, self.alloc, self.page_sizes, self.model.vocab_size,
                                  self.model.spec.max_position, self.device, self.err_flag)
@@ -311,20 +319,23 @@ class ModelRunner:
         self.alloc.commit_many(batch.host_request_ids, batch.host_context_lens)
 
     def _step_shape_graph(self, entries):
-        """Large steps (portions of prompts) whose packed layout was seen before
+        """Steps (portions of prompts) whose packed layout was seen before
         replay a CUDA graph captured for that layout: token counts, wanted places
         and block-table widths fix every shape, everything else is data in the
-        step's one device buffer.  The first step of a layout runs eagerly, the
-        second is captured while it runs, later ones replay; a few layouts
-        (the portions a scheduler cuts are mostly of one size) are kept."""
+        step's one device buffer.  The first steps of a layout run eagerly, the
+        second (of a short step the ``SMALL_GRAPH_AT``-th) is captured while it runs, later
+        ones replay; a few layouts are kept (``SHAPE_GRAPH_MIN_TOKENS``)."""
+        large = sum(len(e.tokens) for e in entries) >= self.shape_graph_min_tokens
+        steps, seen_of = (self._shape_steps, self._shape_seen) if large else (self._small_steps, self._small_seen)
         build = lambda into: build_step_batch(entries, self.alloc, self.page_sizes, self.model.vocab_size,
                                               self.model.spec.max_position, self.device, self.err_flag, into=into)
-        known = lambda key: self._shape_steps[key].dev if key in self._shape_steps else None
+        known = lambda key: steps[key].dev if key in steps else None
         batch = build(known)
         self.last_h2d_bytes = batch.h2d_bytes
         key = batch.graph_key
-        shape = self._shape_steps.get(key)
+        shape = steps.pop(key, None)
         if shape is not None:
+            steps[key] = shape                                     # the one used last
             # the step was packed straight into the graph's buffer: launch
             shape.hold = batch
             shape.graph.replay()
@@ -332,17 +343,17 @@ class ModelRunner:
             ops.mark_tc_unchecked()
             self._commit(entries, batch)
             return shape.logits
-        seen = self._shape_seen.get(key, 0) + 1
-        if len(self._shape_seen) > 64:
-            self._shape_seen.clear()
-        self._shape_seen[key] = seen
-        if seen < 2:
+        seen = seen_of.get(key, 0) + 1
+        if len(seen_of) > SHAPES_COUNTED[0 if large else 1]:
+            seen_of.clear()
+        seen_of[key] = seen
+        if seen < (2 if large else SMALL_GRAPH_AT):
             logits = self.model.forward(batch, self.views)
             self._commit(entries, batch)
             return logits
         # the layout repeats: a static copy of the packed buffer, one eager run over it (this step), the capture
-        if len(self._shape_steps) >= SHAPE_GRAPHS_KEPT:
-            self._shape_steps.pop(next(iter(self._shape_steps)))
+        if len(steps) >= (SHAPE_GRAPHS_KEPT if large else SMALL_GRAPHS_KEPT):
+            steps.pop(next(iter(steps)))
         dev = torch.empty(batch.host_buffer.numel(), dtype=torch.int32, device=self.device)
         batch = build(lambda key: dev)
         side = torch.cuda.Stream(device=self.device)
@@ -359,7 +370,7 @@ class ModelRunner:
             logits = self.model.forward(batch, self.views)
         launches = counter.value - n0
         counter.value = n0
-        self._shape_steps[key] = ShapeGraph(dev, batch, graph, logits, launches)
+        steps[key] = ShapeGraph(dev, batch, graph, logits, launches)
         self._commit(entries, batch)
         return eager
 
