@@ -158,6 +158,25 @@ def test_paged_attention_general(case_id, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("d", [1, 3, 4, 31, 32, 33, 36, 64, 65, 100, 128, 129, 256])
+def test_paged_attention_general_at_every_width(d, dtype):
+    """One, two and four groups of threads over the keys; rows of whole 16-byte pieces and others; pages off such boundaries;
+    contexts below, at and above a block's keys."""
+    from railgun_b200 import ops
+    nh, nkv, page = 4, 2, 4
+    c = make_paged_case(3, [300, 129, 128], [2, 2, 1], nh, nkv, d, page, dtype, seed=d)
+    for window, shift in ((0, 0), (40, 0), (0, 1)):
+        ref = attention_reference(c, nh, nkv, d, page, window, d ** -0.5)
+        q = c["q"].reshape(c["T"], nh * d).contiguous().to(DEV)
+        kv = torch.zeros(c["kv"].numel() + shift, dtype=dtype, device=DEV)[shift:].view(c["kv"].shape)
+        kv.copy_(c["kv"])
+        out = ops.paged_attention_general(
+            q, nh * d, kv, c["bt"].to(DEV), torch.tensor(c["req"], dtype=torch.int32, device=DEV),
+            torch.tensor(c["positions"], dtype=torch.int32, device=DEV), nh, nkv, d, window, d ** -0.5)
+        assert rel_err(out, ref) < (5e-6 if dtype == torch.float32 else 1e-2)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_attention_finds_a_far_key_among_hundreds(dtype):
     """One key far back is made to dominate; losing it (a wrong page, an
     off-by-one at a page's edge) would change the output completely."""
