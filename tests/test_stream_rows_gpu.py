@@ -118,3 +118,36 @@ def test_which_steps_take_it():
     from railgun_b200 import ops
     assert ops.tc_stream_rows(Batch(decode_only=True), 2048) == ops.tc_stream_rows(None, 2048) == 64
     assert [ops.tc_stream_rows(Batch(decode_only=False), w) for w in (64, 2048, 3072, 4096, 16384)] == [255, 255, 170, 128, 64]
+
+
+@pytest.mark.parametrize("rows", [40, 41, 64, 65])
+@pytest.mark.parametrize("N,K", [(37888, 64), (37889, 64), (50000, 264)])
+def test_logits_of_decode_batches(rows, N, K):
+    """Both sides of the rule's edges, against 64 bits."""
+    from railgun_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(rows + N)
+    x = torch.randn(rows, K, device="cuda", generator=g).bfloat16()
+    w = torch.randn(N, K, device="cuda", generator=g).bfloat16()
+    y = ops.linear(x, w, out_dtype=torch.float32)
+    ops.tc_gemm_check()
+    want = x.double() @ w.double().T
+    assert y.dtype == torch.float32 and y.shape == (rows, N)
+    assert float((y.double() - want).abs().max() / want.abs().max()) < K * 2.0 ** -24 + 1e-6
+
+
+@pytest.mark.parametrize("M", [65, 96, 97, 128, 129, 176, 177, 255, 256])
+def test_parts_of_the_tokens(M):
+    """Few tiles of W above 64 rows: two parts of the tokens, of up to 64 and 128 each; a matrix of more tiles than half of the
+    SMs takes them whole.  Residual, norm and partial sums against 64 bits."""
+    from railgun_b200 import ops
+    for N, K in ((256, 264), (2048, 256), (3072, 320)):
+        g = torch.Generator(device="cuda").manual_seed(M + N)
+        x = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+        w = torch.randn(N, K, device="cuda", generator=g).bfloat16()
+        r, nw = torch.randn(M, N, device="cuda", generator=g), torch.rand(N, device="cuda", generator=g) + 0.5
+        want = r.double() + x.double() @ w.double().T
+        h = ops.tc_stream_gemm_residual(x, w, r, nw, 1e-5)
+        ops.tc_gemm_check()
+        err = lambda a, b: float((a.double() - b).abs().max() / b.abs().max())
+        assert err(r, want) < K * 2.0 ** -24 + 1e-6 and err(h.scaled, want * nw.double()) < 2.0 ** -8
+        assert err(h.partials[:h.blocks, :M].double().sum(0), want.pow(2).sum(1)) < 1e-5
