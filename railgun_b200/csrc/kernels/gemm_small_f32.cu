@@ -92,23 +92,29 @@ small_gemm_kernel(const float* __restrict__ x, int ldx, const float* __restrict_
 //   SG_NORM  x_new = x (+ pending), the 32-bit residual, and its rows' RMS norm: x_new / sqrt(mean(x_new^2) + eps) * norm_w.  The
 //            blocks of the first column write x_new, another buffer than x, which the other blocks still read.
 //   SG_SILU  silu(gate) * up of rows [gate K | up K]
-// A block makes its 32 rows once, in shared memory (K <= 256), again in every column of blocks: three to sixteen of them.
-// Two portions of 32 tokens beside three requests that decode, three layers of width 96: 31 launches to 22, 437 to some 405 us a step.
+// A block makes its 32 rows once, in shared memory (K <= 256), again in every column of blocks: three to sixteen of them; its 32
+// rows of W lie there too, asked for before the wait for the kernel before this one, so that behind the rows comes one run over
+// k.  Few blocks run, each once, so the latency of its parts is what counts: 256 threads, a row's numbers in one batch of loads.
+// Two portions of 32 tokens beside three requests that decode, three layers of width 96: 31 launches to 22, 437 to some
+// 405 us a step launched one by one.  With 128 threads, four loads under way and W a piece of 32 numbers at a time the norm's
+// products took 5.05 us each and SiLU-mul and 67 rows by 256 x 96 14.1; so 3.3 and 10.4, the step replayed 120 to 108.
 #define SG_NORM 1
 #define SG_SILU 2
 #define SG_MAX_K 256
+#define SG_ROWS_T 256
 
 template <int PRO, bool VEC>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(SG_ROWS_T)
 small_gemm_rows_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ pending, const float* __restrict__ norm_w,
                        float eps, float* __restrict__ x_new, const float* __restrict__ W, float* __restrict__ out, int ldo, int M,
                        int N, int K) {
-    extern __shared__ __align__(16) float rows[];                        // [SG_T][pitch]
-    __shared__ __align__(16) float sw[SG_T][SG_P];
+    extern __shared__ __align__(16) float rows[];                        // x's [SG_T][pitch], then W's, then SiLU's factors
     const int KP = (K + SG_T - 1) / SG_T * SG_T, pitch = KP + 4;         // pitch 4 mod 32: as SG_P
+    float* sw = rows + SG_T * pitch;
     const int m0 = blockIdx.y * SG_T, n0 = blockIdx.x * SG_T;
-    const int ty = threadIdx.x >> 3, tx = threadIdx.x & 7;
-    const int lr = threadIdx.x >> 2, lk = (threadIdx.x & 3) * 8;
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+    const int lr = threadIdx.x >> 3;                                     // loads: row lr, numbers k_first + 32 i .. + 3
+    const int k_first = (threadIdx.x & 7) * 4;
     const bool xrow = m0 + lr < M, wrow = n0 + lr < N;
     auto load = [&](const float* p, int k) {                             // numbers k .. k + 3 of a row, zeros behind K
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -122,78 +128,86 @@ small_gemm_rows_kernel(const float* __restrict__ x, int ldx, const float* __rest
         }
         return v;
     };
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     const float* wp = W + (size_t)(wrow ? n0 + lr : 0) * K;
-    float4 wv[2];
-    auto fetch_w = [&](int k0) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) wv[h] = wrow ? load(wp, k0 + lk + 4 * h) : make_float4(0.f, 0.f, 0.f, 0.f);
-    };
-    fetch_w(0);
+#pragma unroll 8
+    for (int k = k_first; k < KP; k += SG_T) *reinterpret_cast<float4*>(sw + lr * pitch + k) = wrow ? load(wp, k) : zero;
     pdl_wait();
     pdl_trigger();
-    // ---- the block's rows: four neighbouring threads a row, 16 numbers at a time
+    // ---- the block's rows: eight neighbouring threads a row, all its numbers under way at once
     const size_t row = (size_t)(xrow ? m0 + lr : 0);
     float* mine = rows + lr * pitch;
-    const int k_first = (threadIdx.x & 3) * 4;
-    float ss = 0.f;
-#pragma unroll 4
-    for (int k = k_first; k < KP; k += 16) {
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (xrow) {
-            v = load(x + row * ldx, k);
-            if (PRO == SG_NORM) {
-                if (pending) {
-                    const float4 p = load(pending + row * K, k);
-                    v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
-                    if (blockIdx.x == 0) {
-                        float* o = x_new + row * K + k;
-                        if (VEC) {
-                            if (k < K) *reinterpret_cast<float4*>(o) = v;
-                        } else {
-                            if (k < K) o[0] = v.x;
-                            if (k + 1 < K) o[1] = v.y;
-                            if (k + 2 < K) o[2] = v.z;
-                            if (k + 3 < K) o[3] = v.w;
-                        }
-                    }
-                }
-                ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-            } else {
-                const float4 u = load(x + row * ldx + K, k);
-                v.x = v.x / (1.f + expf(-v.x)) * u.x; v.y = v.y / (1.f + expf(-v.y)) * u.y;
-                v.z = v.z / (1.f + expf(-v.z)) * u.z; v.w = v.w / (1.f + expf(-v.w)) * u.w;
-            }
+    float4 v[SG_MAX_K / SG_T], p[SG_MAX_K / SG_T];
+#pragma unroll
+    for (int i = 0; i < SG_MAX_K / SG_T; ++i) {
+        const int k = k_first + SG_T * i;
+        v[i] = p[i] = zero;
+        if (xrow && k < KP) {
+            v[i] = load(x + row * ldx, k);
+            if (PRO == SG_SILU) p[i] = load(x + row * ldx + K, k);
+            else if (pending) p[i] = load(pending + row * K, k);
         }
-        *reinterpret_cast<float4*>(mine + k) = v;
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < SG_MAX_K / SG_T; ++i) {
+        const int k = k_first + SG_T * i;
+        if (k >= KP) break;
+        if (PRO == SG_NORM) {
+            v[i].x += p[i].x; v[i].y += p[i].y; v[i].z += p[i].z; v[i].w += p[i].w;
+            if (pending && xrow && blockIdx.x == 0) {
+                float* o = x_new + row * K + k;
+                if (VEC) {
+                    if (k < K) *reinterpret_cast<float4*>(o) = v[i];
+                } else {
+                    if (k < K) o[0] = v[i].x;
+                    if (k + 1 < K) o[1] = v[i].y;
+                    if (k + 2 < K) o[2] = v[i].z;
+                    if (k + 3 < K) o[3] = v[i].w;
+                }
+            }
+            ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
+        } else {
+            *reinterpret_cast<float4*>(sw + SG_T * pitch + lr * pitch + k) = p[i];
+        }
+        *reinterpret_cast<float4*>(mine + k) = v[i];
+    }
+    if (PRO == SG_SILU) {
+        // the thread's own numbers, by way of shared memory: written out eight times, the exponentials and divisions are some
+        // 20 KB of code that a block fetches to run once
+#pragma unroll 1
+        for (int k = k_first; k < KP; k += SG_T) {
+            float4 g = *reinterpret_cast<const float4*>(mine + k);
+            const float4 u = *reinterpret_cast<const float4*>(sw + SG_T * pitch + lr * pitch + k);
+            g.x = g.x / (1.f + expf(-g.x)) * u.x; g.y = g.y / (1.f + expf(-g.y)) * u.y;
+            g.z = g.z / (1.f + expf(-g.z)) * u.z; g.w = g.w / (1.f + expf(-g.w)) * u.w;
+            *reinterpret_cast<float4*>(mine + k) = g;
+        }
     }
     if (PRO == SG_NORM) {
         ss += __shfl_xor_sync(0xffffffffu, ss, 1);
         ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+        ss += __shfl_xor_sync(0xffffffffu, ss, 4);
         const float inv = rsqrtf(ss / (float)K + eps);
 #pragma unroll 4
-        for (int k = k_first; k < KP; k += 16) {                         // the thread's own numbers again
+        for (int k = k_first; k < KP; k += SG_T) {                         // the thread's own numbers again
             float4 v = *reinterpret_cast<const float4*>(mine + k);
             const float4 g = load(norm_w, k);
             v.x = v.x * inv * g.x; v.y = v.y * inv * g.y; v.z = v.z * inv * g.z; v.w = v.w * inv * g.w;
             *reinterpret_cast<float4*>(mine + k) = v;
         }
     }
-    // ---- the product, as above
-    float acc[2][4] = {};
+    __syncthreads();                                                      // both operands are there
+    float acc[2][2] = {};
     for (int k0 = 0; k0 < K; k0 += SG_T) {
-        __syncthreads();                                                  // the rows are there; W's numbers before have been used
-#pragma unroll
-        for (int h = 0; h < 2; ++h) *reinterpret_cast<float4*>(&sw[lr][lk + 4 * h]) = wv[h];
-        __syncthreads();
-        if (k0 + SG_T < K) fetch_w(k0 + SG_T);
-        float4 part[2][4] = {};
-        const float *r0 = rows + 2 * ty * pitch + k0, *r1 = r0 + pitch;
+        float4 part[2][2] = {};                                           // four chains of eight, then one of steps, as above
+        const float *r0 = rows + 2 * ty * pitch + k0, *r1 = r0 + pitch, *w0 = sw + tx * pitch + k0;
 #pragma unroll
         for (int k = 0; k < SG_T; k += 4) {
             const float4 a0 = *reinterpret_cast<const float4*>(r0 + k), a1 = *reinterpret_cast<const float4*>(r1 + k);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const float4 b = *reinterpret_cast<const float4*>(&sw[tx + 8 * q][k]);
+            for (int q = 0; q < 2; ++q) {
+                const float4 b = *reinterpret_cast<const float4*>(w0 + 16 * q * pitch + k);
                 part[0][q].x += a0.x * b.x; part[0][q].y += a0.y * b.y; part[0][q].z += a0.z * b.z; part[0][q].w += a0.w * b.w;
                 part[1][q].x += a1.x * b.x; part[1][q].y += a1.y * b.y; part[1][q].z += a1.z * b.z; part[1][q].w += a1.w * b.w;
             }
@@ -201,14 +215,14 @@ small_gemm_rows_kernel(const float* __restrict__ x, int ldx, const float* __rest
 #pragma unroll
         for (int r = 0; r < 2; ++r)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) acc[r][q] += (part[r][q].x + part[r][q].y) + (part[r][q].z + part[r][q].w);
+            for (int q = 0; q < 2; ++q) acc[r][q] += (part[r][q].x + part[r][q].y) + (part[r][q].z + part[r][q].w);
     }
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
         const int m = m0 + 2 * ty + r;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int n = n0 + tx + 8 * q;
+        for (int q = 0; q < 2; ++q) {
+            const int n = n0 + tx + 16 * q;
             if (m < M && n < N) out[(size_t)m * ldo + n] = acc[r][q];
         }
     }
@@ -235,9 +249,13 @@ extern "C" int rg_small_gemm_rows_f32(const float* x, int ldx, const float* pend
         return RG_ERR_UNSUPPORTED;
     const bool vec = K % 4 == 0 && ldx % 4 == 0 &&
                      (((uintptr_t)x | (uintptr_t)W | (uintptr_t)pending | (uintptr_t)norm_w | (uintptr_t)x_new) & 15) == 0;
-    const size_t smem = (size_t)SG_T * ((K + SG_T - 1) / SG_T * SG_T + 4) * sizeof(float);
+    const size_t smem = (size_t)(silu ? 3 : 2) * SG_T * ((K + SG_T - 1) / SG_T * SG_T + 4) * sizeof(float);       // up to 98 KB
     auto kernel = silu ? (vec ? small_gemm_rows_kernel<SG_SILU, true> : small_gemm_rows_kernel<SG_SILU, false>)
                        : (vec ? small_gemm_rows_kernel<SG_NORM, true> : small_gemm_rows_kernel<SG_NORM, false>);
-    return rg_launch(kernel, dim3((N + SG_T - 1) / SG_T, mt), dim3(128), smem, (cudaStream_t)stream, 1, x, ldx, pending, norm_w, eps, x_new,
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+    }
+    return rg_launch(kernel, dim3((N + SG_T - 1) / SG_T, mt), dim3(SG_ROWS_T), smem, (cudaStream_t)stream, 1, x, ldx, pending, norm_w, eps, x_new,
                      W, out, ldo, M, N, K);
 }
