@@ -2625,7 +2625,7 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k, top_p, seed: 
 # over the library's, over 1 to 40 rows, K 64 to 512 and N 96 to 3,000: up to 16 rows the library takes products with a
 # kernel for few rows: 0.67 to 1.01 on average (1.09 at most) up to K 96 and N 8,192, from K 97 on 0.99 to 1.15, from K 192
 # 1.2 to 3.4; from 17 rows 0.61 to 0.93 up to K 448, 512 is 0.94 from 31 rows and 1.04 to 1.08 below, and more 32 x 32 tiles
-# than SMs are up to 1.33 (33 rows by 3,000).
+# than SMs are up to 1.33 (33 rows by 3,000).  (The kernel has since become faster, by 2 to 15 % from 17 rows and K 256 on.)
 SMALL_F32_ROWS = 256
 SMALL_F32_LIMITS = ((96, 256), (448, 148), (512, 148))      # numbers of a row and tiles: up to 16 rows, up to 30, above
 
@@ -2658,15 +2658,7 @@ def small_gemm_f32(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """y = x W^T in 32-bit for a few rows by a small matrix."""
     if not small_gemm_f32_ok(x, weight):
         raise KernelError(f"small_gemm_f32 refuses x {tuple(x.shape)} {x.dtype}, W {tuple(weight.shape)} {weight.dtype}")
-    return _small_gemm_f32(x, weight)
-
-
-def _small_gemm_f32(x, weight):
-    (M, K), N = x.shape, weight.shape[0]
-    out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-    _ok(_fn("gemm_small_f32", "rg_small_gemm_f32")(_ptr(x), c_int(x.stride(0)), _ptr(weight), _ptr(out), c_int(N), c_int(M),
-                                                   c_int(N), c_int(K), _stream()), "small_gemm_f32")
-    return out
+    return _small_rows(x, False, weight)
 
 
 # Products whose rows the small product's kernel makes itself: 32-bit, of numbers that a block keeps in shared memory.
@@ -2710,27 +2702,32 @@ def fresh_norm(resid: torch.Tensor, pending, norm: torch.Tensor, eps: float, wei
     return FreshNorm(resid, pending, norm, eps)
 
 
-def _small_rows(x, ldx: int, pending, norm, eps: float, new, silu: bool, weight, M: int, K: int):
-    N = weight.shape[0]
+def _small_rows(h, gated: bool, weight):
+    """The rows ``h`` (a FreshNorm or a tensor) by ``weight``, or by its two halves and SiLU-mul."""
+    M, K = h.shape
+    N = weight.shape[0] // 2 if gated else weight.shape[0]
     out = torch.empty((M, N), dtype=torch.float32, device=weight.device)
-    _ok(_fn("gemm_small_f32", "rg_small_gemm_rows_f32")(
-        _ptr(x), c_int(ldx), _ptr(pending), _ptr(norm), c_float(eps), _ptr(new), c_int(1 if silu else 0), _ptr(weight), _ptr(out),
-        c_int(N), c_int(M), c_int(N), c_int(K), _stream()), "small_gemm_rows_f32")
+    fresh = isinstance(h, FreshNorm)
+    x, ldx, pending, norm, eps, new = (h.resid, K, h.pending, h.norm, h.eps, h.new) if fresh else (h, h.stride(0), None, None, 0.0, None)
+    _ok(_fn("gemm_small_f32", "rg_small_gemm_f32")(
+        _ptr(x), c_int(ldx), _ptr(pending), _ptr(norm), c_float(eps), _ptr(new), c_int(1 if gated else 0), _ptr(weight), _ptr(out),
+        c_int(N), c_int(M), c_int(N), c_int(K), _stream()), "small_gemm_f32")
     return out
 
 
-def silu_linear_ok(gate_up: torch.Tensor, weight: torch.Tensor) -> bool:
-    """Is the product of silu(gate) * up by ``weight`` one that the small product's kernel can make the rows of?"""
-    return (gate_up.dtype == torch.float32 and gate_up.dim() == 2 and gate_up.is_contiguous() and gate_up.shape[1] % 2 == 0
-            and _small_rows_ok(gate_up.shape[0], gate_up.shape[1] // 2, weight) and _by_address(gate_up, weight))
+def gated_linear_ok(x, weight: torch.Tensor) -> bool:
+    """Is the product by ``weight`` = gate | up one with SiLU-mul in its kernel?"""
+    if isinstance(x, FreshNorm):
+        return weight.shape[0] % 2 == 0 and x.shape[1] == weight.shape[1]           # the rest is why it is a FreshNorm
+    return (x.dtype == torch.float32 and x.dim() == 2 and x.stride(1) == 1 and x.stride(0) >= x.shape[1] and weight.shape[0] % 2 == 0
+            and _small_rows_ok(*x.shape, weight) and _by_address(x, weight))
 
 
-def silu_linear(gate_up: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
-    """(silu(gate) * up) W^T in 32-bit, ``gate_up`` [M, 2 K] = gate | up."""
-    if not silu_linear_ok(gate_up, weight):
-        raise KernelError(f"silu_linear refuses {tuple(gate_up.shape)} {gate_up.dtype}, W {tuple(weight.shape)} {weight.dtype}")
-    M, K2 = gate_up.shape
-    return _small_rows(gate_up, K2, None, None, 0.0, None, True, weight, M, K2 // 2)
+def gated_linear(x, weight: torch.Tensor) -> torch.Tensor:
+    """silu(gate) * up in 32-bit, gate | up = x W^T, ``weight`` [2 I, K] = gate | up."""
+    if not gated_linear_ok(x, weight):
+        raise KernelError(f"gated_linear refuses {tuple(x.shape)} {x.dtype}, W {tuple(weight.shape)} {weight.dtype}")
+    return _small_rows(x, True, weight)
 
 
 # Logits of decode batches by the streaming product: where the library's gets slower with more rows and this one does not.  128,256
@@ -2748,7 +2745,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, bias: torch.Te
     32-bit inputs run in true 32-bit: the reduced-precision matrix mode is
     refused."""
     if isinstance(x, FreshNorm):
-        return _small_rows(x.resid, x.shape[1], x.pending, x.norm, x.eps, x.new, False, weight, *x.shape)
+        return _small_rows(x, False, weight)
     if isinstance(x, NormedRows):
         if (out_dtype is None or out_dtype == torch.bfloat16) and skinny_scaled_ok(x, weight):
             return skinny_gemm_scaled(x, weight)              # the norm is finished inside the product
@@ -2770,7 +2767,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, bias: torch.Te
     if x.shape[0] <= SKINNY_AUTO_ROWS and skinny_gemm_ok(x, weight):
         return skinny_gemm(x, weight, out_dtype)             # small decode batches: stream the weights once
     if (out_dtype is None or out_dtype == torch.float32) and small_gemm_f32_ok(x, weight):
-        return _small_gemm_f32(x, weight)
+        return _small_rows(x, False, weight)
     if out_dtype == torch.float32 and STREAM_HEAD_ROWS[0] <= x.shape[0] <= STREAM_HEAD_ROWS[1] and weight.shape[0] > STREAM_HEAD_WIDTH \
             and tc_stream_ok(x, weight):
         return tc_stream_gemm(x, weight, out_dtype)          # logits of a decode batch over a large vocabulary

@@ -73,10 +73,10 @@ class SwiGLU(FeedForward):
             act = ops.tc_gemm(x, self.w_gate_up, silu_mul=True,
                               tile=ops.tc_pair_tile(x.shape[0], self.w_gate_up.shape[0], x.device))
         else:
-            gate_up = ops.linear(x, self.w_gate_up)
-            if not self.interleaved and ops.silu_linear_ok(gate_up, self.w_down):
-                return ops.silu_linear(gate_up, self.w_down)                     # a small 32-bit product, SiLU-mul in front of it
-            act = ops.silu_mul(gate_up, interleaved=self.interleaved)
+            if not self.interleaved and ops.gated_linear_ok(x, self.w_gate_up):
+                # a small 32-bit product, SiLU-mul behind it; the norm that follows takes the finished product
+                return ops.linear(ops.gated_linear(x, self.w_gate_up), self.w_down)
+            act = ops.silu_mul(ops.linear(x, self.w_gate_up), interleaved=self.interleaved)
         return ops.PendingLinear(act, self.w_down, stream) if defer else ops.linear(act, self.w_down)
 
 

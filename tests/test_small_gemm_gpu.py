@@ -70,7 +70,7 @@ def test_what_stays_the_librarys():
 @pytest.mark.parametrize("M,N,K", [(1, 1, 1), (67, 160, 96), (33, 33, 33), (17, 96, 256), (31, 65, 255), (2, 7, 4), (256, 40, 130)])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_rows_that_the_kernel_makes(M, N, K, shift):
-    """The norm of a residual with and without something pending, and SiLU-mul, in front of the product; on and off 16-byte
+    """The norm of a residual with and without something pending in front of the product, SiLU-mul behind it; on and off 16-byte
     boundaries; the first row of blocks leaves the sum."""
     from railgun_b200 import ops
     g = torch.Generator().manual_seed(M + N + K)
@@ -88,10 +88,14 @@ def test_rows_that_the_kernel_makes(M, N, K, shift):
         # as above; the root mean square and its two products are four more roundings
         assert rel_err(y, unit @ w.double().T) < 3e-6 and torch.equal(h.new, total)
         assert (h.new is x) == (pending is None)
-    gu = new(M, 2 * K)
-    want = (torch.nn.functional.silu(gu[:, :K].double()) * gu[:, K:].double()) @ w.double().T
-    if ops.silu_linear_ok(gu, w):
-        assert rel_err(ops.silu_linear(gu, w), want) < 3e-6
+        if N % 2 == 0:
+            # the same product, the same activation: silu's error is some 4 x 2^-24 of it
+            gate, up = y[:, :N // 2].double(), y[:, N // 2:].double()
+            assert rel_err(ops.gated_linear(h, w), torch.nn.functional.silu(gate) * up) < 5e-7
+    if N % 2 == 0 and ops.gated_linear_ok(x, w):
+        gate, up = (x.double() @ w.double().T).chunk(2, dim=1)
+        # two products' errors (2e-6 each, above), the gate's by silu's slope of at most 1.1
+        assert rel_err(ops.gated_linear(x, w), torch.nn.functional.silu(gate) * up) < 6e-6
 
 
 def test_what_makes_no_rows():
@@ -102,6 +106,7 @@ def test_what_makes_no_rows():
     assert ops.fresh_norm(x, None, n, 1e-5, torch.zeros(8, 65, device=DEV)) is None
     wide = torch.zeros(40, 288, device=DEV)
     assert ops.fresh_norm(wide, None, torch.ones(288, device=DEV), 1e-5, torch.zeros(8, 288, device=DEV)) is None
-    assert not ops.silu_linear_ok(torch.zeros(40, 127, device=DEV), w) and not ops.silu_linear_ok(x, w)
+    assert ops.gated_linear_ok(x, w) and not ops.gated_linear_ok(x, w[:7]) and not ops.gated_linear_ok(x[:, :63], w)
+    assert not ops.gated_linear_ok(x.t(), w) and not ops.gated_linear_ok(wide, torch.zeros(8, 288, device=DEV))
     grown = torch.zeros(8, 64, device=DEV, requires_grad=True)
     assert ops.fresh_norm(x, None, n, 1e-5, grown) is None
