@@ -635,7 +635,11 @@ decode_attention_kernel(const bf16* __restrict__ q, int q_stride, const bf16* __
         cp_async_commit();
     }
     wait_for_input();
-    pdl_trigger();
+    // Who comes next may start now, but for contexts in one part of up to 16 tokens: their output product is the one that streams its
+    // weights past a few rows, and next to this kernel it is slower than behind it.  A step of 60 keys each, 1B model: 4 requests
+    // 777 us beside, 620 behind, 16 requests 947 and 878; above, other products: 32 requests 855 and 877, 64 of 1,024 keys 1,197
+    // and 1,237.  (Behind several parts comes the kernel that adds them up, which waits for them in any case.)
+    if (num_splits > 1 || gridDim.x > 16 || beside) pdl_trigger();
     for (int idx = threadIdx.x; idx < 16 * d8; idx += NTHREADS) {
         const int row = idx / d8, c = idx - row * d8;
         const bool valid = row < nheads;

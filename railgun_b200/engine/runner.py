@@ -47,6 +47,11 @@ SHAPE_GRAPH_MIN_TOKENS = 256
 SHAPE_GRAPHS_KEPT = 4
 SMALL_GRAPH_AT = 4
 SMALL_GRAPHS_KEPT = 8
+# Steps of single tokens have a graph for each power of two of the longest context from 1,024 on, and one for contexts that short:
+# attention in one part (at 1,024 keys in four), so that no kernel adds parts up.  60 keys each, us a step: the 1B model
+# 1 request 641 to 606, 8 678 to 636, 32 910 to 857; kasarax's sizes 198 to 194, 207 to 202, 327 to 316.  At 200 keys the 1B model
+# still gains (637 to 626, 675 to 656, 908 to 875), kasarax loses (198 to 203, 208 to 210), at 400 both lose.
+SHORT_CONTEXT = 128
 SHAPES_COUNTED = 64, 512           # layouts whose steps are counted: of long steps, of short ones
 
 
@@ -397,7 +402,7 @@ class ModelRunner:
         B = _bucket(n_requests, _BATCH_BUCKETS)
         # block tables are as wide as the group with the smallest pages needs
         page = min(self.page_sizes) if self.page_sizes else 16
-        ctx_bucket = 1024
+        ctx_bucket = SHORT_CONTEXT if max_context <= SHORT_CONTEXT else 1024
         while ctx_bucket < max_context:
             ctx_bucket *= 2
         key = (B, -(-ctx_bucket // page))
@@ -475,7 +480,8 @@ class ModelRunner:
         self.last_greedy = None
         if tokens.min() < 0 or tokens.max() >= self.model.vocab_size:
             raise BatchError(f"token ids must be in [0, {self.model.vocab_size})")
-        ctx = max(self._ctx_hint + 1, 1)
+        longest = lambda: 1 + max((self.alloc.num_computed(i) for i in ids.tolist() if self.alloc.has(i)), default=0)  # noqa: E731
+        ctx = self._ctx_hint + 1 if self._ctx_hint else longest()
         while True:
             static = self._static_for(R, ctx)
             static.wait_until_reusable()
@@ -485,7 +491,7 @@ class ModelRunner:
                 break
             except CacheError as e:
                 if "bad argument" in str(e) and ctx < self.model.spec.max_position:
-                    ctx = min(2 * max(ctx, 1024), self.model.spec.max_position)
+                    ctx = min(max(2 * ctx, longest()), self.model.spec.max_position)   # other requests than the last step's
                     continue
                 raise
         B = static.B
