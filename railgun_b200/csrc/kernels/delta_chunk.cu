@@ -16,14 +16,18 @@
 //
 // What bounds it: the 32-bit multiply-adds (128 a cycle and SM, packed or not), and in delta_states the chain from chunk to
 // chunk, 2 x 64 x d of them per column and chunk.  16 columns a block fill 128 of 148 SMs at 16 heads of 128 columns;
-// narrower blocks fetch the same W and K more often.  Measured (2,048 tokens, 16 heads of 128 x 128 on 8): 58 us the
-// systems, 116 the states, 54 the outputs, with products in one chain; all three 269 us on 16 query/key heads since they add up
+// narrower blocks fetch the same W and K more often.  A chunk's 2,048 cycles of multiply-adds stand beside its copies, sums
+// across lanes and three barriers: sixteen warps (d known, eighths of k, quarters of the tokens) overlap those better than
+// eight, 119 us against 141 behind delta_solve at 16 heads of 128 x 128, 93 against 135 at 64 x 64.  Measured (2,048 tokens, 16 heads of 128 x 128 on 8): 58 us the
+// systems, 116 the states (eight warps), 54 the outputs, with products in one chain; all three 269 us on 16 query/key heads since they add up
 // in fours (chunk_scan.cuh), 258 before.  The token-by-token kernel (state_mixers.cu) takes 473 alone in a loop and took 908 in
 // a model's step.  Requests that bring fewer than 256 tokens stay on that one (ops.py, DELTA_CHUNK_MIN_TOKENS).
 #include "chunk_scan.cuh"
 #include <type_traits>
 
 #define DC_CB 16              // columns of S per block of delta_states
+#define DC_TH 512             // threads of delta_states
+#define DC_SP 24              // pitch of S and U in shared memory: eight neighbouring k lie in different banks
 #define DC_WP 72              // pitch of W's rows (k) in shared memory: four neighbouring k lie in different banks
 #define DC_MAX_D 128
 
@@ -229,17 +233,19 @@ __device__ __forceinline__ void dc_copy16(float* dst, const float* src, bool the
 
 // u [T, H, dv]: X on entry, U on return.  before [chunks, H, dv, d]: the state before every chunk.  d % 4 == 0, d <= 128,
 // dv % 4 == 0, rows of k 16-byte aligned.  grid: requests, H, groups of DC_CB columns; a chunk's W, K, X and factors are
-// fetched (cp.async) while the chunk before it is worked on.
-__global__ void __launch_bounds__(NTH)
+// fetched (cp.async) while the chunk before it is worked on.  D: d, or 0.
+template <int D>
+__global__ void __launch_bounds__(DC_TH)
 delta_states_kernel(const float* __restrict__ k, int k_ld, const float* __restrict__ w, const float* __restrict__ factors,
                     const float* __restrict__ decays, float* __restrict__ u, float* __restrict__ before,
                     float* __restrict__ state, const int* __restrict__ cu, const int* __restrict__ start_pos,
-                    const int* __restrict__ slots, int least, int H, int Hqk, int d, int dv) {
+                    const int* __restrict__ slots, int least, int H, int Hqk, int d_arg, int dv) {
     extern __shared__ __align__(16) float sm[];
+    const int d = D ? D : d_arg;
     const int KP = d + 16;                              // pitch of K's rows: two neighbouring tokens lie 16 banks apart
     const int stage_floats = d * DC_WP + CH * KP + CH * DC_CB + CH;
-    float* sS = sm + 2 * stage_floats;                  // [d][16], S
-    float* sU = sS + d * DC_CB;                         // [64][16], exp(c_L - c_i) u_i
+    float* sS = sm + 2 * stage_floats;                  // [d][DC_SP], S
+    float* sU = sS + d * DC_SP;                         // [64][DC_SP], exp(c_L - c_i) u_i
     pdl_wait();
     pdl_trigger();
     const int r = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * DC_CB, hq = h / (H / Hqk);
@@ -254,17 +260,17 @@ delta_states_kernel(const float* __restrict__ k, int k_ld, const float* __restri
         float* st = sm + (c & 1) * stage_floats;
         const int lo = first + c * CH, n = min(CH, last - lo);
         const size_t at = (size_t)(c0 + c) * H + h;
-        for (int e = threadIdx.x; e < d * (CH / 4); e += NTH) {
+        for (int e = threadIdx.x; e < d * (CH / 4); e += DC_TH) {
             const int kk = e / (CH / 4), i = e % (CH / 4) * 4;
             dc_copy16(st + kk * DC_WP + i, w + (at * d + kk) * CH + i, true);
         }
         st += d * DC_WP;
-        for (int e = threadIdx.x; e < CH * d4; e += NTH) {
+        for (int e = threadIdx.x; e < CH * d4; e += DC_TH) {
             const int i = e / d4, kk = (e - i * d4) * 4;
             dc_copy16(st + i * KP + kk, k + (size_t)(lo + min(i, n - 1)) * k_ld + (size_t)hq * d + kk, i < n);
         }
         st += CH * KP;
-        for (int e = threadIdx.x; e < CH * (DC_CB / 4); e += NTH) {
+        for (int e = threadIdx.x; e < CH * (DC_CB / 4); e += DC_TH) {
             const int i = e / (DC_CB / 4), j = e % (DC_CB / 4) * 4;
             const bool there = i < n && j < cols;
             dc_copy16(st + i * DC_CB + j, u + ((size_t)(lo + min(i, n - 1)) * H + h) * dv + j0 + (j < cols ? j : 0), there);
@@ -273,36 +279,30 @@ delta_states_kernel(const float* __restrict__ k, int k_ld, const float* __restri
         asm volatile("cp.async.commit_group;\n" ::);
     };
     issue(0);
-    // S: thread (k tile kt, column tile jt, half ih) keeps rows 4 kt .. + 3 of columns 4 jt + 2 ih and + 1
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int ih = lane >> 4, jt = lane & 3, kt = warp * 4 + ((lane >> 2) & 3);
+    // S: thread (k tile kt, column tile jt, quarter ih of the tokens, interleaved) keeps rows 4 kt .. + 3 of column 4 jt + ih
+    const int ih = lane >> 3, jt = (warp & 1) * 2 + (lane & 1), kt = (warp >> 1) * 4 + ((lane >> 1) & 3);
     const bool owner = kt < d4;
-    const int slot = slots[r];
-    float S[2][4];
-#pragma unroll
-    for (int b = 0; b < 2; ++b) {
-        const int j = 4 * jt + 2 * ih + b;
+    const int slot = slots[r], column = 4 * jt + ih;
+    float S[4];
+    {
         float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (owner && j < cols && slot >= 0 && start_pos[r] > 0)
-            x = *reinterpret_cast<const float4*>(state + (((size_t)slot * H + h) * dv + j0 + j) * d + 4 * kt);
-        S[b][0] = x.x; S[b][1] = x.y; S[b][2] = x.z; S[b][3] = x.w;
+        if (owner && column < cols && slot >= 0 && start_pos[r] > 0)
+            x = *reinterpret_cast<const float4*>(state + (((size_t)slot * H + h) * dv + j0 + column) * d + 4 * kt);
+        S[0] = x.x; S[1] = x.y; S[2] = x.z; S[3] = x.w;
     }
-    // the products W S0: thread (token tile it, column tile ju, quarter kq of the k, interleaved)
-    const int kq = lane >> 3, ju = lane & 3, it = warp * 2 + ((lane >> 2) & 1);
+    // the products W S0: thread (token tile it, column tile ju, eighth kq of the k, interleaved)
+    const int kq = lane >> 2, ju = (warp & 1) * 2 + (lane & 1), it = (warp >> 1) * 2 + ((lane >> 1) & 1);
     for (int c = 0; c < nc; ++c) {
         const int lo = first + c * CH, n = min(CH, last - lo);
         if (c + 1 < nc) issue(c + 1);
+        const float g = decays[(size_t)(c0 + c) * H + h];
         if (owner) {
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
-                *reinterpret_cast<float2*>(sS + (4 * kt + a) * DC_CB + 4 * jt + 2 * ih) = make_float2(S[0][a], S[1][a]);
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                const int j = 4 * jt + 2 * ih + b;
-                if (j < cols)
-                    *reinterpret_cast<float4*>(before + (((size_t)(c0 + c) * H + h) * dv + j0 + j) * d + 4 * kt) =
-                        make_float4(S[b][0], S[b][1], S[b][2], S[b][3]);
-            }
+            for (int a = 0; a < 4; ++a) sS[(4 * kt + a) * DC_SP + column] = S[a];
+            if (column < cols)
+                *reinterpret_cast<float4*>(before + (((size_t)(c0 + c) * H + h) * dv + j0 + column) * d + 4 * kt) =
+                    make_float4(S[0], S[1], S[2], S[3]);
         }
         if (c + 1 < nc) asm volatile("cp.async.wait_group 1;\n" ::);
         else asm volatile("cp.async.wait_group 0;\n" ::);
@@ -318,40 +318,43 @@ delta_states_kernel(const float* __restrict__ k, int k_ld, const float* __restri
 #pragma unroll
                 for (int b = 0; b < 4; ++b) acc[a][b] = 0.f;
 #pragma unroll 8
-            for (int kk = kq; kk < d; kk += 4) {
+            for (int kk = kq; kk < d; kk += 8) {
                 const float4 wv = *reinterpret_cast<const float4*>(sW + kk * DC_WP + 4 * it);
-                const float4 sv = *reinterpret_cast<const float4*>(sS + kk * DC_CB + 4 * ju);
+                const float4 sv = *reinterpret_cast<const float4*>(sS + kk * DC_SP + 4 * ju);
                 acc[0][0] += wv.x * sv.x; acc[0][1] += wv.x * sv.y; acc[0][2] += wv.x * sv.z; acc[0][3] += wv.x * sv.w;
                 acc[1][0] += wv.y * sv.x; acc[1][1] += wv.y * sv.y; acc[1][2] += wv.y * sv.z; acc[1][3] += wv.y * sv.w;
                 acc[2][0] += wv.z * sv.x; acc[2][1] += wv.z * sv.y; acc[2][2] += wv.z * sv.z; acc[2][3] += wv.z * sv.w;
                 acc[3][0] += wv.w * sv.x; acc[3][1] += wv.w * sv.y; acc[3][2] += wv.w * sv.z; acc[3][3] += wv.w * sv.w;
             }
-            // the four quarters' sums: lane kq ends up with token 4 it + kq
-            float half[2][4], one[4];
-            const bool up2 = kq >> 1, up1 = kq & 1;
+            // the eighths' sums: lane kq ends up with token 4 it + kq / 2, its first or second two columns
+            float half[2][4], one[4], two[2];
+            const bool up4 = kq & 4, up2 = kq & 2, up1 = kq & 1;
 #pragma unroll
             for (int a = 0; a < 2; ++a)
 #pragma unroll
                 for (int b = 0; b < 4; ++b) {
-                    const float give = up2 ? acc[a][b] : acc[a + 2][b], keep = up2 ? acc[a + 2][b] : acc[a][b];
+                    const float give = up4 ? acc[a][b] : acc[a + 2][b], keep = up4 ? acc[a + 2][b] : acc[a][b];
                     half[a][b] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
                 }
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
-                const float give = up1 ? half[0][b] : half[1][b], keep = up1 ? half[1][b] : half[0][b];
+                const float give = up2 ? half[0][b] : half[1][b], keep = up2 ? half[1][b] : half[0][b];
                 one[b] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
             }
-            const int i = 4 * it + kq;
-            const float4 xv = *reinterpret_cast<const float4*>(sX + i * DC_CB + 4 * ju);
-            const float4 uv = make_float4(xv.x - one[0], xv.y - one[1], xv.z - one[2], xv.w - one[3]);
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                const float give = up1 ? one[b] : one[b + 2], keep = up1 ? one[b + 2] : one[b];
+                two[b] = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+            }
+            const int i = 4 * it + (kq >> 1), j = 4 * ju + 2 * (kq & 1);
+            const float2 xv = *reinterpret_cast<const float2*>(sX + i * DC_CB + j);
+            const float2 uv = make_float2(xv.x - two[0], xv.y - two[1]);
             const float f = sF[i];
-            if (i < n && 4 * ju < cols) *reinterpret_cast<float4*>(u + ((size_t)(lo + i) * H + h) * dv + j0 + 4 * ju) = uv;
-            *reinterpret_cast<float4*>(sU + i * DC_CB + 4 * ju) =
-                i < n ? make_float4(f * uv.x, f * uv.y, f * uv.z, f * uv.w) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (i < n && j < cols) *reinterpret_cast<float2*>(u + ((size_t)(lo + i) * H + h) * dv + j0 + j) = uv;
+            *reinterpret_cast<float2*>(sU + i * DC_SP + j) = i < n ? make_float2(f * uv.x, f * uv.y) : make_float2(0.f, 0.f);
         }
         __syncthreads();
         {
-            const float g = decays[(size_t)(c0 + c) * H + h];
             float acc[4][4];
 #pragma unroll
             for (int a = 0; a < 4; ++a)
@@ -359,35 +362,33 @@ delta_states_kernel(const float* __restrict__ k, int k_ld, const float* __restri
                 for (int b = 0; b < 4; ++b) acc[a][b] = 0.f;
             if (owner) {
 #pragma unroll 8
-                for (int i = ih; i < n; i += 2) {
+                for (int i = ih; i < n; i += 4) {
                     const float4 kv = *reinterpret_cast<const float4*>(sK + i * KP + 4 * kt);
-                    const float4 uv = *reinterpret_cast<const float4*>(sU + i * DC_CB + 4 * jt);
+                    const float4 uv = *reinterpret_cast<const float4*>(sU + i * DC_SP + 4 * jt);
                     acc[0][0] += kv.x * uv.x; acc[0][1] += kv.x * uv.y; acc[0][2] += kv.x * uv.z; acc[0][3] += kv.x * uv.w;
                     acc[1][0] += kv.y * uv.x; acc[1][1] += kv.y * uv.y; acc[1][2] += kv.y * uv.z; acc[1][3] += kv.y * uv.w;
                     acc[2][0] += kv.z * uv.x; acc[2][1] += kv.z * uv.y; acc[2][2] += kv.z * uv.z; acc[2][3] += kv.z * uv.w;
                     acc[3][0] += kv.w * uv.x; acc[3][1] += kv.w * uv.y; acc[3][2] += kv.w * uv.z; acc[3][3] += kv.w * uv.w;
                 }
             }
-            // the two halves' sums: each keeps its two columns
+            // the quarters' sums: each keeps its column
+            const bool up2 = ih & 2, up1 = ih & 1;
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
+            for (int a = 0; a < 4; ++a) {
+                float pair[2];
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
-                    const float give = ih ? acc[a][b] : acc[a][2 + b], keep = ih ? acc[a][2 + b] : acc[a][b];
-                    S[b][a] = g * S[b][a] + (keep + __shfl_xor_sync(0xffffffffu, give, 16));
+                    const float give = up2 ? acc[a][b] : acc[a][b + 2], keep = up2 ? acc[a][b + 2] : acc[a][b];
+                    pair[b] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
                 }
+                const float give = up1 ? pair[0] : pair[1], keep = up1 ? pair[1] : pair[0];
+                S[a] = g * S[a] + (keep + __shfl_xor_sync(0xffffffffu, give, 8));
+            }
         }
         __syncthreads();                                // the stage and S may be overwritten
     }
-    if (owner && slot >= 0) {
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-            const int j = 4 * jt + 2 * ih + b;
-            if (j < cols)
-                *reinterpret_cast<float4*>(state + (((size_t)slot * H + h) * dv + j0 + j) * d + 4 * kt) =
-                    make_float4(S[b][0], S[b][1], S[b][2], S[b][3]);
-        }
-    }
+    if (owner && slot >= 0 && column < cols)
+        *reinterpret_cast<float4*>(state + (((size_t)slot * H + h) * dv + j0 + column) * d + 4 * kt) = make_float4(S[0], S[1], S[2], S[3]);
 }
 
 // q, k [T, Hqk * d] float rows q_ld, k_ld apart; v [T, H * dv] float or bfloat16, rows v_ld apart; beta, loga [T, H];
@@ -422,10 +423,10 @@ extern "C" int rg_delta_chunk(const float* q, int q_ld, const float* k, int k_ld
     }
 #undef DC_SOLVE
     if (e) return e;
-    const size_t smem = ((size_t)2 * (d * DC_WP + CH * (d + 16) + CH * DC_CB + CH) + (d + CH) * DC_CB) * sizeof(float);
-    cudaError_t ce = cudaFuncSetAttribute(delta_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const size_t smem = ((size_t)2 * (d * DC_WP + CH * (d + 16) + CH * DC_CB + CH) + (d + CH) * DC_SP) * sizeof(float);
+    auto states = d == 128 ? delta_states_kernel<128> : delta_states_kernel<0>;
+    cudaError_t ce = cudaFuncSetAttribute(states, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (ce != cudaSuccess) return (int)ce;
-    return rg_launch(delta_states_kernel, dim3(R, H, groups), dim3(NTH), smem, s, 1, k, k_ld, (const float*)w,
-                     (const float*)factors, (const float*)decays, u, before, state, cu_seqlens, start_pos, slots, least, H, Hqk,
-                     d, dv);
+    return rg_launch(states, dim3(R, H, groups), dim3(DC_TH), smem, s, 1, k, k_ld, (const float*)w, (const float*)factors,
+                     (const float*)decays, u, before, state, cu_seqlens, start_pos, slots, least, H, Hqk, d, dv);
 }
