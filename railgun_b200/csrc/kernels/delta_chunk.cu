@@ -18,10 +18,11 @@
 // chunk, 2 x 64 x d of them per column and chunk.  16 columns a block fill 128 of 148 SMs at 16 heads of 128 columns;
 // narrower blocks fetch the same W and K more often.  A chunk's 2,048 cycles of multiply-adds stand beside its copies, sums
 // across lanes and three barriers: sixteen warps (d known, eighths of k, quarters of the tokens) overlap those better than
-// eight, 119 us against 141 behind delta_solve at 16 heads of 128 x 128, 93 against 135 at 64 x 64.  Measured (2,048 tokens, 16 heads of 128 x 128 on 8): 58 us the
-// systems, 116 the states (eight warps), 54 the outputs, with products in one chain; all three 269 us on 16 query/key heads since they add up
-// in fours (chunk_scan.cuh), 258 before.  The token-by-token kernel (state_mixers.cu) takes 473 alone in a loop and took 908 in
-// a model's step.  Requests that bring fewer than 256 tokens stay on that one (ops.py, DELTA_CHUNK_MIN_TOKENS).
+// eight, 119 us against 141 behind delta_solve at 16 heads of 128 x 128, 93 against 135 at 64 x 64.
+// Measured with eight (2,048 tokens, 16 heads of 128 x 128 on 8): 58 us the systems, 116 the states, 54 the outputs, with products
+// in one chain; all three 269 us on 16 query/key heads since they add up in fours (chunk_scan.cuh), 258 before.  The
+// token-by-token kernel (state_mixers.cu) takes 473 alone in a loop and took 908 in a model's step.  Requests that bring fewer
+// than 256 tokens stay on that one (ops.py, DELTA_CHUNK_MIN_TOKENS).
 #include "chunk_scan.cuh"
 #include <type_traits>
 
