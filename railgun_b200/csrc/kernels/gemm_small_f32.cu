@@ -31,7 +31,7 @@ small_gemm_kernel(const float* __restrict__ x, int ldx, const float* __restrict_
                        float eps, float* __restrict__ x_new, const float* __restrict__ W, float* __restrict__ out, int ldo, int M,
                        int N, int K) {
     extern __shared__ __align__(16) float rows[];                        // x's [SG_T][pitch], then W's
-    const int KP = (K + SG_T - 1) / SG_T * SG_T, pitch = KP + 4;         // pitch 4 mod 32: as SG_P
+    const int KP = (K + SG_T - 1) / SG_T * SG_T, pitch = KP + 4;         // 4 mod 32
     float* sw = rows + SG_T * pitch;
     const int m0 = blockIdx.y * SG_T, n0 = blockIdx.x * (GATED ? SG_T / 2 : SG_T);
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
@@ -120,7 +120,7 @@ small_gemm_kernel(const float* __restrict__ x, int ldx, const float* __restrict_
     __syncthreads();                                                      // both operands are there
     float acc[2][2] = {};
     for (int k0 = 0; k0 < K; k0 += SG_T) {
-        float4 part[2][2] = {};                                           // four chains of eight, then one of steps, as above
+        float4 part[2][2] = {};                                           // four chains of eight, then one of steps
         const float *r0 = rows + 2 * ty * pitch + k0, *r1 = r0 + pitch, *w0 = sw + tx * pitch + k0;
 #pragma unroll
         for (int k = 0; k < SG_T; k += 4) {

@@ -47,10 +47,11 @@ SHAPE_GRAPH_MIN_TOKENS = 256
 SHAPE_GRAPHS_KEPT = 4
 SMALL_GRAPH_AT = 4
 SMALL_GRAPHS_KEPT = 8
-# Steps of single tokens have a graph for each power of two of the longest context from 1,024 on, and one for contexts that short:
-# attention in one part (at 1,024 keys in four), so that no kernel adds parts up.  60 keys each, us a step: the 1B model
+# Steps of single tokens have a graph for each power of two of the longest context from 1,024 on, and one for contexts of up to
+# SHORT_CONTEXT: attention in one part (at 1,024 keys in four), so that no kernel adds parts up.  60 keys each, us a step: the 1B model
 # 1 request 641 to 606, 8 678 to 636, 32 910 to 857; kasarax's sizes 198 to 194, 207 to 202, 327 to 316.  At 200 keys the 1B model
-# still gains (637 to 626, 675 to 656, 908 to 875), kasarax loses (198 to 203, 208 to 210), at 400 both lose.
+# still gains (637 to 626, 675 to 656, 908 to 875), kasarax loses (198 to 203, 208 to 210); at 400 keys
+# both lose up to 8 requests (643 to 652; 198 to 212).
 SHORT_CONTEXT = 128
 SHAPES_COUNTED = 64, 512           # layouts whose steps are counted: of long steps, of short ones
 
