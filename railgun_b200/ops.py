@@ -1768,7 +1768,7 @@ def skinny_gemm_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """Can the weight-streaming decode product take this shape?"""
     return (x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.dim() == 2
             and 0 < x.shape[0] <= SKINNY_MAX_ROWS and x.shape[1] % 8 == 0 and x.stride(1) == 1
-            and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and weight.is_contiguous())
+            and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and weight.is_contiguous() and weight.data_ptr() % 16 == 0)
 
 
 def skinny_gemm(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, silu_mul: bool = False,
@@ -1804,8 +1804,8 @@ def linear_groups(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     G, M, K = x.shape
     N = weight.shape[1]
     if (x.dtype == weight.dtype == torch.bfloat16 and 0 < M <= SKINNY_AUTO_ROWS and N % 32 == 0 and K % 8 == 0
-            and x.is_cuda and x.is_contiguous() and x.data_ptr() % 16 == 0 and weight.is_contiguous()
-            and weight.shape == (G, N, K)):
+            and weight.shape == (G, N, K) and _by_address(x, weight) and x.is_contiguous() and x.data_ptr() % 16 == 0
+            and weight.is_contiguous() and weight.data_ptr() % 16 == 0):
         out = torch.empty((G, M, N), dtype=torch.float32, device=x.device)
         _ok(_fn("gemm_skinny", "rg_skinny_gemm")(
             _ptr(weight), _ptr(x), c_int(K), _ptr(out), c_int(N), c_int(F32), c_int(0), c_int(M), c_int(G * N), c_int(K),
@@ -2244,7 +2244,7 @@ def tc_gemm(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, silu_mul: boo
 def tc_gemm_gated_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """Can ``tc_gemm_gated`` take these operands, and is it worth it?  From as many rows on as the SiLU-mul form."""
     return (isinstance(x, torch.Tensor) and x.dim() == 2 and x.shape[0] >= TC_GEMM_MIN_ROWS and weight.shape[0] % 16 == 0
-            and tc_gemm_ok(x, weight))
+            and _by_address(x, weight) and tc_gemm_ok(x, weight))
 
 
 def tc_gemm_gated(x: torch.Tensor, weight: torch.Tensor, act: str, limit: float = 0.0) -> torch.Tensor:
@@ -2633,13 +2633,14 @@ _PLAIN_TYPES = (torch.Tensor, torch.nn.Parameter)
 _forward_ad, _transforms = torch.autograd.forward_ad, torch._C._functorch.peek_interpreter_stack
 
 
-def _by_address(x: torch.Tensor, weight: torch.Tensor) -> bool:
-    """May a launcher take these by their addresses where the library would take them as tensors?  Both are on the current
+def _by_address(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None) -> bool:
+    """May a launcher take these by their addresses where the library would take them as tensors?  They are on the current
     device, and their product is neither differentiated (either way), mapped nor traced."""
     return (type(x) in _PLAIN_TYPES and type(weight) in _PLAIN_TYPES and x.is_cuda
             and x.get_device() == weight.get_device() == _current_device()
             and not ((x.requires_grad or weight.requires_grad) and torch.is_grad_enabled())
-            and _forward_ad._current_level < 0 and _transforms() is None)
+            and _forward_ad._current_level < 0 and _transforms() is None
+            and (bias is None or _by_address(bias, weight)))
 
 
 def small_gemm_f32_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
@@ -2760,8 +2761,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, bias: torch.Te
         # (up to 16 rows by 2,576 x 2,048: the library's 6.5 us, this package's 2.5)
         if out_dtype is not None and out_dtype != x.dtype:
             raise KernelError("linear: a product with a bias comes out in its input's type")
-        if (x.shape[0] <= SKINNY_AUTO_ROWS and skinny_gemm_ok(x, weight) and bias.dtype == torch.bfloat16
-                and bias.is_contiguous() and bias.shape == weight.shape[:1]):
+        if (x.dim() == weight.dim() == 2 and x.shape[0] <= SKINNY_AUTO_ROWS and x.shape[1] == weight.shape[1]
+                and bias.dtype == torch.bfloat16 and bias.shape == weight.shape[:1] and _by_address(x, weight, bias)
+                and bias.is_contiguous() and skinny_gemm_ok(x, weight)):
             return skinny_gemm(x, weight, bias=bias)
         return torch.addmm(bias, x, weight.t())
     if x.shape[0] <= SKINNY_AUTO_ROWS and skinny_gemm_ok(x, weight):
@@ -2769,7 +2771,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, bias: torch.Te
     if (out_dtype is None or out_dtype == torch.float32) and small_gemm_f32_ok(x, weight):
         return _small_rows(x, False, weight)
     if out_dtype == torch.float32 and STREAM_HEAD_ROWS[0] <= x.shape[0] <= STREAM_HEAD_ROWS[1] and weight.shape[0] > STREAM_HEAD_WIDTH \
-            and tc_stream_ok(x, weight):
+            and _by_address(x, weight) and tc_stream_ok(x, weight):
         return tc_stream_gemm(x, weight, out_dtype)          # logits of a decode batch over a large vocabulary
     if out_dtype is not None and out_dtype != x.dtype:
         return torch.mm(x, weight.t(), out_dtype=out_dtype)

@@ -31,6 +31,41 @@ def test_product_with_a_bias(M, N, K):
         assert torch.equal(ops.linear(x, w, bias=torch.zeros_like(b)), ops.linear(x, w))
 
 
+@pytest.mark.parametrize("M", [4, 48])
+def test_products_that_stay_the_librarys(M):
+    """With a bias, of several inputs, and logits of 41 to 64 rows: a matrix elsewhere is refused, one off a 16-byte boundary is
+    taken, and derivatives and maps go through the product."""
+    from railgun_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(M)
+    N, K = (64, 128) if M <= 16 else (ops.STREAM_HEAD_WIDTH + 64, 64)
+    flat = torch.randn(N * K + 1, device=DEV, generator=g).bfloat16()
+    w, odd = flat[:N * K].view(N, K), flat[1:].view(N, K)
+    x, b = torch.randn(M, K, device=DEV, generator=g).bfloat16(), torch.randn(N, device=DEV, generator=g).bfloat16()
+    bias, out_dtype = (b, None) if M <= 16 else (None, torch.float32)
+    calls = [lambda x, w, b: ops.linear(x, w, out_dtype, bias=bias if b is None else b)]
+    if M <= 16:
+        calls.append(lambda x, w, b: ops.linear_groups(x[None], w[None])[0])
+    for call in calls:
+        exact = lambda w: x.double() @ w.double().T + (b.double() if call is calls[0] and M <= 16 else 0.0)  # noqa: E731
+        # one rounding to bfloat16 at most, of a sum that is off by K 2^-24 of its terms at most
+        assert (call(x, odd, None).double() - exact(odd)).abs().max() <= (2.0 ** -8 + 2.0 ** -14) * exact(odd).abs().max()
+        with pytest.raises(RuntimeError):
+            call(x, w.cpu(), None)
+        with pytest.raises(RuntimeError):
+            call(x.cpu(), w, None)
+    if M <= 16:
+        with pytest.raises(RuntimeError):
+            ops.linear(x, w, bias=b.cpu())
+        xg, wg, bg = (t.clone().requires_grad_() for t in (x, w, b))
+        ops.linear(xg, wg, bias=bg).float().sum().backward()
+        assert torch.allclose(bg.grad.float(), torch.full((N,), float(M), device=DEV))
+        assert rel(wg.grad, x.double().sum(0).expand_as(w)) < 2.0 ** -7 and rel(xg.grad, w.double().sum(0).expand_as(x)) < 2.0 ** -7
+        moved = torch.func.jvp(lambda a: ops.linear(a, w, bias=b), (x,), (torch.ones_like(x),))[1]
+        assert rel(moved, w.double().sum(1).expand(M, N)) < 2.0 ** -7
+        maps = torch.vmap(lambda m: ops.linear(x, m, bias=b))(torch.stack([w, 2 * w]))
+        assert rel(maps[1], 2 * x.double() @ w.double().T + b.double()) < 2.0 ** -7
+
+
 @pytest.mark.parametrize("M,G,N,K", [(1, 4, 1024, 2048), (16, 4, 64, 48), (5, 3, 32, 8), (8, 2, 2400, 72), (17, 4, 64, 64), (3, 4, 48, 64)])
 def test_products_of_several_inputs(M, G, N, K):
     from railgun_b200 import ops

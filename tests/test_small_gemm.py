@@ -1,4 +1,5 @@
-"""Which 32-bit products go to this package's kernel by address: only those whose operands a kernel can read."""
+"""Which products go to this package's kernels by address: only those whose operands a kernel can read."""
+import pytest
 import torch
 
 from railgun_b200 import ops
@@ -8,3 +9,25 @@ def test_an_operand_on_the_host_is_no_operand():
     x, w = torch.zeros(4, 64), torch.zeros(8, 64)
     assert not ops.small_gemm_f32_ok(x, w)
     assert not ops.small_gemm_f32_ok(x.to("meta"), w.to("meta"))
+
+
+@pytest.mark.parametrize("M,dtype", [(4, None), (48, torch.float32)])
+def test_a_product_that_cannot_go_by_address_asks_for_no_address(M, dtype, monkeypatch):
+    """With a bias, and logits of 41 to 64 rows: whether operands may go by address is asked before anything looks at one."""
+    class Operand(torch.Tensor):
+        is_cuda = True
+
+        def data_ptr(self):
+            raise AssertionError("an address")
+    N = 24 if M == 4 else ops.STREAM_HEAD_WIDTH + 8
+    x, w, b = (torch.zeros(*s, dtype=torch.bfloat16).as_subclass(Operand) for s in ((M, 64), (N, 64), (N,)))
+    monkeypatch.setattr(torch, "addmm", lambda *a: "library")
+    monkeypatch.setattr(torch, "mm", lambda *a, **k: "library")
+    monkeypatch.setattr(ops, "SKINNY_AUTO_ROWS", 16 if M == 4 else 0)
+    assert ops.linear(x, w, dtype, bias=b if M == 4 else None) == "library"
+
+
+def test_a_matrix_off_a_16_byte_boundary_is_not_for_16_byte_loads():
+    x, flat = torch.zeros(4, 64).bfloat16(), torch.zeros(24 * 64 + 8).bfloat16()
+    assert flat.data_ptr() % 16 == 0
+    assert [ops.skinny_gemm_ok(x, flat[i:i + 24 * 64].view(24, 64)) for i in (0, 1, 4, 8)] == [True, False, False, True]
