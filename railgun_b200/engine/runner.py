@@ -42,18 +42,21 @@ _DTYPES = {"bfloat16": torch.bfloat16, "bf16": torch.bfloat16, "float32": torch.
 # layout repeats: a portion's size is mostly the scheduler's, and the step of a prompt's next portion beside the same decoding
 # requests has the layout of the one before.  From SHAPE_GRAPH_MIN_TOKENS tokens on at the second step of a layout; shorter
 # steps at the SMALL_GRAPH_AT-th: what a replay saves there is host time (some 30 to 85 launches of 14 to 18 us), a capture
-# costs as much as some of them, and short prompts' layouts are many.  So many layouts of either kind are kept, the ones used last.
+# costs as much as some of them, and short prompts' layouts are many.  So many layouts of either kind are kept.  Where more
+# of them come in turn than are kept, a short step's graph gives way only once it has not been used for so many steps: every
+# step would cost a capture otherwise (RepeatedLayouts).  Long ones, whose captures cost a step or two, give way at once.
 SHAPE_GRAPH_MIN_TOKENS = 256
 SHAPE_GRAPHS_KEPT = 4
 SMALL_GRAPH_AT = 4
-SMALL_GRAPHS_KEPT = 8
+SMALL_GRAPHS_KEPT = 16
+GIVES_WAY_AFTER = 0, 1024          # steps without use: graphs of long steps, of short ones
 # Steps of single tokens have a graph for each power of two of the longest context from 1,024 on, and one for contexts of up to
 # SHORT_CONTEXT: attention in one part (at 1,024 keys in four), so that no kernel adds parts up.  60 keys each, us a step: the 1B model
 # 1 request 641 to 606, 8 678 to 636, 32 910 to 857; kasarax's sizes 198 to 194, 207 to 202, 327 to 316.  At 200 keys the 1B model
 # still gains (637 to 626, 675 to 656, 908 to 875), kasarax loses (198 to 203, 208 to 210); at 400 keys
 # both lose up to 8 requests (643 to 652; 198 to 212).
 SHORT_CONTEXT = 128
-SHAPES_COUNTED = 64, 512           # layouts whose steps are counted: of long steps, of short ones
+LAYOUTS_COUNTED = 64, 512          # layouts whose steps are counted: of long steps, of short ones
 
 
 @contextlib.contextmanager
@@ -242,6 +245,50 @@ class ShapeGraph:
         self.hold = None               # the last packed step (keeps its pinned buffer alive until the copy has run)
 
 
+class RepeatedLayouts:
+    """Which layouts have a captured step (``graphs``), the one used last at the end, and when the next one gets one: at the
+    ``at``-th step of a layout, if there is a place among ``kept`` or a graph that has not been used for ``idle`` steps, which
+    gives way.  The layout of a graph that gave way counts anew.  So there are ``kept`` captures in ``idle`` steps at most,
+    whatever comes in whatever order, and layouts that come in turn keep the graphs that they have."""
+
+    def __init__(self, at: int, kept: int, idle: int, counted: int):
+        self.at, self.kept, self.idle, self.counted = at, kept, idle, counted
+        self.graphs: dict = {}
+        self.seen: dict = {}               # layout -> its steps up to the capture
+        self._used: dict = {}              # the step that used a graph last
+        self._steps = 0
+
+    def replay(self, key):
+        """The graph of a step's layout, or None (``to_capture`` is asked next then)."""
+        graph = self.graphs.pop(key, None)
+        if graph is not None:
+            self._steps += 1
+            self._used[key] = self._steps
+            self.graphs[key] = graph
+        return graph
+
+    def to_capture(self, key) -> bool:
+        """Count a step of a layout without a graph: is it the one to capture?  If so a graph that is in the way is dropped."""
+        self._steps += 1
+        seen = self.seen.get(key, 0) + 1
+        if len(self.seen) > self.counted:
+            self.seen.clear()
+        self.seen[key] = seen
+        if seen < self.at:
+            return False
+        if len(self.graphs) >= self.kept:
+            oldest = next(iter(self.graphs))
+            if self._steps - self._used[oldest] < self.idle:
+                return False
+            del self.graphs[oldest], self._used[oldest]
+            self.seen.pop(oldest, None)
+        return True
+
+    def keep(self, key, graph) -> None:
+        self._used[key] = self._steps
+        self.graphs[key] = graph
+
+
 class CapturedStep:
     def __init__(self, graph, logits, sampled, launches):
         self.graph, self.logits, self.sampled, self.launches = graph, logits, sampled, launches
@@ -278,10 +325,10 @@ class ModelRunner:
         # static and the rows' slots are data of the step (-1 in a padding row).
         self.use_graphs = bool(use_graphs) and self.model.graph_safe
         self._static: dict = {}
-        self._shape_steps: dict = {}       # graph key -> ShapeGraph: steps seen before replay a captured graph
-        self._shape_seen: dict = {}
-        self._small_steps: dict = {}       # the same for steps of fewer than ``shape_graph_min_tokens`` tokens
-        self._small_seen: dict = {}
+        # graph key -> ShapeGraph, of steps of ``shape_graph_min_tokens`` tokens and more and of shorter ones
+        self._long_steps = RepeatedLayouts(2, SHAPE_GRAPHS_KEPT, GIVES_WAY_AFTER[0], LAYOUTS_COUNTED[0])
+        self._short_steps = RepeatedLayouts(SMALL_GRAPH_AT, SMALL_GRAPHS_KEPT, GIVES_WAY_AFTER[1], LAYOUTS_COUNTED[1])
+        self._shape_steps, self._shape_seen = self._long_steps.graphs, self._long_steps.seen
         self.shape_graph_min_tokens = SHAPE_GRAPH_MIN_TOKENS
         self._graph_pool = None
         self._ctx_hint = 0
@@ -330,18 +377,17 @@ class ModelRunner:
         and block-table widths fix every shape, everything else is data in the
         step's one device buffer.  The first steps of a layout run eagerly, the
         second (of a short step the ``SMALL_GRAPH_AT``-th) is captured while it runs, later
-        ones replay; a few layouts are kept (``SHAPE_GRAPH_MIN_TOKENS``)."""
-        large = sum(len(e.tokens) for e in entries) >= self.shape_graph_min_tokens
-        steps, seen_of = (self._shape_steps, self._shape_seen) if large else (self._small_steps, self._small_seen)
+        ones replay; a few layouts are kept (``RepeatedLayouts``)."""
+        steps = (self._long_steps if sum(len(e.tokens) for e in entries) >= self.shape_graph_min_tokens
+                 else self._short_steps)
         build = lambda into: build_step_batch(entries, self.alloc, self.page_sizes, self.model.vocab_size,
                                               self.model.spec.max_position, self.device, self.err_flag, into=into)
-        known = lambda key: steps[key].dev if key in steps else None
+        known = lambda key: steps.graphs[key].dev if key in steps.graphs else None
         batch = build(known)
         self.last_h2d_bytes = batch.h2d_bytes
         key = batch.graph_key
-        shape = steps.pop(key, None)
+        shape = steps.replay(key)
         if shape is not None:
-            steps[key] = shape                                     # the one used last
             # the step was packed straight into the graph's buffer: launch
             shape.hold = batch
             shape.graph.replay()
@@ -349,17 +395,11 @@ class ModelRunner:
             ops.mark_tc_unchecked()
             self._commit(entries, batch)
             return shape.logits
-        seen = seen_of.get(key, 0) + 1
-        if len(seen_of) > SHAPES_COUNTED[0 if large else 1]:
-            seen_of.clear()
-        seen_of[key] = seen
-        if seen < (2 if large else SMALL_GRAPH_AT):
+        if not steps.to_capture(key):
             logits = self.model.forward(batch, self.views)
             self._commit(entries, batch)
             return logits
         # the layout repeats: a static copy of the packed buffer, one eager run over it (this step), the capture
-        if len(steps) >= (SHAPE_GRAPHS_KEPT if large else SMALL_GRAPHS_KEPT):
-            steps.pop(next(iter(steps)))
         dev = torch.empty(batch.host_buffer.numel(), dtype=torch.int32, device=self.device)
         batch = build(lambda key: dev)
         side = torch.cuda.Stream(device=self.device)
@@ -376,7 +416,7 @@ class ModelRunner:
             logits = self.model.forward(batch, self.views)
         launches = counter.value - n0
         counter.value = n0
-        steps[key] = ShapeGraph(dev, batch, graph, logits, launches)
+        steps.keep(key, ShapeGraph(dev, batch, graph, logits, launches))
         self._commit(entries, batch)
         return eager
 
