@@ -21,7 +21,8 @@ import torch
 
 ATTENTION_TILE_ROWS = 64      # query rows per tile of the prefill attention kernel
 # Contexts of portions at which parts choose another attention kernel.  A captured step keeps its choice, so steps on
-# different sides of one are different graphs: what a step computes never depends on which one was captured first.
+# different sides of one are different graphs, and so are steps whose single tokens' contexts are cut into other numbers of
+# parts: what a step computes never depends on which one was captured first.
 PORTION_CONTEXTS = (128, 256)
 
 
@@ -101,7 +102,7 @@ class StepBatch:
 
 
 def build_step_batch(entries, alloc, page_sizes, vocab_size: int, max_position: int, device,
-                     err_flag=None, into=None) -> StepBatch:
+                     err_flag=None, into=None, splits=None) -> StepBatch:
     """Validate the entries against the cache's bookkeeping, reserve pages and
     pack everything into one host buffer that goes to the device in one copy.
 
@@ -110,8 +111,10 @@ def build_step_batch(entries, alloc, page_sizes, vocab_size: int, max_position: 
     Block tables are as wide as the longest one rounded up to a power of two,
     so that steps of the same token counts have the same layout.  ``into``:
     called with the graph key (the layout, that is token counts, wanted places
-    and block-table widths; and whether the longest context of a portion is
-    above each of ``PORTION_CONTEXTS``, at which the attention kernels change)
+    and block-table widths; whether the longest context of a portion is
+    above each of ``PORTION_CONTEXTS``, at which the attention kernels change;
+    and, where there are single tokens, what ``splits(their number, longest
+    context)`` says: into how many parts their contexts are cut)
     once it is known; if it returns a device int32 buffer (of exactly the
     layout's size) the step is copied into that buffer, whose address is what a
     captured graph reads, and the batch's tensors are views of it."""
@@ -168,7 +171,10 @@ def build_step_batch(entries, alloc, page_sizes, vocab_size: int, max_position: 
     slots = host[offs[7]:offs[8]].copy()
     layout = (tuple(count_list), W, max_blocks_t)
     portion_context = max((a + b for a, b in zip(start_list, count_list) if b > 1), default=0)
+    longest = max(a + b for a, b in zip(start_list, count_list))
     key = (layout, tuple(portion_context > n for n in PORTION_CONTEXTS))
+    if n_dec and splits is not None:
+        key += splits(n_dec, longest)
     static = into(key) if into is not None else None
     if static is not None:
         if static.numel() != buf.numel():
@@ -180,7 +186,7 @@ def build_step_batch(entries, alloc, page_sizes, vocab_size: int, max_position: 
     d = dev.split(sizes).__getitem__                       # views, cut in one call
     return StepBatch(
         num_tokens=T, num_requests=R, num_wanted=W,
-        max_query_len=max(count_list), max_context_len=max(a + b for a, b in zip(start_list, count_list)),
+        max_query_len=max(count_list), max_context_len=longest,
         token_ids=d(0), positions=d(1), req_of_token=d(2), want_rows=d(3), cu_seqlens=d(4),
         context_lens=d(5), start_pos=d(6), state_slots=d(7),
         slot_mapping=[d(8 + 2 * g) for g in range(G)],

@@ -381,7 +381,8 @@ class ModelRunner:
         steps = (self._long_steps if sum(len(e.tokens) for e in entries) >= self.shape_graph_min_tokens
                  else self._short_steps)
         build = lambda into: build_step_batch(entries, self.alloc, self.page_sizes, self.model.vocab_size,
-                                              self.model.spec.max_position, self.device, self.err_flag, into=into)
+                                              self.model.spec.max_position, self.device, self.err_flag, into=into,
+                                              splits=self.model.single_token_splits)
         known = lambda key: steps.graphs[key].dev if key in steps.graphs else None
         batch = build(known)
         self.last_h2d_bytes = batch.h2d_bytes

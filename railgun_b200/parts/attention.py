@@ -75,6 +75,7 @@ class PagedAttention(Mixer):
         self.nh, self.nkv, self.d = p["num_heads"], p["num_kv_heads"], p["head_dim"]
         if self.nh % self.nkv:
             raise ValueError(f"{self.nh} heads cannot share {self.nkv} key/value heads")
+        self.kv_tiles = self.nkv * (-(-(self.nh // self.nkv) // 8))
         if self.d > 256:
             raise ValueError(f"head size {self.d} is above the attention kernels' limit of 256")
         self.window = int(p.get("window") or 0)
@@ -99,6 +100,13 @@ class PagedAttention(Mixer):
     takes_normed_rows = True
     defers_output = True
     first_matrix = property(lambda self: self.w_qkv)
+
+    def splits(self, n, longest):
+        return ops.decode_splits(n, self.kv_tiles, longest)
+
+    @property
+    def split_rule(self):
+        return ("paged", self.kv_tiles) if self.env.dtype == torch.bfloat16 and self.d % 16 == 0 else None
 
     def forward(self, x, batch, cache, writes=True, defer=False):
         nh, nkv, d = self.nh, self.nkv, self.d
@@ -141,12 +149,10 @@ class PagedAttention(Mixer):
             return ops.paged_attention_general(qkv, qkv.shape[1], cache.kv, table, batch.req_of_token,
                                                batch.positions, nh, nkv, d, self.window, self.scale)
         out = torch.empty((qkv.shape[0], nh * d), dtype=qkv.dtype, device=qkv.device)
-        kv_tiles = nkv * (-(-(nh // nkv) // 8))
         if batch.decode_only:
             n = batch.num_tokens
             ops.decode_attention(qkv, qkv.shape[1], out, cache.kv, table, None, n, batch.req_of_token,
-                                 batch.positions, nh, nkv, d, self.window, self.scale,
-                                 ops.decode_splits(n, kv_tiles, batch.max_context_len))
+                                 batch.positions, nh, nkv, d, self.window, self.scale, self.splits(n, batch.max_context_len))
             return out
         if batch.num_prefill_tiles:
             if USE_TC_ATTENTION and batch.num_prefill_tiles128 and ops.prefill_attention_tc_ok(
@@ -163,7 +169,7 @@ class PagedAttention(Mixer):
             n = batch.num_decode_rows
             ops.decode_attention(qkv, qkv.shape[1], out, cache.kv, table, batch.decode_rows, n, batch.req_of_token,
                                  batch.positions, nh, nkv, d, self.window, self.scale,
-                                 ops.decode_splits(n, kv_tiles, batch.max_context_len), beside=batch.num_prefill_tiles > 0)
+                                 self.splits(n, batch.max_context_len), beside=batch.num_prefill_tiles > 0)
         return out
 
 
@@ -401,6 +407,20 @@ class NormedAttention(Mixer):
         gate = proj[:, C:] if self.out_gate else None
         return self.attend(q.view(-1, H * D), batch, pages, gate, pooled, out, out_scale)
 
+    def splits(self, n, longest):
+        reach = longest
+        if self.window:
+            reach = min(reach, self.window + self.keep_first + (reach // self.pool if self.pool else 0))
+        if self.chunk:
+            reach = min(reach, self.chunk)
+        return ops.decode_splits(n, self.G * (-(-(self.H // self.G) // 8)), reach)
+
+    @property
+    def split_rule(self):
+        if self.env.dtype != torch.bfloat16:
+            return None
+        return "gqa", self.H, self.G, self.window, self.keep_first, self.pool, self.chunk
+
     def attend(self, q, batch, cache, gate=None, pooled=None, out=None, out_scale: float = 1.0):
         """bfloat16 runs on the tensor cores (requests with several tokens through the flash-style kernel, single
         tokens through the split kernel; both know the window, the kept first tokens or the pooled blocks, the sink
@@ -413,12 +433,6 @@ class NormedAttention(Mixer):
                                                H, G, D, self.window, 1.0, self.keep_first, out=out, **more)
         if out is None:
             out = torch.empty((q.shape[0], H * D), dtype=q.dtype, device=q.device)
-        kv_tiles = G * (-(-(H // G) // 8))
-        reach = batch.max_context_len
-        if self.window:
-            reach = min(reach, self.window + self.keep_first + (reach // self.pool if self.pool else 0))
-        if self.chunk:
-            reach = min(reach, self.chunk)
         if batch.num_prefill_tiles:
             if pooled is None and use_wide_attention(q, out, batch, cache, H, G, D):
                 ops.prefill_attention_wide(q, out, cache.kv, table, batch.prefill_tiles128, batch.positions, H, G, D,
@@ -431,7 +445,7 @@ class NormedAttention(Mixer):
         if n:
             ops.decode_attention(q, q.shape[1], out, cache.kv, table, None if batch.decode_only else batch.decode_rows,
                                  n, batch.req_of_token, batch.positions, H, G, D, self.window, 1.0,
-                                 ops.decode_splits(n, kv_tiles, reach), keep_first=self.keep_first,
+                                 self.splits(n, batch.max_context_len), keep_first=self.keep_first,
                                  beside=batch.num_prefill_tiles > 0, **more)
         return out
 

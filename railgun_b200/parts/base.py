@@ -114,11 +114,22 @@ class Mixer(Part):
     ``ops.PendingLinear``.  A mixer with ``takes_stream`` = True has
     ``forward_stream(stream, batch, cache, writes)``, which adds what is pending
     to the stream and reads it in one kernel, for arrangements without a norm
-    before the part."""
+    before the part.  A mixer that cuts its single tokens' contexts into
+    parts by their number and the step's longest context does so by
+    ``splits(n, longest)`` and says by ``split_rule`` (equal for mixers that
+    cut alike) that it does: the answer is part of what a captured step is
+    known by.  ``nested()``: the mixers that a wrapper runs."""
 
     takes_normed_rows = False
     defers_output = False
     takes_stream = False
+    split_rule = None
+
+    def splits(self, n: int, longest: int) -> int:
+        raise NotImplementedError
+
+    def nested(self):
+        return ()
 
     @classmethod
     def cache_need(cls, params: dict):

@@ -196,7 +196,7 @@ class LatentAttention(Mixer):
             if ops.latent_attention_mma_ok(qa.dtype, H, R, D):
                 ops.latent_attention_mma(qa, o_lat, cache.kv, table, None, batch.decode_rows, n, batch.req_of_token,
                                          batch.positions, R, self.window, self.scale,
-                                         ops.latent_decode_splits(n, -(-H // 64), self._reach(batch)))
+                                         self.splits(n, batch.max_context_len))
             else:
                 o_lat = ops.latent_attention_general(qa, cache.kv, table, batch.req_of_token, batch.positions, R,
                                                      self.window, self.scale)
@@ -209,9 +209,13 @@ class LatentAttention(Mixer):
             ops.sigmoid_gate_(out, proj[:, self.gate_off:self.gate_off + H * dv], dv, d)
         return ops.linear(out, self.w_o_padded)
 
-    def _reach(self, batch) -> int:
-        """How many keys a single token sees at most: that is what its context is cut into shares by."""
-        return min(batch.max_context_len, self.window) if self.window else batch.max_context_len
+    def splits(self, n, longest):
+        # by how many keys a single token sees at most
+        return ops.latent_decode_splits(n, -(-self.H // 64), min(longest, self.window) if self.window else longest)
+
+    @property
+    def split_rule(self):
+        return ("latent", self.H, self.window) if ops.latent_attention_mma_ok(self.env.dtype, self.H, self.R, self.D) else None
 
     def attend(self, qa, batch, cache):
         """bfloat16 with sizes in steps of 16 runs on the tensor cores (requests with several tokens in tiles of
@@ -222,13 +226,11 @@ class LatentAttention(Mixer):
             return ops.latent_attention_general(qa, cache.kv, table, batch.req_of_token, batch.positions, self.R,
                                                 self.window, self.scale, self.sink)
         out = torch.empty((qa.shape[0], self.H, self.R), dtype=qa.dtype, device=qa.device)
-        chunks = -(-self.H // 64)
         args = (batch.req_of_token, batch.positions, self.R, self.window, self.scale)
-        reach = self._reach(batch)
         if batch.decode_only:
             n = batch.num_tokens
             ops.latent_attention_mma(qa, out, cache.kv, table, None, None, n, *args,
-                                     ops.latent_decode_splits(n, chunks, reach), sink=self.sink)
+                                     self.splits(n, batch.max_context_len), sink=self.sink)
             return out
         if batch.num_prefill_tiles:
             ops.latent_attention_mma(qa, out, cache.kv, table, batch.prefill_tiles, None, batch.num_prefill_tiles, *args,
@@ -236,7 +238,7 @@ class LatentAttention(Mixer):
         if batch.num_decode_rows:
             n = batch.num_decode_rows
             ops.latent_attention_mma(qa, out, cache.kv, table, None, batch.decode_rows, n, *args,
-                                     ops.latent_decode_splits(n, chunks, reach), sink=self.sink)
+                                     self.splits(n, batch.max_context_len), sink=self.sink)
         return out
 
 

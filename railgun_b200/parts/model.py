@@ -123,6 +123,7 @@ class DecoderModel:
             ))
             for built, b in zip(self.layers[-1].branches, ls.branches()):
                 built.wiring = self.layers[-1].arrangement.bind(b, ls.prefix, env, tensors)
+        self._cutters = self._find_cutters()
         self.final_norm = NORMS.get(spec.final_norm.kind)(spec.final_norm.params, "", env, tensors)
         self.head = HEADS.get(spec.head.kind)(spec.head.params, "", env, tensors)
         self.stream_ops = [STREAM_OPS.get(op.kind)(op.params, "", env, tensors) for op in spec.stream_ops]
@@ -155,6 +156,20 @@ class DecoderModel:
         yield from self.stream_ops
         yield self.final_norm
         yield self.head
+
+    def single_token_splits(self, n: int, longest: int) -> tuple:
+        """Into how many parts this model's mixers cut the contexts of ``n`` single tokens in a step whose longest context
+        is ``longest``: an answer per way of cutting."""
+        return tuple(mixer.splits(n, longest) for mixer in self._cutters)
+
+    def _find_cutters(self):
+        found, todo = {}, [b.part for layer in self.layers for b in layer.branches if b.role == "mixer"]
+        while todo:
+            mixer = todo.pop()
+            if getattr(mixer, "split_rule", None) is not None:
+                found.setdefault(mixer.split_rule, mixer)
+            todo += getattr(mixer, "nested", tuple)()
+        return list(found.values())
 
     @property
     def graph_safe(self) -> bool:

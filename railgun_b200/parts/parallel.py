@@ -90,6 +90,9 @@ class Parallel(Mixer):
 
     _streams = None             # the further branches' streams, made for the first capture
 
+    def nested(self):
+        return self.parts
+
     def _views(self, cache):
         """The branches' cache views out of this mixer's: a branch that asked for a tuple of needs sees a view with
         one part per need, as it would alone."""

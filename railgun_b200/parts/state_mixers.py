@@ -215,6 +215,9 @@ class InputConv(Mixer):
         self.taps = tensors.get(prefix + p["name"], torch.float32).t().contiguous()                # [taps, channels]
         self.graph_safe = getattr(self.inner, "graph_safe", True)
 
+    def nested(self):
+        return (self.inner,)
+
     def forward(self, x, batch, cache, writes=True):
         state = cache.parts[0].state if self.K > 1 else None
         h = ops.causal_conv(x, 0, self.taps, state, batch, self.env.dtype, residual=True, update=writes)

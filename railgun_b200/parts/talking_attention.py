@@ -90,6 +90,15 @@ class TalkingAttention(Mixer):
         self.freq = tensors.shared_part(("rotary_frequencies", self.rot_dims, base),
                                         lambda: rotary_frequencies(self.rot_dims, base).to(env.device))
 
+    def splits(self, n, longest):
+        return ops.latent_decode_splits(n, -(-self.H // 64), min(longest, self.window) if self.window else longest)
+
+    @property
+    def split_rule(self):
+        R, D = self.G * self.dv, self.G * (self.d + self.dv)
+        own = self.dv % 2 == 0 and ops.latent_attention_mma_ok(self.env.dtype, self.H, R, D)
+        return ("talking", self.H, self.window) if own else None
+
     def mix(self, x, batch, cache, writes=True, out=None, out_scale: float = 1.0, proj=None):
         """The heads' outputs [T, heads * v_dim] times ``out_scale``, before the output product (into ``out``, a
         view whose rows may be further apart, if given).  ``proj``: x times ``w_in``, if the caller has it
@@ -115,12 +124,10 @@ class TalkingAttention(Mixer):
                 out = torch.empty((T, H * dv), dtype=qkv.dtype, device=qkv.device)
             args = (batch.req_of_token, batch.positions, R, self.window, 1.0)
             more = dict(select=(dv, H // G), out_scale=out_scale, score_from=R)     # R = G dv zeros lead the queries
-            reach = min(batch.max_context_len, self.window) if self.window else batch.max_context_len
-            chunks = -(-H // 64)
             if batch.decode_only:
                 n = batch.num_tokens
                 ops.latent_attention_mma(qa, out, cache.kv, table, None, None, n, *args,
-                                         ops.latent_decode_splits(n, chunks, reach), **more)
+                                         self.splits(n, batch.max_context_len), **more)
                 return out
             if flash:
                 ops.talking_prefill_flash(qc, cache.kv, table, batch, G, d, dv, out, out_scale)
@@ -130,7 +137,7 @@ class TalkingAttention(Mixer):
             if batch.num_decode_rows:
                 n = batch.num_decode_rows
                 ops.latent_attention_mma(qa, out, cache.kv, table, None, batch.decode_rows, n, *args,
-                                         ops.latent_decode_splits(n, chunks, reach), **more)
+                                         self.splits(n, batch.max_context_len), **more)
             return out
         q = torch.empty((T, H, d), dtype=qkv.dtype, device=qkv.device)
         ops.talking_prepare(qkv, q, cache.kv, self.q_norm, self.k_norm, self.eps, self.freq, self.rot_dims,

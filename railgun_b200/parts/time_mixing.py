@@ -66,6 +66,9 @@ class TokenShift(Mixer):
     def _inner_view(self, cache):
         return CacheView(cache.cache_id, parts=cache.parts[1:]) if self.inner_composite else cache.parts[1]
 
+    def nested(self):
+        return (self.inner,)
+
     def forward(self, x, batch, cache, writes=True):
         # rows that come from a norm: the shift is a convolution of two taps
         taps = torch.stack([self.share, 1.0 - self.share])

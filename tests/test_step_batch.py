@@ -213,3 +213,19 @@ def test_rows_of_a_step_launched_ahead():
     assert Engine._rows_of_launched(launched, np.array([4, 2, 7], dtype=np.int64)).tolist() == [0, 2, 3]
     assert Engine._rows_of_launched(launched, np.array([7, 4], dtype=np.int64)).tolist() == [3, 0]
     assert Engine._rows_of_launched(launched, np.array([4, 9, 2, 5], dtype=np.int64)) is None
+
+
+def test_the_key_of_a_captured_step_holds_the_parts_of_single_tokens_contexts():
+    alloc = PageAllocator([16], [64], [0], 4)
+    asked = []
+
+    def key(entries):
+        b = build_step_batch(entries, alloc, [16], VOCAB, MAX_POS, "cpu", splits=lambda n, longest: asked.append((n, longest)) or (7, longest > 40))
+        alloc.commit_many(b.host_request_ids, b.host_context_lens)
+        return b.layout, b.graph_key
+    mixed = lambda: key([StepEntry(1, [3], [0]), StepEntry(2, [4, 5], [])])  # noqa: E731
+    assert key([StepEntry(1, [5] * 36, [])])[1] == ((((36,), 0, (4,)),) + ((False, False),)) and not asked
+    keys = [mixed() for _ in range(6)]
+    assert asked == [(1, 37 + i) for i in range(6)]
+    assert len({k[0] for k in keys}) == 1                                   # one layout
+    assert [k[1][2:] for k in keys] == [(7, False)] * 4 + [(7, True)] * 2   # two graphs
