@@ -344,7 +344,8 @@ class ModelRunner:
     def step(self, entries) -> torch.Tensor | None:
         """Run one batch; float32 logits [wanted, vocab] in the order of the
         entries and of each entry's ``want``, or None if nothing is wanted.
-        The result may be a view of a buffer the next step overwrites."""
+        The result may be a view of a buffer the next step overwrites (of steps
+        of single tokens, and of ``shape_graph_min_tokens`` tokens and more)."""
         entries = [e if isinstance(e, StepEntry) else StepEntry(*e) for e in entries]
         if NVTX:
             torch.cuda.nvtx.range_push(f"step {len(entries)} requests {sum(len(e.tokens) for e in entries)} tokens")
@@ -395,7 +396,8 @@ class ModelRunner:
             ops.launch_counter().value += shape.launches
             ops.mark_tc_unchecked()
             self._commit(entries, batch)
-            return shape.logits
+            # a short step's logits are the caller's, as they are where its kernels are launched one by one
+            return shape.logits.clone() if steps is self._short_steps and shape.logits is not None else shape.logits
         if not steps.to_capture(key):
             logits = self.model.forward(batch, self.views)
             self._commit(entries, batch)
