@@ -1,6 +1,7 @@
 // C entry points of the host runtime (cache manager and scheduler), called
 // from Python through ctypes.  Handles are opaque pointers; every function
 // returns a status or a count, never throws across the boundary.
+#include <algorithm>
 #include <cstring>
 #include <unordered_map>
 #include <vector>
@@ -123,9 +124,10 @@ int rg_cache_pack_decode(void* h, const long long* ids, int R, int B, int MB, in
             for (int g = 0; g < G; ++g) {
                 const std::vector<int>& t = r->tables[g];
                 const int ps = c->group(g).page_size;
-                if ((int)t.size() > MB) return CACHE_BAD_ARGUMENT;
+                const size_t need = std::min(t.size(), (size_t)(pos / ps + 1));       // a step further on may have reserved more
+                if (need > (size_t)MB) return CACHE_BAD_ARGUMENT;
                 int* row = tables + ((size_t)g * B + b) * MB;
-                for (size_t i = 0; i < t.size(); ++i) row[i] = t[i] < 0 ? 0 : t[i];
+                for (size_t i = 0; i < need; ++i) row[i] = t[i] < 0 ? 0 : t[i];
                 slot_map[g * B + b] = t[pos / ps] * ps + pos % ps;
             }
         }

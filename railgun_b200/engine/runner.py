@@ -443,12 +443,13 @@ class ModelRunner:
 
     # ---- decode steps from captured graphs -----------------------------------------------------------
     def _static_for(self, n_requests: int, max_context: int) -> StaticDecodeBatch:
+        """The static batch for so many requests whose longest context is this: of the narrowest tables that hold it."""
         B = _bucket(n_requests, _BATCH_BUCKETS)
         # block tables are as wide as the group with the smallest pages needs
         page = min(self.page_sizes) if self.page_sizes else 16
-        ctx_bucket = SHORT_CONTEXT if max_context <= SHORT_CONTEXT else 1024
-        while ctx_bucket < max_context:
-            ctx_bucket *= 2
+        ctx_bucket = SHORT_CONTEXT
+        while -(-ctx_bucket // page) * page < max_context:
+            ctx_bucket = max(1024, 2 * ctx_bucket)
         key = (B, -(-ctx_bucket // page))
         if key not in self._static:
             self._static[key] = StaticDecodeBatch(self, *key)
@@ -525,6 +526,8 @@ class ModelRunner:
         if tokens.min() < 0 or tokens.max() >= self.model.vocab_size:
             raise BatchError(f"token ids must be in [0, {self.model.vocab_size})")
         longest = lambda: 1 + max((self.alloc.num_computed(i) for i in ids.tolist() if self.alloc.has(i)), default=0)  # noqa: E731
+        # mostly the last step's requests, a token further on.  Where they are others the tables may turn out too narrow, or
+        # wider than this step's own: what a step computes does not depend on the one before it, so it is packed anew
         ctx = self._ctx_hint + 1 if self._ctx_hint else longest()
         while True:
             static = self._static_for(R, ctx)
@@ -532,17 +535,18 @@ class ModelRunner:
             try:
                 sampled = self.alloc.pack_decode(ids, static.B, static.MB, static.host_np[static.B:],
                                                  sampling=static.host_np[static.sampling_off:])
-                break
             except CacheError as e:
                 if "bad argument" in str(e) and ctx < self.model.spec.max_position:
-                    ctx = min(max(2 * ctx, longest()), self.model.spec.max_position)   # other requests than the last step's
+                    ctx = min(max(2 * ctx, longest()), self.model.spec.max_position)
                     continue
                 raise
-        B = static.B
-        self._ctx_hint = int(static.host_np[2 * B:2 * B + R].max())
-        if self._ctx_hint > self.model.spec.max_position:
-            raise BatchError(f"position {self._ctx_hint - 1} is beyond the model's max_position_embeddings "
-                             f"{self.model.spec.max_position}")
+            B = static.B
+            ctx = self._ctx_hint = int(static.host_np[2 * B:2 * B + R].max())
+            if ctx > self.model.spec.max_position:
+                raise BatchError(f"position {ctx - 1} is beyond the model's max_position_embeddings "
+                                 f"{self.model.spec.max_position}")
+            if self._static_for(R, ctx) is static:
+                break
         static.host_np[:R] = tokens
         static.host_np[R:B] = 0
         static.packed()

@@ -4,7 +4,7 @@ that must leave the cache's bookkeeping as it was."""
 import numpy as np
 import pytest
 
-from railgun_b200.cache.manager import OutOfPages, PageAllocator
+from railgun_b200.cache.manager import CacheError, OutOfPages, PageAllocator
 from railgun_b200.engine.batch import BatchError, StepEntry, build_step_batch
 
 VOCAB, MAX_POS = 1000, 4096
@@ -229,3 +229,18 @@ def test_the_key_of_a_captured_step_holds_the_parts_of_single_tokens_contexts():
     assert asked == [(1, 37 + i) for i in range(6)]
     assert len({k[0] for k in keys}) == 1                                   # one layout
     assert [k[1][2:] for k in keys] == [(7, False)] * 4 + [(7, True)] * 2   # two graphs
+
+
+def test_a_page_reserved_for_a_later_step_widens_no_table():
+    alloc = PageAllocator([16], [64], [0], 4)
+    b = build_step_batch([StepEntry(1, [5] * 127, [])], alloc, [16], VOCAB, MAX_POS, "cpu")
+    alloc.commit_many(b.host_request_ids, b.host_context_lens)
+    ids, MB = np.array([1], dtype=np.int64), 8
+    first = np.full(4 + 1 + MB, -7, dtype=np.int32)
+    alloc.pack_decode(ids, 1, MB, first)
+    again, wide = first.copy(), np.zeros(4 + 1 + 2 * MB, dtype=np.int32)
+    with pytest.raises(CacheError):
+        alloc.pack_decode(ids, 1, MB, again, ahead=1)                       # 129 tokens: nine pages
+    alloc.pack_decode(ids, 1, 2 * MB, wide, ahead=1)
+    alloc.pack_decode(ids, 1, MB, again)                                    # the step of 128 has its eight
+    assert again.tolist() == first.tolist() and wide[5:13].tolist() == first[5:].tolist() and wide[13] >= 0
