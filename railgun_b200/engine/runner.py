@@ -178,6 +178,7 @@ class StaticDecodeBatch:
         self.step_graphs = {}          # with sampling parameters or greedy -> CapturedStep
         self.follow = [None, None]     # FollowStep: the same step fed with ``sampled`` instead of host tokens
         self.in_flight = None          # an event after the last replay, which writes ``host_out``
+        self.stream = None             # the stream that its last step was launched on
         # the number of the step last packed into ``host`` and of the one whose step has read it (written by that step)
         self.seq = torch.zeros(2, dtype=torch.int32, pin_memory=True)
         self.seq_np = self.seq.numpy()
@@ -243,6 +244,7 @@ class ShapeGraph:
     def __init__(self, dev, batch, graph, logits, launches):
         self.dev, self.batch, self.graph, self.logits, self.launches = dev, batch, graph, logits, launches
         self.hold = None               # the last packed step (keeps its pinned buffer alive until the copy has run)
+        self.stream = None             # the stream that its last step was launched on
 
 
 class RepeatedLayouts:
@@ -369,6 +371,14 @@ class ModelRunner:
         self._commit(entries, batch)
         return logits
 
+    def _in_order(self, owner) -> None:
+        """The buffers of a captured step (``owner``) are its steps' one after the other: launched on another stream than the
+        last time, a step waits for what is on that one."""
+        stream = torch.cuda.current_stream(self.device)
+        if owner.stream is not None and owner.stream != stream:
+            stream.wait_stream(owner.stream)
+        owner.stream = stream
+
     def _commit(self, entries, batch) -> None:
         self.alloc.commit_many(batch.host_request_ids, batch.host_context_lens)
 
@@ -384,7 +394,13 @@ class ModelRunner:
         build = lambda into: build_step_batch(entries, self.alloc, self.page_sizes, self.model.vocab_size,
                                               self.model.spec.max_position, self.device, self.err_flag, into=into,
                                               splits=self.model.single_token_splits)
-        known = lambda key: steps.graphs[key].dev if key in steps.graphs else None
+
+        def known(key):
+            if key not in steps.graphs:
+                return None
+            self._in_order(steps.graphs[key])                      # the step is copied into its buffer next
+            return steps.graphs[key].dev
+
         batch = build(known)
         self.last_h2d_bytes = batch.h2d_bytes
         key = batch.graph_key
@@ -419,7 +435,9 @@ class ModelRunner:
             logits = self.model.forward(batch, self.views)
         launches = counter.value - n0
         counter.value = n0
-        steps.keep(key, ShapeGraph(dev, batch, graph, logits, launches))
+        shape = ShapeGraph(dev, batch, graph, logits, launches)
+        self._in_order(shape)
+        steps.keep(key, shape)
         self._commit(entries, batch)
         return eager
 
@@ -551,6 +569,7 @@ class ModelRunner:
         static.host_np[R:B] = 0
         static.packed()
         self.last_h2d_bytes = static.host.numel() * 4
+        self._in_order(static)
         key = sampled
         logits = None
         if key not in static.step_graphs:
@@ -614,6 +633,7 @@ class ModelRunner:
             return None
         if int(f.host_in_np[2 * B:2 * B + R].max()) > self.model.spec.max_position:
             return None
+        self._in_order(static)
         if key not in f.captured:
             f.captured[key], _ = self._capture(static, follow=f, sampling=key)       # runs this step and captures it
         else:

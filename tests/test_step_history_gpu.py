@@ -72,3 +72,54 @@ def test_single_tokens_after_longer_and_shorter_ones(dtype):
     for other in results[1:]:
         for at in set(other) & set(results[0]):
             assert torch.equal(other[at], results[0][at]), at
+
+
+@pytest.mark.parametrize("kind", ["portions", "single tokens"])
+def test_steps_on_several_streams(kind):
+    """Steps that share a captured step, on two streams in turn, the first of which is busy when its step is launched."""
+    from railgun_b200.engine.batch import StepEntry
+    runner, toks = runner_of("C", "bfloat16", True, max_requests=32)
+    plain, _ = runner_of("C", "bfloat16", True, max_requests=32)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    entries = {"portions": lambda r, i: [StepEntry(10 + i, toks[i % 3][i:i + 9], [8])],
+               "single tokens": lambda r, i: [StepEntry(i % 2, [toks[i % 2][r.alloc.num_computed(i % 2)]], [0])]}[kind]
+    for r in (runner, plain):
+        for rid in (0, 1):
+            r.step([StepEntry(rid, toks[rid][:50 + 10 * rid], [])])
+        for i in range(6):                                              # captured
+            r.step(entries(r, i))
+    want = [plain.step(entries(plain, i)).clone() for i in range(6, 14)]
+    torch.cuda.synchronize()
+    got = []
+    for i in range(6, 14):
+        with torch.cuda.stream(streams[i % 2]):
+            if i % 2 == 0:
+                torch.cuda._sleep(4_000_000)                            # some two milliseconds
+            got.append(runner.step(entries(runner, i)).clone())
+    torch.cuda.synchronize()
+    for i, (a, b) in enumerate(zip(got, want)):
+        assert torch.equal(a, b), i
+
+
+@pytest.mark.parametrize("B", [1, 24])
+def test_steps_that_are_packed_while_the_one_before_runs(B):
+    """No results are read in between and the stream is busy, so that the host packs as soon as a step has read its numbers; 24
+    requests in tables of 64 pages are more numbers than one block reads."""
+    from railgun_b200.engine.batch import StepEntry
+    logits = []
+    for wait in (True, False):
+        runner, toks = runner_of("C", "bfloat16", True, max_requests=32)
+        runner.step([StepEntry(rid, toks[rid % 3][rid:rid + 150], []) for rid in range(B)])
+        ids, out = np.arange(B), []
+        for i in range(12):
+            tokens = np.array([toks[(rid + i) % 3][i + rid] for rid in range(B)], dtype=np.int32)
+            if not wait and i > 2:
+                torch.cuda._sleep(400_000)
+            out.append(runner.decode_step_flat(ids, tokens).clone())
+            out.append(runner.last_greedy.clone())
+            if wait:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        logits.append(out)
+    for i, (a, b) in enumerate(zip(*logits)):
+        assert torch.equal(a, b), i
