@@ -2716,6 +2716,11 @@ def _small_rows(h, gated: bool, weight):
     return out
 
 
+def _refuse_tf32(what: str) -> None:
+    if torch.backends.cuda.matmul.allow_tf32:
+        raise KernelError(f"{what}: TF32 is enabled; the 32-bit path must be true 32-bit")
+
+
 def gated_linear_ok(x, weight: torch.Tensor) -> bool:
     """Is the product by ``weight`` = gate | up one with SiLU-mul in its kernel?"""
     if isinstance(x, FreshNorm):
@@ -2728,6 +2733,7 @@ def gated_linear(x, weight: torch.Tensor) -> torch.Tensor:
     """silu(gate) * up in 32-bit, gate | up = x W^T, ``weight`` [2 I, K] = gate | up."""
     if not gated_linear_ok(x, weight):
         raise KernelError(f"gated_linear refuses {tuple(x.shape)} {x.dtype}, W {tuple(weight.shape)} {weight.dtype}")
+    _refuse_tf32("gated_linear")
     return _small_rows(x, True, weight)
 
 
@@ -2746,6 +2752,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, bias: torch.Te
     32-bit inputs run in true 32-bit: the reduced-precision matrix mode is
     refused."""
     if isinstance(x, FreshNorm):
+        if bias is not None or out_dtype not in (None, torch.float32):
+            raise KernelError("linear: a norm that its product computes has neither a bias behind it nor another type")
+        _refuse_tf32("linear")
         return _small_rows(x, False, weight)
     if isinstance(x, NormedRows):
         if (out_dtype is None or out_dtype == torch.bfloat16) and skinny_scaled_ok(x, weight):
@@ -2755,8 +2764,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, bias: torch.Te
         x = x.materialize()
     if not x.is_cuda:
         raise KernelError("linear: CUDA tensors only (there is no CPU path)")
-    if x.dtype == torch.float32 and torch.backends.cuda.matmul.allow_tf32:
-        raise KernelError("linear: TF32 is enabled; the 32-bit path must be true 32-bit")
+    if x.dtype == torch.float32:
+        _refuse_tf32("linear")
     if bias is not None:
         # (up to 16 rows by 2,576 x 2,048: the library's 6.5 us, this package's 2.5)
         if out_dtype is not None and out_dtype != x.dtype:

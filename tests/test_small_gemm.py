@@ -31,3 +31,23 @@ def test_a_matrix_off_a_16_byte_boundary_is_not_for_16_byte_loads():
     x, flat = torch.zeros(4, 64).bfloat16(), torch.zeros(24 * 64 + 8).bfloat16()
     assert flat.data_ptr() % 16 == 0
     assert [ops.skinny_gemm_ok(x, flat[i:i + 24 * 64].view(24, 64)) for i in (0, 1, 4, 8)] == [True, False, False, True]
+
+
+@pytest.mark.parametrize("what", ["plain", "norm", "gated"])
+def test_32_bit_products_are_refused_while_tf32_is_on(what, monkeypatch):
+    class Operand(torch.Tensor):
+        is_cuda = True
+    x, w = torch.zeros(4, 64).as_subclass(Operand), torch.zeros(8, 64)
+    monkeypatch.setattr(ops, "gated_linear_ok", lambda x, w: True)
+    monkeypatch.setattr(ops, "_small_rows", lambda *a: "launched")
+    call = {"plain": lambda: ops.linear(x, w), "norm": lambda: ops.linear(ops.FreshNorm(torch.zeros(4, 64), None, torch.ones(64), 0.0), w),
+            "gated": lambda: ops.gated_linear(x, w)}[what]
+    monkeypatch.setattr(torch.backends.cuda.matmul, "allow_tf32", True)
+    with pytest.raises(ops.KernelError, match="TF32"):
+        call()
+
+
+def test_a_norm_that_its_product_computes_takes_no_bias():
+    fresh = ops.FreshNorm(torch.zeros(4, 64), None, torch.ones(64), 0.0)
+    with pytest.raises(ops.KernelError, match="bias"):
+        ops.linear(fresh, torch.zeros(8, 64), bias=torch.zeros(8))
