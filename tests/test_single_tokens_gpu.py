@@ -261,6 +261,67 @@ def test_single_tokens_beside_portions(nh, nkv, d, splits, portions):
     ops.tc_gemm_check()
 
 
+@pytest.mark.parametrize("nh,nkv,d", [(32, 8, 64), (24, 8, 128), (4, 2, 48)])
+@pytest.mark.parametrize("splits", [1, 3])
+@pytest.mark.parametrize("portions", [1, 9])
+def test_single_tokens_beside_portions_between_a_steps_kernels(nh, nkv, d, splits, portions):
+    """In the same buffers again and again, launched one by one and as a graph: a kernel that writes the queries and the step's own
+    keys and values directly in front, and one that reads every row of the output directly behind."""
+    from railgun_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(nh * d + portions + splits)
+    page, tokens, singles, ctx, turns = 16, 130, 11, 700, 6
+    R, width = portions + singles, -(-ctx // page)
+    T = portions * tokens + singles
+    first = torch.randn(R * width, 2, nkv, page, d, device=DEV, generator=g).bfloat16()
+    table = torch.randperm(R * width, device=DEV, generator=g).to(torch.int32).view(R, width)
+    news = [torch.randn(T, (nh + 2 * nkv) * d, device=DEV, generator=g).bfloat16() for _ in range(turns)]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    pos = i32([j for _ in range(portions) for j in range(ctx - tokens, ctx)] + [ctx - 1 - 60 * j for j in range(singles)])
+    req = i32([r for r in range(portions) for _ in range(tokens)] + list(range(portions, R)))
+    slots = (table[req.long(), (pos // page).long()] * page + pos % page).to(torch.int32)
+    rows = i32(list(range(portions * tokens, T)))
+    tiles = lambda size: i32([[r * tokens + a, min(size, tokens - a), r] for r in range(portions) for a in range(0, tokens, size)])
+    t128, t64 = tiles(128), tiles(64)
+    angles = torch.randn(ctx, d, device=DEV, generator=g)
+    weight = torch.rand(nh * d, device=DEV, generator=g) + 0.5
+    kv, qkv, resid = first.clone(), news[0].clone(), torch.zeros(T, nh * d, device=DEV)
+
+    def step(new, beside):
+        out = torch.full((T, nh * d), float("nan"), dtype=torch.bfloat16, device=DEV)
+        resid.zero_()
+        qkv.copy_(new)
+        ops.rope_cache_write(qkv, angles, pos, slots, kv, nh, nkv, d, page, None)
+        if d == 64:
+            ops.prefill_attention_tc(qkv, out, kv, table, t128, pos, nh, nkv, d, 0, d ** -0.5)
+        elif d == 128:
+            ops.prefill_attention_wide(qkv, out, kv, table, t128, pos, nh, nkv, d, 0, d ** -0.5)
+        else:
+            ops.prefill_attention(qkv, qkv.shape[1], out, kv, table, t64, pos, nh, nkv, d, 0, d ** -0.5)
+        ops.decode_attention(qkv, qkv.shape[1], out, kv, table, rows, singles, req, pos, nh, nkv, d, 0, d ** -0.5, splits, beside=beside)
+        return ops.add_rmsnorm(resid, out, weight, 1e-5, torch.float32)
+
+    def all_of(run):
+        kv.copy_(first)
+        return [run(new).clone() for new in news * 2]
+
+    want = all_of(lambda new: step(new, False))
+    assert all(bool(t.isfinite().all()) for t in want)
+    for got, one in zip(all_of(lambda new: step(new, True)), want):
+        assert torch.equal(got, one)
+    source, graph = news[0].clone(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        result = step(source, True)
+
+    def replay(new):
+        source.copy_(new)
+        graph.replay()
+        return result
+    for got, one in zip(all_of(replay), want):
+        assert torch.equal(got, one)
+    ops.tc_gemm_check()
+
+
 @pytest.mark.parametrize("nh,nkv,d", [(1, 1, 16), (32, 8, 64), (32, 8, 128), (64, 16, 128), (8, 8, 256)])
 @pytest.mark.parametrize("paired", [False, True])
 def test_rotation_and_cache_write(nh, nkv, d, paired):
