@@ -12,7 +12,6 @@
 // a new sampler from the wall clock every step (crates/vllm-engine/src/sampling.rs:19-30).
 #include "common.cuh"
 #include <cooperative_groups.h>
-#include <utility>
 namespace cg = cooperative_groups;
 
 #define SAMPLE_THREADS 1024
@@ -534,7 +533,8 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, 2) argmax_cluster_kernel(const
     __shared__ int part_i[ARGMAX_CLUSTER];
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank(), r = blockIdx.x / ARGMAX_CLUSTER;
-    auto started = cl.barrier_arrive();                                 // this block runs: the others may write its memory
+    // this block runs: the others may write its memory (nothing has been written yet that they would have to see)
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     pdl_wait();
     pdl_trigger();
     const float* row = logits + (size_t)r * V;
@@ -568,7 +568,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, 2) argmax_cluster_kernel(const
         }
     }
     block_argmax(best, bi, sv, si);
-    cl.barrier_wait(std::move(started));                                // the first block runs (its loads covered the wait)
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");         // the first block runs; the loads covered the wait
     if (threadIdx.x == 0) {
         *cl.map_shared_rank(&part_v[rank], 0) = best;
         *cl.map_shared_rank(&part_i[rank], 0) = bi;

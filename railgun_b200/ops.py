@@ -2196,11 +2196,17 @@ def tc_pair_tile(M: int, N: int, device) -> str:
     A narrower tile has to save a twelfth of that: it moves more of x per result, and where nearly every pair is busy the
     power limit, not the rounds, is the bound.  Back to back with SiLU-mul, 256 / 224 / 192 columns: 1,056 rows by 3,072 x
     16,384 150 / 135 / 140 us, 1,701 by 2,048 x 16,384 195 / 165 / 172, 2,048 by 4,096 x 28,672 417 / 448 / 473."""
-    pairs = num_sms(device) // 2
+    return f"256x{_pair_tile(M, N, num_sms(device) // 2)[0]}"
+
+
+def _pair_tile(M: int, N: int, pairs: int) -> tuple:
+    """The tile's width and the rounds it takes."""
     m_tiles = -(-M // 256)
-    cost = {n: -(-(m_tiles * -(-N // n)) // pairs) * (n + 8) for n in (256, 224, 192)}
+    rounds = {n: -(-(m_tiles * -(-N // n)) // pairs) for n in (256, 224, 192)}
+    cost = {n: r * (n + 8) for n, r in rounds.items()}
     best = min(cost, key=lambda n: (cost[n], -n))
-    return f"256x{best if 12 * cost[best] <= 11 * cost[256] else 256}"
+    best = best if 12 * cost[best] <= 11 * cost[256] else 256
+    return best, rounds[best]
 
 
 def tc_gemm(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, silu_mul: bool = False, wide: bool = True,
@@ -2242,9 +2248,19 @@ def tc_gemm(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, silu_mul: boo
 
 
 def tc_gemm_gated_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
-    """Can ``tc_gemm_gated`` take these operands, and is it worth it?  From as many rows on as the SiLU-mul form."""
+    """Can ``tc_gemm_gated`` take these operands?  From as many rows on as the SiLU-mul form (and see ``tc_gemm_gated_pays``)."""
     return (isinstance(x, torch.Tensor) and x.dim() == 2 and x.shape[0] >= TC_GEMM_MIN_ROWS and weight.shape[0] % 16 == 0
             and _by_address(x, weight) and tc_gemm_ok(x, weight))
+
+
+def tc_gemm_gated_pays(M: int, N: int, pairs: int) -> bool:
+    """Is the product with the activation in its epilogue faster than the library's with the activation's kernel behind it?
+    Where its tiles are worked off in three rounds or more and are mostly filled: five sixths of what the rounds' tiles
+    hold.  Its time over the other's (49 shapes, gelu, 1,024 to 4,096 rows): at least three rounds, filled 0.84 and more 0.74 to
+    0.99; filled 0.82 and less (1,057 rows, whose last row of tiles is nearly empty) 1.01 to 1.11; two rounds 0.94 to 1.34 (2,048 rows by
+    2,048 x 4,096 33.2 and 32.0 us, 1,500 rows 37.0 and 27.7); one round 1.15 to 1.43."""
+    width, rounds = _pair_tile(M, N, pairs)
+    return rounds >= 3 and 6 * M * N >= 5 * rounds * pairs * 256 * width
 
 
 def tc_gemm_gated(x: torch.Tensor, weight: torch.Tensor, act: str, limit: float = 0.0) -> torch.Tensor:
@@ -2739,9 +2755,15 @@ def gated_linear(x, weight: torch.Tensor) -> torch.Tensor:
 
 # Logits of decode batches by the streaming product: where the library's gets slower with more rows and this one does not.  128,256
 # rows of W, the library's and this one: 40 rows by 2,048 83.2 / 86.2 us, 48 95.8 / 87.4, 64 99.0 / 89.2, by 4,096 48 185 / 179, 64 188 / 181;
-# 32,768 rows of W are level (two tiles of W an SM, which start at once).
+# Level or slower with fewer tiles of W to an SM, the last of which are a larger part of all: 41 to 64 rows by 100,352 x 3,072 0.98
+# to 0.99, by 65,536 x 4,096 1.01 to 1.02, by 50,000 x 2,048 0.98 to 1.01; so from more than five an SM on.  Where a row of logits ends off a
+# 16-byte boundary the library takes five times as long (48 rows by 37,889 x 2,048 195 / 36 us): from more than two an SM on.
 STREAM_HEAD_ROWS = 41, 64
-STREAM_HEAD_WIDTH = 2 * 148 * 128
+STREAM_HEAD_TILES, STREAM_HEAD_ODD_TILES = 5, 2
+
+
+def _stream_head_pays(N: int, sms: int) -> bool:
+    return N > (STREAM_HEAD_ODD_TILES if N % 4 else STREAM_HEAD_TILES) * sms * 128
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, bias: torch.Tensor | None = None) -> torch.Tensor:
@@ -2779,8 +2801,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, bias: torch.Te
         return skinny_gemm(x, weight, out_dtype)             # small decode batches: stream the weights once
     if (out_dtype is None or out_dtype == torch.float32) and small_gemm_f32_ok(x, weight):
         return _small_rows(x, False, weight)
-    if out_dtype == torch.float32 and STREAM_HEAD_ROWS[0] <= x.shape[0] <= STREAM_HEAD_ROWS[1] and weight.shape[0] > STREAM_HEAD_WIDTH \
-            and _by_address(x, weight) and tc_stream_ok(x, weight):
+    if out_dtype == torch.float32 and STREAM_HEAD_ROWS[0] <= x.shape[0] <= STREAM_HEAD_ROWS[1] and _by_address(x, weight) \
+            and _stream_head_pays(weight.shape[0], num_sms(x.device)) and tc_stream_ok(x, weight):
         return tc_stream_gemm(x, weight, out_dtype)          # logits of a decode batch over a large vocabulary
     if out_dtype is not None and out_dtype != x.dtype:
         return torch.mm(x, weight.t(), out_dtype=out_dtype)

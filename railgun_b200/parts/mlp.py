@@ -50,7 +50,9 @@ class SwiGLU(FeedForward):
         if self.act != "silu":
             if isinstance(x, ops.NormedRows):
                 x = x.materialize()
-            act = (ops.tc_gemm_gated(x, self.w_gate_up, self.act) if ops.tc_gemm_gated_ok(x, self.w_gate_up)
+            own = ops.tc_gemm_gated_ok(x, self.w_gate_up) and ops.tc_gemm_gated_pays(
+                x.shape[0], self.w_gate_up.shape[0], ops.num_sms(x.device) // 2)
+            act = (ops.tc_gemm_gated(x, self.w_gate_up, self.act) if own
                    else ops.gated_activation(ops.linear(x, self.w_gate_up), self.act))
             return ops.PendingLinear(act, self.w_down, stream) if defer else ops.linear(act, self.w_down)
         if isinstance(x, ops.NormedRows):

@@ -6,7 +6,7 @@ import pytest
 
 KERNELS = Path(__file__).resolve().parents[1] / "railgun_b200" / "csrc" / "kernels"
 REACHES = re.compile(r"map_shared_rank\(|mapa_shared\(")
-MEETS = re.compile(r"\.sync\(\);|barrier_wait\(|cluster_sync_all\(\);")
+MEETS = re.compile(r"\.sync\(\);|barrier\.cluster\.wait|cluster_sync_all\(\);")
 
 
 def bodies(text):

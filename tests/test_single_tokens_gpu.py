@@ -37,7 +37,7 @@ def test_products_that_stay_the_librarys(M):
     taken, and derivatives and maps go through the product."""
     from railgun_b200 import ops
     g = torch.Generator(device=DEV).manual_seed(M)
-    N, K = (64, 128) if M <= 16 else (ops.STREAM_HEAD_WIDTH + 64, 64)
+    N, K = (64, 128) if M <= 16 else (5 * 148 * 128 + 64, 64)
     flat = torch.randn(N * K + 1, device=DEV, generator=g).bfloat16()
     w, odd = flat[:N * K].view(N, K), flat[1:].view(N, K)
     x, b = torch.randn(M, K, device=DEV, generator=g).bfloat16(), torch.randn(N, device=DEV, generator=g).bfloat16()

@@ -19,7 +19,8 @@ def test_a_product_that_cannot_go_by_address_asks_for_no_address(M, dtype, monke
 
         def data_ptr(self):
             raise AssertionError("an address")
-    N = 24 if M == 4 else ops.STREAM_HEAD_WIDTH + 8
+    N = 24
+    monkeypatch.setattr(ops, "_stream_head_pays", lambda N, sms: True)
     x, w, b = (torch.zeros(*s, dtype=torch.bfloat16).as_subclass(Operand) for s in ((M, 64), (N, 64), (N,)))
     monkeypatch.setattr(torch, "addmm", lambda *a: "library")
     monkeypatch.setattr(torch, "mm", lambda *a, **k: "library")
@@ -51,3 +52,17 @@ def test_a_norm_that_its_product_computes_takes_no_bias():
     fresh = ops.FreshNorm(torch.zeros(4, 64), None, torch.ones(64), 0.0)
     with pytest.raises(ops.KernelError, match="bias"):
         ops.linear(fresh, torch.zeros(8, 64), bias=torch.zeros(8))
+
+
+@pytest.mark.parametrize("M,N,pays", [
+    (1024, 16384, True), (1057, 16384, False), (1280, 16384, True), (2048, 16384, True), (1024, 28672, True), (1057, 28672, False),
+    (1024, 4096, False), (1500, 4096, False), (2048, 4096, False), (3000, 4096, True), (4096, 4096, True), (1024, 2048, False),
+    (4096, 2048, False), (1057, 8192, False), (1500, 8192, True), (2048, 8192, True)])
+def test_which_gated_products_run_with_their_activation_inside(M, N, pays):
+    """On both sides of the lines, on 74 pairs."""
+    assert ops.tc_gemm_gated_pays(M, N, 74) == pays
+
+
+@pytest.mark.parametrize("N,pays", [(128256, True), (94720, False), (94724, True), (50000, False), (37889, True), (37888, False), (32769, False)])
+def test_which_logits_are_streamed(N, pays):
+    assert ops._stream_head_pays(N, 148) == pays
