@@ -17,12 +17,12 @@
 // What bounds it: the 32-bit multiply-adds (128 a cycle and SM, packed or not), and in delta_states the chain from chunk to
 // chunk, 2 x 64 x d of them per column and chunk.  16 columns a block fill 128 of 148 SMs at 16 heads of 128 columns;
 // narrower blocks fetch the same W and K more often.  A chunk's 2,048 cycles of multiply-adds stand beside its copies, sums
-// across lanes and three barriers: sixteen warps (d known, eighths of k, quarters of the tokens) overlap those better than
-// eight, 119 us against 141 behind delta_solve at 16 heads of 128 x 128, 93 against 135 at 64 x 64.
-// Measured with eight (2,048 tokens, 16 heads of 128 x 128 on 8): 58 us the systems, 116 the states, 54 the outputs, with products
-// in one chain; all three 269 us on 16 query/key heads since they add up in fours (chunk_scan.cuh), 258 before.  The
-// token-by-token kernel (state_mixers.cu) takes 473 alone in a loop and took 908 in a model's step.  Requests that bring fewer
-// than 256 tokens stay on that one (ops.py, DELTA_CHUNK_MIN_TOKENS).
+// across lanes and three barriers: sixteen warps (eighths of k, quarters of the tokens) overlap those better than eight, 119 us
+// against 141 behind delta_solve at 16 heads of 128 x 128, where d is also a compile-time number, 93 against 135 at 64 x 64, where
+// it is not.
+// Measured (2,048 tokens, 16 heads of 128 x 128 on 8, under ncu): 70 us the systems, 122 the states, 65 the outputs, their products
+// in fours (chunk_scan.cuh).  The token-by-token kernel (state_mixers.cu) takes 473 alone in a loop and took 908 in a model's
+// step.  Requests that bring fewer than 256 tokens stay on that one (ops.py, DELTA_CHUNK_MIN_TOKENS).
 #include "chunk_scan.cuh"
 #include <type_traits>
 

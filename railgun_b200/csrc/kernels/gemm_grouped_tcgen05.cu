@@ -5,8 +5,8 @@
 // next tile's products.
 //
 // What bounds it: every byte of the experts' matrices once from HBM (32 experts of 4,096 x 2,048: 537 MB, 82 us) beside as much time
-// of the tensor cores (8,192 places: 84 us), and what crosses L2 -> SM, which this form cuts: a pair's tile of 256 x 256 fetches 512
-// bytes of operands per place and row of W where one CTA's tile of 128 x 256 fetched 768.  Gate and up rows meet in the
+// of the tensor cores (8,192 places: 84 us), and what crosses L2 -> SM, which this form cuts: a pair's tile of 256 x 256 fetches
+// 1,024 bytes of operands per number of k for 65,536 results where one CTA's tile of 128 x 256 fetched 768 for 32,768.  Gate and up rows meet in the
 // epilogue: the tensor map walks the matrix [gate rows; up rows] in blocks of 8 gate and the 8 matching up rows, so that lanes
 // l and l + 8 of a warp hold a pair, and the activation is applied to 32-bit sums and written once.  2,048 tokens with four choices
 // each among 32 experts: gathered rows by 4,096 x 2,048 with the activation 222 us as tiles of 128 x 256 a CTA with a kernel behind

@@ -1,7 +1,7 @@
 // Weight-streaming matrix product for steps of 17 to 256 rows on the 5th-generation tensor cores:
 // y[M, N] = x[M, K] W[N, K]^T with the operands swapped, so that 128 rows of W fill the M side of tcgen05.mma
-// and the step's tokens (padded to 64, 128 or 256) its N side: D[128 weight rows, tokens] accumulates in tensor memory while W
-// streams through a ring of TMA stages exactly once.  At these sizes the product is bound by reading W, and a
+// and the step's tokens (in steps of 16) its N side: D[128 weight rows, tokens] accumulates in tensor memory while W
+// streams through a ring of TMA stages once (twice where the tokens go in two parts, dispatch_ts).  At these sizes the product is bound by reading W, and a
 // product with few rows of W (q|k|v, O, down) has too few 128-row tiles to occupy the GPU, so K is split over the
 // CTAs of a thread-block cluster: every CTA accumulates its K range of the cluster's tile, leaves the partial sums
 // in its shared memory (over the stages, which are done with by then), and the cluster's CTAs add them, each for its
@@ -23,7 +23,7 @@
 #include "tcgen05.cuh"
 
 #define TS_ROWS 128               // rows of W per tile (the MMA's M)
-#define TS_MAX_TOK 256            // tokens per tile (the MMA's N): 64, 128 or 256; fewer are padded with zeros by TMA
+#define TS_MAX_TOK 256            // tokens per tile, at most: a kernel is made for 64, 128 or 256; boxes and the MMA's N are of those that are there, in steps of 16 (zeros from TMA behind them)
 #define TS_BK 64
 #define TS_MAX_SPLITS 8
 #define TS_EPI_NONE 0

@@ -524,7 +524,8 @@ sample_kernel(const float* __restrict__ logits, int V,
 // Wide rows: a cluster of eight blocks per row, each on a contiguous part of it with every load under way at once; the
 // blocks' best meet in the first block's shared memory.  What bounds it: latency (few rows), then the rows' bytes from L2.
 // As two kernels with the parts' best in global memory between them (256 threads a block, one number a load) rows of 128,256
-// took 4.4 us for one and 13.0 for 64, rows of 32,768 4.1 and 6.1, of 4,096 4.0; this one 2.9 and 7.7, 2.5 and 6.1, 2.4.
+// took 4.4 us for one and 13.0 for 64, rows of 32,768 4.1 and 6.1, of 4,096 4.0; this one 3.0 and 7.7, 2.5 and 6.1, 2.3 (the
+// blocks' first meeting, which covers the first one's start, is some 0.1 of them).
 #define ARGMAX_CLUSTER 8
 __global__ void __launch_bounds__(SAMPLE_THREADS, 2) argmax_cluster_kernel(const float* __restrict__ logits, int V, int* __restrict__ out) {
     __shared__ float sv[32];

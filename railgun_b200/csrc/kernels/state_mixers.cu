@@ -66,7 +66,8 @@ __global__ void causal_conv_kernel(const A* __restrict__ x, int ld, int x_off, c
 }
 
 // The same for bfloat16 inputs with eight channels per thread (16-byte loads), where rows and offsets allow it.  What the
-// step's description and the taps say is asked for before the wait for the kernel before this one.
+// step's description says is asked for before the wait for the kernel before this one; the taps behind it, since a token
+// shift's are made by a kernel of the same step.
 template <typename O>
 __global__ void causal_conv8_kernel(const bf16* __restrict__ x, int ld, int x_off, const float* __restrict__ taps,
                                     const float* __restrict__ bias, float* state,

@@ -69,7 +69,8 @@ extern "C" int rg_step_in(void* host, int* dev, int first, int n, void* seq, uns
     if (e) return e;
     e = device_address(seq, &s);
     if (e) return e;
-    // four 16-byte requests a thread at most before there are 64 blocks: 64 KB of the bus's 50 GB/s are 1.3 us
+    // one 16-byte request a thread, all under way at once, up to 64 blocks (256 KB; 64 KB of the bus's 50 GB/s are 1.3 us); a
+    // larger step is a few requests a thread one after another
     const int blocks = min(64, (n + 4 * STEP_IN_THREADS - 1) / (4 * STEP_IN_THREADS));
     return rg_launch(step_in_kernel, dim3(blocks), dim3(STEP_IN_THREADS), 0, (cudaStream_t)stream, 1, (const int*)h, dev, first, n,
                      (volatile int*)s, done);

@@ -303,7 +303,8 @@ class ModelRunner:
     live at a time; ``page_size``: tokens per page (the reference's
     ``--block-size``, default 16, crates/vllm-scheduler/src/scheduler.rs:53).
     ``use_graphs``: steps in which every request brings exactly one token and
-    wants its logits are replayed from a captured CUDA graph."""
+    wants its logits are replayed from a captured CUDA graph, other steps once
+    their layout repeats (``RepeatedLayouts``)."""
 
     def __init__(self, model_dir, dtype="bfloat16", device="cuda:0", page_size: int = 16,
                  max_tokens: int = 16384, max_requests: int = 64, spec_override=None, use_graphs: bool = True):

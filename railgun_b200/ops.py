@@ -650,8 +650,8 @@ def moe_grouped_gemm(a: torch.Tensor, src, src_div: int, w: torch.Tensor, tiles:
     ``plain_act`` names an activation on the product, see ``ACTIVATIONS``).  Row ``pos`` of the input is ``a[src[pos] // src_div]``
     or, without ``src``, ``a[pos]``.  Returns [places, N]; rows that belong to no
     tile are not written.  bfloat16 with rows on 16-byte boundaries runs on the
-    tensor cores (tiles of 32 places: mma.sync, weight-streaming; tiles of 128 or 256:
-    the grouped tcgen05 product, whose bounded waits ``tc_gemm_check`` reports
+    tensor cores (tiles of 32 places: mma.sync, weight-streaming; tiles of 256, or of 128
+    where a caller made such: the grouped tcgen05 product, whose bounded waits ``tc_gemm_check`` reports
     on), everything else in 32-bit arithmetic on the CUDA cores (tiles of 32)."""
     _check(a, "a")
     _check(w, "w", a.dtype)
@@ -719,7 +719,7 @@ def moe_grouped_gemm_tc_ok(dtype, K: int, lda: int) -> bool:
 
 def moe_tile_rows(dtype, pairs: int, num_experts: int, K1: int, K2: int) -> int:
     """Places per tile of the grouped products: 256 (the tcgen05 product) once an expert gets 64 places on
-    average (prompts: every weight row that is read serves 128 rows), else 32."""
+    average (prompts: every weight row that is read serves up to 256 places), else 32."""
     tc = moe_grouped_gemm_tc_ok(dtype, K1, K1) and moe_grouped_gemm_tc_ok(dtype, K2, K2)
     return MOE_TC_TILE_ROWS if tc and pairs >= 64 * max(1, num_experts) else MOE_TILE_ROWS
 
@@ -2638,10 +2638,10 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k, top_p, seed: 
 
 # 32-bit products that run in this package's kernel instead of the library's.  What it saves is host time (7 against 15 us),
 # which counts for nothing where a step is replayed from a graph, so only where it is no slower on the GPU either.  Its time
-# over the library's, over 1 to 40 rows, K 64 to 512 and N 96 to 3,000: up to 16 rows the library takes products with a
-# kernel for few rows: 0.67 to 1.01 on average (1.09 at most) up to K 96 and N 8,192, from K 97 on 0.99 to 1.15, from K 192
-# 1.2 to 3.4; from 17 rows 0.61 to 0.93 up to K 448, 512 is 0.94 from 31 rows and 1.04 to 1.08 below, and more 32 x 32 tiles
-# than SMs are up to 1.33 (33 rows by 3,000).  (The kernel has since become faster, by 2 to 15 % from 17 rows and K 256 on.)
+# over the library's (595 shapes, 1 to 256 rows, K 32 to 512, N 64 to 8,192): up to 16 rows the library takes products with a
+# kernel for few rows: 0.72 to 0.86 on average up to K 96 (at most 1.09, one row by 8,192 x 64: 3.4 and 3.1 us), from K 128 on
+# 1.1 to 3.5; from 17 rows 0.56 to 0.87 up to K 448, and 512 from 31 rows 0.81.  More 32 x 32 tiles than SMs were up to 1.33 (33
+# rows by 3,000, with this kernel's earlier form).
 SMALL_F32_ROWS = 256
 SMALL_F32_LIMITS = ((96, 256), (448, 148), (512, 148))      # numbers of a row and tiles: up to 16 rows, up to 30, above
 
@@ -2767,8 +2767,9 @@ def _stream_head_pays(N: int, sms: int) -> bool:
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype=None, bias: torch.Tensor | None = None) -> torch.Tensor:
-    """y = x W^T (+ ``bias``, added inside the product), W stored [out, in].  Up to 64 bfloat16 rows go through the
-    weight-streaming kernel of this package; everything else through the
+    """y = x W^T (+ ``bias``, added inside the product), W stored [out, in].  Up to ``SKINNY_AUTO_ROWS`` bfloat16 rows, 41 to
+    64 whose 32-bit result is wide enough, and 32-bit products of a few rows by small matrices go through kernels of
+    this package; everything else through the
     library matrix product (cuBLAS), as in the reference, whose projections
     are library GEMMs (crates/vllm-models/src/llama/attention.rs:94-96,133).
     32-bit inputs run in true 32-bit: the reduced-precision matrix mode is

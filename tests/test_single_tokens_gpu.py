@@ -155,7 +155,7 @@ def test_norm_and_gate(H, dv, types, whole):
 
 @pytest.mark.parametrize("T,H", [(1, 4), (3, 4096), (592, 2048), (593, 2048), (149, 4100), (2, 16384), (160, 16384), (2, 16388), (150, 32768), (2, 32772)])
 def test_rows_kept_in_registers(T, H):
-    """One, two, four and eight pieces a thread, and rows that are too wide for that; rows picked out; nothing pending."""
+    """One, two and four pieces a thread, and rows that are too wide for that; rows picked out; nothing pending."""
     from railgun_b200 import ops
     g = torch.Generator(device=DEV).manual_seed(H)
     x, w = torch.randn(T, H, device=DEV, generator=g), torch.rand(H, device=DEV, generator=g) + 0.5
