@@ -54,6 +54,23 @@ __global__ void step_out_kernel(const int* __restrict__ dev, int* __restrict__ h
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) host[i] = dev[i];
 }
 
+// The result of a step that a graph replays, to where the step's packed buffer says (0: nowhere): a tensor of its own per step,
+// as a step launched one kernel at a time returns.  What bounds it: its launch as the graph's last node (a result of 5 x 500
+// numbers), or its bytes.  A copy behind the graph instead: a step of 22 small kernels 130 us, 120 with this.
+__global__ void step_result_kernel(const float* __restrict__ src, const unsigned long long* __restrict__ where, size_t n) {
+    float* dst = reinterpret_cast<float*>(*where);                 // the step's description: in place before the step's first kernel
+    pdl_wait();
+    pdl_trigger();
+    if (dst == nullptr) return;
+    const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+    if ((((uintptr_t)src | (uintptr_t)dst) & 15u) == 0) {
+        for (size_t i = first; i < n >> 2; i += step) reinterpret_cast<float4*>(dst)[i] = reinterpret_cast<const float4*>(src)[i];
+        for (size_t i = (n & ~(size_t)3) + first; i < n; i += step) dst[i] = src[i];
+    } else {
+        for (size_t i = first; i < n; i += step) dst[i] = src[i];
+    }
+}
+
 // What the GPU calls a page-locked host address.
 static int device_address(void* host, void** dev) {
     *dev = nullptr;
@@ -82,4 +99,13 @@ extern "C" int rg_step_out(const int* dev, void* host, int n, void* stream) {
     const int e = device_address(host, &h);
     if (e) return e;
     return rg_launch(step_out_kernel, dim3(1), dim3(min(512, (n + 31) / 32 * 32)), 0, (cudaStream_t)stream, 1, dev, (int*)h, n);
+}
+
+// where: 8-byte aligned, on the device: the address of n floats, or 0.
+extern "C" int rg_step_result(const float* src, const void* where, long long n, void* stream) {
+    if (n <= 0) return 0;
+    if ((uintptr_t)where & 7u) return RG_ERR_UNSUPPORTED;
+    const long long blocks = (n + 1023) / 1024;
+    return rg_launch(step_result_kernel, dim3((unsigned)(blocks < 592 ? blocks : 592)), dim3(256), 0, (cudaStream_t)stream, 1, src,
+                     (const unsigned long long*)where, (size_t)n);
 }

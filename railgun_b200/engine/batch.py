@@ -98,6 +98,7 @@ class StepBatch:
     prefill_tiles128: torch.Tensor | None = None     # the same requests in tiles of up to 128 positions
     num_prefill_tiles128: int = 0
     max_portion_context: int = 0     # the longest context among those requests (of several tokens)
+    result_address: torch.Tensor | None = None       # [2]: where a replayed step's result goes, 64 bits (0: nowhere)
     graph_key: tuple = ()            # the layout and what else decides which kernels the step takes: see build_step_batch
 
 
@@ -116,8 +117,9 @@ def build_step_batch(entries, alloc, page_sizes, vocab_size: int, max_position: 
     and, where there are single tokens, what ``splits(their number, longest
     context)`` says: into how many parts their contexts are cut)
     once it is known; if it returns a device int32 buffer (of exactly the
-    layout's size) the step is copied into that buffer, whose address is what a
-    captured graph reads, and the batch's tensors are views of it."""
+    layout's size) and an address, the step is copied into that buffer, which is
+    what a captured graph reads, with the address (where its result goes, or 0)
+    as its last two numbers, and the batch's tensors are views of it."""
     if not entries:
         raise BatchError("a step needs at least one entry")
     R = len(entries)
@@ -160,6 +162,9 @@ def build_step_batch(entries, alloc, page_sizes, vocab_size: int, max_position: 
         sizes += [T, R * max_blocks_t[g]]
     sizes += [3 * n_tiles, n_dec, 3 * n_tiles128]
     offs = [0, *accumulate(sizes)]
+    for n in (offs[-1] % 2, 2):                             # one 64-bit number
+        sizes.append(n)
+        offs.append(offs[-1] + n)
     buf = torch.empty(offs[-1], dtype=torch.int32, pin_memory=_pinned())
     tokens = token_arrays[0] if R == 1 else np.concatenate(token_arrays)
     if tokens.dtype != np.int64:
@@ -176,6 +181,10 @@ def build_step_batch(entries, alloc, page_sizes, vocab_size: int, max_position: 
     if n_dec and splits is not None:
         key += splits(n_dec, longest)
     static = into(key) if into is not None else None
+    address = 0
+    if static is not None:
+        static, address = static
+    host[-2:].view(np.int64)[0] = address
     if static is not None:
         if static.numel() != buf.numel():
             raise BatchError(f"the step packs {buf.numel()} ints, the buffer to copy into holds {static.numel()}")
@@ -199,5 +208,5 @@ def build_step_batch(entries, alloc, page_sizes, vocab_size: int, max_position: 
         prefill_tiles=d(8 + 2 * G).view(-1, 3) if n_tiles else None, num_prefill_tiles=n_tiles,
         decode_rows=d(9 + 2 * G) if n_dec else None, num_decode_rows=n_dec,
         prefill_tiles128=d(10 + 2 * G).view(-1, 3) if n_tiles128 else None, num_prefill_tiles128=n_tiles128,
-        max_portion_context=portion_context, graph_key=key,
+        max_portion_context=portion_context, graph_key=key, result_address=d(12 + 2 * G),
     )

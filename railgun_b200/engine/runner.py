@@ -178,7 +178,7 @@ class StaticDecodeBatch:
         self.step_graphs = {}          # with sampling parameters or greedy -> CapturedStep
         self.follow = [None, None]     # FollowStep: the same step fed with ``sampled`` instead of host tokens
         self.in_flight = None          # an event after the last replay, which writes ``host_out``
-        self.stream = None             # the stream that its last step was launched on
+        self.stream = self.stream_handle = None     # the stream that its last step was launched on
         # the number of the step last packed into ``host`` and of the one whose step has read it (written by that step)
         self.seq = torch.zeros(2, dtype=torch.int32, pin_memory=True)
         self.seq_np = self.seq.numpy()
@@ -244,7 +244,7 @@ class ShapeGraph:
     def __init__(self, dev, batch, graph, logits, launches):
         self.dev, self.batch, self.graph, self.logits, self.launches = dev, batch, graph, logits, launches
         self.hold = None               # the last packed step (keeps its pinned buffer alive until the copy has run)
-        self.stream = None             # the stream that its last step was launched on
+        self.stream = self.stream_handle = None     # the stream that its last step was launched on
 
 
 class RepeatedLayouts:
@@ -375,10 +375,13 @@ class ModelRunner:
     def _in_order(self, owner) -> None:
         """The buffers of a captured step (``owner``) are its steps' one after the other: launched on another stream than the
         last time, a step waits for what is on that one."""
+        handle = ops.current_stream_handle()
+        if owner.stream_handle == handle:
+            return
         stream = torch.cuda.current_stream(self.device)
-        if owner.stream is not None and owner.stream != stream:
+        if owner.stream is not None:
             stream.wait_stream(owner.stream)
-        owner.stream = stream
+        owner.stream, owner.stream_handle = stream, handle
 
     def _commit(self, entries, batch) -> None:
         self.alloc.commit_many(batch.host_request_ids, batch.host_context_lens)
@@ -396,11 +399,17 @@ class ModelRunner:
                                               self.model.spec.max_position, self.device, self.err_flag, into=into,
                                               splits=self.model.single_token_splits)
 
+        result = None
+
         def known(key):
-            if key not in steps.graphs:
+            nonlocal result
+            shape = steps.graphs.get(key)
+            if shape is None:
                 return None
-            self._in_order(steps.graphs[key])                      # the step is copied into its buffer next
-            return steps.graphs[key].dev
+            self._in_order(shape)                                  # the step is copied into its buffer next
+            # a short step's logits are the caller's, as they are where its kernels are launched one by one
+            result = shape.logits if steps is self._long_steps or shape.logits is None else torch.empty_like(shape.logits)
+            return shape.dev, (0 if result is shape.logits else result.data_ptr())
 
         batch = build(known)
         self.last_h2d_bytes = batch.h2d_bytes
@@ -413,15 +422,14 @@ class ModelRunner:
             ops.launch_counter().value += shape.launches
             ops.mark_tc_unchecked()
             self._commit(entries, batch)
-            # a short step's logits are the caller's, as they are where its kernels are launched one by one
-            return shape.logits.clone() if steps is self._short_steps and shape.logits is not None else shape.logits
+            return result
         if not steps.to_capture(key):
             logits = self.model.forward(batch, self.views)
             self._commit(entries, batch)
             return logits
         # the layout repeats: a static copy of the packed buffer, one eager run over it (this step), the capture
         dev = torch.empty(batch.host_buffer.numel(), dtype=torch.int32, device=self.device)
-        batch = build(lambda key: dev)
+        batch = build(lambda key: (dev, 0))
         side = torch.cuda.Stream(device=self.device)
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
@@ -434,6 +442,9 @@ class ModelRunner:
         graph = torch.cuda.CUDAGraph()
         with capture(graph):
             logits = self.model.forward(batch, self.views)
+            if steps is self._short_steps and logits is not None:
+                logits = logits.contiguous()
+                ops.step_result(logits, batch.result_address)
         launches = counter.value - n0
         counter.value = n0
         shape = ShapeGraph(dev, batch, graph, logits, launches)

@@ -87,6 +87,11 @@ def _stream():
     return c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
+def current_stream_handle() -> int:
+    """The current stream of the current device, as a number."""
+    return _raw_stream(_current_device()) if _raw_stream is not None else torch.cuda.current_stream().cuda_stream
+
+
 def _ok(code: int, what: str) -> None:
     if code == 0:
         return
@@ -2606,6 +2611,16 @@ def step_out(dev: torch.Tensor, host: torch.Tensor) -> None:
     if not (host.dtype == torch.int32 and host.is_pinned() and host.is_contiguous() and host.numel() == dev.numel()):
         raise KernelError(f"step_out: host must be {dev.numel()} page-locked int32 numbers")
     _ok(_fn("step_io", "rg_step_out")(_ptr(dev), c_void_p(host.data_ptr()), c_int(dev.numel()), _stream()), "step_out")
+
+
+def step_result(src: torch.Tensor, where: torch.Tensor) -> None:
+    """The float32 numbers of ``src``, copied to the address that ``where`` (two int32 of the device: one 64-bit number, 0 for
+    nowhere) holds when the kernel runs."""
+    _check(src, "src", torch.float32)
+    _check(where, "where", torch.int32)
+    if where.numel() != 2 or where.data_ptr() % 8:
+        raise KernelError("step_result: where must be two numbers on an 8-byte boundary")
+    _ok(_fn("step_io", "rg_step_result")(_ptr(src), _ptr(where), c_longlong(src.numel()), _stream()), "step_result")
 
 
 def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k, top_p, seed: torch.Tensor,

@@ -123,3 +123,18 @@ def test_steps_that_are_packed_while_the_one_before_runs(B):
         logits.append(out)
     for i, (a, b) in enumerate(zip(*logits)):
         assert torch.equal(a, b), i
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 1023, 4 * 256 * 592 + 5])
+@pytest.mark.parametrize("at", [0, 1])
+def test_a_result_goes_where_the_step_says(n, at):
+    from railgun_b200 import ops
+    src = torch.randn(n, device="cuda")
+    room = torch.full((n + at + 1,), 7.0, device="cuda")
+    where = torch.tensor([0, room[at:].data_ptr()], dtype=torch.int64, device="cuda").view(torch.int32)
+    ops.step_result(src, where[:2])
+    assert bool((room == 7.0).all())
+    ops.step_result(src, where[2:])
+    assert torch.equal(room[at:at + n], src) and bool((room[:at] == 7.0).all()) and float(room[-1]) == 7.0
+    with pytest.raises(ops.KernelError):
+        ops.step_result(src, where[1:3])
