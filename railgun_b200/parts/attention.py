@@ -99,7 +99,7 @@ class PagedAttention(Mixer):
 
     takes_normed_rows = True
     defers_output = True
-    first_matrix = property(lambda self: self.w_qkv)
+    first_matrix = property(lambda self: self.w_qkv if type(self).forward is PagedAttention.forward else None)
 
     def splits(self, n, longest):
         return ops.decode_splits(n, self.kv_tiles, longest)

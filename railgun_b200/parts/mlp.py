@@ -43,7 +43,7 @@ class SwiGLU(FeedForward):
 
     takes_normed_rows = True
     defers_output = True
-    first_matrix = property(lambda self: self.w_gate_up)
+    first_matrix = property(lambda self: self.w_gate_up if type(self).forward is SwiGLU.forward else None)
 
     def forward(self, x, batch, defer=False):
         stream = ops.tc_stream_rows(batch, self.w_down.shape[0])

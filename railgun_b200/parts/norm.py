@@ -51,7 +51,8 @@ class RMSNorm(Norm):
     fuses_pending_linear = True
     fuses_post_norm = True
     fuses_pending_sum = True
-    plain_rms = property(lambda self: self.groups == 1)          # over the whole row, with ``weight`` and ``eps`` alone
+    # over the whole row, with ``weight`` and ``eps`` alone (not where a derived class adds and norms in its own way)
+    plain_rms = property(lambda self: self.groups == 1 and type(self).add_norm is RMSNorm.add_norm)
 
     def add_norm(self, resid, pending, rows=None):
         if self.groups > 1 or isinstance(pending, ops.PendingSum):

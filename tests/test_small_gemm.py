@@ -3,6 +3,9 @@ import pytest
 import torch
 
 from railgun_b200 import ops
+from railgun_b200.parts.attention import PagedAttention
+from railgun_b200.parts.mlp import SwiGLU
+from railgun_b200.parts.norm import RMSNorm
 
 
 def test_an_operand_on_the_host_is_no_operand():
@@ -66,3 +69,16 @@ def test_which_gated_products_run_with_their_activation_inside(M, N, pays):
 @pytest.mark.parametrize("N,pays", [(128256, True), (94720, False), (94724, True), (50000, False), (37889, True), (37888, False), (32769, False)])
 def test_which_logits_are_streamed(N, pays):
     assert ops._stream_head_pays(N, 148) == pays
+
+
+@pytest.mark.parametrize("base,own,asked", [(RMSNorm, "add_norm", "plain_rms"), (PagedAttention, "forward", "first_matrix"),
+                                            (SwiGLU, "forward", "first_matrix")])
+def test_a_part_that_does_it_its_own_way_is_given_rows(base, own, asked):
+    """A norm moves into the product that reads it only past the two classes' own code."""
+    part = base.__new__(base)
+    part.groups, part.w_qkv, part.w_gate_up = 1, "matrix", "matrix"
+    assert getattr(part, asked)
+    other = type("Other", (base,), {own: lambda self, *a, **k: None})
+    part = other.__new__(other)
+    part.groups, part.w_qkv, part.w_gate_up = 1, "matrix", "matrix"
+    assert not getattr(part, asked)
