@@ -98,7 +98,7 @@ class StepBatch:
     prefill_tiles128: torch.Tensor | None = None     # the same requests in tiles of up to 128 positions
     num_prefill_tiles128: int = 0
     max_portion_context: int = 0     # the longest context among those requests (of several tokens)
-    result_address: torch.Tensor | None = None       # [2]: where a replayed step's result goes, 64 bits (0: nowhere)
+    result_address: torch.Tensor | None = None       # its last two numbers: where a replayed step's result goes, 64 bits (0: nowhere)
     graph_key: tuple = ()            # the layout and what else decides which kernels the step takes: see build_step_batch
 
 
@@ -162,9 +162,8 @@ def build_step_batch(entries, alloc, page_sizes, vocab_size: int, max_position: 
         sizes += [T, R * max_blocks_t[g]]
     sizes += [3 * n_tiles, n_dec, 3 * n_tiles128]
     offs = [0, *accumulate(sizes)]
-    for n in (offs[-1] % 2, 2):                             # one 64-bit number
-        sizes.append(n)
-        offs.append(offs[-1] + n)
+    sizes.append(2 + offs[-1] % 2)                          # a 64-bit number at the end
+    offs.append(offs[-1] + sizes[-1])
     buf = torch.empty(offs[-1], dtype=torch.int32, pin_memory=_pinned())
     tokens = token_arrays[0] if R == 1 else np.concatenate(token_arrays)
     if tokens.dtype != np.int64:
@@ -181,17 +180,15 @@ def build_step_batch(entries, alloc, page_sizes, vocab_size: int, max_position: 
     if n_dec and splits is not None:
         key += splits(n_dec, longest)
     static = into(key) if into is not None else None
-    address = 0
-    if static is not None:
-        static, address = static
-    host[-2:].view(np.int64)[0] = address
-    if static is not None:
+    if static is None:
+        host[-2:] = 0
+        dev = buf.to(device, non_blocking=True)
+    else:
+        static, host[-2:].view(np.int64)[0] = static
         if static.numel() != buf.numel():
             raise BatchError(f"the step packs {buf.numel()} ints, the buffer to copy into holds {static.numel()}")
         static.copy_(buf, non_blocking=True)
         dev = static
-    else:
-        dev = buf.to(device, non_blocking=True)
     d = dev.split(sizes).__getitem__                       # views, cut in one call
     return StepBatch(
         num_tokens=T, num_requests=R, num_wanted=W,
@@ -208,5 +205,5 @@ def build_step_batch(entries, alloc, page_sizes, vocab_size: int, max_position: 
         prefill_tiles=d(8 + 2 * G).view(-1, 3) if n_tiles else None, num_prefill_tiles=n_tiles,
         decode_rows=d(9 + 2 * G) if n_dec else None, num_decode_rows=n_dec,
         prefill_tiles128=d(10 + 2 * G).view(-1, 3) if n_tiles128 else None, num_prefill_tiles128=n_tiles128,
-        max_portion_context=portion_context, graph_key=key, result_address=d(12 + 2 * G),
+        max_portion_context=portion_context, graph_key=key, result_address=d(11 + 2 * G),
     )

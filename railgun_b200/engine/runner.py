@@ -444,7 +444,7 @@ class ModelRunner:
             logits = self.model.forward(batch, self.views)
             if steps is self._short_steps and logits is not None:
                 logits = logits.contiguous()
-                ops.step_result(logits, batch.result_address)
+                ops.step_result(logits, batch.result_address[-2:])
         launches = counter.value - n0
         counter.value = n0
         shape = ShapeGraph(dev, batch, graph, logits, launches)
